@@ -417,16 +417,18 @@ FO_DEVI uint32_t exp_field(float lpf) {
   if constexpr (PDT == FO_F16) eb = max(eb, 113u << 23);  // zero / subnormal halves use the min normal exponent
   return eb;
 }
-// master weight from (stored value as fp32, ECC as fp32) for ordinary values (see fast::Ordinary)
+// master weight from (stored value as fp32, ECC as fp32) for ordinary values (see fast::Ordinary).
+// The fraction times a power of two is exact (ordinary values: no underflow), so one fma rounds as the
+// product and the sum the reference writes.
 template <int PDT, int ECC_BITS>
-FO_DEVI f2 reconstruct_ordinary2(f2 lpf, f2 ef, f2 one) {
+FO_DEVI f2 reconstruct_ordinary2(f2 lpf, f2 ef) {
   using K = EccConst<PDT, ECC_BITS>;
   // RN(e / MAX) for every integer e of the ECC type: e*hi + RN(e*lo) carries the quotient to
   // about 2^-48, which no e/MAX comes that close to a rounding boundary without being exact
   // (all 2^ECC_BITS values are compared with the IEEE division by the self-test)
   f2 fr = fma2(ef, sp(K::rcp_hi()), mul2(ef, sp(K::rcp_lo())));
   f2 sc = mk(__uint_as_float(exp_field<PDT>(lpf.x)), __uint_as_float(exp_field<PDT>(lpf.y)));
-  return sum2(mul2(fr, sc), lpf, one);
+  return fma2(fr, sc, lpf);
 }
 // 2^(1 - exponent of lpf) as float bits: the inverted exponent field (one logic operation)
 template <int PDT>
@@ -435,17 +437,38 @@ FO_DEVI uint32_t inv_exp_field(float lpf) {
   if constexpr (PDT == FO_F16) ib = min(ib, 142u << 23);  // zero / subnormal halves use the min normal exponent
   return ib;
 }
-// ECC of theta given lpf = RN_lp(theta) as fp32, for kMin <= |lpf| <= 1e38 (see fast::Ordinary):
-// err * 2^-log_half_ulp * MAX, |.| <= MAX without clipping because |err| is at most half an ULP of lpf
+// ECC of theta given lpf = RN_lp(theta) as fp32, for kMin <= |lpf| <= 1e38 (see fast::Ordinary), as words
+// whose low ECC_BITS bits are the code.
+// bf16: theta carries 16 bits below lpf's, so err is j half-ULPs / 2^15 for an integer |j| <= 2^15 (or / 2^16
+// just below a power of two), and the reference's product, two roundings and floor(|.| + 0.5) reduce to a
+// step function of j.  One fma reproduces it: err * (2^k * K) + magic, where the inverted exponent field and
+// K's mantissa are merged by one logic operation, the addition of 1.5 * 2^23 units rounds to the nearest
+// integer, and the power of two left over sits in the magic constant.  MAX = 32767: the reference gives j for
+// |j| <= 16416 and one less beyond (j * 32767 / 32768 is rounded to 24 bits first, and those ties go away from
+// zero), so K = 1 - c needs 0.5/16417 < c < 0.5/16416; c = 511 * 2^-24 does.  MAX = 127: j * 127 / 32768 is
+// exact and its only tie is 63.5, where nearest-even agrees.  Compared with the IEEE text for every fp32 by
+// the self-test.  (Five packed instructions and two conversions with two sign copies per pair before, two
+// packed and two logic ones now: 3 of AdamW's 64.5 instructions per element.)
 template <int PDT, int ECC_BITS>
-FO_DEVI void ecc_ordinary2(f2 theta, f2 lpf, int& e0, int& e1) {
-  constexpr float kC = Ecc<ECC_BITS>::MAX * (PDT == FO_BF16 ? 128.0f : 1024.0f);  // MAX * 2^MANT, exact
+FO_DEVI void ecc_ordinary2(f2 theta, f2 lpf, uint32_t& e0, uint32_t& e1) {
   f2 err = fma2(lpf, sp(-1.0f), theta);
-  f2 sc = mk(__uint_as_float(inv_exp_field<PDT>(lpf.x)), __uint_as_float(inv_exp_field<PDT>(lpf.y)));
-  f2 s = mul2(mul2(err, sc), sp(kC));  // the first product is exact (a power of two, no underflow: err is a multiple of theta's ULP)
-  f2 y = add2(s, mk(copysignf(0.5f, s.x), copysignf(0.5f, s.y)));  // round half away from zero ...
-  e0 = __float2int_rz(y.x);                                        // ... by truncation
-  e1 = __float2int_rz(y.y);
+  if constexpr (PDT == FO_BF16) {
+    constexpr uint32_t kMant = ECC_BITS == 16 ? 0x7FFE01u : 0x7E0000u;     // mantissas of 2K = 2 - 511 * 2^-23 and of 127/64
+    constexpr float kMagic = ECC_BITS == 16 ? 6.0f : 1536.0f;              // 1.5 * 2^23 units of 2^-21 / 2^-13
+    const f2 sc = mk(__uint_as_float((~__float_as_uint(lpf.x) & 0x7F800000u) | kMant),
+                     __uint_as_float((~__float_as_uint(lpf.y) & 0x7F800000u) | kMant));
+    const f2 r = fma2(err, sc, sp(kMagic));
+    e0 = __float_as_uint(r.x);
+    e1 = __float_as_uint(r.y);
+  } else {
+    constexpr float kC = Ecc<ECC_BITS>::MAX * 1024.0f;  // MAX * 2^MANT, exact
+    // err * 2^-log_half_ulp * MAX, |.| <= MAX without clipping because |err| is at most half an ULP of lpf
+    f2 sc = mk(__uint_as_float(inv_exp_field<PDT>(lpf.x)), __uint_as_float(inv_exp_field<PDT>(lpf.y)));
+    f2 s = mul2(mul2(err, sc), sp(kC));  // the first product is exact (a power of two, no underflow: err is a multiple of theta's ULP)
+    f2 y = add2(s, mk(copysignf(0.5f, s.x), copysignf(0.5f, s.y)));  // round half away from zero ...
+    e0 = (uint32_t)__float2int_rz(y.x);                              // ... by truncation
+    e1 = (uint32_t)__float2int_rz(y.y);
+  }
 }
 
 // RN(c/255) for the codes c in bytes b and b+1 of w (flashoptim_jax/quantization.py:74), without a
@@ -459,23 +482,25 @@ FO_DEVI f2 codes_over_255(uint32_t w, int b) {
   return fma2(cf, sp(__uint_as_float(0x3B808081u)), mul2(cf, sp(__uint_as_float(0xAF7EFEFFu))));
 }
 
-// bits whose low byte is floor(127 * 2n/(1+|n|) + 0.5), |n| <= 1
-FO_DEVI void softsign_code_bits2(f2 n, f2 one, uint32_t& c0, uint32_t& c1) {
-  f2 d = add2(mk(fabsf(n.x), fabsf(n.y)), sp(1.0f));
-  f2 ny = neg_rcp2(d);
+// bits whose low byte is floor(127 * 2n/(1+|n|) + 0.5), |n| <= 1.  Only the code has to be the reference's,
+// and n has 2^31 values: what follows was cut down to what gives the right code for each of them (self-test).
+// The approximate reciprocal needs no Newton step in front of the residual correction, which squares its
+// error anyway, and 254 q + 0.5 may be rounded once instead of twice.
+FO_DEVI void softsign_code_bits2(f2 n, uint32_t& c0, uint32_t& c1) {
+  f2 d = mk(fadd(1.0f, fabsf(n.x)), fadd(1.0f, fabsf(n.y)));  // scalar: the absolute value is free there
+  f2 ny = mk(rcp_approx(-d.x), rcp_approx(-d.y));
   f2 nq0 = mul2(n, ny);
   f2 r = fma2(d, nq0, n);                      // n - d*q0
   f2 nq = fma2(r, ny, nq0);                    // -n/(1+|n|); 2n/(1+|n|) * 127 == nq * -254 exactly
-  f2 c = sum2(mul2(nq, sp(-254.0f)), sp(0.5f), one);
-  f2 fl = add2_rd(c, sp(12582912.0f));
+  f2 fl = add2_rd(fma2(nq, sp(-254.0f), sp(0.5f)), sp(12582912.0f));
   c0 = __float_as_uint(fl.x);
   c1 = __float_as_uint(fl.y);
 }
-// bits whose low byte is floor(255 * root/av + 0.5); nroot = -root, nrcp = -RN(1/av)
-FO_DEVI void quant_v_bits2(f2 nroot, f2 av, f2 nrcp, f2 one, uint32_t& c0, uint32_t& c1) {
+// bits whose low byte is floor(255 * root/av + 0.5); nroot = -root, nrcp = -RN(1/av).  RN(255 t + 0.5) has the
+// same floor as RN(RN(255 t) + 0.5) for every fp32 t in [0, 1].
+FO_DEVI void quant_v_bits2(f2 nroot, f2 av, f2 nrcp, uint32_t& c0, uint32_t& c1) {
   f2 t = div_negnum_by_rcp2(nroot, av, nrcp);
-  f2 c = sum2(mul2(t, sp(255.0f)), sp(0.5f), one);
-  f2 fl = add2_rd(c, sp(12582912.0f));
+  f2 fl = add2_rd(fma2(t, sp(255.0f), sp(0.5f)), sp(12582912.0f));
   c0 = __float_as_uint(fl.x);
   c1 = __float_as_uint(fl.y);
 }

@@ -43,7 +43,7 @@ __global__ void selftest_softsign(const float one, unsigned long long* out) {
       float n = __uint_as_float((uint32_t)b | (s ? 0x80000000u : 0u));
       bad += fast::softsign_code(n) != ieee::quant_m(n, 1.0f);
       uint32_t c0, c1;
-      fast2::softsign_code_bits2(make_float2(n, -n), fast2::sp(one), c0, c1);
+      fast2::softsign_code_bits2(make_float2(n, -n), c0, c1);
       bad += (int)(signed char)(c0 & 0xFFu) != ieee::quant_m(n, 1.0f);
       bad += (int)(signed char)(c1 & 0xFFu) != ieee::quant_m(-n, 1.0f);
     }
@@ -67,7 +67,7 @@ __global__ void selftest_reconstruct(const float one, unsigned long long* out) {
     {
       bad += !same_float(fast::reconstruct_ordinary<PDT, ECC_BITS>(lpf, (float)e), want);
       const int en = (e == -(1 << (ECC_BITS - 1))) ? e : -e;  // the most negative pattern has no negation
-      const float2 t2 = fast2::reconstruct_ordinary2<PDT, ECC_BITS>(make_float2(lpf, -lpf), make_float2((float)e, (float)en), fast2::sp(one));
+      const float2 t2 = fast2::reconstruct_ordinary2<PDT, ECC_BITS>(make_float2(lpf, -lpf), make_float2((float)e, (float)en));
       const float want_neg = ieee::reconstruct<PDT, ECC_BITS>(bits ^ 0x8000u, en);
       bad += !same_float(t2.x, want) || !same_float(t2.y, want_neg);
     }
@@ -91,9 +91,10 @@ __global__ void selftest_split(const float one, unsigned long long* out) {
     if (fabsf(lpf) >= fast::Ordinary<PDT>::kMin && fabsf(lpf) <= 3.0e38f)
     {
       bad += fast::ecc_ordinary<PDT, ECC_BITS>(theta, lpf) != e1;
-      int p0, p1;
+      uint32_t p0, p1;  // the code is in the low ECC_BITS bits
       fast2::ecc_ordinary2<PDT, ECC_BITS>(make_float2(theta, -theta), make_float2(lpf, -lpf), p0, p1);
-      bad += (p0 != e1) || (p1 != -e1);
+      constexpr uint32_t kMask = (1u << ECC_BITS) - 1u;
+      bad += (((p0 ^ (uint32_t)e1) | (p1 ^ (uint32_t)-e1)) & kMask) != 0u;
     }
     // the packed conversion the hot path uses must agree with the scalar one
     float lo, hi;
@@ -127,10 +128,10 @@ __global__ void selftest_group_div(const float one, unsigned long long pairs, un
     bad += fast::quant_v(x, gs) != ieee::quant_v(x, safe);
     if (gs.tame) {
       uint32_t c0, c1;
-      fast2::softsign_code_bits2(fast2::div_by_rcp2(make_float2(x, -x), fast2::sp(-safe), fast2::sp(gs.rcp)), fast2::sp(one), c0, c1);
+      fast2::softsign_code_bits2(fast2::div_by_rcp2(make_float2(x, -x), fast2::sp(-safe), fast2::sp(gs.rcp)), c0, c1);
       bad += (int)(signed char)(c0 & 0xFFu) != ieee::quant_m(x, safe);
       bad += (int)(signed char)(c1 & 0xFFu) != ieee::quant_m(-x, safe);
-      fast2::quant_v_bits2(make_float2(-x, -safe), fast2::sp(safe), fast2::sp(-gs.rcp), fast2::sp(one), c0, c1);
+      fast2::quant_v_bits2(make_float2(-x, -safe), fast2::sp(safe), fast2::sp(-gs.rcp), c0, c1);
       bad += (int)(c0 & 0xFFu) != ieee::quant_v(x, safe);
       bad += (int)(c1 & 0xFFu) != 255;
       bad += (int)(signed char)(fast::softsign_code_bits(fast::div_by_rcp(x, safe, gs.rcp)) & 0xFFu) != ieee::quant_m(x, safe);

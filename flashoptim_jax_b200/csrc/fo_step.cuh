@@ -735,7 +735,7 @@ FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, 
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        theta[k] = reconstruct_ordinary2<PDT, ECC_BITS>(old_lp[k], mk(ef[2 * k], ef[2 * k + 1]), one2);
+        theta[k] = reconstruct_ordinary2<PDT, ECC_BITS>(old_lp[k], mk(ef[2 * k], ef[2 * k + 1]));
       if constexpr (PDT == FO_BF16) {
         // a value too small for the exponent-field shortcut (zero included)
         if (!(minabs8(old_lp) >= fast::Ordinary<PDT>::kMin)) {
@@ -772,7 +772,7 @@ FO_DEVI bool stored_form(const float2 (&theta)[4], uint32_t (&nw)[4], uint4& ecc
       unpack2<PDT>(nw[k], new_lp[k].x, new_lp[k].y);
     }
     if constexpr (ECC_BITS != 0) {
-      int ne[8];
+      uint32_t ne[8];
 #pragma unroll
       for (int k = 0; k < 4; ++k) ecc_ordinary2<PDT, ECC_BITS>(theta[k], new_lp[k], ne[2 * k], ne[2 * k + 1]);
       {
@@ -785,8 +785,8 @@ FO_DEVI bool stored_form(const float2 (&theta)[4], uint32_t (&nw)[4], uint4& ecc
           if constexpr (REPAIR) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              ne[2 * k] = repair_ecc<PDT, ECC_BITS>(theta[k].x);
-              ne[2 * k + 1] = repair_ecc<PDT, ECC_BITS>(theta[k].y);
+              ne[2 * k] = (uint32_t)repair_ecc<PDT, ECC_BITS>(theta[k].x);
+              ne[2 * k + 1] = (uint32_t)repair_ecc<PDT, ECC_BITS>(theta[k].y);
             }
           }
         }
@@ -1156,7 +1156,7 @@ FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uin
     uint32_t q[8];
     const float2 nam = sp(-am), rm2 = sp(fast::rcp_rn(am));
 #pragma unroll
-    for (int k = 0; k < 4; ++k) softsign_code_bits2(div_by_rcp2(m[k], nam, rm2), one2, q[2 * k], q[2 * k + 1]);
+    for (int k = 0; k < 4; ++k) softsign_code_bits2(div_by_rcp2(m[k], nam, rm2), q[2 * k], q[2 * k + 1]);
     if (!(am >= 1.0e-12f && am <= 1.0e30f)) {  // all-zero group, or a scale outside the reciprocal's range
       rare = true;
       if constexpr (REPAIR) {
@@ -1174,7 +1174,7 @@ FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uin
       av = group_max(av_lane);
       const float2 av2 = sp(av), nrv2 = sp(-fast::rcp_rn(av));
 #pragma unroll
-      for (int k = 0; k < 4; ++k) quant_v_bits2(nroot[k], av2, nrv2, one2, q[2 * k], q[2 * k + 1]);
+      for (int k = 0; k < 4; ++k) quant_v_bits2(nroot[k], av2, nrv2, q[2 * k], q[2 * k + 1]);
       if (!(av >= 1.0e-12f && av <= 1.0737418e9f)) {  // 2^30: also the limit of the packed Adam division
         rare = true;
         if constexpr (REPAIR) {
