@@ -18,6 +18,7 @@ FO_F32, FO_BF16, FO_F16 = 0, 1, 2
 FO_OPT_ADAM, FO_OPT_LION, FO_OPT_SGD = 0, 1, 2
 FO_STATE_QUANT, FO_STATE_FULL, FO_STATE_NONE = 0, 1, 2
 FO_FLAG_DECOUPLED_WD, FO_FLAG_NESTEROV, FO_FLAG_LION_LERP, FO_FLAG_LP_DELTA, FO_FLAG_SCALE_FLOOR = 1, 2, 4, 8, 16
+FO_LAUNCH_CHAINED = 1
 FO_MAX_HYPERS = 16
 FO_MAX_PEERS = 7
 FO_SELFTEST_STATIC_MAX_COUNTERS = 4
@@ -53,6 +54,10 @@ class FoLeaf(ctypes.Structure):
     ]
 
 
+class FoLeafOut(ctypes.Structure):
+    _fields_ = [(name, ctypes.c_void_p) for name in ("param", "ecc", "mu", "mu_scales", "nu", "nu_scales")]
+
+
 class FoStepDesc(ctypes.Structure):
     _fields_ = [
         ("struct_size", ctypes.c_uint32),
@@ -64,6 +69,7 @@ class FoStepDesc(ctypes.Structure):
         ("peer_grad_offsets", ctypes.c_void_p),
         ("grad_sq_norm", ctypes.c_void_p), ("max_grad_norm", ctypes.c_float), ("reserved2", ctypes.c_uint32),
         ("mc_param_offset", ctypes.c_int64), ("mc_grad_offset", ctypes.c_int64),
+        ("outs", ctypes.c_void_p), ("launch_flags", ctypes.c_uint32), ("reserved3", ctypes.c_uint32),
     ]
 
 

@@ -1,6 +1,6 @@
 """Builds libflashoptim_b200.so in-tree with nvcc for sm_100a.
 
-The step-kernel family is split into ten instantiation slices (optimizer x state kind)
+The step-kernel family is split into instantiation slices (optimizer x state kind x kernel)
 compiled from one source with different -D switches, so the build runs in parallel.
 Objects go to csrc/build/, the library to lib/.  Nothing is compiled at import time:
 call build_native() (or `python -m flashoptim_jax_b200.build`).
@@ -35,12 +35,22 @@ _OPTS = (("adam", "FO_OPT_ADAM"), ("lion", "FO_OPT_LION"), ("sgd", "FO_OPT_SGD")
 _KINDS = (("quant", 0), ("full", 1), ("generic", 3))
 
 
-# block shape of a slice: (threads per block, resident blocks per SM).  Measured on B200: the plain
+# block shape of a slice: (threads per block, resident blocks per SM).  Measured on B200: the
 # Adam kernels run best as one 512-thread block per SM (all warps of an SM share one instruction
 # stream and one set of tables); the kernels that also read peers' gradients keep 256-thread blocks,
 # whose smaller stages leave room for a deeper copy pipeline.  Lion gains 2 % from one 768-thread block
 # over three of 256; SGD measures the same either way and keeps the default (256 x 3).
-_SHAPES = {("adam", 0): (512, 1), ("lion", 0): (768, 1)}
+_SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1), ("adam", "group"): (512, 1),
+           ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1),
+           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "group"): (512, 1), ("lion", "all"): (512, 1),
+           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "group"): (512, 1), ("sgd", "all"): (512, 1)}
+# name and feature mask (fo_step.cuh) of the kernels of a slice
+_MODES = (("plain", 0), ("clip", 1), ("out", 2), ("group", 4), ("delta", 8), ("all", 15), ("peer", 16), ("piece", -1))
+
+
+def _has_kernel(oname: str, kname: str, mname: str) -> bool:
+    """Group sizes concern quantized moments only, the parameter hand-back Adam only."""
+    return not (mname == "group" and kname != "quant") and not (mname == "delta" and oname != "adam")
 
 
 def _units(shapes=None, ffi_dir: str | None = None) -> List[Tuple[str, str, List[str]]]:
@@ -49,26 +59,29 @@ def _units(shapes=None, ffi_dir: str | None = None) -> List[Tuple[str, str, List
     if ffi_dir is not None:
         units.append(("fo_ffi", "fo_ffi.cc", ["-x", "cu", f"-I{ffi_dir}"]))
 
-    def step_unit(oname: str, omacro: str, kname: str, kind: int, aux: int | None):
-        suffix = "" if aux is None else ("_aux" if aux else "_plain")
-        flags = [f"-DFO_INST_OPT={omacro}", f"-DFO_INST_KIND={kind}", f"-DFO_INST_AUX={aux or 0}",
+    def step_unit(oname: str, omacro: str, kname: str, kind: int, mname: str, mode: int):
+        suffix = f"_{mname}" if mname else ""
+        flags = [f"-DFO_INST_OPT={omacro}", f"-DFO_INST_KIND={kind}", f"-DFO_INST_MODE={mode}",
                  f"-DFO_INST_NAME=lookup_{oname}_{kname}{suffix}"]
-        shape = shapes.get((oname, aux))
+        shape = shapes.get((oname, mname))
         if shape is not None and kind != 3:
             flags += [f"-DFO_THREADS={shape[0]}", f"-DFO_MIN_BLOCKS_ADAM={shape[1]}", f"-DFO_MIN_BLOCKS_MOMENTUM={shape[1]}"]
             if len(shape) > 2:
                 flags.append(f"-DFO_PLAIN_STAGES={shape[2]}")
+            flags.append("-DFO_SHAPE_NS=shape_" + "_".join(str(x) for x in shape))
         units.append((f"fo_step_{oname}_{kname}{suffix}", "fo_step_inst.cu", flags))
 
     for oname, omacro in _OPTS:
         for kname, kind in _KINDS:
             if kind == 3:
-                step_unit(oname, omacro, kname, kind, None)
+                step_unit(oname, omacro, kname, kind, "", 1)
             else:
-                for aux in (0, 1):
-                    step_unit(oname, omacro, kname, kind, aux)
-    for aux in (0, 1):
-        step_unit("sgd", "FO_OPT_SGD", "none", 2, aux)
+                for mname, mode in _MODES:
+                    if _has_kernel(oname, kname, mname):
+                        step_unit(oname, omacro, kname, kind, mname, mode)
+    for mname, mode in _MODES:
+        if _has_kernel("sgd", "none", mname):
+            step_unit("sgd", "FO_OPT_SGD", "none", 2, mname, mode)
     return units
 
 
@@ -107,7 +120,7 @@ def _sources_digest(extra: List[str], units=None) -> str:
 def build_native(force: bool = False, jobs: int | None = None, extra_flags: List[str] | None = None,
                  lib_path: str = LIB_PATH, verbose: bool = False, shapes=None) -> str:
     """Compile every CUDA source for sm_100a and link the shared object; returns its path.
-    `shapes` overrides the block shapes of the step slices ({(optimizer, aux): (threads, blocks per SM)})."""
+    `shapes` overrides the block shapes of the step slices ({(optimizer, kernel): (threads, blocks per SM)})."""
     extra = list(extra_flags or [])
     units = _units(shapes, ffi_include_dir())
     os.makedirs(OBJ_DIR, exist_ok=True)

@@ -18,25 +18,50 @@ int fail(int code, const char* fmt, ...) {
   return code;
 }
 
-static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool generic, bool aux) {
-#define FO_PICK(stem) return aux ? stem##_aux(pdt, ecc_bits) : stem##_plain(pdt, ecc_bits)
+// the kernel with the asked features: one of its own for one feature, else the one that carries them all
+static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool generic, int mode) {
+#define FO_PICK(stem)                                                    \
+  switch (mode) {                                                        \
+    case kPlain: return stem##_plain(pdt, ecc_bits);                     \
+    case kClip: return stem##_clip(pdt, ecc_bits);                       \
+    case kOut: return stem##_out(pdt, ecc_bits);                         \
+    case kPeer: return stem##_peer(pdt, ecc_bits);                       \
+    default: return stem##_all(pdt, ecc_bits);                           \
+  }
   if (opt == FO_OPT_ADAM) {
     if (generic) return lookup_adam_generic(pdt, ecc_bits);
-    if (state == FO_STATE_QUANT) FO_PICK(lookup_adam_quant);
-    if (state == FO_STATE_FULL) FO_PICK(lookup_adam_full);
+    if (mode == kGroup) return lookup_adam_quant_group(pdt, ecc_bits);
+    if (mode == kDelta) return state == FO_STATE_QUANT ? lookup_adam_quant_delta(pdt, ecc_bits) : lookup_adam_full_delta(pdt, ecc_bits);
+    if (state == FO_STATE_QUANT) { FO_PICK(lookup_adam_quant) }
+    if (state == FO_STATE_FULL) { FO_PICK(lookup_adam_full) }
   } else if (opt == FO_OPT_LION) {
     if (generic) return lookup_lion_generic(pdt, ecc_bits);
-    if (state == FO_STATE_QUANT) FO_PICK(lookup_lion_quant);
-    if (state == FO_STATE_FULL) FO_PICK(lookup_lion_full);
+    if (mode == kGroup) return lookup_lion_quant_group(pdt, ecc_bits);
+    if (state == FO_STATE_QUANT) { FO_PICK(lookup_lion_quant) }
+    if (state == FO_STATE_FULL) { FO_PICK(lookup_lion_full) }
   } else if (opt == FO_OPT_SGD) {
     if (generic) return lookup_sgd_generic(pdt, ecc_bits);
-    if (state == FO_STATE_QUANT) FO_PICK(lookup_sgd_quant);
-    if (state == FO_STATE_FULL) FO_PICK(lookup_sgd_full);
-    if (state == FO_STATE_NONE) FO_PICK(lookup_sgd_none);
+    if (mode == kGroup) return lookup_sgd_quant_group(pdt, ecc_bits);
+    if (state == FO_STATE_QUANT) { FO_PICK(lookup_sgd_quant) }
+    if (state == FO_STATE_FULL) { FO_PICK(lookup_sgd_full) }
+    if (state == FO_STATE_NONE) { FO_PICK(lookup_sgd_none) }
   }
 #undef FO_PICK
   return Launcher{nullptr, 0u};
 }
+static PieceFn find_pieces(int opt, int pdt, int ecc_bits, int state) {
+  if (opt == FO_OPT_ADAM) return state == FO_STATE_QUANT ? lookup_adam_quant_piece(pdt, ecc_bits) : lookup_adam_full_piece(pdt, ecc_bits);
+  if (opt == FO_OPT_LION) return state == FO_STATE_QUANT ? lookup_lion_quant_piece(pdt, ecc_bits) : lookup_lion_full_piece(pdt, ecc_bits);
+  if (state == FO_STATE_NONE) return lookup_sgd_none_piece(pdt, ecc_bits);
+  return state == FO_STATE_QUANT ? lookup_sgd_quant_piece(pdt, ecc_bits) : lookup_sgd_full_piece(pdt, ecc_bits);
+}
+
+// Up to this many elements in whole chunks a call goes through piece_kernel alone: its blocks of 1024
+// elements spread a small problem over all SMs in one launch, where step_kernel has one block of 4096 to 6144
+// elements on few of them and leaves the ragged ends to a second launch.
+#ifndef FO_SMALL_ELEMS
+#define FO_SMALL_ELEMS (148ull * 8192ull)
+#endif
 
 static DevHyper make_dev_hyper(const FoHyper& h, int opt) {
   DevHyper d;
@@ -96,16 +121,19 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
   if (d->n_hypers == 0) return fail(FO_ERR_INVALID_ARG, "fo_step: no hyper-parameter set");
   if (d->n_hypers > FO_MAX_HYPERS) return fail(FO_ERR_TOO_LARGE, "fo_step: %u hyper sets, at most %d per call", d->n_hypers, FO_MAX_HYPERS);
   bool generic = false;
+  int group_shift = 5;
   if (d->state == FO_STATE_QUANT) {
     if (d->group_size < 1) return fail(FO_ERR_INVALID_ARG, "fo_step: group_size %d", d->group_size);
     if (d->group_size > kGenericTile) return fail(FO_ERR_UNSUPPORTED, "fo_step: group_size %d > %d", d->group_size, kGenericTile);
-    generic = d->group_size != 32;
+    // a group is 1 to 32 lanes of 8 elements for 8, 16, ..., 256; other sizes run a kernel of their own
+    generic = d->group_size < 8 || d->group_size > 256 || (d->group_size & (d->group_size - 1)) != 0;
+    for (group_shift = 0; (2 << group_shift) <= d->group_size; ++group_shift) {}
   }
   if (d->n_peers > (uint32_t)kMaxPeers) return fail(FO_ERR_TOO_LARGE, "fo_step: %u peers, at most %d", d->n_peers, kMaxPeers);
   if (d->n_peers > 0 && d->peer_param_offsets == nullptr && d->peer_grad_offsets == nullptr)
     return fail(FO_ERR_INVALID_ARG, "fo_step: n_peers without peer_param_offsets or peer_grad_offsets");
-  if (d->n_peers > 0 && generic) return fail(FO_ERR_UNSUPPORTED, "fo_step: peer replicas need group_size 32");
-  if (find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, false).launch == nullptr)
+  if (d->n_peers > 0 && d->state == FO_STATE_QUANT && d->group_size != 32) return fail(FO_ERR_UNSUPPORTED, "fo_step: peer replicas need group_size 32");
+  if (find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, kPlain).launch == nullptr)
     return fail(FO_ERR_UNSUPPORTED, "fo_step: no kernel for this combination");
 
   const bool need_mu = d->state != FO_STATE_NONE;
@@ -120,60 +148,81 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
     if (need_nu && L.nu == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null nu", i);
     if (need_scales && L.mu_scales == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null mu_scales", i);
     if (need_scales && need_nu && L.nu_scales == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null nu_scales", i);
+    if (d->outs != nullptr) {
+      const FoLeafOut& O = d->outs[i];
+      if (O.param == nullptr || (d->ecc_bits != 0 && O.ecc == nullptr) || (need_mu && O.mu == nullptr) || (need_nu && O.nu == nullptr) ||
+          (need_scales && O.mu_scales == nullptr) || (need_scales && need_nu && O.nu_scales == nullptr))
+        return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null output", i);
+    }
     if (L.hyper >= d->n_hypers) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: hyper index %u out of range", i, L.hyper);
   }
 
-  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  LaunchInfo info;
-  info.sm_count = sm_count_of_current_device();
-  if (info.sm_count <= 0) return fail(FO_ERR_CUDA, "fo_step: cannot query the current device");
-  const unsigned long long kMaxBlocks = 0x7FFFFFFFull;
+  if (d->outs != nullptr && d->n_peers > 0) return fail(FO_ERR_UNSUPPORTED, "fo_step: peers and separate outputs");
 
-  StepParams p;
-  memset(&p, 0, sizeof(p));
-  for (uint32_t h = 0; h < d->n_hypers; ++h) p.hyper[h] = make_dev_hyper(d->hypers[h], d->opt);
-  p.grad_dtype = d->grad_dtype;
-  p.group_size = d->state == FO_STATE_QUANT ? d->group_size : 32;
-  p.one = 1.0f;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  DevHyper hyper[FO_MAX_HYPERS];
+  bool lp_delta = false;
+  for (uint32_t h = 0; h < d->n_hypers; ++h) {
+    hyper[h] = make_dev_hyper(d->hypers[h], d->opt);
+    lp_delta = lp_delta || (hyper[h].flags & FO_FLAG_LP_DELTA) != 0;
+  }
+  Peers peers;
+  memset(&peers, 0, sizeof(peers));
   if (d->peer_param_offsets != nullptr) {
-    p.peers.n = (int)d->n_peers;
-    for (uint32_t r = 0; r < d->n_peers; ++r) p.peers.delta[r] = (long long)d->peer_param_offsets[r];
+    peers.n = (int)d->n_peers;
+    for (uint32_t r = 0; r < d->n_peers; ++r) peers.delta[r] = (long long)d->peer_param_offsets[r];
   }
   if (d->peer_grad_offsets != nullptr && d->n_peers > 0) {
     const uint32_t ranks = d->n_peers + 1;
-    p.peers.ng = (int)d->n_peers;
-    for (uint32_t r = 0; r < d->n_peers; ++r) p.peers.gdelta[r] = (long long)d->peer_grad_offsets[r];
-    p.peers.neg_ranks = -(float)ranks;
-    p.peers.rcp_ranks = 1.0f / (float)ranks;  // correctly rounded (IEEE division on the host)
-    p.peers.ranks_pow2 = (ranks & (ranks - 1)) == 0;
+    peers.ng = (int)d->n_peers;
+    for (uint32_t r = 0; r < d->n_peers; ++r) peers.gdelta[r] = (long long)d->peer_grad_offsets[r];
+    peers.neg_ranks = -(float)ranks;
+    peers.rcp_ranks = 1.0f / (float)ranks;  // correctly rounded (IEEE division on the host)
+    peers.ranks_pow2 = (ranks & (ranks - 1)) == 0;
   }
-
   if (d->mc_param_offset != 0) {
     if (d->peer_param_offsets == nullptr || d->n_peers == 0) return fail(FO_ERR_INVALID_ARG, "fo_step: mc_param_offset without peer_param_offsets");
-    p.peers.mc_pdelta = (long long)d->mc_param_offset;
+    peers.mc_pdelta = (long long)d->mc_param_offset;
   }
   if (d->mc_grad_offset != 0) {
     if (d->peer_grad_offsets == nullptr || d->n_peers == 0) return fail(FO_ERR_INVALID_ARG, "fo_step: mc_grad_offset without peer_grad_offsets");
-    p.peers.mc_gdelta = (long long)d->mc_grad_offset;
+    peers.mc_gdelta = (long long)d->mc_grad_offset;
   }
-  p.sq_norm = d->grad_sq_norm;
-  p.max_norm = d->max_grad_norm;
-  // the slice that runs this step, and the elements one of its chunks covers
-  const Launcher launcher = find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, step_needs_aux(p));
-  if (launcher.launch == nullptr) return fail(FO_ERR_UNSUPPORTED, "fo_step: no kernel for this combination");
-  const LaunchFn launch = launcher.launch;
-  const unsigned long long chunk = generic ? generic_tile_elems(d->group_size) : launcher.chunk;
+  const bool with_peers = peers.n > 0 || peers.ng > 0;
+  const int features = (d->grad_sq_norm != nullptr ? kClip : 0) | (d->outs != nullptr ? kOut : 0) |
+                       (d->state == FO_STATE_QUANT && d->group_size != 32 ? kGroup : 0) | (lp_delta ? kDelta : 0);
+  const int mode = with_peers ? kPeer : features;
+  const Launcher launcher = find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, mode);
+  const PieceFn pieces = generic ? nullptr : find_pieces(d->opt, d->param_dtype, d->ecc_bits, d->state);
+  if (launcher.launch == nullptr || (!generic && pieces == nullptr)) return fail(FO_ERR_UNSUPPORTED, "fo_step: no kernel for this combination");
 
-  int count = 0;
-  unsigned long long blocks = 0;
+  HostLeaf table[kMaxLeaves];
+  HostStep hs;
+  hs.leaf = table; hs.n_leaves = 0;
+  hs.hyper = hyper; hs.n_hypers = (int)d->n_hypers;
+  hs.grad_dtype = d->grad_dtype; hs.group_shift = group_shift; hs.group_size = d->state == FO_STATE_QUANT ? d->group_size : 32;
+  hs.sm_count = sm_count_of_current_device();
+  if (hs.sm_count <= 0) return fail(FO_ERR_CUDA, "fo_step: cannot query the current device");
+  hs.sq_norm = d->grad_sq_norm; hs.max_norm = d->max_grad_norm;
+  hs.peers = &peers;
+  bool chained = (d->launch_flags & FO_LAUNCH_CHAINED) != 0;
+  const int most_leaves = (mode == kPlain || mode == kPeer) && !generic ? kMaxLeaves : kMaxLeavesFlex;
+  const unsigned long long unit = generic ? generic_tile_elems(d->group_size) : kPieceElems;
+  const unsigned long long kMaxBlocks = 0x7FFFFFFFull;
+  unsigned long long blocks = 0, whole = 0;
   auto flush = [&]() -> int {
-    if (count == 0) return FO_OK;
-    p.n_leaves = count;
-    p.first_block[count] = (uint32_t)blocks;
-    info.total_chunks = (unsigned int)blocks;
-    cudaError_t e = launch(p, info, stream);
-    count = 0;
-    blocks = 0;
+    if (hs.n_leaves == 0) return FO_OK;
+    cudaError_t e = cudaSuccess;
+    if (generic) {
+      e = launcher.launch(hs, chained, stream);
+    } else {
+      // with peers the whole chunks always take the kernel that knows them (the pieces' path is scalar there)
+      const unsigned int main_chunk = (with_peers ? whole > 0 : whole > FO_SMALL_ELEMS) ? launcher.chunk : 0u;
+      if (main_chunk != 0) e = launcher.launch(hs, chained, stream);
+      if (e == cudaSuccess) e = pieces(hs, main_chunk, chained, stream);
+    }
+    hs.n_leaves = 0;
+    blocks = whole = 0;
     if (e != cudaSuccess) return fail(FO_ERR_CUDA, "fo_step: launch failed: %s", cudaGetErrorString(e));
     return FO_OK;
   };
@@ -186,30 +235,51 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
   auto advance = [](const void* base, unsigned long long elems, size_t size) -> void* {
     return base == nullptr ? nullptr : (void*)((const char*)base + elems * size);
   };
+  auto distance = [](const void* to, const void* from) -> long long { return from == nullptr ? 0ll : (long long)((const char*)to - (const char*)from); };
   for (uint32_t i = 0; i < d->n_leaves; ++i) {
     const FoLeaf& L = d->leaves[i];
+    DevOut out = {};
+    bool aligned = aligned16(L.grad) && aligned16(L.param) && aligned16(L.ecc) && aligned16(L.mu) && aligned16(L.nu);
+    if (d->outs != nullptr && L.n != 0) {
+      const FoLeafOut& O = d->outs[i];
+      out.param = distance(O.param, L.param);
+      out.ecc = distance(O.ecc, L.ecc);
+      out.mu = distance(O.mu, L.mu);
+      out.mu_scales = distance(O.mu_scales, L.mu_scales);
+      out.nu = distance(O.nu, L.nu);
+      out.nu_scales = distance(O.nu_scales, L.nu_scales);
+      aligned = aligned && ((out.param | out.ecc | out.mu | out.nu) & 15) == 0;
+    }
     for (unsigned long long done = 0; done < L.n; done += kMaxLeafElems) {
       const unsigned long long n = L.n - done < kMaxLeafElems ? L.n - done : kMaxLeafElems;
-      const unsigned long long nb = (n + chunk - 1) / chunk;
+      const unsigned long long nb = (n + unit - 1) / unit;
       if (nb > kMaxBlocks) return fail(FO_ERR_TOO_LARGE, "fo_step: leaf %u with %llu elements exceeds one launch", i, (unsigned long long)L.n);
-      if (count == kMaxLeaves || blocks + nb > kMaxBlocks) {
+      if (hs.n_leaves == most_leaves || blocks + nb > kMaxBlocks) {
         int rc = flush();
         if (rc != FO_OK) return rc;
       }
-      DevLeaf& D = p.leaf[count];
+      HostLeaf& H = table[hs.n_leaves];
+      DevLeaf& D = H.src;
       D.grad = advance(L.grad, done, grad_size);
       D.param = advance(L.param, done, param_size);
       D.ecc = advance(L.ecc, done, ecc_size);
       D.mu = advance(L.mu, done, moment_size);
       D.nu = advance(L.nu, done, moment_size);
-      D.mu_scales = advance(L.mu_scales, done / 32, 2);
-      D.nu_scales = advance(L.nu_scales, done / 32, 2);
+      D.mu_scales = advance(L.mu_scales, done >> group_shift, 2);
+      D.nu_scales = advance(L.nu_scales, done >> group_shift, 2);
       D.n = n;
-      p.first_block[count] = (uint32_t)blocks;
-      p.hyper_of[count] = (uint8_t)L.hyper;
-      p.aligned[count] = aligned16(D.grad) && aligned16(D.param) && aligned16(D.ecc) && aligned16(D.mu) && aligned16(D.nu);
+      H.out = out;
+      H.hyper = (uint8_t)L.hyper;
+      const DevHyper& dh = hyper[L.hyper];
+      bool hot = aligned && !(mode == kPeer && (dh.flags & FO_FLAG_LP_DELTA) != 0);
+      if (d->opt == FO_OPT_ADAM && dh.dyn == nullptr) hot = hot && (dh.flags & kFlagTameAdam) != 0;
+#ifdef FO_NAIVE_MATH
+      hot = false;
+#endif
+      H.hot = hot ? 1 : 0;
+      if (hot && !generic) whole += n / launcher.chunk * launcher.chunk;
       blocks += nb;
-      ++count;
+      ++hs.n_leaves;
     }
   }
   return flush();

@@ -53,17 +53,15 @@ template <bool VARIANCE>
 __global__ void __launch_bounds__(kCodecThreads) dequantize_kernel(const void* __restrict__ values,
                                                               const __half* __restrict__ scales, float* __restrict__ out,
                                                               unsigned long long n, int G) {
-  __shared__ float lut_m[256], lut_v[256];
-  build_luts(lut_m, lut_v);
   const unsigned long long stride = (unsigned long long)gridDim.x * kCodecThreads;
   for (unsigned long long i = (unsigned long long)blockIdx.x * kCodecThreads + threadIdx.x; i < n; i += stride) {
     const float sc = __half2float(scales[i / G]);
     const unsigned int b = ((const unsigned char*)values)[i];
     if (VARIANCE) {
-      float s = fmul(lut_v[b], sc);
+      float s = fmul(ieee::deq_v_norm((int)b), sc);
       out[i] = fmul(s, s);
     } else {
-      out[i] = fmul(lut_m[b], sc);
+      out[i] = fmul(kDeqM.v[b], sc);
     }
   }
 }

@@ -1,23 +1,26 @@
 // Multi-tensor fused optimizer step for sm_100a.
 //
-// One launch walks a table of pytree leaves.  The leaves are cut into chunks of 2048
-// elements; a persistent grid of blocks strides over the chunk list.  Inside a chunk a
-// thread owns 8 consecutive elements, so every warp-wide access is a run of 256
+// A call walks a table of pytree leaves.  Two kernels share the work:
+//   step_kernel   the whole chunks of the leaves (a chunk: threads per block x 8 elements), a persistent
+//                 grid with a copy pipeline through shared memory, one block (or a few) per SM;
+//   piece_kernel  everything else in pieces of 1024 elements, one 128-thread block each: the ragged ends,
+//                 leaves shorter than a chunk, leaves the vector path cannot take, and whole small problems.
+// In both a thread owns 8 consecutive elements, so every warp-wide access is a run of 256
 // consecutive elements: 16 B per lane for the 2-byte streams (grad, param, int16 ECC), 8 B
 // per lane for the 1-byte streams (int8/uint8 codes, int8 ECC).  A 32-element quantization
-// group is 4 adjacent lanes; its absmax is two xor-shuffles.  Everything between load and
-// store lives in registers: reconstruct the fp32 master weight, dequantize the moments,
-// apply the update, split the weight back, requantize with fresh group scales.  All arrays
-// are updated in place; a group is read and written by the same 4 lanes only.
+// group is 4 adjacent lanes; its absmax is two xor-shuffles (groups of 8 to 256: none to five).
+// Everything between load and store lives in registers: reconstruct the fp32 master weight, dequantize the
+// moments, apply the update, split the weight back, requantize with fresh group scales.  A group is read and
+// written by the same lanes only, so the arrays may be updated in place.
 //
-// Two code paths produce the same bits:
-//   hot   full, 16-byte-aligned chunks under ordinary hyper-parameters: vector accesses and
-//         the fast:: arithmetic of fo_math.cuh, with per-piece checks that send unusual
-//         values (|param| < 2^-118, second moment < 1e-30, group scale outside
-//         [1e-12, 1e30]) to the IEEE formulation;
-//   cold  everything else (leaf tails, unaligned leaves, eps or bias correction outside the
-//         range the shortcut division is proven for): scalar guarded accesses and ieee::
-//         arithmetic only.
+// Three paths produce the same bits:
+//   hot   straight-line vector code on the fast:: arithmetic of fo_math.cuh, with per-piece checks that send
+//         a warp that holds an unusual value (|param| < 2^-100, second moment < 1e-30, group scale outside
+//         [1e-12, 1e30]) to the repairing pass;
+//   repairing pass (REPAIR = true)  the same code with the affected lanes redone in IEEE arithmetic; all of
+//         piece_kernel's vector work runs it, with a limit for ragged ends;
+//   cold  scalar guarded accesses and ieee:: arithmetic only (unaligned leaves, eps or bias correction
+//         outside the range the shortcut division is proven for, pieces under peer replicas).
 //
 // The arithmetic follows flashoptim_jax/adamw.py:76-131 and
 // flashoptim_jax/momentum_kernel.py:62-103 operation by operation (see fo_math.cuh).
@@ -31,6 +34,29 @@
 
 namespace fo {
 
+constexpr int kMaxLeaves = 320;      // leaves per launch of the plain and the peers' kernel (kernel-parameter table)
+constexpr int kMaxLeavesFlex = 240;  // of the kernel that can also write elsewhere: its table entries are larger
+constexpr int kMaxPeers = 7;
+constexpr int kGenericTile = 1024;   // slots per block of the any-group-size kernel
+constexpr int kPieceThreads = 128, kPieceElems = kPieceThreads * 8;
+constexpr uint32_t kFlagTameAdam = 1u << 31;  // internal: sqrt(nu)/sqrt(bc2) may use the reciprocal shortcut
+
+// Which features a step_kernel instantiation carries beyond the plain step (in place, groups of 32, no clipping).
+// One feature at a time is what steps ask for, and each has a kernel of its own: a kernel that carries them all as
+// run-time switches needs 80 instructions per element where the plain one needs 60, and spills (AdamW, 124 M
+// parameters: 344 us plain, 494 with all features switched off).  kAll serves the combinations.
+constexpr int kPlain = 0;
+constexpr int kClip = 1;   // gradients rescaled by their global norm
+constexpr int kOut = 2;    // results written elsewhere
+constexpr int kGroup = 4;  // quantization groups of 8, 16, 64, 128 or 256
+constexpr int kDelta = 8;  // FO_FLAG_LP_DELTA
+constexpr int kAll = 15;
+constexpr int kPeer = 16;  // peers' gradients and parameter replicas, clipping; groups of 32, in place
+
+// Names below depend on the block shape of the translation unit (FO_THREADS): each shape has its own.
+#ifndef FO_SHAPE_NS
+#define FO_SHAPE_NS shape_default
+#endif
 // Tuning (measured on B200): 256-thread blocks; Adam's working set wants 128 registers
 // (2 resident blocks per SM), Lion / SGD fit 3 blocks.
 #ifndef FO_THREADS
@@ -48,14 +74,6 @@ namespace fo {
 #ifndef FO_LUT_COPIES
 #define FO_LUT_COPIES 8
 #endif
-constexpr int kThreads = FO_THREADS;
-constexpr int min_blocks(int opt) { return opt == FO_OPT_ADAM ? FO_MIN_BLOCKS_ADAM : FO_MIN_BLOCKS_MOMENTUM; }
-constexpr int kPiece = 8;
-constexpr int kLutCopies = FO_LUT_COPIES;                 // copies of the momentum dequantization table in shared memory
-constexpr int kChunk = kThreads * kPiece;      // elements per chunk
-constexpr int kMaxLeaves = 320;                // leaves per launch (kernel-parameter table)
-constexpr int kGenericTile = 1024;             // slots per block of the any-group-size kernel
-constexpr uint32_t kFlagTameAdam = 1u << 31;   // internal: sqrt(nu)/sqrt(bc2) may use the reciprocal shortcut
 
 struct DevLeaf {
   const void* grad;
@@ -66,6 +84,10 @@ struct DevLeaf {
   void* nu;
   void* nu_scales;
   unsigned long long n;
+};
+// where a leaf's results go: byte distances from the arrays they are computed from (0: in place)
+struct DevOut {
+  long long param, ecc, mu, mu_scales, nu, nu_scales;
 };
 
 struct DevHyper {
@@ -79,7 +101,6 @@ struct DevHyper {
 // Replicas of the parameter arrays on peer GPUs (ZeRO-1 all-gather folded into the step): every
 // updated parameter vector is also stored `delta[r]` bytes away from its local address, i.e. at the
 // same element of peer r's replica.  Plain stores through peer-mapped memory; no waiting on peers.
-constexpr int kMaxPeers = 7;
 // Reduce-scatter folded into the step: the gradient of an element is the mean over this rank's
 // value and the values `gdelta[r]` bytes away (the same element of peer r's gradient buffer):
 // fp32 sum in the order own, peer 0, peer 1, ..., divided by the number of ranks, rounded once to
@@ -120,22 +141,66 @@ FO_DEVI void store_to_peers(const Peers& peers, T* local, const T& v) {
   for (int r = 0; r < peers.n; ++r) *reinterpret_cast<T*>(reinterpret_cast<char*>(local) + peers.delta[r]) = v;
 }
 
-struct StepParams {
-  DevLeaf leaf[kMaxLeaves];
-  uint32_t first_block[kMaxLeaves + 1];  // first chunk of each leaf; [n_leaves] = total chunks
-  uint8_t hyper_of[kMaxLeaves];
-  uint8_t aligned[kMaxLeaves];
+// Kernel parameters of step_kernel: the whole chunks of the hot leaves form one sequence.
+struct StepCommon {
   DevHyper hyper[FO_MAX_HYPERS];
   int32_t n_leaves;
   int32_t grad_dtype;
-  int32_t group_size;
-  float one;  // 1.0f the compiler cannot see through (see fast2::sum2)
-  int32_t stages;  // shared-memory stages of the copy pipeline (2..8), set by the launcher
-  Peers peers;
+  int32_t group_shift;  // log2 of the group size
+  float one;            // 1.0f the compiler cannot see through (see fast2::sum2)
+  int32_t stages;       // shared-memory stages of the copy pipeline (2..8), set by the launcher
+  uint32_t run_chunks;  // consecutive chunks a block takes at a time (set by the launcher)
   const double* sq_norm;  // device: sum of squares of all gradients of the step (nullptr: no clipping)
   float max_norm;
-  uint32_t run_chunks;  // consecutive chunks a block takes at a time (set by the launcher)
+  int32_t group_size;   // of the any-group-size kernel
 };
+template <int N>
+struct LeafTable {
+  DevLeaf leaf[N];
+  uint32_t first_block[N + 1];  // first chunk of each leaf; [n_leaves] = total chunks
+  uint8_t hyper_of[N];
+};
+template <bool OUT, bool PEER>
+struct StepTables;
+template <>
+struct StepTables<false, false> : StepCommon {
+  LeafTable<kMaxLeaves> t;
+};
+template <>
+struct StepTables<true, false> : StepCommon {
+  LeafTable<kMaxLeavesFlex> t;
+  DevOut out[kMaxLeavesFlex];
+};
+template <>
+struct StepTables<false, true> : StepCommon {
+  LeafTable<kMaxLeaves> t;
+  Peers peers;
+};
+template <int MODE>
+using StepParams = StepTables<(MODE & kOut) != 0, MODE == kPeer>;
+// Kernel parameters of piece_kernel.  Two table sizes: a launch copies its whole parameter block, and 2 KB
+// instead of 31 saves about 1.5 us of host time on a call for a leaf or two.
+template <int N>
+struct PieceParams : StepCommon {
+  DevLeaf leaf[N];
+  DevOut out[N];
+  uint32_t first_piece[N + 1];
+  uint32_t start[N];    // first piece of the leaf this launch takes (the ones before went through step_kernel)
+  uint8_t hyper_of[N];
+  uint8_t hot[N];       // the vector path may take the leaf (alignment; hyper-parameters known on the host)
+  Peers peers;
+};
+constexpr int kPieceLeavesSmall = 12, kPieceLeavesLarge = 236;
+static_assert(sizeof(PieceParams<kPieceLeavesLarge>) <= 32764 && sizeof(StepParams<kOut>) <= 32764 && sizeof(StepParams<kPeer>) <= 32764,
+              "kernel parameters");
+
+inline namespace FO_SHAPE_NS {
+
+constexpr int kThreads = FO_THREADS;
+constexpr int min_blocks(int opt) { return opt == FO_OPT_ADAM ? FO_MIN_BLOCKS_ADAM : FO_MIN_BLOCKS_MOMENTUM; }
+constexpr int kPiece = 8;
+constexpr int kLutCopies = FO_LUT_COPIES;                 // copies of the momentum dequantization table in shared memory
+constexpr int kChunk = kThreads * kPiece;      // elements per chunk
 
 // true when the quotient sqrt(nu)/sqrt(bc2) may be formed as div_by_rcp without changing
 // (quotient + eps): for sqrt(nu) >= 2^-100 the shortcut is exact, below it the quotient is
@@ -268,6 +333,7 @@ struct Clip {
   float n_g;     // norm rounded to the gradient dtype
   float rcp_n;   // RN(1 / n_g)
   float m_g;     // max_norm rounded to the gradient dtype
+  FO_DEVI const Clip& get() const { return *this; }
 };
 FO_DEVI Clip load_clip(const double* sq_norm, float max_norm, int gdt) {
   Clip c;
@@ -295,15 +361,36 @@ FO_DEVI float load_grad_mean(const void* grad, int gdt, unsigned long long i, co
   return round_to_grad_dtype(fdiv(g, -peers.neg_ranks), gdt);
 }
 
-// One chunk, any alignment, any length: thread t owns elements base + 8t .. base + 8t + 7,
-// out-of-range elements count as zeros (flashoptim_jax/quantization.py:20-26).
+// Momentum dequantization values, entry = code byte as unsigned: evaluated by the compiler with the formula's
+// own fp32 operations (compared with the device's by the self-test).
+struct DeqTable {
+  float v[256];
+  constexpr DeqTable() : v() {
+    for (int b = 0; b < 256; ++b) {
+      const int q = b < 128 ? b : b - 256;
+      const float t = (float)q / 127.0f;
+      v[b] = t / (2.0f - (t < 0.0f ? -t : t));
+    }
+  }
+};
+static __device__ const DeqTable kDeqM{};
+
+// Eight elements from i0 on, any alignment, any length: out-of-range elements count as zeros
+// (flashoptim_jax/quantization.py:20-26).  All lanes of a warp call this together (group maxima).
 template <int OPT, int PDT, int ECC_BITS, int STATE>
-__device__ __noinline__ void cold_chunk(const DevLeaf& L, const Hyp& h, int gdt, unsigned long long base,
-                                        const float* lut_m, const float* lut_v, const Peers& peers, const Clip& clip) {
+__device__ __noinline__ void cold_piece(const DevLeaf& L, const DevOut* out, const DevHyper& dh, const int gdt, const int gshift,
+                                        const unsigned long long i0, const Peers* peers, const double* sq_norm, const float max_norm) {
+  const Hyp h = load_hyper<OPT>(dh);
+  const Clip clip = load_clip(sq_norm, max_norm, gdt);
   const unsigned long long n = L.n;
-  const unsigned long long i0 = base + (unsigned long long)threadIdx.x * kPiece;
-  const unsigned long long gi = i0 >> 5;
+  const unsigned long long gi = i0 >> gshift;
+  const int group_lanes = 1 << (gshift - 3);
   const bool live = i0 < n;
+  auto to = [&](void* base, long long DevOut::*d) { return (char*)base + (out != nullptr ? out->*d : 0ll); };
+  char* const o_param = to(L.param, &DevOut::param);
+  char* const o_ecc = to(L.ecc, &DevOut::ecc);
+  char* const o_mu = to(L.mu, &DevOut::mu);
+  char* const o_nu = to(L.nu, &DevOut::nu);
   float m[8], root[8];
   float msc = 0.0f, vsc = 0.0f;
   if constexpr (STATE == FO_STATE_QUANT) {
@@ -317,7 +404,7 @@ __device__ __noinline__ void cold_chunk(const DevLeaf& L, const Hyp& h, int gdt,
     const unsigned long long i = i0 + j;
     m[j] = 0.0f; root[j] = 0.0f;
     if (i < n) {
-      const float g = clip_ieee(load_grad_mean(L.grad, gdt, i, peers), clip, gdt);
+      const float g = clip_ieee(peers != nullptr ? load_grad_mean(L.grad, gdt, i, *peers) : load_grad(L.grad, gdt, i), clip, gdt);
       float theta, old_f32 = 0.0f;
       uint32_t pb = 0;
       if constexpr (PDT == FO_F32) {
@@ -332,9 +419,9 @@ __device__ __noinline__ void cold_chunk(const DevLeaf& L, const Hyp& h, int gdt,
       }
       float mm = 0.0f, vv = 0.0f, rr = 0.0f;
       if constexpr (STATE == FO_STATE_QUANT) {
-        mm = fmul(lut_m[((const unsigned char*)L.mu)[i]], msc);
+        mm = fmul(kDeqM.v[((const unsigned char*)L.mu)[i]], msc);
         if constexpr (OPT == FO_OPT_ADAM) {
-          float s = fmul(lut_v[((const unsigned char*)L.nu)[i]], vsc);
+          float s = fmul(ieee::deq_v_norm(((const unsigned char*)L.nu)[i]), vsc);
           vv = fmul(s, s);
         }
       } else if constexpr (STATE == FO_STATE_FULL) {
@@ -344,45 +431,45 @@ __device__ __noinline__ void cold_chunk(const DevLeaf& L, const Hyp& h, int gdt,
       update_element_ieee<OPT, STATE>(h, g, theta, mm, vv, rr);
       if constexpr (PDT == FO_F32) {
         if (h.flags & FO_FLAG_LP_DELTA) theta = fadd(old_f32, fsub(theta, old_f32));
-        ((float*)L.param)[i] = theta;
-        store_to_peers(peers, (float*)L.param + i, theta);
+        ((float*)o_param)[i] = theta;
+        if (peers != nullptr) store_to_peers(*peers, (float*)o_param + i, theta);
       } else {
         uint32_t nb;
         int e;
         store_form_ieee<PDT, ECC_BITS>(h.flags, theta, pb, nb, e);
-        ((unsigned short*)L.param)[i] = (unsigned short)nb;
-        store_to_peers(peers, (unsigned short*)L.param + i, (unsigned short)nb);
-        if constexpr (ECC_BITS == 16) ((short*)L.ecc)[i] = (short)e;
-        if constexpr (ECC_BITS == 8) ((signed char*)L.ecc)[i] = (signed char)e;
+        ((unsigned short*)o_param)[i] = (unsigned short)nb;
+        if (peers != nullptr) store_to_peers(*peers, (unsigned short*)o_param + i, (unsigned short)nb);
+        if constexpr (ECC_BITS == 16) ((short*)o_ecc)[i] = (short)e;
+        if constexpr (ECC_BITS == 8) ((signed char*)o_ecc)[i] = (signed char)e;
       }
       if constexpr (STATE == FO_STATE_FULL) {
-        ((float*)L.mu)[i] = mm;
-        if constexpr (OPT == FO_OPT_ADAM) ((float*)L.nu)[i] = vv;
+        ((float*)o_mu)[i] = mm;
+        if constexpr (OPT == FO_OPT_ADAM) ((float*)o_nu)[i] = vv;
       }
       m[j] = mm; root[j] = rr;
     }
   }
   if constexpr (STATE == FO_STATE_QUANT) {
     const bool floor_mode = (h.flags & FO_FLAG_SCALE_FLOOR) != 0;
-    const bool writer = (threadIdx.x & 3) == 0 && live;
+    const bool writer = (threadIdx.x & (group_lanes - 1)) == 0 && live;
     float am = 0.0f, av = 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) { am = fmaxf(am, fabsf(m[j])); av = fmaxf(av, root[j]); }
-    am = fmaxf(am, __shfl_xor_sync(0xFFFFFFFFu, am, 1));
-    am = fmaxf(am, __shfl_xor_sync(0xFFFFFFFFu, am, 2));
+    for (int o = 1; o < group_lanes; o <<= 1) {
+      am = fmaxf(am, __shfl_xor_sync(0xFFFFFFFFu, am, o));
+      av = fmaxf(av, __shfl_xor_sync(0xFFFFFFFFu, av, o));
+    }
     const float sm = ieee::safe_scale(am, floor_mode);
 #pragma unroll 1
     for (int j = 0; j < 8; ++j)
-      if (i0 + j < n) ((signed char*)L.mu)[i0 + j] = (signed char)ieee::quant_m(m[j], sm);
-    if (writer) ((__half*)L.mu_scales)[gi] = __float2half_rn(am);
+      if (i0 + j < n) ((signed char*)o_mu)[i0 + j] = (signed char)ieee::quant_m(m[j], sm);
+    if (writer) ((__half*)to(L.mu_scales, &DevOut::mu_scales))[gi] = __float2half_rn(am);
     if constexpr (OPT == FO_OPT_ADAM) {
-      av = fmaxf(av, __shfl_xor_sync(0xFFFFFFFFu, av, 1));
-      av = fmaxf(av, __shfl_xor_sync(0xFFFFFFFFu, av, 2));
       const float sv = ieee::safe_scale(av, floor_mode);
 #pragma unroll 1
       for (int j = 0; j < 8; ++j)
-        if (i0 + j < n) ((unsigned char*)L.nu)[i0 + j] = (unsigned char)ieee::quant_v(root[j], sv);
-      if (writer) ((__half*)L.nu_scales)[gi] = __float2half_rn(av);
+        if (i0 + j < n) ((unsigned char*)o_nu)[i0 + j] = (unsigned char)ieee::quant_v(root[j], sv);
+      if (writer) ((__half*)to(L.nu_scales, &DevOut::nu_scales))[gi] = __float2half_rn(av);
     }
   }
 }
@@ -413,7 +500,13 @@ FO_DEVI uint32_t pack2(float lo, float hi) {
   }
 }
 
-FO_DEVI float group_max(float a) {
+// maximum over the lanes that share a quantization group: four for groups of 32, 2^(gshift - 3) in general
+template <bool ANY>
+FO_DEVI float group_max(float a, const int gshift) {
+  if constexpr (ANY) {
+    for (int o = 1; o < (1 << (gshift - 3)); o <<= 1) a = fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, o));
+    return a;
+  }
   a = fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, 1));
   return fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, 2));
 }
@@ -468,7 +561,7 @@ struct Raw {
 };
 
 template <int OPT, int PDT, int ECC_BITS, int STATE>
-FO_DEVI void hot_load(const DevLeaf& L, const int gdt, const uint32_t i0, Raw<OPT, PDT, ECC_BITS, STATE>& r) {
+FO_DEVI void hot_load(const DevLeaf& L, const int gdt, const int gshift, const uint32_t i0, Raw<OPT, PDT, ECC_BITS, STATE>& r) {
   if constexpr (PDT == FO_F32) {
     r.p0 = __ldcs((const uint4*)((const float*)L.param + i0));
     r.p1 = __ldcs((const uint4*)((const float*)L.param + i0) + 1);
@@ -482,10 +575,10 @@ FO_DEVI void hot_load(const DevLeaf& L, const int gdt, const uint32_t i0, Raw<OP
   }
   if constexpr (STATE == FO_STATE_QUANT) {
     r.mq = __ldcs((const uint2*)((const unsigned char*)L.mu + i0));
-    r.msc = ((const __half*)L.mu_scales)[i0 >> 5];
+    r.msc = ((const __half*)L.mu_scales)[i0 >> gshift];
     if constexpr (OPT == FO_OPT_ADAM) {
       r.vq = __ldcs((const uint2*)((const unsigned char*)L.nu + i0));
-      r.vsc = ((const __half*)L.nu_scales)[i0 >> 5];
+      r.vsc = ((const __half*)L.nu_scales)[i0 >> gshift];
     }
   } else if constexpr (STATE == FO_STATE_FULL) {
     r.m0 = __ldcs((const uint4*)((const float*)L.mu + i0));
@@ -552,6 +645,19 @@ FO_DEVI uint4 lds128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
   return v;
 }
+// The same constants kept in shared memory and read where they are used (broadcast reads): held in registers they
+// push step_kernel's loop over its limit.
+struct SharedClip {
+  bool active;
+  uint32_t at;  // shared address of {n_g, 1 / n_g, m_g, div_ok}
+  FO_DEVI Clip get() const {
+    const uint4 v = lds128(at);
+    Clip c;
+    c.active = active; c.div_ok = v.w != 0u;
+    c.n_g = __uint_as_float(v.x); c.rcp_n = __uint_as_float(v.y); c.m_g = __uint_as_float(v.z);
+    return c;
+  }
+};
 FO_DEVI uint2 lds64(uint32_t a) {
   uint2 v;
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
@@ -667,6 +773,15 @@ FO_DEVI float maxabs8(const float2 (&x)[4]) {
 // byte k of a word as an index
 FO_DEVI uint32_t byte_of(uint32_t w, int k) { return __byte_perm(w, 0u, 0x4440u | (uint32_t)k); }
 
+// Where the momentum dequantization values come from.
+struct LutGlobal {  // the constant table through L1 (pieces and repairs: a handful of chunks, no table to build first)
+  FO_DEVI float2 pair(uint32_t w, int k) const { return make_float2(__ldg(&kDeqM.v[byte_of(w, k)]), __ldg(&kDeqM.v[byte_of(w, k + 1)])); }
+};
+struct LutWide {  // kLutCopies interleaved copies in shared memory (see build_wide_lut)
+  const float* base;
+  FO_DEVI float2 pair(uint32_t w, int k) const { return make_float2(base[byte_of(w, k) * kLutCopies], base[byte_of(w, k + 1) * kLutCopies]); }
+};
+
 // Addresses of the eight elements a thread owns in the current chunk, one per stream.  Inside a run
 // of consecutive chunks they advance by compile-time constants, so a later chunk's address is this
 // one plus an immediate.
@@ -680,22 +795,39 @@ struct Piece {
   char* vsc;
 };
 template <int PDT, int ECC_BITS, int STATE>
-FO_DEVI Piece piece_at(const DevLeaf& L, const int gdt, const uint32_t i0) {
+FO_DEVI Piece piece_at(const DevLeaf& L, const int gdt, const int gshift, const uint32_t i0) {
   Piece a;
   a.grad = (const char*)L.grad + (size_t)i0 * (gdt == FO_F32 ? 4u : 2u);
   a.param = (char*)L.param + (size_t)i0 * (PDT == FO_F32 ? 4u : 2u);
   a.ecc = (char*)L.ecc + (size_t)i0 * (ECC_BITS == 16 ? 2u : 1u);
   a.mu = (char*)L.mu + (size_t)i0 * (STATE == FO_STATE_FULL ? 4u : 1u);
   a.nu = (char*)L.nu + (size_t)i0 * (STATE == FO_STATE_FULL ? 4u : 1u);
-  a.msc = (char*)L.mu_scales + (size_t)(i0 >> 5) * 2u;
-  a.vsc = (char*)L.nu_scales + (size_t)(i0 >> 5) * 2u;
+  a.msc = (char*)L.mu_scales + (size_t)(i0 >> gshift) * 2u;
+  a.vsc = (char*)L.nu_scales + (size_t)(i0 >> gshift) * 2u;
   return a;
 }
+// The distances from a leaf's arrays to where its results go.
+struct OutAt {  // read through a pointer: pieces and repairs
+  const DevOut* out;
+  FO_DEVI long long operator()(long long DevOut::*d) const { return out->*d; }
+};
+// read from the kernel's parameters where they are used, through an index the compiler cannot follow: hoisted
+// out of the chunk loop the six distances cost twelve registers, and what the loop then spills goes to L2 (the
+// shared-memory carve-out leaves L1 little room): 700 instead of 450 us on 124 M parameters
+struct OutOf {
+  const StepParams<kOut>& p;
+  int leaf;
+  FO_DEVI long long operator()(long long DevOut::*d) const {
+    int l = leaf;
+    asm volatile("" : "+r"(l));
+    return p.out[l].*d;
+  }
+};
 
 // master weights of a piece from the stored parameter words (p0, p1) and ECC words (e_in); same
 // contract for REPAIR as hot_unpack
 template <bool REPAIR, int PDT, int ECC_BITS>
-FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, const float2 one2, float2 (&theta)[4]) {
+FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, float2 (&theta)[4]) {
   using namespace fast2;
   bool rare = false;
   if constexpr (PDT == FO_F32) {
@@ -812,11 +944,10 @@ FO_DEVI bool stored_form(const float2 (&theta)[4], uint32_t (&nw)[4], uint4& ecc
 // Returns false when a parameter lies outside the range of the packed split (the caller then takes
 // the repairing pass); nothing has been stored in that case.
 template <int OPT, int PDT, int ECC_BITS>
-__device__ __noinline__ bool zero_chunk(const uint32_t flags, const float wd, const float decay, const int gdt, const float one,
+__device__ __noinline__ bool zero_chunk(const uint32_t flags, const float wd, const float decay, const int gdt,
                                         const char* p_grad, char* p_param, char* p_ecc, char* p_mu, char* p_nu, char* p_msc, char* p_vsc) {
   // (addresses and scalars by value: a structure passed by reference would have to live in local memory)
   using namespace fast2;
-  const float2 one2 = sp(one);
   struct { const char* grad; char* param; char* ecc; char* mu; char* nu; char* msc; char* vsc; } at = {p_grad, p_param, p_ecc, p_mu, p_nu, p_msc, p_vsc};
   struct { uint32_t flags; float wd, decay; } h = {flags, wd, decay};
   // the test, on what is in memory: gradients +-0, all codes 0 (then the moments are zero whatever the
@@ -846,7 +977,7 @@ __device__ __noinline__ bool zero_chunk(const uint32_t flags, const float wd, co
     e.x = t.x; e.y = t.y;
   }
   float2 theta[4];
-  bool rare = unpack_master<false, PDT, ECC_BITS>(p0, p1, e, one2, theta);
+  bool rare = unpack_master<false, PDT, ECC_BITS>(p0, p1, e, theta);
   if (OPT == FO_OPT_LION || (h.flags & FO_FLAG_DECOUPLED_WD) != 0) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) theta[k] = mul2(theta[k], sp(h.decay));
@@ -875,23 +1006,22 @@ __device__ __noinline__ bool zero_chunk(const uint32_t flags, const float wd, co
 // REPAIR = false: straight-line code; returns true when a value lies outside a shortcut's proven
 // range (the results are then not to be stored).  REPAIR = true: the affected lane redoes the stage
 // with IEEE operations and the results are always good.
-template <bool REPAIR, int OPT, int PDT, int ECC_BITS, int STATE>
-FO_DEVI bool hot_unpack(const Raw<OPT, PDT, ECC_BITS, STATE>& r, const int gdt, const float* lut_mw, const float one, Unpacked& u) {
+template <bool REPAIR, int OPT, int PDT, int ECC_BITS, int STATE, typename LUT>
+FO_DEVI bool hot_unpack(const Raw<OPT, PDT, ECC_BITS, STATE>& r, const int gdt, const LUT& lut, Unpacked& u) {
   using namespace fast2;
-  const float2 one2 = sp(one);
   bool rare = false;
   if (gdt == FO_F32) pairs_of(r.g0, r.g1, u.g);
   else if (gdt == FO_BF16) pairs_of16<FO_BF16>(r.g0, u.g);
   else pairs_of16<FO_F16>(r.g0, u.g);
 
-  rare = unpack_master<REPAIR, PDT, ECC_BITS>(r.p0, r.p1, r.e, one2, u.theta);
+  rare = unpack_master<REPAIR, PDT, ECC_BITS>(r.p0, r.p1, r.e, u.theta);
 
   if constexpr (STATE == FO_STATE_QUANT) {
     const float2 msc = sp(__half2float(r.msc));
     const uint32_t mw[2] = {r.mq.x, r.mq.y};
 #pragma unroll
     for (int k = 0; k < 4; ++k)  // quantization.py:52-55
-      u.m[k] = mul2(mk(lut_mw[byte_of(mw[k >> 1], 2 * (k & 1)) * kLutCopies], lut_mw[byte_of(mw[k >> 1], 2 * (k & 1) + 1) * kLutCopies]), msc);
+      u.m[k] = mul2(lut.pair(mw[k >> 1], 2 * (k & 1)), msc);
     if constexpr (OPT == FO_OPT_ADAM) {
       const float2 vsc = sp(__half2float(r.vsc));
       const uint32_t vw[2] = {r.vq.x, r.vq.y};
@@ -966,9 +1096,35 @@ FO_DEVI bool mean_of_sum(float2 (&g)[4], const int gdt, const Peers& peers) {
 
 // Global-norm clipping of a piece (see Clip), for gradients already known to be rescaled.
 // Same contract for REPAIR as hot_unpack.
-template <bool REPAIR>
-FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const Clip& c) {
+template <bool REPAIR, typename CLIP>
+FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const CLIP& source) {
   using namespace fast2;
+  const Clip c = source.get();
+  bool rare = !c.div_ok;
+  if (gdt == FO_BF16) {
+    // g and n_g have 8-bit mantissas, so g / n_g is never halfway between two bf16 values and no closer to
+    // that than 2^-17 of itself: the product with the fp32 reciprocal (off by 2^-23 at most) rounds to the same
+    // bf16 value as the quotient, and the second product is one bf16 instruction.  Holds while the quotient is
+    // normal: |g| >= 2^-100 (n_g <= 2^20), or zero.  Twice the magnitude bits minus one, as unsigned: zero wraps
+    // to the top and passes.  (With the exact division and both conversions the same took 11 instructions per
+    // element instead of 4.)
+    uint32_t lo = 0xFFFFFFFFu;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      lo = min(lo, min(2u * __float_as_uint(g[k].x) - 1u, 2u * __float_as_uint(g[k].y) - 1u));
+    rare = rare || lo < 2u * 0x0D800000u - 1u;
+    const __nv_bfloat162 mg = __float2bfloat162_rn(c.m_g);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 q = mul2(g[k], sp(c.rcp_n));
+      if constexpr (REPAIR) {
+        if (rare) q = mk(fdiv(g[k].x, c.n_g), fdiv(g[k].y, c.n_g));
+      }
+      const __nv_bfloat162 r = __hmul2_rn(__floats2bfloat162_rn(q.x, q.y), mg);
+      unpack2<FO_BF16>(*reinterpret_cast<const uint32_t*>(&r), g[k].x, g[k].y);
+    }
+    return rare;
+  }
   // The reciprocal shortcut is exact for 2^-100 <= |g| <= 2^100, and for zeros up to their sign,
   // which is put back below.  Magnitude bits minus one, as unsigned: zero wraps to the top and passes.
   uint32_t lo = 0xFFFFFFFFu, hi = 0u;
@@ -978,7 +1134,7 @@ FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const Clip& c) {
     lo = min(lo, min(a, b));
     hi = max(hi, max(a + 1u, b + 1u));
   }
-  const bool rare = !c.div_ok || lo < 0x0D800000u - 1u || hi > 0x71800000u;  // 2^-100, 2^100
+  rare = rare || lo < 0x0D800000u - 1u || hi > 0x71800000u;  // 2^-100, 2^100
   float2 q[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -991,14 +1147,7 @@ FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const Clip& c) {
       for (int k = 0; k < 4; ++k) q[k] = mk(fdiv(g[k].x, c.n_g), fdiv(g[k].y, c.n_g));
     }
   }
-  if (gdt == FO_BF16) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      unpack2<FO_BF16>(pack2<FO_BF16>(q[k].x, q[k].y), q[k].x, q[k].y);
-      q[k] = mul2(q[k], sp(c.m_g));
-      unpack2<FO_BF16>(pack2<FO_BF16>(q[k].x, q[k].y), g[k].x, g[k].y);
-    }
-  } else if (gdt == FO_F16) {
+  if (gdt == FO_F16) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       unpack2<FO_F16>(pack2<FO_F16>(q[k].x, q[k].y), q[k].x, q[k].y);
@@ -1014,22 +1163,49 @@ FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const Clip& c) {
 
 FO_DEVI float sign_of(float x);
 
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__device__ __noinline__ void warm_chunk(const DevLeaf& L, const Hyp& h, const int gdt, const uint32_t base,
-                                        const float one, const float* lut_mw, const Peers& peers, const Clip* clip);
+template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
+__device__ __noinline__ void warm_chunk(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t i0, const Peers* peers);
+
+// FO_FLAG_LP_DELTA: the parameter handed back is old + lp(new - old), each operation rounded to the parameter's
+// dtype (flashoptim_jax/adamw.py:411,415,463); o0, o1 are the old parameter's words
+template <int PDT>
+FO_DEVI void hand_back_delta(const uint4& o0, const uint4& o1, uint32_t (&nw)[4], float2 (&theta)[4]) {
+  using namespace fast2;
+  if constexpr (PDT == FO_F32) {
+    float2 old[4];
+    pairs_of(o0, o1, old);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) theta[k] = add2(old[k], fma2(old[k], sp(-1.0f), theta[k]));
+  } else {
+    float2 old[4];
+    pairs_of16<PDT>(o0, old);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 nv, d;
+      unpack2<PDT>(nw[k], nv.x, nv.y);
+      nv = fma2(old[k], sp(-1.0f), nv);
+      unpack2<PDT>(pack2<PDT>(nv.x, nv.y), d.x, d.y);
+      nv = add2(old[k], d);
+      nw[k] = pack2<PDT>(nv.x, nv.y);
+    }
+  }
+}
 
 // Second half of a hot chunk: update, split, requantize, store.  Each stage runs its packed
 // shortcut unconditionally.
 // REPAIR = false (first pass): a value outside the range a shortcut is proven for only raises
 // `rare`; nothing is stored until the end, and if any lane of the warp saw such a value the warp's
 // 256 elements are redone from memory by warm_chunk, otherwise the results are written.
-// REPAIR = true (warm_chunk): the lane that holds such a value (exact zeros are the common case:
+// REPAIR = true (warm_chunk, pieces): the lane that holds such a value (exact zeros are the common case:
 // untouched rows, padding, zero gradients) redoes that stage with IEEE operations, then stores.
 // The stored bits are those of the IEEE path in every case.
-template <bool REPAIR, int OPT, int PDT, int ECC_BITS, int STATE, bool AUX, bool MASKED = false>
-FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uint32_t base, const Piece& at, const float one,
-                        bool rare, Unpacked& u, const float* lut_mw, const Peers& peers, const Clip* clip,
+// `at` is the piece the operands came from, `distance` (kOut) tells how far away the results go;
+// old_param(w0, w1) delivers the words of the old parameter.
+template <bool REPAIR, int OPT, int PDT, int ECC_BITS, int STATE, int MODE, bool MASKED = false, typename OUT, typename OLD>
+FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const int gdt, const uint32_t i0,
+                        const Piece& at, bool rare, Unpacked& u, const OUT& distance, OLD old_param, const Peers* peers,
                         const int n_valid = kPiece, const bool group_valid = true) {
+  const float one = c.one;
   using namespace fast2;
   const float2 one2 = sp(one);
   float2 (&g)[4] = u.g;
@@ -1152,7 +1328,7 @@ FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uin
   float am = 0.0f, av = 0.0f;
   if constexpr (STATE == FO_STATE_QUANT) {
     const bool floor_mode = (h.flags & FO_FLAG_SCALE_FLOOR) != 0;
-    am = group_max(am_lane);
+    am = group_max<(MODE & kGroup) != 0>(am_lane, c.group_shift);
     uint32_t q[8];
     const float2 nam = sp(-am), rm2 = sp(fast::rcp_rn(am));
 #pragma unroll
@@ -1171,7 +1347,7 @@ FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uin
     mq.x = pack_bytes(q[0], q[1], q[2], q[3]);
     mq.y = pack_bytes(q[4], q[5], q[6], q[7]);
     if constexpr (OPT == FO_OPT_ADAM) {
-      av = group_max(av_lane);
+      av = group_max<(MODE & kGroup) != 0>(av_lane, c.group_shift);
       const float2 av2 = sp(av), nrv2 = sp(-fast::rcp_rn(av));
 #pragma unroll
       for (int k = 0; k < 4; ++k) quant_v_bits2(nroot[k], av2, nrv2, q[2 * k], q[2 * k + 1]);
@@ -1195,42 +1371,60 @@ FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uin
   (void)rare;
   if constexpr (!REPAIR) {
     if (__any_sync(0xFFFFFFFFu, rare)) {
-      if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && !AUX) {
+      if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && (MODE & ~(kClip | kGroup)) == 0) {
         // no new first moment of the warp differs from zero: look whether the whole piece is at rest
-        if (__all_sync(0xFFFFFFFFu, am_lane == 0.0f) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, one, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
+        if (__all_sync(0xFFFFFFFFu, am_lane == 0.0f) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
       }
-      warm_chunk<OPT, PDT, ECC_BITS, STATE, AUX>(L, h, gdt, base, one, lut_mw, peers, clip);
+      warm_chunk<OPT, PDT, ECC_BITS, STATE, MODE>(c, L, out, dh, i0, peers);
       return;
     }
   }
+  if constexpr ((MODE & kDelta) != 0) {
+    if (h.flags & FO_FLAG_LP_DELTA) {
+      uint4 o0, o1 = make_uint4(0u, 0u, 0u, 0u);
+      old_param(o0, o1);
+      hand_back_delta<PDT>(o0, o1, nw, theta);
+    }
+  }
   // ---- stores ---------------------------------------------------------------------------------------------
+  Piece to = at;
+  if constexpr ((MODE & kOut) != 0) {
+    to.param += distance(&DevOut::param);
+    if constexpr (ECC_BITS != 0) to.ecc += distance(&DevOut::ecc);
+    if constexpr (STATE != FO_STATE_NONE) to.mu += distance(&DevOut::mu);
+    if constexpr (STATE != FO_STATE_NONE && OPT == FO_OPT_ADAM) to.nu += distance(&DevOut::nu);
+    if constexpr (STATE == FO_STATE_QUANT) to.msc += distance(&DevOut::mu_scales);
+    if constexpr (STATE == FO_STATE_QUANT && OPT == FO_OPT_ADAM) to.vsc += distance(&DevOut::nu_scales);
+  }
   if constexpr (REPAIR && MASKED) {
-    // the ragged end of a leaf (ragged_chunk only): the piece that straddles the end stores its
+    // the ragged end of a leaf (pieces only): the piece that straddles the end stores its
     // valid elements one by one, pieces beyond it store nothing; a group's scale is stored by the
     // lanes of a group that has an element at all
     if (n_valid < kPiece) {
-      for (int j = 0; j < n_valid; ++j) {
+#pragma unroll
+      for (int j = 0; j < kPiece; ++j) {
+        if (j >= n_valid) continue;
         const float2 t = theta[j >> 1];
         if constexpr (PDT == FO_F32) {
-          ((float*)at.param)[j] = (j & 1) ? t.y : t.x;
+          ((float*)to.param)[j] = (j & 1) ? t.y : t.x;
         } else {
-          ((unsigned short*)at.param)[j] = (unsigned short)(nw[j >> 1] >> (16 * (j & 1)));
+          ((unsigned short*)to.param)[j] = (unsigned short)(nw[j >> 1] >> (16 * (j & 1)));
           const uint32_t ew[4] = {ecc_out.x, ecc_out.y, ecc_out.z, ecc_out.w};
-          if constexpr (ECC_BITS == 16) ((unsigned short*)at.ecc)[j] = (unsigned short)(ew[j >> 1] >> (16 * (j & 1)));
-          if constexpr (ECC_BITS == 8) ((unsigned char*)at.ecc)[j] = (unsigned char)(ew[j >> 2] >> (8 * (j & 3)));
+          if constexpr (ECC_BITS == 16) ((unsigned short*)to.ecc)[j] = (unsigned short)(ew[j >> 1] >> (16 * (j & 1)));
+          if constexpr (ECC_BITS == 8) ((unsigned char*)to.ecc)[j] = (unsigned char)(ew[j >> 2] >> (8 * (j & 3)));
         }
         if constexpr (STATE == FO_STATE_FULL) {
-          ((float*)at.mu)[j] = (j & 1) ? m[j >> 1].y : m[j >> 1].x;
-          if constexpr (OPT == FO_OPT_ADAM) ((float*)at.nu)[j] = (j & 1) ? v[j >> 1].y : v[j >> 1].x;
+          ((float*)to.mu)[j] = (j & 1) ? m[j >> 1].y : m[j >> 1].x;
+          if constexpr (OPT == FO_OPT_ADAM) ((float*)to.nu)[j] = (j & 1) ? v[j >> 1].y : v[j >> 1].x;
         } else if constexpr (STATE == FO_STATE_QUANT) {
-          ((unsigned char*)at.mu)[j] = (unsigned char)(((j & 4) ? mq.y : mq.x) >> (8 * (j & 3)));
-          if constexpr (OPT == FO_OPT_ADAM) ((unsigned char*)at.nu)[j] = (unsigned char)(((j & 4) ? vq.y : vq.x) >> (8 * (j & 3)));
+          ((unsigned char*)to.mu)[j] = (unsigned char)(((j & 4) ? mq.y : mq.x) >> (8 * (j & 3)));
+          if constexpr (OPT == FO_OPT_ADAM) ((unsigned char*)to.nu)[j] = (unsigned char)(((j & 4) ? vq.y : vq.x) >> (8 * (j & 3)));
         }
       }
       if constexpr (STATE == FO_STATE_QUANT) {
         if (group_valid) {
-          *(__half*)at.msc = __float2half_rn(am);
-          if constexpr (OPT == FO_OPT_ADAM) *(__half*)at.vsc = __float2half_rn(av);
+          *(__half*)to.msc = __float2half_rn(am);
+          if constexpr (OPT == FO_OPT_ADAM) *(__half*)to.vsc = __float2half_rn(av);
         }
       }
       return;
@@ -1239,44 +1433,44 @@ FO_DEVI void hot_finish(const DevLeaf& L, const Hyp& h, const int gdt, const uin
   if constexpr (PDT == FO_F32) {
     const float4 lo = make_float4(theta[0].x, theta[0].y, theta[1].x, theta[1].y);
     const float4 hi = make_float4(theta[2].x, theta[2].y, theta[3].x, theta[3].y);
-    if (AUX && peers.mc_pdelta != 0) {
-      char* mc = at.param + peers.mc_pdelta;
+    if (MODE == kPeer && peers->mc_pdelta != 0) {
+      char* mc = to.param + peers->mc_pdelta;
       multicast_store(mc, make_uint4(__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(lo.z), __float_as_uint(lo.w)));
       multicast_store(mc + 16, make_uint4(__float_as_uint(hi.x), __float_as_uint(hi.y), __float_as_uint(hi.z), __float_as_uint(hi.w)));
     } else {
-      __stcs((float4*)at.param, lo);
-      __stcs((float4*)at.param + 1, hi);
-      if constexpr (AUX) {
-        store_to_peers(peers, (float4*)at.param, lo);
-        store_to_peers(peers, (float4*)at.param + 1, hi);
+      __stcs((float4*)to.param, lo);
+      __stcs((float4*)to.param + 1, hi);
+      if constexpr (MODE == kPeer) {
+        store_to_peers(*peers, (float4*)to.param, lo);
+        store_to_peers(*peers, (float4*)to.param + 1, hi);
       }
     }
   } else {
     const uint4 w = make_uint4(nw[0], nw[1], nw[2], nw[3]);
-    if (AUX && peers.mc_pdelta != 0) {
-      multicast_store(at.param + peers.mc_pdelta, w);
+    if (MODE == kPeer && peers->mc_pdelta != 0) {
+      multicast_store(to.param + peers->mc_pdelta, w);
     } else {
-      __stcs((uint4*)at.param, w);
-      if constexpr (AUX) store_to_peers(peers, (uint4*)at.param, w);
+      __stcs((uint4*)to.param, w);
+      if constexpr (MODE == kPeer) store_to_peers(*peers, (uint4*)to.param, w);
     }
-    if constexpr (ECC_BITS == 16) __stcs((uint4*)at.ecc, ecc_out);
-    if constexpr (ECC_BITS == 8) __stcs((uint2*)at.ecc, make_uint2(ecc_out.x, ecc_out.y));
+    if constexpr (ECC_BITS == 16) __stcs((uint4*)to.ecc, ecc_out);
+    if constexpr (ECC_BITS == 8) __stcs((uint2*)to.ecc, make_uint2(ecc_out.x, ecc_out.y));
   }
   if constexpr (STATE == FO_STATE_FULL) {
-    __stcs((float4*)at.mu, make_float4(m[0].x, m[0].y, m[1].x, m[1].y));
-    __stcs((float4*)at.mu + 1, make_float4(m[2].x, m[2].y, m[3].x, m[3].y));
+    __stcs((float4*)to.mu, make_float4(m[0].x, m[0].y, m[1].x, m[1].y));
+    __stcs((float4*)to.mu + 1, make_float4(m[2].x, m[2].y, m[3].x, m[3].y));
     if constexpr (OPT == FO_OPT_ADAM) {
-      __stcs((float4*)at.nu, make_float4(v[0].x, v[0].y, v[1].x, v[1].y));
-      __stcs((float4*)at.nu + 1, make_float4(v[2].x, v[2].y, v[3].x, v[3].y));
+      __stcs((float4*)to.nu, make_float4(v[0].x, v[0].y, v[1].x, v[1].y));
+      __stcs((float4*)to.nu + 1, make_float4(v[2].x, v[2].y, v[3].x, v[3].y));
     }
   } else if constexpr (STATE == FO_STATE_QUANT) {
     // the four lanes of a group all store its scale: same value to the same address, one
     // unpredicated instruction
-    __stcs((uint2*)at.mu, mq);
-    *(__half*)at.msc = __float2half_rn(am);
+    __stcs((uint2*)to.mu, mq);
+    *(__half*)to.msc = __float2half_rn(am);
     if constexpr (OPT == FO_OPT_ADAM) {
-      __stcs((uint2*)at.nu, vq);
-      *(__half*)at.vsc = __float2half_rn(av);
+      __stcs((uint2*)to.nu, vq);
+      *(__half*)to.vsc = __float2half_rn(av);
     }
   }
 }
@@ -1286,14 +1480,16 @@ template <int BYTES>
 FO_DEVI void masked_words(const void* src, const int n_valid, uint32_t (&w)[2 * BYTES]) {
 #pragma unroll
   for (int k = 0; k < 2 * BYTES; ++k) w[k] = 0u;
-  for (int j = 0; j < n_valid; ++j) {
+#pragma unroll
+  for (int j = 0; j < kPiece; ++j) {  // unrolled, so that the words stay in registers
+    if (j >= n_valid) continue;
     if constexpr (BYTES == 4) w[j] = ((const uint32_t*)src)[j];
     if constexpr (BYTES == 2) w[j >> 1] |= (uint32_t)((const unsigned short*)src)[j] << (16 * (j & 1));
     if constexpr (BYTES == 1) w[j >> 2] |= (uint32_t)((const unsigned char*)src)[j] << (8 * (j & 3));
   }
 }
 template <int OPT, int PDT, int ECC_BITS, int STATE>
-__device__ __noinline__ void masked_load(const Piece& at, const int gdt, const int n_valid, Raw<OPT, PDT, ECC_BITS, STATE>& r) {
+FO_DEVI void masked_load(const Piece& at, const int gdt, const int n_valid, Raw<OPT, PDT, ECC_BITS, STATE>& r) {
   uint32_t w4[8], w2[4], w1[2];
   if constexpr (PDT == FO_F32) {
     masked_words<4>(at.param, n_valid, w4);
@@ -1324,22 +1520,20 @@ __device__ __noinline__ void masked_load(const Piece& at, const int gdt, const i
   }
 }
 
-// The repairing pass with a limit, for a leaf's ragged last chunk and for leaves shorter than a chunk
-// (called from the tail kernel only): elements from n_limit on do not exist; they read as
-// zeros (flashoptim_jax/quantization.py:20-26) and nothing is stored for them.  Warps that lie wholly
-// beyond the end return at once.  (Not with peer replicas: their stores are whole vectors.)
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__device__ __noinline__ void ragged_chunk(const DevLeaf& L, const Hyp& h, const int gdt, const uint32_t base,
-                                        const float one, const float* lut_mw, const Peers& peers, const Clip* clip,
-                                        const uint32_t n_limit) {
-  const uint32_t i0 = base + threadIdx.x * kPiece;
+// The repairing pass with a limit, for piece_kernel: elements from n_limit on do not exist; they read as
+// zeros (flashoptim_jax/quantization.py:20-26) and nothing is stored for them.  A warp that lies wholly
+// beyond the end returns at once.
+template <int OPT, int PDT, int ECC_BITS, int STATE>
+FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut& out, const DevHyper& dh, const Hyp& h, const Clip& clip,
+                          const uint32_t i0, const uint32_t n_limit) {
   if ((i0 & ~255u) >= n_limit) return;  // the warp's first element: the same answer in all its lanes
+  const int gdt = c.grad_dtype, gshift = c.group_shift;
   const int n_valid = i0 >= n_limit ? 0 : (n_limit - i0 < (uint32_t)kPiece ? (int)(n_limit - i0) : kPiece);
-  const bool group_valid = (i0 & ~31u) < n_limit;
-  const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, i0);
+  const bool group_valid = (i0 >> gshift << gshift) < n_limit;
+  const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, gshift, i0);
   Raw<OPT, PDT, ECC_BITS, STATE> raw;
   if (n_valid == kPiece) {
-    hot_load<OPT, PDT, ECC_BITS, STATE>(L, gdt, i0, raw);
+    hot_load<OPT, PDT, ECC_BITS, STATE>(L, gdt, gshift, i0, raw);
   } else {
     masked_load<OPT, PDT, ECC_BITS, STATE>(at, gdt, n_valid, raw);
     if constexpr (STATE == FO_STATE_QUANT) {
@@ -1348,56 +1542,55 @@ __device__ __noinline__ void ragged_chunk(const DevLeaf& L, const Hyp& h, const 
     }
   }
   Unpacked u;
-  hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, lut_mw, one, u);
-  if (AUX && peers.ng > 0) {
-    merge_peer_grads<true>(u.g, gdt, peers, [&](int r, uint4& w0, uint4& w1) {
-      const char* g = (const char*)L.grad + peers.gdelta[r];
-      if (gdt == FO_F32) {
-        w0 = __ldcs((const uint4*)((const float*)g + i0));
-        w1 = __ldcs((const uint4*)((const float*)g + i0) + 1);
-      } else {
-        w0 = __ldcs((const uint4*)((const unsigned short*)g + i0));
-      }
-    });
-  }
-  if (AUX && clip->active) clip_grads<true>(u.g, gdt, *clip);
-  hot_finish<true, OPT, PDT, ECC_BITS, STATE, AUX, true>(L, h, gdt, base, at, one, false, u, lut_mw, peers, clip, n_valid, group_valid);
+  hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, LutGlobal{}, u);
+  if (clip.active) clip_grads<true>(u.g, gdt, clip);
+  hot_finish<true, OPT, PDT, ECC_BITS, STATE, kAll, true>(c, L, &out, dh, h, gdt, i0, at, false, u, OutAt{&out},
+                                                           [&](uint4& w0, uint4& w1) { w0 = raw.p0; w1 = raw.p1; }, nullptr, n_valid, group_valid);
 }
 
 // Second chance for a warp whose first pass met a value outside a shortcut's range: the same
 // packed arithmetic from a fresh load, with per-lane IEEE repairs.  About twice the cost of a
-// first pass for that warp, against about seven times for the scalar IEEE path.
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__device__ __noinline__ void warm_chunk(const DevLeaf& L, const Hyp& h, const int gdt, const uint32_t base,
-                                        const float one, const float* lut_mw, const Peers& peers, const Clip* clip) {
+// first pass for that warp, against about seven times for the scalar IEEE path.  (Everything it needs comes
+// from the kernel's parameters: a structure of the caller's would have to live in local memory.)
+template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
+__device__ __noinline__ void warm_chunk(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t i0, const Peers* peers) {
+  const int gdt = c.grad_dtype, gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;
+  const Hyp h = load_hyper<OPT>(dh);
   Raw<OPT, PDT, ECC_BITS, STATE> raw;
-  hot_load<OPT, PDT, ECC_BITS, STATE>(L, gdt, base + threadIdx.x * kPiece, raw);
+  hot_load<OPT, PDT, ECC_BITS, STATE>(L, gdt, gshift, i0, raw);
   Unpacked u;
-  hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, lut_mw, one, u);
-  if (AUX && peers.ng > 0) {
-    const uint32_t i0 = base + threadIdx.x * kPiece;
-    merge_peer_grads<true>(u.g, gdt, peers, [&](int r, uint4& w0, uint4& w1) {
-      const char* g = (const char*)L.grad + peers.gdelta[r];
-      if (gdt == FO_F32) {
-        w0 = __ldcs((const uint4*)((const float*)g + i0));
-        w1 = __ldcs((const uint4*)((const float*)g + i0) + 1);
-      } else {
-        w0 = __ldcs((const uint4*)((const unsigned short*)g + i0));
-      }
-    });
+  hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, LutGlobal{}, u);
+  if constexpr (MODE == kPeer) {
+    if (peers->ng > 0) {
+      merge_peer_grads<true>(u.g, gdt, *peers, [&](int r, uint4& w0, uint4& w1) {
+        const char* g = (const char*)L.grad + peers->gdelta[r];
+        if (gdt == FO_F32) {
+          w0 = __ldcs((const uint4*)((const float*)g + i0));
+          w1 = __ldcs((const uint4*)((const float*)g + i0) + 1);
+        } else {
+          w0 = __ldcs((const uint4*)((const unsigned short*)g + i0));
+        }
+      });
+    }
   }
-  if (AUX && clip->active) clip_grads<true>(u.g, gdt, *clip);
-  const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, base + threadIdx.x * kPiece);
-  hot_finish<true, OPT, PDT, ECC_BITS, STATE, AUX>(L, h, gdt, base, at, one, false, u, lut_mw, peers, clip);
+  if constexpr ((MODE & (kClip | kPeer)) != 0) {
+    const Clip clip = load_clip(c.sq_norm, c.max_norm, gdt);
+    if (clip.active) clip_grads<true>(u.g, gdt, clip);
+  }
+  const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, gshift, i0);
+  hot_finish<true, OPT, PDT, ECC_BITS, STATE, MODE>(c, L, out, dh, h, gdt, i0, at, false, u, OutAt{out},
+                                                    [&](uint4& w0, uint4& w1) { w0 = raw.p0; w1 = raw.p1; }, peers);
 }
 
-// One block's run of consecutive whole chunks [ch, hot_end) of a leaf, for the kernel without peer or
-// clipping code.  Three stages of compile-time size; the loop body is unrolled three times, so
+// One block's run of consecutive whole chunks [ch, hot_end) of a leaf, for the kernels without peer code.  Three stages of compile-time size; the loop body is unrolled three times, so
 // that the stage an iteration reads and the one it fills are fixed, and the thread's addresses
 // move once per three chunks: every access inside is a register plus an immediate.
-template <int OPT, int PDT, int ECC_BITS, int STATE>
-FO_DEVI void hot_run(const DevLeaf& L, const Hyp& h, const int gdt, const uint32_t ch, const uint32_t hot_end, const uint32_t stage0,
-                     const float one, const float* lut_mw, const Peers& peers) {
+template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE, typename LUT, typename OUT>
+FO_DEVI void hot_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const SharedClip& clip,
+                     const uint32_t ch, const uint32_t hot_end, const uint32_t stage0, const LUT& lut, const OUT& distance) {
+  const int gdt = c.grad_dtype;
+  const int gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;
+  const int kScB = (kChunk >> gshift) * 2;  // bytes of scales per chunk
   using S = Stage<OPT, PDT, ECC_BITS, STATE>;
   constexpr int kPsz = PDT == FO_F32 ? 4 : 2, kEsz = ECC_BITS == 16 ? 2 : 1;
   constexpr int kSsz = STATE == FO_STATE_FULL ? 4 : 1;   // bytes per element of a moment stream
@@ -1406,7 +1599,7 @@ FO_DEVI void hot_run(const DevLeaf& L, const Hyp& h, const int gdt, const uint32
   uint32_t base = ch * (uint32_t)kChunk;
   uint32_t tid;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));  // read once: otherwise re-read at every use
-  Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, base + tid * kPiece);
+  Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, gshift, base + tid * kPiece);
   const uint32_t s16 = stage0 + tid * 16u, s8 = stage0 + tid * 8u;
   const int gsz = gdt == FO_F32 ? 4 : 2;
   // copies of the chunk `ahead` chunks after the one `at` points to, into stage `slot`
@@ -1485,21 +1678,32 @@ FO_DEVI void hot_run(const DevLeaf& L, const Hyp& h, const int gdt, const uint32
       raw.msc = msc; raw.vsc = vsc;
       if constexpr (STATE == FO_STATE_QUANT) {
         if (it + (uint32_t)(k + 1) < n_it) {
-          msc = *(const __half*)(at.msc + (k + 1) * (kChunk / 32 * 2));
-          if constexpr (OPT == FO_OPT_ADAM) vsc = *(const __half*)(at.vsc + (k + 1) * (kChunk / 32 * 2));
+          msc = *(const __half*)(at.msc + (k + 1) * kScB);
+          if constexpr (OPT == FO_OPT_ADAM) vsc = *(const __half*)(at.vsc + (k + 1) * kScB);
         }
       }
       Unpacked u;
-      const bool rare = hot_unpack<false, OPT, PDT, ECC_BITS, STATE>(raw, gdt, lut_mw, one, u);
+      bool rare = hot_unpack<false, OPT, PDT, ECC_BITS, STATE>(raw, gdt, lut, u);
+      if constexpr ((MODE & kClip) != 0) {
+        if (clip.active) {
+          const bool odd = clip_grads<false>(u.g, gdt, clip);
+          rare = rare || odd;
+        }
+      }
       Piece cur;
       cur.grad = at.grad + k * (kChunk * gsz);
       cur.param = at.param + k * (kChunk * kPsz);
       cur.ecc = at.ecc + k * (kChunk * kEsz);
       cur.mu = at.mu + k * (kChunk * kSsz);
       cur.nu = at.nu + k * (kChunk * kSsz);
-      cur.msc = at.msc + k * (kChunk / 32 * 2);
-      cur.vsc = at.vsc + k * (kChunk / 32 * 2);
-      hot_finish<false, OPT, PDT, ECC_BITS, STATE, false>(L, h, gdt, base + (uint32_t)k * kChunk, cur, one, rare, u, lut_mw, peers, nullptr);
+      cur.msc = at.msc + k * kScB;
+      cur.vsc = at.vsc + k * kScB;
+      // (the old parameter is still in the stage this chunk was read from)
+      hot_finish<false, OPT, PDT, ECC_BITS, STATE, MODE>(c, L, out, dh, h, gdt, base + (uint32_t)k * kChunk + tid * kPiece, cur, rare, u, distance,
+                                                         [&](uint4& w0, uint4& w1) {
+                                                           w0 = lds128(s16 + (uint32_t)k * kSB);
+                                                           if constexpr (PDT == FO_F32) w1 = lds128(s16 + (uint32_t)k * kSB + 16u * kThreads);
+                                                         }, nullptr);
     }
     base += (uint32_t)(kS * kChunk);
     at.grad += kS * kChunk * gsz;
@@ -1510,123 +1714,22 @@ FO_DEVI void hot_run(const DevLeaf& L, const Hyp& h, const int gdt, const uint32
       if constexpr (OPT == FO_OPT_ADAM) at.nu += kS * kChunk * kSsz;
     }
     if constexpr (STATE == FO_STATE_QUANT) {
-      at.msc += kS * (kChunk / 32 * 2);
-      if constexpr (OPT == FO_OPT_ADAM) at.vsc += kS * (kChunk / 32 * 2);
+      at.msc += kS * kScB;
+      if constexpr (OPT == FO_OPT_ADAM) at.vsc += kS * kScB;
     }
   }
 }
 
-// exact dequantization tables, one entry per code byte (built once per block)
-FO_DEVI void build_luts(float* lut_m, float* lut_v) {
-  for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-    lut_m[b] = ieee::deq_m_norm((int)(signed char)b);
-    lut_v[b] = ieee::deq_v_norm(b);
-  }
-  __syncthreads();
-}
-// The momentum table once more in kLutCopies interleaved copies (entry of code b for lane l at
-// b*kLutCopies + l % kLutCopies): the straight-line path looks eight random codes up per
-// thread, and with a single copy a warp's 32 look-ups fall three deep on some bank.
-FO_DEVI void build_wide_lut(const float* lut_m, float* lut_mw) {
-  for (int i = threadIdx.x; i < 256 * kLutCopies; i += blockDim.x) lut_mw[i] = lut_m[i / kLutCopies];
-  __syncthreads();
-}
-
-template <int OPT>
-FO_DEVI bool leaf_is_hot(const StepParams& p, int l) {
-#ifdef FO_NAIVE_MATH
-  return false;
-#else
-  return p.aligned[l] != 0;
-#endif
-}
-
-// The chunks [ch, end) of leaf l that the straight-line path does not take.  An aligned leaf under
-// ordinary hyper-parameters goes through the repairing pass with a limit (vector accesses, masked at
-// the leaf's end); the scalar path keeps unaligned leaves, the CPU-path parameter hand-back and peer
-// replicas.  Out of line and fed by reference to the kernel's parameters, so that the persistent loop's
-// register allocation does not see it.
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__device__ __noinline__ void leaf_tail(const StepParams& p, const int l, uint32_t ch, const uint32_t end, const float* lut_all,
-                                       const Clip* clip) {
-  const DevLeaf& L = p.leaf[l];
-  const Hyp h = load_hyper<OPT>(p.hyper[p.hyper_of[l]]);
-  const float* lut_m = lut_all;
-  const float* lut_v = lut_all + 256;
-  const float* lut_mw = lut_all + 512 + (STATE == FO_STATE_QUANT ? (threadIdx.x & (kLutCopies - 1)) : 0);
-  bool hyper_ok = (h.flags & FO_FLAG_LP_DELTA) == 0;  // as in the kernel: what the straight-line arithmetic may take
-  if constexpr (OPT == FO_OPT_ADAM) hyper_ok = hyper_ok && (h.flags & kFlagTameAdam) != 0;
-  const bool vector_ok = leaf_is_hot<OPT>(p, l) && hyper_ok &&
-                         (!AUX || (p.peers.n == 0 && p.peers.ng == 0 && p.peers.mc_pdelta == 0 && p.peers.mc_gdelta == 0));
-  Clip none;
-  none.active = false; none.div_ok = true; none.n_g = 1.0f; none.rcp_n = 1.0f; none.m_g = 1.0f;
-  for (; ch < end; ++ch) {
-    if (vector_ok)
-      ragged_chunk<OPT, PDT, ECC_BITS, STATE, AUX>(L, h, p.grad_dtype, ch * (uint32_t)kChunk, p.one, lut_mw, p.peers, clip, (uint32_t)L.n);
-    else
-      cold_chunk<OPT, PDT, ECC_BITS, STATE>(L, h, p.grad_dtype, (unsigned long long)ch * kChunk, lut_m, lut_v, p.peers, clip != nullptr ? *clip : none);
-  }
-}
-
-// Second walk over the runs of this block, for what the straight-line loop of step_kernel skipped.
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__device__ __noinline__ void block_tails(const StepParams& p, const float* lut_all) {
-  const Clip clip = load_clip(AUX ? p.sq_norm : nullptr, p.max_norm, p.grad_dtype);
-  const uint32_t total = p.first_block[p.n_leaves];
-  for (uint32_t run0 = blockIdx.x * p.run_chunks; run0 < total; run0 += gridDim.x * p.run_chunks) {
-    uint32_t c = run0;
-    const uint32_t c_hi = min(total, run0 + p.run_chunks);
-    int l_first = 0;
-    for (int l_end = p.n_leaves; l_end - l_first > 1;) {
-      const int mid = (l_first + l_end) >> 1;
-      if (p.first_block[mid] <= c) l_first = mid; else l_end = mid;
-    }
-    for (int l = l_first; l < p.n_leaves && c < c_hi; ++l) {
-      const uint32_t first = p.first_block[l];
-      const uint32_t next = min(p.first_block[l + 1], c_hi);
-      if (c >= next) continue;
-      const uint32_t end = next - first;
-      uint32_t ch = c - first;
-      const uint32_t flags = p.hyper[p.hyper_of[l]].dyn != nullptr ? load_hyper<OPT>(p.hyper[p.hyper_of[l]]).flags : p.hyper[p.hyper_of[l]].flags;
-      bool hyper_ok = (flags & FO_FLAG_LP_DELTA) == 0;
-      if constexpr (OPT == FO_OPT_ADAM) hyper_ok = hyper_ok && (flags & kFlagTameAdam) != 0;
-      const uint32_t hot_end = (leaf_is_hot<OPT>(p, l) && hyper_ok) ? min(end, (uint32_t)(p.leaf[l].n / kChunk)) : 0u;
-      if (ch < hot_end) ch = hot_end;  // those were done
-      if (ch < end) leaf_tail<OPT, PDT, ECC_BITS, STATE, AUX>(p, l, ch, end, lut_all, AUX ? &clip : nullptr);
-      c = next;
-    }
-  }
-}
-
-// Persistent grid.  The chunks of all leaves form one sequence (first_block[] gives each leaf's
-// first position in it) and block b takes positions b, b + grid, b + 2*grid, ...: at any moment
-// the blocks work on neighbouring chunks, which keeps the DRAM pages they stream from few.
-// Every block walks the leaves in order.  Inside a leaf its whole aligned chunks are taken by
-// the straight-line path with nothing per chunk but a counter and the prefetch of the block's
-// next chunk; what is left (a ragged last chunk, unaligned leaves, hyper-parameter sets outside
-// the shortcuts' range) goes to the scalar IEEE path.
-// AUX: the instantiation that also averages the peers' gradients and / or clips by the global
-// norm; the plain one carries none of that code or state.
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const __grid_constant__ StepParams p) {
-  // one array for the three tables, so that the out-of-line paths need one pointer: [0, 256) momentum,
-  // [256, 512) second moment, [512, 512 + 256 * kLutCopies) the interleaved momentum copies
-  __shared__ float lut_all[512 + (STATE == FO_STATE_QUANT ? 256 * kLutCopies : 1)];
-  float* const lut_m = lut_all;
-  float* const lut_v = lut_all + 256;
-  float* const lut_m_wide = lut_all + 512;
-  if constexpr (STATE == FO_STATE_QUANT) {
-    build_luts(lut_m, lut_v);
-    build_wide_lut(lut_m, lut_m_wide);
-  }
-  const float* lut_mw = lut_m_wide + (STATE == FO_STATE_QUANT ? (threadIdx.x & (kLutCopies - 1)) : 0);
-  extern __shared__ __align__(16) unsigned char stage_mem[];  // p.stages stages of Stage::bytes(grad dtype)
+// The same for the kernel that also averages the peers' gradients and / or stores into their replicas.
+template <int OPT, int PDT, int ECC_BITS, int STATE, typename LUT>
+FO_DEVI void peer_run(const StepParams<kPeer>& p, const DevLeaf& L, const DevHyper& dh, const Hyp& h, const SharedClip& clip, uint32_t ch,
+                      const uint32_t hot_end, const uint32_t stage0, const LUT& lut) {
   using S = Stage<OPT, PDT, ECC_BITS, STATE>;
+  const int gdt = p.grad_dtype;
   // gradients summed in the NVLink switch (16-bit gradients only; fp32 leaves take the point-to-point route)
-  const bool switch_sum = AUX && p.peers.mc_gdelta != 0 && p.grad_dtype != FO_F32;
-  const int ng = (AUX && !switch_sum) ? p.peers.ng : 0;
-  const uint32_t stage_bytes = (uint32_t)S::bytes(p.grad_dtype, ng);
-  const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(stage_mem);
+  const bool switch_sum = p.peers.mc_gdelta != 0 && gdt != FO_F32;
+  const int ng = switch_sum ? 0 : p.peers.ng;
+  const uint32_t stage_bytes = (uint32_t)S::bytes(gdt, ng);
   const uint32_t stage_end = stage0 + (uint32_t)p.stages * stage_bytes;
   // Ring of kSwitchBatch thread-private slots behind the stages.  A multicast load-reduce takes
   // several microseconds and no asynchronous copy can issue one, so each thread keeps a batch of
@@ -1634,175 +1737,243 @@ __global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const _
   // the ring (the sums for this and the next iterations) and issues the next batch.
   const uint32_t ring0 = stage_end;
   const uint32_t toff = threadIdx.x * kPiece;
-  const Clip clip = load_clip(AUX ? p.sq_norm : nullptr, p.max_norm, p.grad_dtype);
-  // The chunks of all leaves form one sequence, cut into runs of p.run_chunks consecutive chunks; block b
-  // takes runs b, b + grid, b + 2 grid, ...  Inside a run every address advances by compile-time
-  // constants; dealing the runs out in turn spreads regions that cost more (rows at rest, ragged ends,
-  // values outside the shortcuts' ranges) over all blocks.
-  const uint32_t total = p.first_block[p.n_leaves];
-  constexpr uint32_t grid = 1u;   // chunk stride inside a run
-  for (uint32_t run0 = blockIdx.x * p.run_chunks; run0 < total; run0 += gridDim.x * p.run_chunks) {
-  uint32_t c = run0;  // this block's next position in the sequence
-  const uint32_t c_hi = min(total, run0 + p.run_chunks);
-  int l_first = 0;
-  for (int l_end = p.n_leaves; l_end - l_first > 1;) {  // the leaf that holds position c
-    const int mid = (l_first + l_end) >> 1;
-    if (p.first_block[mid] <= c) l_first = mid; else l_end = mid;
+  const uint32_t stride = (uint32_t)kChunk;
+  uint32_t base = ch * (uint32_t)kChunk;
+  // Copy pipeline: one group per chunk (empty past the end of the run, so that the count of
+  // groups still pending always tells which chunk has landed).  The stage filled in an
+  // iteration is the one read in the iteration before, whose values have been consumed.
+  uint32_t fill_ch = ch, fill_base = base, wr = stage0;
+  uint4 batch[kSwitchBatch] = {};
+  uint32_t turn = 0;  // iteration number inside the run, modulo kSwitchBatch
+  const char* mc_grad = (const char*)L.grad + p.peers.mc_gdelta;
+  if (switch_sum) {
+#pragma unroll
+    for (int k = 0; k < kSwitchBatch; ++k)
+      if (ch + (uint32_t)k < hot_end)
+        batch[k] = multicast_sum(mc_grad + (size_t)(base + (uint32_t)k * stride + toff) * 2u, gdt);
   }
-  for (int l = l_first; l < p.n_leaves; ++l) {
-    const uint32_t first = p.first_block[l];
-    if (c >= c_hi) break;
-    const uint32_t next = min(p.first_block[l + 1], c_hi);
-    if (c >= next) continue;
-    const uint32_t end = next - first;  // chunks in this leaf
-    uint32_t ch = c - first;            // this block's first chunk inside the leaf
-    const DevLeaf& L = p.leaf[l];
-    const Hyp h = load_hyper<OPT>(p.hyper[p.hyper_of[l]]);
-    // the CPU-path parameter hand-back (FO_FLAG_LP_DELTA) needs the old stored value to the end: IEEE path only
-    bool hyper_ok = (h.flags & FO_FLAG_LP_DELTA) == 0;
-    if constexpr (OPT == FO_OPT_ADAM) hyper_ok = hyper_ok && (h.flags & kFlagTameAdam) != 0;  // the reciprocal shortcut in the denominator
-    const uint32_t hot_end = (leaf_is_hot<OPT>(p, l) && hyper_ok) ? min(end, (uint32_t)(L.n / kChunk)) : 0u;  // whole chunks
-    if constexpr (!AUX) {
-      if (ch < hot_end) {
-        hot_run<OPT, PDT, ECC_BITS, STATE>(L, h, p.grad_dtype, ch, hot_end, stage0, p.one, lut_mw, p.peers);
-        ch = hot_end;
-      }
-    } else if (ch < hot_end) {
-      const uint32_t stride = grid * (uint32_t)kChunk;
-      uint32_t base = ch * (uint32_t)kChunk;
-      // Copy pipeline: one group per chunk (empty past the end of the run, so that the count of
-      // groups still pending always tells which chunk has landed).  The stage filled in an
-      // iteration is the one read in the iteration before, whose values have been consumed.
-      uint32_t fill_ch = ch, fill_base = base, wr = stage0;
-      uint4 batch[kSwitchBatch] = {};
-      uint32_t turn = 0;  // iteration number inside the run, modulo kSwitchBatch
-      const char* mc_grad = (const char*)L.grad + p.peers.mc_gdelta;
-      if (switch_sum) {
+  for (int k = 1; k < p.stages; ++k) {
+    if (fill_ch < hot_end) stage_fill<OPT, PDT, ECC_BITS, STATE>(L, gdt, fill_base + toff, wr, p.peers, ng, !switch_sum);
+    copy_commit();
+    ++fill_ch; fill_base += stride; wr += stage_bytes;
+  }
+  uint32_t rd = stage0;
+  // the group scales go through registers, one chunk ahead
+  __half msc = __float2half(0.0f), vsc = msc;
+  if constexpr (STATE == FO_STATE_QUANT) {
+    msc = ((const __half*)L.mu_scales)[(base + toff) >> 5];
+    if constexpr (OPT == FO_OPT_ADAM) vsc = ((const __half*)L.nu_scales)[(base + toff) >> 5];
+  }
+  for (; ch < hot_end; ++ch, base += stride) {
+    if (switch_sum && turn == 0) {
 #pragma unroll
-        for (int k = 0; k < kSwitchBatch; ++k)
-          if (ch + (uint32_t)k * grid < hot_end)
-            batch[k] = multicast_sum(mc_grad + (size_t)(base + (uint32_t)k * stride + toff) * 2u, p.grad_dtype);
-      }
-      for (int k = 1; k < p.stages; ++k) {
-        if (fill_ch < hot_end) stage_fill<OPT, PDT, ECC_BITS, STATE>(L, p.grad_dtype, fill_base + toff, wr, p.peers, ng, !switch_sum);
-        copy_commit();
-        fill_ch += grid; fill_base += stride; wr += stage_bytes;
-      }
-      uint32_t rd = stage0;
-      // the group scales go through registers, one chunk ahead
-      __half msc = __float2half(0.0f), vsc = msc;
-      if constexpr (STATE == FO_STATE_QUANT) {
-        msc = ((const __half*)L.mu_scales)[(base + toff) >> 5];
-        if constexpr (OPT == FO_OPT_ADAM) vsc = ((const __half*)L.nu_scales)[(base + toff) >> 5];
-      }
-      for (; ch < hot_end; ch += grid, base += stride) {
-        if (switch_sum && turn == 0) {
-#pragma unroll
-          for (int k = 0; k < kSwitchBatch; ++k) {  // park what has arrived, ask for the batch after it
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(ring0 + (uint32_t)k * (16u * kThreads) + threadIdx.x * 16u),
-                         "r"(batch[k].x), "r"(batch[k].y), "r"(batch[k].z), "r"(batch[k].w) : "memory");
-            if (ch + (uint32_t)(kSwitchBatch + k) * grid < hot_end)
-              batch[k] = multicast_sum(mc_grad + (size_t)(base + (uint32_t)(kSwitchBatch + k) * stride + toff) * 2u, p.grad_dtype);
-          }
-        }
-        if (fill_ch < hot_end) stage_fill<OPT, PDT, ECC_BITS, STATE>(L, p.grad_dtype, fill_base + toff, wr, p.peers, ng, !switch_sum);
-        copy_commit();
-        fill_ch += grid; fill_base += stride;
-        wr += stage_bytes;
-        if (wr == stage_end) wr = stage0;
-        if (!AUX || p.stages <= 3) {  // all but the oldest group may still be pending; local streams use 2 or 3 stages
-          if (p.stages == 3) copy_wait<2>();
-          else copy_wait<1>();
-        } else switch (p.stages) {
-          case 2: copy_wait<1>(); break;
-          case 3: copy_wait<2>(); break;
-          case 4: copy_wait<3>(); break;
-          case 5: copy_wait<4>(); break;
-          case 6: copy_wait<5>(); break;
-          case 7: copy_wait<6>(); break;
-          default: copy_wait<7>(); break;
-        }
-        Raw<OPT, PDT, ECC_BITS, STATE> raw;
-        stage_read<OPT, PDT, ECC_BITS, STATE>(p.grad_dtype, rd, raw);
-        const uint32_t peer_grads = rd + S::kOffGrad + (uint32_t)S::grad_bytes(p.grad_dtype);
-        rd += stage_bytes;
-        if (rd == stage_end) rd = stage0;
-        raw.msc = msc; raw.vsc = vsc;
-        if constexpr (STATE == FO_STATE_QUANT) {
-          if (ch + grid < hot_end) {
-            msc = ((const __half*)L.mu_scales)[(base + stride + toff) >> 5];
-            if constexpr (OPT == FO_OPT_ADAM) vsc = ((const __half*)L.nu_scales)[(base + stride + toff) >> 5];
-          }
-        }
-        Unpacked u;
-        bool rare = hot_unpack<false, OPT, PDT, ECC_BITS, STATE>(raw, p.grad_dtype, lut_mw, p.one, u);
-        if (switch_sum) {
-          const uint4 sum = lds128(ring0 + turn * (16u * kThreads) + threadIdx.x * 16u);
-          turn = turn + 1 == kSwitchBatch ? 0u : turn + 1;
-          grad_pairs(sum, sum, p.grad_dtype, u.g);
-          const bool odd = mean_of_sum<false>(u.g, p.grad_dtype, p.peers);
-          rare = rare || odd;
-        }
-        if (AUX && ng > 0) {
-          const bool odd = merge_peer_grads<false>(u.g, p.grad_dtype, p.peers, [&](int r, uint4& w0, uint4& w1) {
-            const uint32_t at = peer_grads + (uint32_t)r * (uint32_t)S::grad_bytes(p.grad_dtype) + threadIdx.x * 16u;
-            w0 = lds128(at);
-            if (p.grad_dtype == FO_F32) w1 = lds128(at + 16u * kThreads);
-          });
-          rare = rare || odd;
-        }
-        if (AUX && clip.active) {
-          const bool odd = clip_grads<false>(u.g, p.grad_dtype, clip);
-          rare = rare || odd;
-        }
-        const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, p.grad_dtype, base + toff);
-        hot_finish<false, OPT, PDT, ECC_BITS, STATE, AUX>(L, h, p.grad_dtype, base, at, p.one, rare, u, lut_mw, p.peers, AUX ? &clip : nullptr);
+      for (int k = 0; k < kSwitchBatch; ++k) {  // park what has arrived, ask for the batch after it
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(ring0 + (uint32_t)k * (16u * kThreads) + threadIdx.x * 16u),
+                     "r"(batch[k].x), "r"(batch[k].y), "r"(batch[k].z), "r"(batch[k].w) : "memory");
+        if (ch + (uint32_t)(kSwitchBatch + k) < hot_end)
+          batch[k] = multicast_sum(mc_grad + (size_t)(base + (uint32_t)(kSwitchBatch + k) * stride + toff) * 2u, gdt);
       }
     }
-    ch = end;  // the rest of the leaf in this run is taken after the loop (block_tails)
-    c = first + ch;
+    if (fill_ch < hot_end) stage_fill<OPT, PDT, ECC_BITS, STATE>(L, gdt, fill_base + toff, wr, p.peers, ng, !switch_sum);
+    copy_commit();
+    ++fill_ch; fill_base += stride;
+    wr += stage_bytes;
+    if (wr == stage_end) wr = stage0;
+    if (p.stages <= 3) {  // all but the oldest group may still be pending; local streams use 2 or 3 stages
+      if (p.stages == 3) copy_wait<2>();
+      else copy_wait<1>();
+    } else switch (p.stages) {
+      case 2: copy_wait<1>(); break;
+      case 3: copy_wait<2>(); break;
+      case 4: copy_wait<3>(); break;
+      case 5: copy_wait<4>(); break;
+      case 6: copy_wait<5>(); break;
+      case 7: copy_wait<6>(); break;
+      default: copy_wait<7>(); break;
+    }
+    Raw<OPT, PDT, ECC_BITS, STATE> raw;
+    stage_read<OPT, PDT, ECC_BITS, STATE>(gdt, rd, raw);
+    const uint32_t peer_grads = rd + S::kOffGrad + (uint32_t)S::grad_bytes(gdt);
+    rd += stage_bytes;
+    if (rd == stage_end) rd = stage0;
+    raw.msc = msc; raw.vsc = vsc;
+    if constexpr (STATE == FO_STATE_QUANT) {
+      if (ch + 1u < hot_end) {
+        msc = ((const __half*)L.mu_scales)[(base + stride + toff) >> 5];
+        if constexpr (OPT == FO_OPT_ADAM) vsc = ((const __half*)L.nu_scales)[(base + stride + toff) >> 5];
+      }
+    }
+    Unpacked u;
+    bool rare = hot_unpack<false, OPT, PDT, ECC_BITS, STATE>(raw, gdt, lut, u);
+    if (switch_sum) {
+      const uint4 sum = lds128(ring0 + turn * (16u * kThreads) + threadIdx.x * 16u);
+      turn = turn + 1 == kSwitchBatch ? 0u : turn + 1;
+      grad_pairs(sum, sum, gdt, u.g);
+      const bool odd = mean_of_sum<false>(u.g, gdt, p.peers);
+      rare = rare || odd;
+    }
+    if (ng > 0) {
+      const bool odd = merge_peer_grads<false>(u.g, gdt, p.peers, [&](int r, uint4& w0, uint4& w1) {
+        const uint32_t at = peer_grads + (uint32_t)r * (uint32_t)S::grad_bytes(gdt) + threadIdx.x * 16u;
+        w0 = lds128(at);
+        if (gdt == FO_F32) w1 = lds128(at + 16u * kThreads);
+      });
+      rare = rare || odd;
+    }
+    if (clip.active) {
+      const bool odd = clip_grads<false>(u.g, gdt, clip);
+      rare = rare || odd;
+    }
+    const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, 5, base + toff);
+    hot_finish<false, OPT, PDT, ECC_BITS, STATE, kPeer>(p, L, nullptr, dh, h, gdt, base + toff, at, rare, u, OutAt{nullptr}, [](uint4&, uint4&) {}, &p.peers);
   }
-  }
-  // What the loop left (ragged last chunks, leaves the straight-line path does not take) is the work of
-  // step_tail_kernel, a launch of its own: measured on the 80-register Lion / SGD kernels, a call to
-  // that code from this kernel, inside the leaf loop or after it, cost a quarter of their throughput
-  // (spills in the loop, no uniform registers).
 }
 
-// The same walk over the same runs for what step_kernel skipped; launched after it with the same grid
-// when the leaf table has a ragged end, an unaligned leaf or hyper-parameters outside the shortcuts'
-// range (the launcher looks).
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-__global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_tail_kernel(const __grid_constant__ StepParams p) {
-  __shared__ float lut_all[512 + (STATE == FO_STATE_QUANT ? 256 * kLutCopies : 1)];
-  if constexpr (STATE == FO_STATE_QUANT) {
-    build_luts(lut_all, lut_all + 256);
-    build_wide_lut(lut_all, lut_all + 512);
+// The momentum table in kLutCopies interleaved copies (entry of code b for lane l at
+// b*kLutCopies + l % kLutCopies): the straight-line path looks eight random codes up per
+// thread, and with a single copy a warp's 32 look-ups fall three deep on some bank.
+FO_DEVI void build_wide_lut(float* lut_mw) {
+  for (int i = threadIdx.x; i < 256 * kLutCopies; i += blockDim.x) lut_mw[i] = __ldg(&kDeqM.v[i / kLutCopies]);
+  __syncthreads();
+}
+
+// Launches of one call are chained: a kernel lets the next one start as soon as its own blocks are resident
+// (they work on different leaves), and no kernel completes before the one in front of it has, so that whatever
+// the stream holds next sees all of them done.  One thread's wait is enough for that.
+FO_DEVI void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+FO_DEVI void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+FO_DEVI void chain_end() {
+  if (blockIdx.x == 0 && threadIdx.x == 0) chain_wait();
+}
+
+// the leaf of a table that holds position c of the common sequence
+FO_DEVI int leaf_of(const uint32_t* first, const int n_leaves, const uint32_t c) {
+  int lo = 0;
+  for (int hi = n_leaves; hi - lo > 1;) {
+    const int mid = (lo + hi) >> 1;
+    if (first[mid] <= c) lo = mid; else hi = mid;
   }
-  block_tails<OPT, PDT, ECC_BITS, STATE, AUX>(p, lut_all);
+  return lo;
+}
+
+// Persistent grid over whole chunks.  The chunks of all leaves form one sequence, cut into runs of
+// p.run_chunks consecutive chunks; block b takes runs b, b + grid, b + 2 grid, ...  Inside a run every
+// address advances by compile-time constants; dealing the runs out in turn spreads regions that cost more
+// (rows at rest, values outside the shortcuts' ranges) over all blocks.  The kernel holds nothing but this:
+// measured on the 80-register Lion / SGD kernels, a call to the code for ragged ends from here, inside the leaf
+// loop or after it, cost a quarter of their throughput (spills in the loop, no uniform registers).
+template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
+__global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const __grid_constant__ StepParams<MODE> p) {
+  chain_release();
+  __shared__ float lut_wide[STATE == FO_STATE_QUANT ? 256 * kLutCopies : 1];
+  if constexpr (STATE == FO_STATE_QUANT) build_wide_lut(lut_wide);
+  const LutWide lut{lut_wide + (STATE == FO_STATE_QUANT ? (threadIdx.x & (kLutCopies - 1)) : 0)};
+  extern __shared__ __align__(16) unsigned char stage_mem[];  // p.stages stages of Stage::bytes(grad dtype)
+  using S = Stage<OPT, PDT, ECC_BITS, STATE>;
+  const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(stage_mem);
+  const int gdt = p.grad_dtype;
+  if ((MODE & (kClip | kPeer)) != 0 && p.sq_norm != nullptr) chain_wait();  // the norm comes from a kernel in front of this one
+  SharedClip clip{false, 0u};
+  if constexpr ((MODE & (kClip | kPeer)) != 0) {
+    __shared__ float4 clip_constants;
+    const Clip k = load_clip(p.sq_norm, p.max_norm, gdt);
+    if (threadIdx.x == 0) clip_constants = make_float4(k.n_g, k.rcp_n, k.m_g, __uint_as_float(k.div_ok ? 1u : 0u));
+    __syncthreads();
+    clip.active = k.active;
+    clip.at = (uint32_t)__cvta_generic_to_shared(&clip_constants);
+  }
+  const uint32_t total = p.t.first_block[p.n_leaves];
+  for (uint32_t run0 = blockIdx.x * p.run_chunks; run0 < total; run0 += gridDim.x * p.run_chunks) {
+    uint32_t c = run0;  // this block's next position in the sequence
+    const uint32_t c_hi = min(total, run0 + p.run_chunks);
+    for (int l = leaf_of(p.t.first_block, p.n_leaves, c); l < p.n_leaves; ++l) {
+      if (c >= c_hi) break;
+      const uint32_t first = p.t.first_block[l];
+      const uint32_t next = min(p.t.first_block[l + 1], c_hi);
+      if (c >= next) continue;
+      const uint32_t end = next - first;  // chunks of this leaf in this run
+      uint32_t ch = c - first;            // the first of them
+      c = next;
+      const DevLeaf& L = p.t.leaf[l];
+      const DevHyper& dh = p.hyper[p.t.hyper_of[l]];
+      const DevOut* out = nullptr;
+      if constexpr ((MODE & kOut) != 0) out = &p.out[l];
+      const Hyp h = load_hyper<OPT>(dh);
+      if constexpr (OPT == FO_OPT_ADAM) {
+        // device-resident scalars can leave the range the reciprocal shortcut in the denominator is proven for
+        if ((h.flags & kFlagTameAdam) == 0) {
+          const Peers* peers = nullptr;
+          if constexpr (MODE == kPeer) peers = &p.peers;
+          for (; ch < end; ++ch)
+            cold_piece<OPT, PDT, ECC_BITS, STATE>(L, out, dh, gdt, (MODE & kGroup) != 0 ? p.group_shift : 5, (unsigned long long)ch * kChunk + threadIdx.x * kPiece, peers,
+                                                  (MODE & (kClip | kPeer)) != 0 ? p.sq_norm : nullptr, p.max_norm);
+          continue;
+        }
+      }
+      if constexpr (MODE != kPeer) {
+        if constexpr ((MODE & kOut) != 0)
+          hot_run<OPT, PDT, ECC_BITS, STATE, MODE>(p, L, out, dh, h, clip, ch, end, stage0, lut, OutOf{p, l});
+        else
+          hot_run<OPT, PDT, ECC_BITS, STATE, MODE>(p, L, out, dh, h, clip, ch, end, stage0, lut, OutAt{nullptr});
+      } else {
+        peer_run<OPT, PDT, ECC_BITS, STATE>(p, L, dh, h, clip, ch, end, stage0, lut);
+      }
+    }
+  }
+  chain_end();
+}
+
+// Everything the chunks of step_kernel leave over, in pieces of 1024 elements dealt out to 128-thread blocks.
+// Latency bound (a piece is one load, one pass of arithmetic, one store), hence many small blocks; measured
+// against the same work on step_kernel's grid of 512- and 768-thread blocks, which took 10 to 17 us for a single
+// ragged end, see launch_pieces.
+template <int OPT, int PDT, int ECC_BITS, int STATE, int N>
+__global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_constant__ PieceParams<N> p) {
+  chain_release();
+  const bool with_peers = p.peers.n > 0 || p.peers.ng > 0 || p.peers.mc_pdelta != 0 || p.peers.mc_gdelta != 0;
+  if (p.sq_norm != nullptr) chain_wait();
+  const Clip clip = load_clip(p.sq_norm, p.max_norm, p.grad_dtype);
+  const uint32_t total = p.first_piece[p.n_leaves];
+  for (uint32_t q = blockIdx.x; q < total; q += gridDim.x) {
+    const int l = leaf_of(p.first_piece, p.n_leaves, q);
+    const DevLeaf& L = p.leaf[l];
+    const DevHyper& dh = p.hyper[p.hyper_of[l]];
+    const uint32_t i0 = (p.start[l] + (q - p.first_piece[l])) * (uint32_t)kPieceElems + threadIdx.x * kPiece;
+    bool vector_ok = p.hot[l] != 0 && !with_peers;
+    const Hyp h = load_hyper<OPT>(dh);
+    if constexpr (OPT == FO_OPT_ADAM) vector_ok = vector_ok && (h.flags & kFlagTameAdam) != 0;
+    if (vector_ok)
+      ragged_piece<OPT, PDT, ECC_BITS, STATE>(p, L, p.out[l], dh, h, clip, i0, (uint32_t)L.n);
+    else
+      cold_piece<OPT, PDT, ECC_BITS, STATE>(L, &p.out[l], dh, p.grad_dtype, p.group_shift, i0, with_peers ? &p.peers : nullptr, p.sq_norm, p.max_norm);
+  }
+  chain_end();
 }
 
 // ---- any group size (1..1024): one block per tile of whole groups, group maxima through
-// shared-memory atomics on the (non-negative) float bit patterns; IEEE arithmetic only ------
+// shared-memory atomics on the (non-negative) float bit patterns; IEEE arithmetic only.  For group sizes that
+// are not 8, 16, ..., 256 (those run step_kernel and piece_kernel) ------------------------------------------
 template <int OPT, int PDT, int ECC_BITS>
-__global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant__ StepParams p) {
-  __shared__ float lut_m[256], lut_v[256];
+__global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant__ StepParams<kOut> p) {
+  chain_release();
   __shared__ unsigned int smax_m[kGenericTile], smax_v[kGenericTile];
-  build_luts(lut_m, lut_v);
+  if (p.sq_norm != nullptr) chain_wait();
   const Clip clip = load_clip(p.sq_norm, p.max_norm, p.grad_dtype);
-  int lo = 0, hi = p.n_leaves;
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if (p.first_block[mid] <= blockIdx.x) lo = mid; else hi = mid;
-  }
-  const int l = lo;
-  const DevLeaf& L = p.leaf[l];
-  const Hyp h = load_hyper<OPT>(p.hyper[p.hyper_of[l]]);
+  const int l = leaf_of(p.t.first_block, p.n_leaves, blockIdx.x);
+  const DevLeaf& L = p.t.leaf[l];
+  const DevOut& out = p.out[l];
+  const Hyp h = load_hyper<OPT>(p.hyper[p.t.hyper_of[l]]);
   const int G = p.group_size;
   const int groups_per_tile = max(1, kGenericTile / G);
   const int tile = groups_per_tile * G;
   const unsigned long long n = L.n;
-  const unsigned long long base = (unsigned long long)(blockIdx.x - p.first_block[l]) * tile;
+  const unsigned long long base = (unsigned long long)(blockIdx.x - p.t.first_block[l]) * tile;
+  char* const o_param = (char*)L.param + out.param;
+  char* const o_ecc = (char*)L.ecc + out.ecc;
+  char* const o_mu = (char*)L.mu + out.mu;
+  char* const o_nu = (char*)L.nu + out.nu;
+  __half* const o_msc = (__half*)((char*)L.mu_scales + out.mu_scales);
+  __half* const o_vsc = (__half*)((char*)L.nu_scales + out.nu_scales);
   for (int i = threadIdx.x; i < groups_per_tile; i += 256) { smax_m[i] = 0u; smax_v[i] = 0u; }
   __syncthreads();
   constexpr int kPer = kGenericTile / 256;
@@ -1827,23 +1998,23 @@ __global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant
         if constexpr (ECC_BITS == 8) e = ((const signed char*)L.ecc)[i];
         theta = master_of_ieee<PDT, ECC_BITS>(pb, e);
       }
-      float mm = fmul(lut_m[((const unsigned char*)L.mu)[i]], __half2float(((const __half*)L.mu_scales)[gi]));
+      float mm = fmul(kDeqM.v[((const unsigned char*)L.mu)[i]], __half2float(((const __half*)L.mu_scales)[gi]));
       float vv = 0.0f, rr = 0.0f;
       if constexpr (OPT == FO_OPT_ADAM) {
-        float s = fmul(lut_v[((const unsigned char*)L.nu)[i]], __half2float(((const __half*)L.nu_scales)[gi]));
+        float s = fmul(ieee::deq_v_norm(((const unsigned char*)L.nu)[i]), __half2float(((const __half*)L.nu_scales)[gi]));
         vv = fmul(s, s);
       }
       update_element_ieee<OPT, FO_STATE_QUANT>(h, g, theta, mm, vv, rr);
       if constexpr (PDT == FO_F32) {
         if (h.flags & FO_FLAG_LP_DELTA) theta = fadd(old_f32, fsub(theta, old_f32));
-        ((float*)L.param)[i] = theta;
+        ((float*)o_param)[i] = theta;
       } else {
         uint32_t nb;
         int e;
         store_form_ieee<PDT, ECC_BITS>(h.flags, theta, pb, nb, e);
-        ((unsigned short*)L.param)[i] = (unsigned short)nb;
-        if constexpr (ECC_BITS == 16) ((short*)L.ecc)[i] = (short)e;
-        if constexpr (ECC_BITS == 8) ((signed char*)L.ecc)[i] = (signed char)e;
+        ((unsigned short*)o_param)[i] = (unsigned short)nb;
+        if constexpr (ECC_BITS == 16) ((short*)o_ecc)[i] = (short)e;
+        if constexpr (ECC_BITS == 8) ((signed char*)o_ecc)[i] = (signed char)e;
       }
       m[k] = mm; root[k] = rr;
       atomicMax(&smax_m[li / G], __float_as_uint(fabsf(mm)));
@@ -1858,15 +2029,16 @@ __global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant
     const unsigned long long i = base + li;
     if (li < tile && i < n) {
       const float am = __uint_as_float(smax_m[li / G]);
-      ((signed char*)L.mu)[i] = (signed char)ieee::quant_m(m[k], ieee::safe_scale(am, floor_mode));
-      if (li % G == 0) ((__half*)L.mu_scales)[i / G] = __float2half_rn(am);
+      ((signed char*)o_mu)[i] = (signed char)ieee::quant_m(m[k], ieee::safe_scale(am, floor_mode));
+      if (li % G == 0) o_msc[i / G] = __float2half_rn(am);
       if constexpr (OPT == FO_OPT_ADAM) {
         const float av = __uint_as_float(smax_v[li / G]);
-        ((unsigned char*)L.nu)[i] = (unsigned char)ieee::quant_v(root[k], ieee::safe_scale(av, floor_mode));
-        if (li % G == 0) ((__half*)L.nu_scales)[i / G] = __float2half_rn(av);
+        ((unsigned char*)o_nu)[i] = (unsigned char)ieee::quant_v(root[k], ieee::safe_scale(av, floor_mode));
+        if (li % G == 0) o_vsc[i / G] = __float2half_rn(av);
       }
     }
   }
+  chain_end();
 }
 
 // elements one block of the any-group-size kernel covers
@@ -1874,35 +2046,79 @@ inline unsigned int generic_tile_elems(int group_size) {
   return (unsigned int)(kGenericTile / group_size > 0 ? kGenericTile / group_size : 1) * (unsigned int)group_size;
 }
 
-// grid of the persistent kernel: resident blocks per SM x SMs of the current device
-struct LaunchInfo {
-  unsigned int total_chunks;
-  int sm_count;
+}  // namespace FO_SHAPE_NS
+
+// ---- host side --------------------------------------------------------------------------------------------
+
+// What a call hands to the launchers of its kernel slice (host memory).
+struct HostLeaf {
+  DevLeaf src;
+  DevOut out;
+  uint8_t hyper;
+  uint8_t hot;  // aligned, and its hyper-parameters are in the range of the vector path as far as the host knows
 };
-using LaunchFn = cudaError_t (*)(const StepParams&, const LaunchInfo&, cudaStream_t);
-// A kernel slice and the elements one of its chunks covers.  Block size, and with it the chunk, is a
-// property of the slice (the slices are compiled with their own FO_THREADS): the host builds
-// first_block[] from this number.
+struct HostStep {
+  const HostLeaf* leaf;
+  int n_leaves;
+  const DevHyper* hyper;
+  int n_hypers;
+  int grad_dtype, group_shift, group_size;
+  int sm_count;
+  const double* sq_norm;
+  float max_norm;
+  const Peers* peers;
+};
+// `chained`: the launch in front of this one on the stream is one of this library's and works on other leaves
+// (or is the one whose result chain_wait() in the kernel waits for); set to true by a launch.
+using MainFn = cudaError_t (*)(const HostStep&, bool& chained, cudaStream_t);
+using PieceFn = cudaError_t (*)(const HostStep&, unsigned int main_chunk, bool& chained, cudaStream_t);
+// A slice of step_kernel and the elements one of its chunks covers.  Block size, and with it the chunk, is a
+// property of the slice (the slices are compiled with their own FO_THREADS).
 struct Launcher {
-  LaunchFn launch;
+  MainFn launch;
   unsigned int chunk;
 };
+
+template <typename P>
+cudaError_t launch_chained(void (*kernel)(P), unsigned int grid, unsigned int threads, int smem, bool& chained, cudaStream_t s, const P& p) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = (size_t)smem;
+  c.stream = s;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = a;
+  c.numAttrs = chained ? 1 : 0;
+  chained = true;
+  return cudaLaunchKernelEx(&c, kernel, p);
+}
+
+inline void fill_common(StepCommon& p, const HostStep& s) {
+  for (int i = 0; i < s.n_hypers; ++i) p.hyper[i] = s.hyper[i];
+  p.n_leaves = 0;
+  p.grad_dtype = s.grad_dtype;
+  p.group_shift = s.group_shift;
+  p.group_size = s.group_size;
+  p.one = 1.0f;
+  p.stages = 0;
+  p.run_chunks = 1;
+  p.sq_norm = s.sq_norm;
+  p.max_norm = s.max_norm;
+}
+
+inline namespace FO_SHAPE_NS {
 
 // Shared memory of one SM that blocks may use, and what each block loses to the system.
 constexpr int kSmemPerSm = 227 * 1024, kSmemReservedPerBlock = 1024;
 
-// whether a step needs the kernel that carries the peer and clipping code
-inline bool step_needs_aux(const StepParams& p) {
-  return p.peers.n > 0 || p.peers.ng > 0 || p.sq_norm != nullptr || p.peers.mc_pdelta != 0 || p.peers.mc_gdelta != 0;
-}
-
-template <int OPT, int PDT, int ECC_BITS, int STATE, bool AUX>
-cudaError_t launch_step(const StepParams& p_in, const LaunchInfo& info, cudaStream_t s) {
-  constexpr bool aux = AUX;
-  if (step_needs_aux(p_in) != aux) return cudaErrorInvalidValue;
-  const bool switch_sum = p_in.peers.mc_gdelta != 0 && p_in.grad_dtype != FO_F32;
+template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
+cudaError_t launch_main(const HostStep& hs, bool& chained, cudaStream_t s) {
+  constexpr bool peer = MODE == kPeer;
+  const bool switch_sum = peer && hs.peers->mc_gdelta != 0 && hs.grad_dtype != FO_F32;
   const int ring_bytes = switch_sum ? kSwitchBatch * 16 * kThreads : 0;
-  auto kernel = step_kernel<OPT, PDT, ECC_BITS, STATE, AUX>;
+  auto kernel = step_kernel<OPT, PDT, ECC_BITS, STATE, MODE>;
   // Two caches, per instantiation of this function (one kernel each): the kernel's static shared memory
   // (the same on every device) and whether a device's copy of the function has been opted in above
   // 48 KB.  Atomics: concurrent first calls may both query and both set, which is harmless (same
@@ -1918,17 +2134,17 @@ cudaError_t launch_step(const StepParams& p_in, const LaunchInfo& info, cudaStre
   }
   // as many stages as fit beside the tables with min_blocks(OPT) blocks on an SM; when the peers'
   // gradient pieces make a stage too large for two of them, with one block on an SM
-  // (the plain kernel runs three stages, each with room for fp32 gradients: see hot_run)
-  const int per_stage = Stage<OPT, PDT, ECC_BITS, STATE>::bytes(aux ? p_in.grad_dtype : FO_F32, switch_sum ? 0 : p_in.peers.ng);
+  // (the kernels without peers run three stages, each with room for fp32 gradients: see hot_run)
+  const int per_stage = Stage<OPT, PDT, ECC_BITS, STATE>::bytes(peer ? hs.grad_dtype : FO_F32, (!peer || switch_sum) ? 0 : hs.peers->ng);
   int blocks_per_sm = min_blocks(OPT);
   int stages = (kSmemPerSm / blocks_per_sm - kSmemReservedPerBlock - static_smem - ring_bytes) / per_stage;
-  while (stages < (aux ? 2 : kPlainStages) && blocks_per_sm > 1) {
+  while (stages < (peer ? 2 : kPlainStages) && blocks_per_sm > 1) {
     --blocks_per_sm;
     stages = (kSmemPerSm / blocks_per_sm - kSmemReservedPerBlock - static_smem - ring_bytes) / per_stage;
   }
-  const int max_stages = !aux ? kPlainStages : ((p_in.peers.ng > 0 && !switch_sum) ? kMaxStagesPeers : kMaxStages);
+  const int max_stages = !peer ? kPlainStages : ((hs.peers->ng > 0 && !switch_sum) ? kMaxStagesPeers : kMaxStages);
   if (stages > max_stages) stages = max_stages;
-  if (stages < (aux ? 2 : kPlainStages)) return cudaErrorInvalidConfiguration;
+  if (stages < (peer ? 2 : kPlainStages)) return cudaErrorInvalidConfiguration;
   const int dynamic_smem = stages * per_stage + ring_bytes;
   static std::atomic<bool> opted_in[64];  // per device ordinal (zero-initialised)
   int dev = 0;
@@ -1941,10 +2157,28 @@ cudaError_t launch_step(const StepParams& p_in, const LaunchInfo& info, cudaStre
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 64) opted_in[dev].store(true, std::memory_order_release);
   }
-  StepParams p = p_in;
+  StepParams<MODE> p;  // filled as far as it is used
+  fill_common(p, hs);
   p.stages = stages;
-  unsigned int grid = (unsigned int)info.sm_count * blocks_per_sm;
-  if (grid > info.total_chunks) grid = info.total_chunks;
+  if constexpr (peer) p.peers = *hs.peers;
+  uint32_t total = 0;
+  int n = 0;
+  for (int i = 0; i < hs.n_leaves; ++i) {
+    const HostLeaf& l = hs.leaf[i];
+    const uint32_t chunks = l.hot ? (uint32_t)(l.src.n / kChunk) : 0u;
+    if (chunks == 0) continue;
+    p.t.leaf[n] = l.src;
+    p.t.hyper_of[n] = l.hyper;
+    p.t.first_block[n] = total;
+    if constexpr ((MODE & kOut) != 0) p.out[n] = l.out;
+    total += chunks;
+    ++n;
+  }
+  if (n == 0) return cudaSuccess;
+  p.n_leaves = n;
+  p.t.first_block[n] = total;
+  unsigned int grid = (unsigned int)(hs.sm_count * blocks_per_sm);
+  if (grid > total) grid = total;
   // Run length: at most FO_RUN_MAX chunks (filling and draining the copy pipeline at a run's ends costs
   // about one chunk's time, 0.5 % of such a run), and for small launches a quarter of a block's share,
   // rounded up, so that no block gets more than four runs.
@@ -1954,62 +2188,101 @@ cudaError_t launch_step(const StepParams& p_in, const LaunchInfo& info, cudaStre
 #ifndef FO_RUN_MAX
 #define FO_RUN_MAX 192u
 #endif
-  unsigned int run = (info.total_chunks + grid * FO_RUN_DIV - 1u) / (grid * FO_RUN_DIV);
-  // is there anything the straight-line loop leaves (a ragged end, a misaligned leaf, hyper-parameters
-  // outside the shortcuts' range)?  Device-resident scalars can move Adam's hyper-parameters out of that
-  // range at run time: then the tail kernel is launched to look for itself.
-  bool dynamic = false;
-  int tails = 0;  // leaves with work for the tail kernel
-  for (int l = 0; l < p.n_leaves; ++l) {
-    const DevHyper& h = p.hyper[p.hyper_of[l]];
-    bool ok = (h.flags & FO_FLAG_LP_DELTA) == 0 && p.aligned[l] != 0;
-    if (OPT == FO_OPT_ADAM) {
-      ok = ok && (h.flags & kFlagTameAdam) != 0;
-      dynamic = dynamic || h.dyn != nullptr;
-    }
-    if (!ok || p.leaf[l].n % (unsigned long long)kChunk != 0) ++tails;
-  }
-#ifdef FO_NAIVE_MATH
-  tails = p.n_leaves;
-#endif
-  const bool ragged = tails > 0;
-  // A launch of at most FO_RUN_WHOLE chunks per block with next to no tail work is dealt out as one run
-  // per block: it lasts tens of microseconds, a second fill and drain of the pipeline per block shows
-  // (4 M parameters: 31 -> 24 us), and an uneven count of short runs per block costs more than it
-  // spreads.  (With many ragged leaves in the table the short runs stay: they spread the tail kernel's
-  // work, which follows the same runs, over four times as many blocks.)
+  unsigned int run = (total + grid * FO_RUN_DIV - 1u) / (grid * FO_RUN_DIV);
+  // A launch of at most FO_RUN_WHOLE chunks per block is dealt out as one run per block: it lasts tens of
+  // microseconds, a second fill and drain of the pipeline per block shows (4 M parameters: 31 -> 24 us), and an
+  // uneven count of short runs per block costs more than it spreads.
 #ifndef FO_RUN_WHOLE
 #define FO_RUN_WHOLE 32u
 #endif
-  const unsigned int share = (info.total_chunks + grid - 1u) / grid;
-  if (share <= FO_RUN_WHOLE && tails <= 4) run = share;
+  const unsigned int share = (total + grid - 1u) / grid;
+  if (share <= FO_RUN_WHOLE) run = share;
   p.run_chunks = run < 1u ? 1u : (run > FO_RUN_MAX ? FO_RUN_MAX : run);
-  kernel<<<grid, kThreads, dynamic_smem, s>>>(p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const bool need_tails = ragged || dynamic;
-  if (need_tails) {
-    step_tail_kernel<OPT, PDT, ECC_BITS, STATE, AUX><<<grid, kThreads, 0, s>>>(p);
-    e = cudaGetLastError();
-  }
-  return e;
-}
-template <int OPT, int PDT, int ECC_BITS>
-cudaError_t launch_step_generic(const StepParams& p, const LaunchInfo& info, cudaStream_t s) {
-  step_kernel_generic<OPT, PDT, ECC_BITS><<<info.total_chunks, 256, 0, s>>>(p);
-  return cudaGetLastError();
+  return launch_chained(kernel, grid, kThreads, dynamic_smem, chained, s, p);
 }
 
+// The pieces that the whole chunks (of main_chunk elements; 0: step_kernel is not used) of the hot leaves leave over.
+template <int OPT, int PDT, int ECC_BITS, int STATE, int N>
+cudaError_t launch_piece_table(const HostStep& hs, const int* which, int n, unsigned int main_chunk, bool& chained, cudaStream_t s) {
+  PieceParams<N> p;  // filled as far as it is used
+  fill_common(p, hs);
+  p.peers = *hs.peers;
+  uint32_t total = 0;
+  for (int k = 0; k < n; ++k) {
+    const HostLeaf& l = hs.leaf[which[k]];
+    const unsigned long long done = l.hot && main_chunk != 0 ? l.src.n / main_chunk * main_chunk : 0ull;
+    p.leaf[k] = l.src;
+    p.out[k] = l.out;
+    p.hyper_of[k] = l.hyper;
+    p.hot[k] = l.hot;
+    p.start[k] = (uint32_t)(done / kPieceElems);
+    p.first_piece[k] = total;
+    total += (uint32_t)((l.src.n - done + kPieceElems - 1) / kPieceElems);
+  }
+  p.n_leaves = n;
+  p.first_piece[n] = total;
+  const unsigned int most = (unsigned int)hs.sm_count * 64u;  // a misaligned leaf can be large: blocks then take several pieces
+  return launch_chained(piece_kernel<OPT, PDT, ECC_BITS, STATE, N>, total < most ? total : most, kPieceThreads, 0, chained, s, p);
+}
+template <int OPT, int PDT, int ECC_BITS, int STATE>
+cudaError_t launch_pieces(const HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
+  int which[kPieceLeavesLarge];
+  int n = 0;
+  for (int i = 0; i <= hs.n_leaves; ++i) {
+    if (i < hs.n_leaves) {
+      const HostLeaf& l = hs.leaf[i];
+      if (l.src.n == 0 || (l.hot && main_chunk != 0 && l.src.n % main_chunk == 0)) continue;
+      which[n++] = i;
+    }
+    if (n == kPieceLeavesLarge || (i == hs.n_leaves && n > 0)) {
+      const cudaError_t e = n <= kPieceLeavesSmall ? launch_piece_table<OPT, PDT, ECC_BITS, STATE, kPieceLeavesSmall>(hs, which, n, main_chunk, chained, s)
+                                                   : launch_piece_table<OPT, PDT, ECC_BITS, STATE, kPieceLeavesLarge>(hs, which, n, main_chunk, chained, s);
+      if (e != cudaSuccess) return e;
+      n = 0;
+    }
+  }
+  return cudaSuccess;
+}
+template <int OPT, int PDT, int ECC_BITS>
+cudaError_t launch_generic(const HostStep& hs, bool& chained, cudaStream_t s) {
+  StepParams<kOut> p;
+  fill_common(p, hs);
+  const unsigned int tile = generic_tile_elems(hs.group_size);
+  uint32_t total = 0;
+  for (int i = 0; i < hs.n_leaves; ++i) {
+    p.t.leaf[i] = hs.leaf[i].src;
+    p.out[i] = hs.leaf[i].out;
+    p.t.hyper_of[i] = hs.leaf[i].hyper;
+    p.t.first_block[i] = total;
+    total += (uint32_t)((hs.leaf[i].src.n + tile - 1) / tile);
+  }
+  p.n_leaves = hs.n_leaves;
+  p.t.first_block[hs.n_leaves] = total;
+  return launch_chained(step_kernel_generic<OPT, PDT, ECC_BITS>, total, 256u, 0, chained, s, p);
+}
+
+}  // namespace FO_SHAPE_NS
+
 // lookups implemented by the instantiation units (fo_step_inst.cu, one per slice: optimizer x state
-// kind x with / without the peer and clipping code); each returns {nullptr, 0} for a (param dtype,
-// ecc width) pair that does not exist
-#define FO_DECLARE_LOOKUP(name) Launcher name(int pdt, int ecc_bits);
-#define FO_DECLARE_PAIR(stem) FO_DECLARE_LOOKUP(stem##_plain) FO_DECLARE_LOOKUP(stem##_aux)
-FO_DECLARE_PAIR(lookup_adam_quant) FO_DECLARE_PAIR(lookup_adam_full) FO_DECLARE_LOOKUP(lookup_adam_generic)
-FO_DECLARE_PAIR(lookup_lion_quant) FO_DECLARE_PAIR(lookup_lion_full) FO_DECLARE_LOOKUP(lookup_lion_generic)
-FO_DECLARE_PAIR(lookup_sgd_quant) FO_DECLARE_PAIR(lookup_sgd_full) FO_DECLARE_LOOKUP(lookup_sgd_generic)
-FO_DECLARE_PAIR(lookup_sgd_none)
-#undef FO_DECLARE_PAIR
-#undef FO_DECLARE_LOOKUP
+// kind x kernel); each returns null for a (param dtype, ecc width) pair that does not exist
+#define FO_DECLARE_SLICE(stem)                       \
+  Launcher stem##_plain(int pdt, int ecc_bits);      \
+  Launcher stem##_clip(int pdt, int ecc_bits);       \
+  Launcher stem##_out(int pdt, int ecc_bits);        \
+  Launcher stem##_all(int pdt, int ecc_bits);        \
+  Launcher stem##_peer(int pdt, int ecc_bits);       \
+  PieceFn stem##_piece(int pdt, int ecc_bits);
+FO_DECLARE_SLICE(lookup_adam_quant) FO_DECLARE_SLICE(lookup_adam_full)
+FO_DECLARE_SLICE(lookup_lion_quant) FO_DECLARE_SLICE(lookup_lion_full)
+FO_DECLARE_SLICE(lookup_sgd_quant) FO_DECLARE_SLICE(lookup_sgd_full) FO_DECLARE_SLICE(lookup_sgd_none)
+Launcher lookup_adam_quant_group(int pdt, int ecc_bits);
+Launcher lookup_lion_quant_group(int pdt, int ecc_bits);
+Launcher lookup_sgd_quant_group(int pdt, int ecc_bits);
+Launcher lookup_adam_quant_delta(int pdt, int ecc_bits);
+Launcher lookup_adam_full_delta(int pdt, int ecc_bits);
+Launcher lookup_adam_generic(int pdt, int ecc_bits);
+Launcher lookup_lion_generic(int pdt, int ecc_bits);
+Launcher lookup_sgd_generic(int pdt, int ecc_bits);
+#undef FO_DECLARE_SLICE
 
 }  // namespace fo

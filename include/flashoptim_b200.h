@@ -6,8 +6,8 @@
  * descriptors) are HOST memory and are copied into kernel parameters at launch.  The
  * library never allocates, frees or keeps caller memory, never synchronises the device
  * and launches only on the stream it is given, so a call can sit inside any framework's
- * stream order (XLA custom call, PyTorch, CUDA graph).  All updates are in place: the
- * reference's fused kernels alias every output onto its input
+ * stream order (XLA custom call, PyTorch, CUDA graph).  Updates are in place unless told
+ * otherwise: the reference's fused kernels alias every output onto its input
  * (flashoptim_jax/adamw.py:268,293; flashoptim_jax/momentum_kernel.py:222,246).
  *
  * All functions return FO_OK or an FO_ERR_* code; fo_status_string() names a code and
@@ -165,7 +165,24 @@ typedef struct FoStepDesc {
    * Both need the matching point-to-point table as well, which serves ragged ends and rare values. */
   int64_t mc_param_offset;
   int64_t mc_grad_offset;
+  /* Where the results go, one entry per leaf (host table); NULL: every array is updated in place.  With it the
+   * leaf's arrays are only read: a caller that keeps the old parameters and state needs no copy of them.
+   * Not together with peers. */
+  const struct FoLeafOut* outs;
+  uint32_t launch_flags; /* FO_LAUNCH_* */
+  uint32_t reserved3;
 } FoStepDesc;
+typedef struct FoLeafOut {
+  void* param;
+  void* ecc;
+  void* mu;
+  void* mu_scales;
+  void* nu;
+  void* nu_scales;
+} FoLeafOut;
+/* The launch in front of this one on the stream is another fo_step of the same pytree step (other leaves), or
+ * the fo_sq_norm* call that forms its grad_sq_norm: the kernels may start before that launch has drained. */
+#define FO_LAUNCH_CHAINED 1u
 #define FO_MAX_PEERS 7
 
 /* Replaces pl.pallas_call(...) of _fused_flash_adamw_leaf_impl (adamw.py:225-353) and of

@@ -1,0 +1,125 @@
+"""The routes a call can take through the step kernels, bit for bit against the CPU oracle: whole chunks through
+step_kernel (problems above 148 * 8192 elements) with the rest in pieces of 1024, small problems in pieces alone; groups of
+8 to 256, parameters handed back as old + lp(new - old), results written elsewhere, clipping, and combinations."""
+
+import ctypes
+
+import ml_dtypes
+import numpy as np
+import pytest
+
+from oracle import c_oracle as C
+from oracle import flashoptim_oracle as O
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+MAIN = 148 * 8192 + 5 * 6144  # above the limit for every chunk size (2048, 4096, 6144)
+G_NP = {0: np.float32, 1: ml_dtypes.bfloat16, 2: np.float16}
+
+
+def _step(opt, grads, leaves, outs, state, group, hp, pdt, gdt, ecc_bits, sq=None, max_norm=0.0):
+    from flashoptim_jax_b200 import _lib
+
+    L = (_lib.FoLeaf * len(leaves))()
+    X = (_lib.FoLeafOut * len(leaves))()
+    for i, (g, lf) in enumerate(zip(grads, leaves)):
+        L[i].grad, L[i].n, L[i].hyper = g.data_ptr(), lf.param.numel(), 0
+        for name in lf.fields():
+            t = getattr(lf, name)
+            setattr(L[i], name, None if t is None else t.data_ptr())
+            if outs is not None and t is not None:
+                setattr(X[i], name, getattr(outs[i], name).data_ptr())
+    hy = _lib.FoHyper()
+    for k, name in enumerate(("lr", "wd", "b1", "b2", "one_minus_b1", "one_minus_b2", "eps", "bc1", "bc2")):
+        setattr(hy, name, float(hp[k]))
+    hy.flags = int(hp[9])
+    d = _lib.FoStepDesc(struct_size=ctypes.sizeof(_lib.FoStepDesc), opt=opt, param_dtype=pdt, grad_dtype=gdt, ecc_bits=ecc_bits,
+                        state=state, group_size=group, n_leaves=len(leaves), n_hypers=1, leaves=ctypes.cast(L, ctypes.c_void_p),
+                        hypers=ctypes.cast(ctypes.pointer(hy), ctypes.c_void_p))
+    if outs is not None:
+        d.outs = ctypes.cast(X, ctypes.c_void_p)
+    if sq is not None:
+        d.grad_sq_norm, d.max_grad_norm = sq.data_ptr(), max_norm
+    _lib.check(_lib.lib().fo_step(ctypes.byref(d), 0))
+
+
+def _run(opt, pdt, ecc_bits, state, group, conv, sizes, *, gdt=1, elsewhere=False, max_norm=None, offset=0, steps=3):
+    import torch
+
+    from flashoptim_jax_b200 import _engine as eng
+
+    rng = np.random.default_rng(sum(sizes) + group)
+    refs = [H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), opt, state, ecc_bits, group) for n in sizes]
+    for r in refs:
+        r.param[: r.param.size // 50] = 0  # values outside the shortcuts' ranges
+    devs = [r.copy().to_device() for r in refs]
+    if offset:  # a leaf that does not start on a 16-byte boundary
+        for d in devs:
+            d.param = torch.cat([d.param[:offset], d.param])[offset:]
+    for t in range(1, steps + 1):
+        grads = [H.make_grad(rng, n, 1e-2, G_NP[gdt], outliers=1e-3) for n in sizes]
+        for g in grads:
+            g[: g.size // 3: 7] = 0
+        hp = H.hyper_tuple(opt, conv, t, lr=1e-3, wd=1e-2)
+        dev_g = [H.to_torch(g) for g in grads]
+        sq = None
+        if max_norm is not None:
+            sq = eng.sq_norm_of(dev_g)
+            grads = O.clip_by_global_norm(grads, max_norm, sq_norm=float(sq.cpu()))
+        for g, r in zip(grads, refs):
+            H.oracle_step(opt, g, r, state, group, hp)
+        old = [H.LeafArrays(*[None if getattr(d, f) is None else getattr(d, f).clone() for f in d.fields()]) for d in devs] if elsewhere else None
+        outs = [H.LeafArrays(*[None if getattr(d, f) is None else torch.empty_like(getattr(d, f)) for f in d.fields()]) for d in devs] if elsewhere else None
+        _step(opt, dev_g, devs, outs, state, group, hp, pdt, gdt, ecc_bits, sq, max_norm or 0.0)
+        torch.cuda.synchronize()
+        if elsewhere:
+            for a, b in zip(devs, old):  # the inputs are left alone
+                H.assert_leaf_equal(a.to_host(), b.to_host(), f"inputs of step {t}")
+            devs = outs
+        for i, (d, r) in enumerate(zip(devs, refs)):
+            H.assert_leaf_equal(d.to_host(), r, f"step {t} leaf {i} n={sizes[i]}")
+
+
+@pytest.mark.parametrize("n", [MAIN, MAIN + 1, MAIN + 1023 * 3 + 5])
+@pytest.mark.parametrize("opt,pdt,ecc_bits,state", [(C.ADAM, 1, 16, C.STATE_QUANT), (C.ADAM, 2, 8, C.STATE_QUANT), (C.ADAM, 0, 0, C.STATE_QUANT),
+                                                    (C.ADAM, 1, 8, C.STATE_FULL), (C.LION, 1, 8, C.STATE_QUANT), (C.LION, 2, 16, C.STATE_FULL),
+                                                    (C.SGD, 1, 16, C.STATE_QUANT), (C.SGD, 0, 0, C.STATE_FULL), (C.SGD, 2, 8, C.STATE_NONE)])
+def test_whole_chunks_and_their_rest(opt, pdt, ecc_bits, state, n):
+    _run(opt, pdt, ecc_bits, state, 32, O.FUSED, [n, 77], steps=2)
+
+
+@pytest.mark.parametrize("group", [8, 16, 64, 128, 256])
+@pytest.mark.parametrize("opt,pdt,ecc_bits", [(C.ADAM, 1, 16), (C.LION, 2, 8), (C.SGD, 0, 0)])
+def test_group_sizes(opt, pdt, ecc_bits, group):
+    _run(opt, pdt, ecc_bits, C.STATE_QUANT, group, O.FUSED, [MAIN + group + 3], gdt=0, steps=2)
+    _run(opt, pdt, ecc_bits, C.STATE_QUANT, group, O.FUSED, [1, 7, group, group + 1, 1023, 1024, 1025, 5 * 1024 - group - 1])
+
+
+@pytest.mark.parametrize("pdt,ecc_bits,state", [(1, 8, C.STATE_QUANT), (1, 16, C.STATE_FULL), (2, 0, C.STATE_QUANT), (0, 0, C.STATE_QUANT)])
+def test_parameter_handed_back_as_a_delta(pdt, ecc_bits, state):
+    _run(C.ADAM, pdt, ecc_bits, state, 32, O.UNFUSED, [MAIN + 1029], steps=2)
+    _run(C.ADAM, pdt, ecc_bits, state, 32, O.UNFUSED, [3, 1024, 2047])
+
+
+@pytest.mark.parametrize("opt,pdt,ecc_bits,state,group,conv", [
+    (C.ADAM, 1, 8, C.STATE_QUANT, 32, O.FUSED), (C.ADAM, 1, 16, C.STATE_QUANT, 64, O.UNFUSED), (C.ADAM, 0, 0, C.STATE_FULL, 32, O.FUSED),
+    (C.LION, 2, 16, C.STATE_QUANT, 32, O.FUSED), (C.SGD, 1, 0, C.STATE_NONE, 32, O.FUSED), (C.SGD, 1, 8, C.STATE_QUANT, 40, O.FUSED)])
+def test_results_elsewhere(opt, pdt, ecc_bits, state, group, conv):
+    _run(opt, pdt, ecc_bits, state, group, conv, [MAIN + 517, 33], elsewhere=True, steps=2)
+    _run(opt, pdt, ecc_bits, state, group, conv, [1, 1000, 4096], elsewhere=True)
+    _run(opt, pdt, ecc_bits, state, group, conv, [1500], elsewhere=True, offset=1)  # scalar path
+
+
+@pytest.mark.parametrize("gdt", [0, 1, 2])
+@pytest.mark.parametrize("max_norm", [0.5, 1e6])
+def test_clipping_on_whole_chunks(gdt, max_norm):
+    _run(C.ADAM, 1, 16, C.STATE_QUANT, 32, O.FUSED, [MAIN + 100, 2048], gdt=gdt, max_norm=max_norm, steps=2)
+    _run(C.LION, 1, 8, C.STATE_QUANT, 64, O.FUSED, [MAIN], gdt=gdt, max_norm=max_norm, elsewhere=True, steps=2)
+
+
+def test_many_leaves_need_several_tables():
+    rng = np.random.default_rng(3)
+    sizes = [int(x) for x in rng.integers(1, 9000, 500)]
+    _run(C.ADAM, 1, 8, C.STATE_QUANT, 32, O.FUSED, sizes, steps=2)
+    _run(C.ADAM, 1, 8, C.STATE_QUANT, 64, O.FUSED, sizes, steps=1, elsewhere=True)
