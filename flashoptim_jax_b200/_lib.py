@@ -26,7 +26,7 @@ FO_SELFTEST_SQRT, FO_SELFTEST_SOFTSIGN, FO_SELFTEST_RECONSTRUCT, FO_SELFTEST_SPL
 FO_SELFTEST_GROUP_DIV, FO_SELFTEST_CODE_TABLES, FO_SELFTEST_RCP, FO_SELFTEST_PACKED = 4, 5, 6, 7
 
 EXPORTS = (
-    "fo_step", "fo_quantize_momentum", "fo_dequantize_momentum", "fo_quantize_variance",
+    "fo_step", "fo_step_ex", "fo_quantize_momentum", "fo_dequantize_momentum", "fo_quantize_variance",
     "fo_dequantize_variance", "fo_split", "fo_reconstruct", "fo_selftest", "fo_selftest_static", "fo_version",
     "fo_status_string", "fo_last_error", "fo_sq_norm", "fo_mean_sq_norm", "fo_step_scalars", "fo_step_scalars_schedule",
 )
@@ -69,8 +69,11 @@ class FoStepDesc(ctypes.Structure):
         ("peer_grad_offsets", ctypes.c_void_p),
         ("grad_sq_norm", ctypes.c_void_p), ("max_grad_norm", ctypes.c_float), ("reserved2", ctypes.c_uint32),
         ("mc_param_offset", ctypes.c_int64), ("mc_grad_offset", ctypes.c_int64),
-        ("outs", ctypes.c_void_p), ("launch_flags", ctypes.c_uint32), ("reserved3", ctypes.c_uint32),
     ]
+
+
+class FoStepMore(ctypes.Structure):
+    _fields_ = [("struct_size", ctypes.c_uint32), ("launch_flags", ctypes.c_uint32), ("outs", ctypes.c_void_p)]
 
 
 class FoArray(ctypes.Structure):
@@ -101,6 +104,8 @@ def lib() -> ctypes.CDLL:
     vp, u64, i32 = ctypes.c_void_p, ctypes.c_uint64, ctypes.c_int32
     cdll.fo_step.restype = ctypes.c_int
     cdll.fo_step.argtypes = [ctypes.POINTER(FoStepDesc), vp]
+    cdll.fo_step_ex.restype = ctypes.c_int
+    cdll.fo_step_ex.argtypes = [ctypes.POINTER(FoStepDesc), ctypes.POINTER(FoStepMore), vp]
     for name in ("fo_quantize_momentum", "fo_quantize_variance"):
         fn = getattr(cdll, name)
         fn.restype = ctypes.c_int

@@ -105,10 +105,15 @@ static int sm_count_of_current_device() {
 
 using namespace fo;
 
-extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
+extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) { return fo_step_ex(d, nullptr, cuda_stream); }
+
+extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cuda_stream) {
   if (d == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: null descriptor");
   if (d->struct_size != sizeof(FoStepDesc))
     return fail(FO_ERR_INVALID_ARG, "fo_step: struct_size %u != %zu (ABI mismatch)", d->struct_size, sizeof(FoStepDesc));
+  if (more != nullptr && more->struct_size != sizeof(FoStepMore))
+    return fail(FO_ERR_INVALID_ARG, "fo_step_ex: struct_size %u != %zu (ABI mismatch)", more->struct_size, sizeof(FoStepMore));
+  const FoLeafOut* const outs = more != nullptr ? more->outs : nullptr;
   if (d->opt < FO_OPT_ADAM || d->opt > FO_OPT_SGD) return fail(FO_ERR_INVALID_ARG, "fo_step: bad opt %d", d->opt);
   if (d->param_dtype < FO_F32 || d->param_dtype > FO_F16) return fail(FO_ERR_INVALID_ARG, "fo_step: bad param_dtype %d", d->param_dtype);
   if (d->grad_dtype < FO_F32 || d->grad_dtype > FO_F16) return fail(FO_ERR_INVALID_ARG, "fo_step: bad grad_dtype %d", d->grad_dtype);
@@ -148,8 +153,8 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
     if (need_nu && L.nu == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null nu", i);
     if (need_scales && L.mu_scales == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null mu_scales", i);
     if (need_scales && need_nu && L.nu_scales == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null nu_scales", i);
-    if (d->outs != nullptr) {
-      const FoLeafOut& O = d->outs[i];
+    if (outs != nullptr) {
+      const FoLeafOut& O = outs[i];
       if (O.param == nullptr || (d->ecc_bits != 0 && O.ecc == nullptr) || (need_mu && O.mu == nullptr) || (need_nu && O.nu == nullptr) ||
           (need_scales && O.mu_scales == nullptr) || (need_scales && need_nu && O.nu_scales == nullptr))
         return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: null output", i);
@@ -157,7 +162,7 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
     if (L.hyper >= d->n_hypers) return fail(FO_ERR_INVALID_ARG, "fo_step: leaf %u: hyper index %u out of range", i, L.hyper);
   }
 
-  if (d->outs != nullptr && d->n_peers > 0) return fail(FO_ERR_UNSUPPORTED, "fo_step: peers and separate outputs");
+  if (outs != nullptr && d->n_peers > 0) return fail(FO_ERR_UNSUPPORTED, "fo_step: peers and separate outputs");
 
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   DevHyper hyper[FO_MAX_HYPERS];
@@ -189,7 +194,7 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
     peers.mc_gdelta = (long long)d->mc_grad_offset;
   }
   const bool with_peers = peers.n > 0 || peers.ng > 0;
-  const int features = (d->grad_sq_norm != nullptr ? kClip : 0) | (d->outs != nullptr ? kOut : 0) |
+  const int features = (d->grad_sq_norm != nullptr ? kClip : 0) | (outs != nullptr ? kOut : 0) |
                        (d->state == FO_STATE_QUANT && d->group_size != 32 ? kGroup : 0) | (lp_delta ? kDelta : 0);
   const int mode = with_peers ? kPeer : features;
   const Launcher launcher = find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, mode);
@@ -205,7 +210,7 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
   if (hs.sm_count <= 0) return fail(FO_ERR_CUDA, "fo_step: cannot query the current device");
   hs.sq_norm = d->grad_sq_norm; hs.max_norm = d->max_grad_norm;
   hs.peers = &peers;
-  bool chained = (d->launch_flags & FO_LAUNCH_CHAINED) != 0;
+  bool chained = more != nullptr && (more->launch_flags & FO_LAUNCH_CHAINED) != 0;
   const int most_leaves = (mode == kPlain || mode == kPeer) && !generic ? kMaxLeaves : kMaxLeavesFlex;
   const unsigned long long unit = generic ? generic_tile_elems(d->group_size) : kPieceElems;
   const unsigned long long kMaxBlocks = 0x7FFFFFFFull;
@@ -240,8 +245,8 @@ extern "C" int fo_step(const FoStepDesc* d, void* cuda_stream) {
     const FoLeaf& L = d->leaves[i];
     DevOut out = {};
     bool aligned = aligned16(L.grad) && aligned16(L.param) && aligned16(L.ecc) && aligned16(L.mu) && aligned16(L.nu);
-    if (d->outs != nullptr && L.n != 0) {
-      const FoLeafOut& O = d->outs[i];
+    if (outs != nullptr && L.n != 0) {
+      const FoLeafOut& O = outs[i];
       out.param = distance(O.param, L.param);
       out.ecc = distance(O.ecc, L.ecc);
       out.mu = distance(O.mu, L.mu);

@@ -165,13 +165,14 @@ typedef struct FoStepDesc {
    * Both need the matching point-to-point table as well, which serves ragged ends and rare values. */
   int64_t mc_param_offset;
   int64_t mc_grad_offset;
-  /* Where the results go, one entry per leaf (host table); NULL: every array is updated in place.  With it the
-   * leaf's arrays are only read: a caller that keeps the old parameters and state needs no copy of them.
-   * Not together with peers. */
-  const struct FoLeafOut* outs;
-  uint32_t launch_flags; /* FO_LAUNCH_* */
-  uint32_t reserved3;
 } FoStepDesc;
+#define FO_MAX_PEERS 7
+
+/* Replaces pl.pallas_call(...) of _fused_flash_adamw_leaf_impl (adamw.py:225-353) and of
+ * fused_momentum_leaf_impl (momentum_kernel.py:183-302), for a whole pytree at once. */
+int fo_step(const FoStepDesc* desc, void* cuda_stream);
+
+/* fo_step with what its descriptor has no room for (more == NULL: the same call). */
 typedef struct FoLeafOut {
   void* param;
   void* ecc;
@@ -180,14 +181,18 @@ typedef struct FoLeafOut {
   void* nu;
   void* nu_scales;
 } FoLeafOut;
-/* The launch in front of this one on the stream is another fo_step of the same pytree step (other leaves), or
+typedef struct FoStepMore {
+  uint32_t struct_size;  /* sizeof(FoStepMore) */
+  uint32_t launch_flags; /* FO_LAUNCH_* */
+  /* Where the results go, one entry per leaf (host table); NULL: every array is updated in place.  With it the
+   * leaf's arrays are only read: a caller that keeps the old parameters and state needs no copy of them.
+   * Not together with peers. */
+  const FoLeafOut* outs;
+} FoStepMore;
+/* The launch in front of this one on the stream is another fo_step* of the same pytree step (other leaves), or
  * the fo_sq_norm* call that forms its grad_sq_norm: the kernels may start before that launch has drained. */
 #define FO_LAUNCH_CHAINED 1u
-#define FO_MAX_PEERS 7
-
-/* Replaces pl.pallas_call(...) of _fused_flash_adamw_leaf_impl (adamw.py:225-353) and of
- * fused_momentum_leaf_impl (momentum_kernel.py:183-302), for a whole pytree at once. */
-int fo_step(const FoStepDesc* desc, void* cuda_stream);
+int fo_step_ex(const FoStepDesc* desc, const FoStepMore* more, void* cuda_stream);
 
 /* Per-step scalars formed on the device, so that a whole step can be captured in a CUDA graph
  * with no host scalar in it (the reference forms them as traced values inside its jitted step:

@@ -37,11 +37,10 @@ def _step(opt, grads, leaves, outs, state, group, hp, pdt, gdt, ecc_bits, sq=Non
     d = _lib.FoStepDesc(struct_size=ctypes.sizeof(_lib.FoStepDesc), opt=opt, param_dtype=pdt, grad_dtype=gdt, ecc_bits=ecc_bits,
                         state=state, group_size=group, n_leaves=len(leaves), n_hypers=1, leaves=ctypes.cast(L, ctypes.c_void_p),
                         hypers=ctypes.cast(ctypes.pointer(hy), ctypes.c_void_p))
-    if outs is not None:
-        d.outs = ctypes.cast(X, ctypes.c_void_p)
+    more = _lib.FoStepMore(struct_size=ctypes.sizeof(_lib.FoStepMore), outs=None if outs is None else ctypes.cast(X, ctypes.c_void_p))
     if sq is not None:
         d.grad_sq_norm, d.max_grad_norm = sq.data_ptr(), max_norm
-    _lib.check(_lib.lib().fo_step(ctypes.byref(d), 0))
+    _lib.check(_lib.lib().fo_step_ex(ctypes.byref(d), ctypes.byref(more), 0))
 
 
 def _run(opt, pdt, ecc_bits, state, group, conv, sizes, *, gdt=1, elsewhere=False, max_norm=None, offset=0, steps=3):
