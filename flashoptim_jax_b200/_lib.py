@@ -27,8 +27,8 @@ FO_SELFTEST_GROUP_DIV, FO_SELFTEST_CODE_TABLES, FO_SELFTEST_RCP, FO_SELFTEST_PAC
 
 EXPORTS = (
     "fo_step", "fo_step_ex", "fo_quantize_momentum", "fo_dequantize_momentum", "fo_quantize_variance",
-    "fo_dequantize_variance", "fo_split", "fo_reconstruct", "fo_selftest", "fo_selftest_static", "fo_version",
-    "fo_status_string", "fo_last_error", "fo_sq_norm", "fo_mean_sq_norm", "fo_step_scalars", "fo_step_scalars_schedule",
+    "fo_dequantize_variance", "fo_split", "fo_reconstruct", "fo_split_many", "fo_reconstruct_many", "fo_selftest", "fo_selftest_static", "fo_version",
+    "fo_status_string", "fo_last_error", "fo_sq_norm", "fo_sq_norm_mixed", "fo_mean_sq_norm", "fo_step_scalars", "fo_step_scalars_schedule",
 )
 FO_SQ_NORM_WORKSPACE_BYTES = 16384
 
@@ -76,6 +76,10 @@ class FoStepMore(ctypes.Structure):
     _fields_ = [("struct_size", ctypes.c_uint32), ("launch_flags", ctypes.c_uint32), ("outs", ctypes.c_void_p)]
 
 
+class FoSplitLeaf(ctypes.Structure):
+    _fields_ = [("theta", ctypes.c_void_p), ("lp", ctypes.c_void_p), ("ecc", ctypes.c_void_p), ("n", ctypes.c_uint64)]
+
+
 class FoArray(ctypes.Structure):
     _fields_ = [("data", ctypes.c_void_p), ("n", ctypes.c_uint64)]
 
@@ -118,12 +122,18 @@ def lib() -> ctypes.CDLL:
         fn = getattr(cdll, name)
         fn.restype = ctypes.c_int
         fn.argtypes = [vp, vp, vp, i32, i32, u64, vp]
+    for name in ("fo_split_many", "fo_reconstruct_many"):
+        fn = getattr(cdll, name)
+        fn.restype = ctypes.c_int
+        fn.argtypes = [ctypes.POINTER(FoSplitLeaf), ctypes.c_uint32, i32, i32, vp]
     cdll.fo_selftest.restype = ctypes.c_int
     cdll.fo_selftest.argtypes = [i32, ctypes.c_int64, ctypes.POINTER(ctypes.c_uint64), vp]
     cdll.fo_selftest_static.restype = ctypes.c_int
     cdll.fo_selftest_static.argtypes = [i32, ctypes.c_int64, ctypes.POINTER(ctypes.c_uint64), ctypes.c_uint32, vp]
     cdll.fo_sq_norm.restype = ctypes.c_int
     cdll.fo_sq_norm.argtypes = [ctypes.POINTER(FoArray), ctypes.c_uint32, i32, i32, vp, vp, vp]
+    cdll.fo_sq_norm_mixed.restype = ctypes.c_int
+    cdll.fo_sq_norm_mixed.argtypes = [ctypes.POINTER(FoArray), ctypes.POINTER(i32), ctypes.c_uint32, i32, vp, vp, vp]
     cdll.fo_mean_sq_norm.restype = ctypes.c_int
     cdll.fo_mean_sq_norm.argtypes = [vp, vp, ctypes.c_uint64, i32, vp, ctypes.c_uint32, i32, vp, vp, vp]
     cdll.fo_step_scalars.restype = ctypes.c_int
@@ -138,6 +148,28 @@ def lib() -> ctypes.CDLL:
     cdll.fo_last_error.argtypes = []
     _lib = cdll
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The host extension (csrc/fo_host.cc), bound to the library of lib(); raises loudly when it is absent."""
+    global _host
+    if _host is None:
+        l = lib()
+        try:
+            from . import _fo_host
+        except ImportError as e:
+            raise NativeLibraryError(
+                f"cannot load flashoptim_jax_b200._fo_host: {e}; build it with `python -m flashoptim_jax_b200.build`") from e
+        from .quantization import QuantizedArray
+
+        names = ("fo_step_ex", "fo_sq_norm_mixed", "fo_split_many", "fo_reconstruct_many", "fo_quantize_momentum", "fo_quantize_variance",
+                 "fo_dequantize_momentum", "fo_dequantize_variance", "fo_status_string", "fo_last_error")
+        _fo_host.bind({name: ctypes.cast(getattr(l, name), ctypes.c_void_p).value for name in names}, QuantizedArray)
+        _host = _fo_host
+    return _host
 
 
 def check(status: int) -> None:

@@ -7,7 +7,7 @@
 namespace fo {
 int fail(int code, const char* fmt, ...);
 
-constexpr int kNormMaxArrays = 160;   // per launch (kernel-parameter table)
+constexpr int kNormMaxArrays = 320;   // per launch (kernel-parameter table)
 constexpr int kNormBlocksPerSm = 8;
 constexpr int kNormMaxBlocks = 2048;  // doubles in the workspace
 
@@ -16,8 +16,8 @@ struct NormParams {
   unsigned long long n[kNormMaxArrays];
   uint32_t first_chunk[kNormMaxArrays + 1];
   uint8_t aligned[kNormMaxArrays];
+  uint8_t dtype[kNormMaxArrays];
   int32_t n_arrays;
-  int32_t dtype;
 };
 
 FO_DEVI float sq_run(const uint4& w0, const uint4& w1, int dt) {
@@ -36,38 +36,43 @@ constexpr unsigned long long kNormChunk = (unsigned long long)kChunk * kNormPiec
 
 __global__ void __launch_bounds__(kThreads) sq_norm_partial(const __grid_constant__ NormParams p, double* partials) {
   __shared__ double warp_sums[kThreads / 32];
+  chain_release();
   double acc = 0.0;
   const uint32_t total = p.first_chunk[p.n_arrays];
-  int a = 0;
   for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
-    while (c >= p.first_chunk[a + 1]) ++a;
+    const int a = leaf_of(p.first_chunk, p.n_arrays, c);
     const unsigned long long base = (unsigned long long)(c - p.first_chunk[a]) * kNormChunk + (unsigned long long)threadIdx.x * kPiece;
     const unsigned long long n = p.n[a];
-    if (p.aligned[a] && base + (kNormPieces - 1) * (unsigned long long)kChunk + kPiece <= n) {
+    const int dt = p.dtype[a];
+    const void* data = p.data[a];
+    if (p.aligned[a]) {
       uint4 w0[kNormPieces], w1[kNormPieces];
 #pragma unroll
       for (int k = 0; k < kNormPieces; ++k) {
         const unsigned long long i0 = base + (unsigned long long)k * kChunk;
-        w1[k] = make_uint4(0u, 0u, 0u, 0u);
-        if (p.dtype == FO_F32) {
-          w0[k] = __ldcs((const uint4*)((const float*)p.data[a] + i0));
-          w1[k] = __ldcs((const uint4*)((const float*)p.data[a] + i0) + 1);
+        w0[k] = w1[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (i0 + kPiece > n) continue;  // the array's ragged end: below
+        if (dt == FO_F32) {
+          w0[k] = __ldcs((const uint4*)((const float*)data + i0));
+          w1[k] = __ldcs((const uint4*)((const float*)data + i0) + 1);
         } else {
-          w0[k] = __ldcs((const uint4*)((const unsigned short*)p.data[a] + i0));
+          w0[k] = __ldcs((const uint4*)((const unsigned short*)data + i0));
         }
       }
 #pragma unroll
-      for (int k = 0; k < kNormPieces; ++k) acc += (double)sq_run(w0[k], w1[k], p.dtype);
-    } else {
-      for (int k = 0; k < kNormPieces; ++k) {
-        const unsigned long long i0 = base + (unsigned long long)k * kChunk;
-        float s = 0.0f;
-        for (int j = 0; j < kPiece && i0 + j < n; ++j) {
-          const float g = load_grad(p.data[a], p.dtype, i0 + j);
-          s = __fmaf_rn(g, g, s);
-        }
-        acc += (double)s;
+      for (int k = 0; k < kNormPieces; ++k) acc += (double)sq_run(w0[k], w1[k], dt);
+    }
+#pragma unroll 1
+    for (int k = 0; k < kNormPieces; ++k) {
+      const unsigned long long i0 = base + (unsigned long long)k * kChunk;
+      if (i0 >= n || (p.aligned[a] && i0 + kPiece <= n)) continue;
+      float s = 0.0f;
+#pragma unroll
+      for (int j = 0; j < kPiece; ++j) {
+        const float g = i0 + j < n ? load_grad(data, dt, i0 + j) : 0.0f;
+        s = __fmaf_rn(g, g, s);
       }
+      acc += (double)s;
     }
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
@@ -145,6 +150,8 @@ __global__ void __launch_bounds__(kThreads) mean_sq_norm_partial(const __grid_co
 constexpr int kFinalThreads = 256;
 __global__ void __launch_bounds__(kFinalThreads) sq_norm_final(const double* partials, int n, double* out, int accumulate) {
   __shared__ double warp_sums[kFinalThreads / 32];
+  chain_release();
+  chain_wait();  // launched behind the blocks' sums
   double s = 0.0;
 #pragma unroll
   for (int k = 0; k < kNormMaxBlocks / kFinalThreads; ++k) {
@@ -196,20 +203,16 @@ __global__ void step_scalars_schedule_kernel(const int32_t* count, int32_t sched
 
 using namespace fo;
 
-extern "C" int fo_sq_norm(const FoArray* arrays, uint32_t n_arrays, int32_t dtype, int32_t accumulate, double* out,
-                          void* workspace, void* cuda_stream) {
+static int sq_norm_entry(const char* who, const FoArray* arrays, const int32_t* dtypes, int32_t dtype, uint32_t n_arrays, int32_t accumulate, double* out,
+                         void* workspace, cudaStream_t stream) {
   static_assert(kNormMaxBlocks * sizeof(double) <= FO_SQ_NORM_WORKSPACE_BYTES, "workspace too small");
-  if (out == nullptr || workspace == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_sq_norm: null out / workspace");
-  if (dtype < FO_F32 || dtype > FO_F16) return fail(FO_ERR_INVALID_ARG, "fo_sq_norm: bad dtype %d", dtype);
-  if (n_arrays > 0 && arrays == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_sq_norm: null table");
-  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  if (out == nullptr || workspace == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: null out / workspace", who);
+  if (n_arrays > 0 && arrays == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: null table", who);
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return fail(FO_ERR_CUDA, "fo_sq_norm: cannot query the current device");
+    return fail(FO_ERR_CUDA, "%s: cannot query the current device", who);
   double* partials = static_cast<double*>(workspace);
-  NormParams p;
-  memset(&p, 0, sizeof(p));
-  p.dtype = dtype;
+  NormParams p;  // filled as far as it is used
   int count = 0;
   unsigned long long chunks = 0;
   bool launched = false;
@@ -221,20 +224,22 @@ extern "C" int fo_sq_norm(const FoArray* arrays, uint32_t n_arrays, int32_t dtyp
     unsigned int grid = (unsigned int)(sms * kNormBlocksPerSm);
     if (grid > kNormMaxBlocks) grid = kNormMaxBlocks;
     if (grid > chunks) grid = (unsigned int)chunks;
-    if (grid > 0) sq_norm_partial<<<grid, kThreads, 0, stream>>>(p, partials);
-    sq_norm_final<<<1, kFinalThreads, 0, stream>>>(partials, (int)grid, out, launched ? 1 : accumulate);
+    bool chained = false;
+    cudaError_t e = grid > 0 ? launch_chained(sq_norm_partial, grid, kThreads, 0, chained, stream, p, partials) : cudaSuccess;
+    if (e == cudaSuccess) e = launch_chained(sq_norm_final, 1u, (unsigned int)kFinalThreads, 0, chained, stream, (const double*)partials, (int)grid, out, launched ? 1 : (int)accumulate);
     launched = true;
     count = 0;
     chunks = 0;
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(FO_ERR_CUDA, "fo_sq_norm: launch failed: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return fail(FO_ERR_CUDA, "%s: launch failed: %s", who, cudaGetErrorString(e));
     return FO_OK;
   };
   for (uint32_t i = 0; i < n_arrays; ++i) {
+    const int32_t dt = dtypes != nullptr ? dtypes[i] : dtype;
+    if (dt < FO_F32 || dt > FO_F16) return fail(FO_ERR_INVALID_ARG, "%s: bad dtype %d", who, dt);
     if (arrays[i].n == 0) continue;
-    if (arrays[i].data == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_sq_norm: array %u: null data", i);
+    if (arrays[i].data == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: array %u: null data", who, i);
     const unsigned long long nc = (arrays[i].n + kNormChunk - 1) / kNormChunk;
-    if (nc > 0x7FFFFFFFull) return fail(FO_ERR_TOO_LARGE, "fo_sq_norm: array %u with %llu elements exceeds one launch", i, (unsigned long long)arrays[i].n);
+    if (nc > 0x7FFFFFFFull) return fail(FO_ERR_TOO_LARGE, "%s: array %u with %llu elements exceeds one launch", who, i, (unsigned long long)arrays[i].n);
     if (count == kNormMaxArrays || chunks + nc > 0x7FFFFFFFull) {
       int rc = flush();
       if (rc != FO_OK) return rc;
@@ -243,10 +248,22 @@ extern "C" int fo_sq_norm(const FoArray* arrays, uint32_t n_arrays, int32_t dtyp
     p.n[count] = arrays[i].n;
     p.first_chunk[count] = (uint32_t)chunks;
     p.aligned[count] = ((uintptr_t)arrays[i].data & 15u) == 0;
+    p.dtype[count] = (uint8_t)dt;
     chunks += nc;
     ++count;
   }
   return flush();
+}
+
+extern "C" int fo_sq_norm(const FoArray* arrays, uint32_t n_arrays, int32_t dtype, int32_t accumulate, double* out,
+                          void* workspace, void* cuda_stream) {
+  if (dtype < FO_F32 || dtype > FO_F16) return fail(FO_ERR_INVALID_ARG, "fo_sq_norm: bad dtype %d", dtype);
+  return sq_norm_entry("fo_sq_norm", arrays, nullptr, dtype, n_arrays, accumulate, out, workspace, static_cast<cudaStream_t>(cuda_stream));
+}
+extern "C" int fo_sq_norm_mixed(const FoArray* arrays, const int32_t* dtypes, uint32_t n_arrays, int32_t accumulate, double* out,
+                                void* workspace, void* cuda_stream) {
+  if (n_arrays > 0 && dtypes == nullptr) return fail(FO_ERR_INVALID_ARG, "fo_sq_norm_mixed: null table");
+  return sq_norm_entry("fo_sq_norm_mixed", arrays, dtypes, FO_F32, n_arrays, accumulate, out, workspace, static_cast<cudaStream_t>(cuda_stream));
 }
 
 extern "C" int fo_mean_sq_norm(const void* grad, void* mean_out, uint64_t n, int32_t dtype, const int64_t* peer_grad_offsets,

@@ -153,6 +153,7 @@ struct StepCommon {
   const double* sq_norm;  // device: sum of squares of all gradients of the step (nullptr: no clipping)
   float max_norm;
   int32_t group_size;   // of the any-group-size kernel
+  int32_t after_norm;   // the launch in front of this one forms sq_norm: wait for it
 };
 template <int N>
 struct LeafTable {
@@ -1838,7 +1839,7 @@ FO_DEVI void build_wide_lut(float* lut_mw) {
 }
 
 // Launches of one call are chained: a kernel lets the next one start as soon as its own blocks are resident
-// (they work on different leaves), and no kernel completes before the one in front of it has, so that whatever
+// (they work on different leaves; the first of a clipped step waits for the norm before it does), and no kernel completes before the one in front of it has, so that whatever
 // the stream holds next sees all of them done.  One thread's wait is enough for that.
 FO_DEVI void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 FO_DEVI void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -1864,7 +1865,8 @@ FO_DEVI int leaf_of(const uint32_t* first, const int n_leaves, const uint32_t c)
 // loop or after it, cost a quarter of their throughput (spills in the loop, no uniform registers).
 template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
 __global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const __grid_constant__ StepParams<MODE> p) {
-  chain_release();
+  if ((MODE & (kClip | kPeer)) != 0 && p.after_norm) chain_wait();
+  chain_release();  // (only now: a launch behind this one may rely on the norm)
   __shared__ float lut_wide[STATE == FO_STATE_QUANT ? 256 * kLutCopies : 1];
   if constexpr (STATE == FO_STATE_QUANT) build_wide_lut(lut_wide);
   const LutWide lut{lut_wide + (STATE == FO_STATE_QUANT ? (threadIdx.x & (kLutCopies - 1)) : 0)};
@@ -1872,7 +1874,6 @@ __global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const _
   using S = Stage<OPT, PDT, ECC_BITS, STATE>;
   const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(stage_mem);
   const int gdt = p.grad_dtype;
-  if ((MODE & (kClip | kPeer)) != 0 && p.sq_norm != nullptr) chain_wait();  // the norm comes from a kernel in front of this one
   SharedClip clip{false, 0u};
   if constexpr ((MODE & (kClip | kPeer)) != 0) {
     __shared__ float4 clip_constants;
@@ -1929,9 +1930,9 @@ __global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const _
 // ragged end, see launch_pieces.
 template <int OPT, int PDT, int ECC_BITS, int STATE, int N>
 __global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_constant__ PieceParams<N> p) {
+  if (p.after_norm) chain_wait();
   chain_release();
   const bool with_peers = p.peers.n > 0 || p.peers.ng > 0 || p.peers.mc_pdelta != 0 || p.peers.mc_gdelta != 0;
-  if (p.sq_norm != nullptr) chain_wait();
   const Clip clip = load_clip(p.sq_norm, p.max_norm, p.grad_dtype);
   const uint32_t total = p.first_piece[p.n_leaves];
   for (uint32_t q = blockIdx.x; q < total; q += gridDim.x) {
@@ -1955,9 +1956,9 @@ __global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_const
 // are not 8, 16, ..., 256 (those run step_kernel and piece_kernel) ------------------------------------------
 template <int OPT, int PDT, int ECC_BITS>
 __global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant__ StepParams<kOut> p) {
+  if (p.after_norm) chain_wait();
   chain_release();
   __shared__ unsigned int smax_m[kGenericTile], smax_v[kGenericTile];
-  if (p.sq_norm != nullptr) chain_wait();
   const Clip clip = load_clip(p.sq_norm, p.max_norm, p.grad_dtype);
   const int l = leaf_of(p.t.first_block, p.n_leaves, blockIdx.x);
   const DevLeaf& L = p.t.leaf[l];
@@ -2067,11 +2068,12 @@ struct HostStep {
   const double* sq_norm;
   float max_norm;
   const Peers* peers;
+  bool after_norm;  // of the next launch
 };
 // `chained`: the launch in front of this one on the stream is one of this library's and works on other leaves
 // (or is the one whose result chain_wait() in the kernel waits for); set to true by a launch.
-using MainFn = cudaError_t (*)(const HostStep&, bool& chained, cudaStream_t);
-using PieceFn = cudaError_t (*)(const HostStep&, unsigned int main_chunk, bool& chained, cudaStream_t);
+using MainFn = cudaError_t (*)(HostStep&, bool& chained, cudaStream_t);
+using PieceFn = cudaError_t (*)(HostStep&, unsigned int main_chunk, bool& chained, cudaStream_t);
 // A slice of step_kernel and the elements one of its chunks covers.  Block size, and with it the chunk, is a
 // property of the slice (the slices are compiled with their own FO_THREADS).
 struct Launcher {
@@ -2079,8 +2081,8 @@ struct Launcher {
   unsigned int chunk;
 };
 
-template <typename P>
-cudaError_t launch_chained(void (*kernel)(P), unsigned int grid, unsigned int threads, int smem, bool& chained, cudaStream_t s, const P& p) {
+template <typename... P>
+cudaError_t launch_chained(void (*kernel)(P...), unsigned int grid, unsigned int threads, int smem, bool& chained, cudaStream_t s, const P&... p) {
   cudaLaunchConfig_t c = {};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(threads);
@@ -2092,10 +2094,10 @@ cudaError_t launch_chained(void (*kernel)(P), unsigned int grid, unsigned int th
   c.attrs = a;
   c.numAttrs = chained ? 1 : 0;
   chained = true;
-  return cudaLaunchKernelEx(&c, kernel, p);
+  return cudaLaunchKernelEx(&c, kernel, p...);
 }
 
-inline void fill_common(StepCommon& p, const HostStep& s) {
+inline void fill_common(StepCommon& p, HostStep& s) {
   for (int i = 0; i < s.n_hypers; ++i) p.hyper[i] = s.hyper[i];
   p.n_leaves = 0;
   p.grad_dtype = s.grad_dtype;
@@ -2106,6 +2108,8 @@ inline void fill_common(StepCommon& p, const HostStep& s) {
   p.run_chunks = 1;
   p.sq_norm = s.sq_norm;
   p.max_norm = s.max_norm;
+  p.after_norm = s.after_norm && s.sq_norm != nullptr ? 1 : 0;
+  s.after_norm = false;
 }
 
 inline namespace FO_SHAPE_NS {
@@ -2114,7 +2118,7 @@ inline namespace FO_SHAPE_NS {
 constexpr int kSmemPerSm = 227 * 1024, kSmemReservedPerBlock = 1024;
 
 template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
-cudaError_t launch_main(const HostStep& hs, bool& chained, cudaStream_t s) {
+cudaError_t launch_main(HostStep& hs, bool& chained, cudaStream_t s) {
   constexpr bool peer = MODE == kPeer;
   const bool switch_sum = peer && hs.peers->mc_gdelta != 0 && hs.grad_dtype != FO_F32;
   const int ring_bytes = switch_sum ? kSwitchBatch * 16 * kThreads : 0;
@@ -2203,7 +2207,7 @@ cudaError_t launch_main(const HostStep& hs, bool& chained, cudaStream_t s) {
 
 // The pieces that the whole chunks (of main_chunk elements; 0: step_kernel is not used) of the hot leaves leave over.
 template <int OPT, int PDT, int ECC_BITS, int STATE, int N>
-cudaError_t launch_piece_table(const HostStep& hs, const int* which, int n, unsigned int main_chunk, bool& chained, cudaStream_t s) {
+cudaError_t launch_piece_table(HostStep& hs, const int* which, int n, unsigned int main_chunk, bool& chained, cudaStream_t s) {
   PieceParams<N> p;  // filled as far as it is used
   fill_common(p, hs);
   p.peers = *hs.peers;
@@ -2225,7 +2229,7 @@ cudaError_t launch_piece_table(const HostStep& hs, const int* which, int n, unsi
   return launch_chained(piece_kernel<OPT, PDT, ECC_BITS, STATE, N>, total < most ? total : most, kPieceThreads, 0, chained, s, p);
 }
 template <int OPT, int PDT, int ECC_BITS, int STATE>
-cudaError_t launch_pieces(const HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
+cudaError_t launch_pieces(HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
   int which[kPieceLeavesLarge];
   int n = 0;
   for (int i = 0; i <= hs.n_leaves; ++i) {
@@ -2244,7 +2248,7 @@ cudaError_t launch_pieces(const HostStep& hs, unsigned int main_chunk, bool& cha
   return cudaSuccess;
 }
 template <int OPT, int PDT, int ECC_BITS>
-cudaError_t launch_generic(const HostStep& hs, bool& chained, cudaStream_t s) {
+cudaError_t launch_generic(HostStep& hs, bool& chained, cudaStream_t s) {
   StepParams<kOut> p;
   fill_common(p, hs);
   const unsigned int tile = generic_tile_elems(hs.group_size);

@@ -189,9 +189,11 @@ typedef struct FoStepMore {
    * Not together with peers. */
   const FoLeafOut* outs;
 } FoStepMore;
-/* The launch in front of this one on the stream is another fo_step* of the same pytree step (other leaves), or
- * the fo_sq_norm* call that forms its grad_sq_norm: the kernels may start before that launch has drained. */
+/* What the launch in front of this one on the stream is; the kernels then start before it has drained.
+ * CHAINED: another fo_step* of the same pytree step (other leaves).  AFTER_NORM: the fo_sq_norm* call that forms
+ * this step's grad_sq_norm (the kernels wait for its result). */
 #define FO_LAUNCH_CHAINED 1u
+#define FO_LAUNCH_AFTER_NORM 2u
 int fo_step_ex(const FoStepDesc* desc, const FoStepMore* more, void* cuda_stream);
 
 /* Per-step scalars formed on the device, so that a whole step can be captured in a CUDA graph
@@ -227,6 +229,9 @@ typedef struct FoArray {
 #define FO_SQ_NORM_WORKSPACE_BYTES 16384
 int fo_sq_norm(const FoArray* arrays, uint32_t n_arrays, int32_t dtype, int32_t accumulate, double* out,
                void* workspace, void* cuda_stream);
+/* The same over arrays of several dtypes: dtypes[i] (host table) is the dtype of arrays[i]. */
+int fo_sq_norm_mixed(const FoArray* arrays, const int32_t* dtypes, uint32_t n_arrays, int32_t accumulate, double* out,
+                     void* workspace, void* cuda_stream);
 
 /* Reduce-scatter and norm in one sweep, for ZeRO-1 steps that clip by the global norm: this rank's
  * slice of the averaged gradient is needed twice (for the norm of the whole averaged gradient, then
@@ -263,6 +268,16 @@ int fo_split(const float* theta, void* param_lp, void* ecc, int32_t param_dtype,
              void* cuda_stream);
 int fo_reconstruct(const void* param_lp, const void* ecc, float* theta, int32_t param_dtype, int32_t ecc_bits,
                    uint64_t n, void* cuda_stream);
+/* The same for a pytree's leaves at once (host table; leaves that share param_dtype and ecc_bits):
+ * fo_split_many reads theta and writes lp and ecc, fo_reconstruct_many reads lp and ecc and writes theta. */
+typedef struct FoSplitLeaf {
+  float* theta;
+  void* lp;
+  void* ecc;
+  uint64_t n;
+} FoSplitLeaf;
+int fo_split_many(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t param_dtype, int32_t ecc_bits, void* cuda_stream);
+int fo_reconstruct_many(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t param_dtype, int32_t ecc_bits, void* cuda_stream);
 
 /*
  * Device self-checks of the exact-arithmetic shortcuts the kernels use (no counterpart in
