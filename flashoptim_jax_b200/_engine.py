@@ -22,8 +22,10 @@ from . import tree as pytree
 from ._dev import DTYPE_CODE, ECC_BITS_OF, as_tensor, require_cuda, stream_ptr
 from .quantization import QuantizedArray
 from .utils import (
+    GroupResolver,
     _group_config_for_path,
     _is_quantized_leaf,
+    _resolve_learning_rate,
     _tree_leaves_with_paths,
     _use_ecc_leaf,
     _validate_fused_group_size,
@@ -85,21 +87,19 @@ _clip = threading.local()
 
 
 @contextlib.contextmanager
-def grad_clip(sq_norm: torch.Tensor, max_norm: float):
+def grad_clip(sq_norm: torch.Tensor, max_norm: float, fresh: bool = False):
     """While active, every launch rescales its gradients as optax.clip_by_global_norm does
     (examples/train_gpt2_pretrain.py:56-70): `sq_norm` is a one-element float64 device tensor with the
-    sum of squares of all gradients of the step (see sq_norm_of)."""
+    sum of squares of all gradients of the step (see sq_norm_of).  `fresh`: the launch that forms it is the last thing
+    on the stream, so that the step's first launch may be chained to it."""
     if sq_norm.dtype != torch.float64 or sq_norm.numel() != 1 or not sq_norm.is_cuda:
         raise ValueError("sq_norm must be a one-element float64 CUDA tensor")
     previous = getattr(_clip, "value", None)
-    _clip.value = (sq_norm, float(max_norm))
+    _clip.value = (sq_norm, float(max_norm), bool(fresh))
     try:
         yield
     finally:
         _clip.value = previous
-
-
-_workspaces: Dict[int, torch.Tensor] = {}
 
 
 def sq_norm_of(tensors: List[torch.Tensor], out: Optional[torch.Tensor] = None, accumulate: bool = False) -> torch.Tensor:
@@ -112,9 +112,7 @@ def sq_norm_of(tensors: List[torch.Tensor], out: Optional[torch.Tensor] = None, 
     if out is None:
         out = torch.zeros(1, dtype=torch.float64, device=device)
     lib = _lib.lib()
-    ws = _workspaces.get(device.index)
-    if ws is None:
-        ws = _workspaces[device.index] = torch.empty(_lib.FO_SQ_NORM_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
+    ws = torch.empty(_lib.FO_SQ_NORM_WORKSPACE_BYTES, dtype=torch.uint8, device=device)  # its own: streams do not share one
     by_dtype: Dict[torch.dtype, List[torch.Tensor]] = {}
     for t in tensors:
         if t.dtype not in DTYPE_CODE:
@@ -145,9 +143,7 @@ def mean_sq_norm(grad_slice: torch.Tensor, mean_out: torch.Tensor, peer_grad_off
     device = grad_slice.device
     if grad_slice.numel() != mean_out.numel() or grad_slice.dtype != mean_out.dtype:
         raise ValueError("mean_sq_norm: slice and output differ")
-    ws = _workspaces.get(device.index)
-    if ws is None:
-        ws = _workspaces[device.index] = torch.empty(_lib.FO_SQ_NORM_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
+    ws = torch.empty(_lib.FO_SQ_NORM_WORKSPACE_BYTES, dtype=torch.uint8, device=device)  # its own: streams do not share one
     peers = np.asarray(peer_grad_offsets, dtype=np.int64)
     with torch.cuda.device(device):
         _lib.check(_lib.lib().fo_mean_sq_norm(grad_slice.data_ptr(), mean_out.data_ptr(), grad_slice.numel(), DTYPE_CODE[grad_slice.dtype],
@@ -275,12 +271,6 @@ class PreparedLaunch:
                                    "keep": ws})  # the tensors stay alive as long as their addresses are in the tables
                 start = end
 
-    def set_grads(self, grad_ptrs: np.ndarray, keep: List[torch.Tensor]) -> None:
-        """New gradient buffers for the same leaves (addresses in the order of the work list this was built from)."""
-        for call in self.calls:
-            call["leaves"]["grad"] = grad_ptrs[call["index"]]
-        self._grads_alive = keep
-
     def run(self, hyper_of_group: Dict[int, Tuple[Any, ...]]) -> int:
         lib = _lib.lib()
         clip = getattr(_clip, "value", None)
@@ -304,87 +294,97 @@ class PreparedLaunch:
         return len(self.calls)
 
 
-class DonatedStepCache:
-    """The functional tx.step for callers that donate their buffers and hand each step's outputs to the
-    next: the parameter and state tensors are then the same objects step after step, and only the gradients
-    and the scalars change.  After one step through the general path this remembers the prepared launch of
-    that step, keyed on the identity and the addresses of every tensor of the returned trees; a later call
-    whose trees consist of exactly those tensors skips the per-leaf host work (path normalisation, param-group
-    matching, validation, table building: about 12 us per leaf) and replays the launch with new gradient
-    addresses and hyper-parameter values.  Anything else (other tensors, other gradient dtypes, non-contiguous
-    gradients) falls back to the general path, which then re-primes the cache.  A replayed step keeps the
-    param-group membership of the remembered call: selectors are functions of the path and of the leaf's
-    shape / dtype in every use the reference shows, and a selector that reads a leaf's *values* is not
-    re-evaluated while the same tensors come back."""
+def _static_selector(spec: Any) -> bool:
+    """A selector that gives the same answer for the same path: a name or a path, or a list of those."""
+    if isinstance(spec, (str, tuple)):
+        return True
+    return type(spec) is list and all(isinstance(x, (str, tuple)) for x in spec)
 
-    def __init__(self):
-        self.entry = None
 
-    @staticmethod
-    def _tensors(params: Any, state_trees: List[Any]) -> Tuple[List[torch.Tensor], List[Any]]:
-        """Every tensor of the trees in flattening order, and the trees' structural signature."""
-        out, sig = pytree.tree_leaves_and_signature(params)
-        sig.append(len(out))
-        for tree in state_trees:
-            leaves, s = pytree.tree_leaves_and_signature(tree, is_leaf=_is_quantized_leaf)
-            sig.append(s)
-            for leaf in leaves:
-                if isinstance(leaf, QuantizedArray):
-                    out.append(leaf.values)
-                    out.append(leaf.scales)
-                else:
-                    out.append(leaf)
-        return out, sig
+class NativeStep:
+    """tx.step without the per-leaf Python work: the general path runs once per kind of pytree (structure, shapes, dtypes,
+    param-group membership) and leaves a compiled plan behind (csrc/fo_host.cc); a later call that fits it is one native call
+    that checks the leaves again, fills in addresses and hyper-parameter values, allocates what must not overwrite
+    its operands, and launches.  Anything else (other dtypes, non-contiguous tensors, edited param groups, tensor subclasses, a
+    launch observer) takes the general path.
 
-    def remember(self, opt: int, work: List[LeafWork], configs: List[Dict[str, Any]], params_out: Any, state_trees_out: List[Any]) -> None:
-        groups: List[Dict[str, Any]] = []
-        gids = []
-        for c in configs:
-            for i, g in enumerate(groups):
-                if g is c or g == c:
-                    gids.append(i)
-                    break
-            else:
-                groups.append(c)
-                gids.append(len(groups) - 1)
-        tensors, sig = self._tensors(params_out, state_trees_out)
-        if not all(isinstance(t, torch.Tensor) for t in tensors):
-            self.entry = None
+    Selectors that are functions are asked again whenever the parameters are not the very tensors of the last step,
+    which with donated buffers they are: a selector that reads a leaf's *values* is not re-evaluated while
+    the same tensors come back."""
+
+    MOST_PLANS = 4
+
+    def __init__(self, opt: int, donate: bool, defaults: Dict[str, Any], param_groups: Any, hyper_of_config):
+        self.opt, self.donate, self.defaults, self.param_groups = opt, bool(donate), defaults, param_groups
+        self.hyper_of_config = hyper_of_config  # config -> hyper-parameter tuple (lr and bias corrections are filled in per step)
+        self.plans: List[Any] = []
+        self.wait = self.backoff = 0
+
+    def run(self, params: Any, count: Any, states: Tuple[Any, ...], grads: Any):
+        """(params, state trees, count) after the step, or None when no plan fits."""
+        if not self.plans or _observer is not None:
+            return None
+        clip = getattr(_clip, "value", None)
+        sq, max_norm, chained = (0, 0.0, False) if clip is None else (clip[0].data_ptr(), clip[1], clip[2])
+        for i, (host_run, plan) in enumerate(self.plans):
+            hit = host_run(plan, params, count, states, grads, sq, max_norm, chained)
+            if hit is not None:
+                if i:
+                    self.plans.insert(0, self.plans.pop(i))
+                self.backoff = 0
+                return hit
+        return None
+
+    def remember(self, params: Any, path_leaves, work: List[LeafWork], configs: List[Dict[str, Any]], n_states: int) -> None:
+        """Compile the step the general path has just taken."""
+        if _observer is not None:
             return
-        self.entry = {
-            "plan": PreparedLaunch(opt, work, gids), "groups": groups, "ids": [id(t) for t in tensors],
-            "sig": sig,
-            "ptrs": [t.data_ptr() for t in tensors], "alive": tensors, "params": params_out, "state": state_trees_out,
-            "grad_spec": [(w.grad.dtype, w.grad.shape, w.grad.device) for w in work],
-        }
-
-    def replay(self, params: Any, state_trees: List[Any], grads: Any, hyper_of_group) -> Optional[Tuple[Any, List[Any]]]:
-        """Runs the remembered launch if (params, state) are the remembered tensors; returns (params, state trees)
-        or None.  `hyper_of_group(config)` gives the hyper-parameter tuple of a param group for this step."""
-        e = self.entry
-        if e is None:
-            return None
-        tensors, sig = self._tensors(params, state_trees)
-        if len(tensors) != len(e["ids"]) or sig != e["sig"]:
-            return None
-        try:  # the same objects at the same addresses (C-level loops: this check runs on every step)
-            if list(map(id, tensors)) != e["ids"] or list(map(torch.Tensor.data_ptr, tensors)) != e["ptrs"]:
-                return None
-        except TypeError:  # something that is not a tensor
-            return None
-        g_leaves = pytree.tree_leaves(grads)
-        spec = e["grad_spec"]
-        if len(g_leaves) != len(spec):
-            return None
-        ptrs = np.empty(len(spec), dtype=np.uint64)
-        for k, (g, (dtype, shape, device)) in enumerate(zip(g_leaves, spec)):
-            if not isinstance(g, torch.Tensor) or g.dtype != dtype or g.shape != shape or g.device != device or not g.is_contiguous():
-                return None
-            ptrs[k] = g.data_ptr()
-        plan = e["plan"]
-        plan.set_grads(ptrs, g_leaves)
-        plan.run({gid: hyper_of_group(config) for gid, config in enumerate(e["groups"])})
-        return e["params"], e["state"]
+        if self.wait:  # steps of this kind keep missing their plans: making them is not free
+            self.wait -= 1
+            return
+        self.backoff = min(2 * self.backoff + 1, 1023)
+        self.wait = self.backoff - 1
+        if not work or any(w.bucket[0] != work[0].bucket[0] for w in work):
+            return
+        groups: List[Dict[str, Any]] = []
+        group_of: Dict[int, int] = {}
+        for c in configs:
+            if id(c) not in group_of:
+                group_of[id(c)] = len(groups)
+                groups.append(c)
+        hypers = []
+        for c in groups:
+            if not all(type(c[k]) in (float, int) for k in ("weight_decay", "b1", "b2", "eps", "momentum", "dampening") if k in c):
+                return
+            _, wd, b1, b2, omb1, omb2, eps, _, _, flags = self.hyper_of_config(c)
+            hypers.append((c["learning_rate"], float(wd), float(b1), float(b2), float(omb1), float(omb2), float(eps), int(flags)))
+        calls: List[Tuple[Tuple[Any, ...], List[int]]] = []
+        open_call: Dict[Tuple[Any, ...], int] = {}
+        leaves = []
+        for w, c in zip(work, configs):
+            gid = group_of[id(c)]
+            k = open_call.get(w.bucket)
+            if k is None or (gid not in calls[k][1] and len(calls[k][1]) == _lib.FO_MAX_HYPERS):
+                k = open_call[w.bucket] = len(calls)
+                calls.append((w.bucket, []))
+            if gid not in calls[k][1]:
+                calls[k][1].append(gid)
+            _, pdt, gdt, ecc_bits, state, group_size = w.bucket
+            leaves.append((tuple(w.param.shape), pdt, gdt, ecc_bits, state, group_size, gid, k, calls[k][1].index(gid)))
+        if self.param_groups is not None and type(self.param_groups) not in (list, tuple):
+            return
+        param_groups = self.param_groups
+        watched = tuple(param_groups or ())
+        member = GroupResolver(self.defaults, param_groups).member
+        host = _lib.host()
+        plan = host.make_plan(
+            self.opt, self.donate, work[0].bucket[0], params, n_states, tuple(leaves), tuple(hypers),
+            tuple((*bucket[1:5], bucket[5], tuple(slots)) for bucket, slots in calls), param_groups, watched,
+            not all(_static_selector(g["params"]) for g in watched), member, tuple(path for path, _ in path_leaves),
+            tuple(member(path, leaf) for path, leaf in path_leaves), _resolve_learning_rate)
+        if plan is not None:
+            self.plans.insert(0, (host.run, plan))
+            del self.plans[self.MOST_PLANS:]
 
 
 def launch(opt: int, work: List[LeafWork], peer_param_offsets: Optional[List[int]] = None,

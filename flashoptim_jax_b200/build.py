@@ -1,4 +1,4 @@
-"""Builds libflashoptim_b200.so in-tree with nvcc for sm_100a.
+"""Builds libflashoptim_b200.so in-tree with nvcc for sm_100a, and the host extension over it.
 
 The step-kernel family is split into instantiation slices (optimizer x state kind x kernel)
 compiled from one source with different -D switches, so the build runs in parallel.
@@ -21,6 +21,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ_DIR = os.path.join(CSRC, "build")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libflashoptim_b200.so")
+HOST_PATH = os.path.join(HERE, "_fo_host.so")  # the host side (csrc/fo_host.cc): a Python extension over torch's C++ tensors
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -155,6 +156,32 @@ def build_native(force: bool = False, jobs: int | None = None, extra_flags: List
     return lib_path
 
 
+def build_host(force: bool = False) -> str:
+    """Compile the extension module flashoptim_jax_b200._fo_host with the host compiler; returns its path."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    source = os.path.join(CSRC, "fo_host.cc")
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    dirs = [*include_paths(), sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{d}" for d in dirs], source, "-o", HOST_PATH, f"-L{libs}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda",
+           "-lc10", "-lc10_cuda"]
+    stamp = HOST_PATH + ".digest"
+    digest = _sources_digest([torch.__version__, sys.version, *cmd], [])
+    if not force and os.path.exists(HOST_PATH) and os.path.exists(stamp) and open(stamp).read() == digest:
+        return HOST_PATH
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"host build failed:\n{' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+    with open(stamp, "w") as f:
+        f.write(digest)
+    return HOST_PATH
+
+
 if __name__ == "__main__":
     path = build_native(force="--force" in sys.argv, verbose="-v" in sys.argv)
+    print(build_host(force="--force" in sys.argv))
     print(path)

@@ -16,6 +16,7 @@ from __future__ import annotations
 from typing import Any
 
 from . import _engine as eng
+from . import _lib
 from . import tree as pytree
 from ._dev import as_tensor
 from .utils import FlashOptimizer
@@ -23,7 +24,8 @@ from .utils import FlashOptimizer
 
 def global_sq_norm(grads: Any):
     """One-element float64 CUDA tensor with the sum of squares of every leaf of `grads`."""
-    return eng.sq_norm_of([as_tensor(g) for g in pytree.tree_leaves(grads)])
+    sq = _lib.host().sq_norm(grads)
+    return eng.sq_norm_of([as_tensor(g) for g in pytree.tree_leaves(grads)]) if sq is None else sq
 
 
 def clip_by_global_norm(tx: FlashOptimizer, max_norm: float) -> FlashOptimizer:
@@ -36,7 +38,7 @@ def clip_by_global_norm(tx: FlashOptimizer, max_norm: float) -> FlashOptimizer:
 
     def step_fn(params: Any, state: Any, grads: Any):
         sq = global_sq_norm(grads)
-        with eng.grad_clip(sq, max_norm):
+        with eng.grad_clip(sq, max_norm, fresh=True):
             params, opt_state = tx.step(params, state["opt"], grads)
         return params, {"clip": (), "opt": opt_state}
 

@@ -83,11 +83,16 @@ def reconstruct_leaf(theta_lp, rho) -> torch.Tensor:
 
 def reconstruct_weights(params_lp: Any, errors: Any) -> Any:
     """fp32 weights of a whole pytree (flashoptim_jax/compression.py:124-126)."""
-    return pytree.tree_map(reconstruct_leaf, params_lp, errors)
+    out = _lib.host().reconstruct(params_lp, errors)  # one launch per dtype; None: not a pytree of contiguous CUDA tensors
+    return pytree.tree_map(reconstruct_leaf, params_lp, errors) if out is None else out
 
 
 def set_fp32_params(fp32_params: Any, param_template: Any, master_weight_bits: Optional[int] = 24) -> Tuple[Any, Any]:
     """fp32 weights -> (stored params, ECC tree) with the template's dtypes (flashoptim_jax/compression.py:129-146)."""
+    _validate_master_weight_bits(master_weight_bits)
+    pair = _lib.host().split(fp32_params, param_template, 0 if master_weight_bits is None else master_weight_bits - 16)
+    if pair is not None:
+        return pair
     leaves, treedef = pytree.tree_flatten(fp32_params)
     template_leaves, template_def = pytree.tree_flatten(param_template)
     if treedef != template_def:

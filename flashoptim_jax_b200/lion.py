@@ -68,16 +68,13 @@ def flash_lion(learning_rate=1e-4, b1: float = 0.9, b2: float = 0.99, weight_dec
         eng.launch(_lib.FO_OPT_LION, work)
         return treedef.unflatten(new_p), FlashLionState(count=count, mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
 
-    cache = eng.DonatedStepCache()
+    native = eng.NativeStep(_lib.FO_OPT_LION, donate, defaults, param_groups, lambda c: lion_hyper(c, 0.0))
 
     def step_fn(params: Any, state: FlashLionState, grads: Any):
+        hit = native.run(params, state.count, (state.ecc, state.mu), grads)
+        if hit is not None:
+            return hit[0], FlashLionState(hit[2], hit[1][1], hit[1][0])
         old_count = as_tensor(state.count, dtype=torch.int32).cpu()
-        if donate:
-            hit = cache.replay(params, [state.ecc, state.mu], grads, lambda config: lion_hyper(
-                config, utils._resolve_learning_rate(config["learning_rate"], old_count)))
-            if hit is not None:
-                ecc_t, mu_t = hit[1]
-                return hit[0], FlashLionState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32), mu=mu_t, ecc=ecc_t)
         configs = []
         param_pl, grad_leaves, (ecc_leaves, mu_leaves), treedef = eng.flatten_step_inputs(
             name, params, grads, [state.ecc, state.mu])
@@ -97,8 +94,7 @@ def flash_lion(learning_rate=1e-4, b1: float = 0.9, b2: float = 0.99, weight_dec
         new_state = FlashLionState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32),
                                    mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        if donate:
-            cache.remember(_lib.FO_OPT_LION, work, configs, new_params, [new_state.ecc, new_state.mu])
+        native.remember(params, param_pl, work, configs, 2)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

@@ -27,6 +27,9 @@ def _num_groups(n: int, group_size: int) -> int:
 
 
 def _quantize(x, group_size: int, variance: bool) -> QuantizedArray:
+    q = _lib.host().quantize(x, group_size, variance)  # None: something to convert first, or an error to report
+    if q is not None:
+        return q
     x = as_tensor(x)
     require_cuda(x, "x")
     xf = x.to(torch.float32).contiguous()
@@ -40,6 +43,9 @@ def _quantize(x, group_size: int, variance: bool) -> QuantizedArray:
 
 
 def _dequantize(q: QuantizedArray, group_size: int, variance: bool) -> torch.Tensor:
+    out = _lib.host().dequantize(q, group_size, variance)
+    if out is not None:
+        return out
     values, scales = q.values, q.scales
     require_cuda(values, "values")
     values = values.contiguous()

@@ -87,16 +87,13 @@ def _make_sgd_transform(learning_rate, momentum, dampening, weight_decay, nester
         eng.launch(_lib.FO_OPT_SGD, work)
         return treedef.unflatten(new_p), FlashSGDState(count=count, mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
 
-    cache = eng.DonatedStepCache()
+    native = eng.NativeStep(_lib.FO_OPT_SGD, donate, defaults, param_groups, lambda c: sgd_hyper(c, 0.0, decoupled_weight_decay))
 
     def step_fn(params: Any, state: FlashSGDState, grads: Any):
+        hit = native.run(params, state.count, (state.ecc, state.mu), grads)
+        if hit is not None:
+            return hit[0], FlashSGDState(hit[2], hit[1][1], hit[1][0])
         old_count = as_tensor(state.count, dtype=torch.int32).cpu()
-        if donate:
-            hit = cache.replay(params, [state.ecc, state.mu], grads, lambda config: sgd_hyper(
-                config, utils._resolve_learning_rate(config["learning_rate"], old_count), decoupled_weight_decay))
-            if hit is not None:
-                ecc_t, mu_t = hit[1]
-                return hit[0], FlashSGDState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32), mu=mu_t, ecc=ecc_t)
         configs = []
         param_pl, grad_leaves, (ecc_leaves, mu_leaves), treedef = eng.flatten_step_inputs(
             name, params, grads, [state.ecc, state.mu])
@@ -121,8 +118,7 @@ def _make_sgd_transform(learning_rate, momentum, dampening, weight_decay, nester
         new_state = FlashSGDState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32),
                                   mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        if donate:
-            cache.remember(_lib.FO_OPT_SGD, work, configs, new_params, [new_state.ecc, new_state.mu])
+        native.remember(params, param_pl, work, configs, 2)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

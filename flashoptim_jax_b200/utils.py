@@ -94,12 +94,15 @@ class GroupResolver:
                 raise ValueError("Each param group must define a 'params' matcher")
         self._configs: Dict[int, Dict[str, Any]] = {}
 
-    def __call__(self, path, leaf) -> Dict[str, Any]:
-        index = -1
+    def member(self, path, leaf) -> int:
+        """Index of the first group whose matcher accepts the leaf, -1 for the defaults."""
         for i, group in enumerate(self.groups):
             if _path_matches(path, leaf, group["params"]):
-                index = i
-                break
+                return i
+        return -1
+
+    def __call__(self, path, leaf) -> Dict[str, Any]:
+        index = self.member(path, leaf)
         config = self._configs.get(index)
         if config is None:
             config = dict(self.defaults)
