@@ -1,0 +1,209 @@
+"""tx.step through the compiled plan (csrc/fo_host.cc) against the general path, bit for bit: trees of every container, each
+optimizer, donated and not; and what must make a plan give way (edited param groups, selectors that change their mind,
+gradients that need a conversion, several threads)."""
+
+import collections
+import contextlib
+import threading
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+Pair = collections.namedtuple("Pair", "kernel bias")
+
+
+def _params(seed=0):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(s, device="cuda", generator=g) * 0.02
+    return {"b": [Pair(r(33, 7).bfloat16(), r(7)), None], "a": {"w": r(70, 64).to(torch.float16), "z": (r(5).bfloat16(), r(2048).bfloat16())}}
+
+
+def _grads(params, seed):
+    import torch
+
+    from flashoptim_jax_b200 import tree
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return tree.tree_map(lambda p: (torch.randn(p.shape, device="cuda", generator=g) * 1e-2).to(p.dtype), params)
+
+
+def _leaves(x):
+    from flashoptim_jax_b200 import tree
+
+    return tree.tree_leaves(x)
+
+
+def _same(a, b):
+    import torch
+
+    la, lb = _leaves(a), _leaves(b)
+    assert len(la) == len(lb)
+    for x, y in zip(la, lb):
+        assert x.dtype == y.dtype and x.shape == y.shape and torch.equal(x.view(torch.uint8) if x.dim() else x, y.view(torch.uint8) if y.dim() else y)
+
+
+@contextlib.contextmanager
+def _general_path():
+    from flashoptim_jax_b200 import _engine as eng
+
+    eng.set_launch_observer(lambda key, n: contextlib.nullcontext())
+    try:
+        yield
+    finally:
+        eng.set_launch_observer(None)
+
+
+FACTORIES = [("flash_adamw", dict(learning_rate=1e-3)), ("flash_adam", dict(learning_rate=lambda c: 1e-3 / (1 + int(c)), master_weight_bits=32, group_size=64)),
+             ("flash_adamw", dict(learning_rate=1e-3, fused=False, quantize=False)), ("flash_lion", dict(weight_decay=1e-2)),
+             ("flash_sgd", dict(learning_rate=1e-2)), ("flash_sgdw", dict(learning_rate=1e-2, momentum=0.9, nesterov=True, group_size=40, fused=False))]
+
+
+@pytest.mark.parametrize("donate", [False, True])
+@pytest.mark.parametrize("name,kw", FACTORIES)
+def test_planned_steps_equal_general_steps(name, kw, donate):
+    import flashoptim_jax_b200 as fo
+
+    groups = [{"params": ["bias", "a/z/1"], "weight_decay": 0.0, "learning_rate": 5e-3}, {"params": lambda p, leaf: leaf.dim() == 1, "weight_decay": 0.1}]
+    tx = getattr(fo, name)(param_groups=groups, donate=donate, **kw)
+    ref = getattr(fo, name)(param_groups=groups, **kw)
+    p, q = _params(), _params()
+    s, t = tx.init(p), ref.init(q)
+    for k in range(4):
+        g = _grads(q, k)
+        before = [x.clone() for x in _leaves((p, s))]
+        old = (p, s)
+        p, s = tx.step(p, s, g)
+        with _general_path():
+            q, t = ref.step(q, t, g)
+        _same((p, tuple(s)), (q, tuple(t)))
+        assert type(p["b"]) is list and type(p["b"][0]) is Pair and p["b"][1] is None and int(s.count) == k + 1
+        if not donate:
+            _same(old, before)
+
+
+def test_edited_groups_and_selectors_are_honoured():
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    frozen = set()
+    groups = [{"params": lambda path, leaf: path[0] in frozen, "learning_rate": 0.0, "weight_decay": 0.0}, {"params": "y", "learning_rate": 2e-2}]
+    tx = fo.flash_adamw(learning_rate=1e-2, param_groups=groups)
+    p = {k: torch.ones(100, device="cuda", dtype=torch.bfloat16) for k in ("x", "y")}
+    s, g = tx.init(p), {k: torch.full((100,), 0.1, device="cuda", dtype=torch.bfloat16) for k in ("x", "y")}
+    for _ in range(3):
+        p, s = tx.step(p, s, g)
+    frozen.add("x")
+    q, s = tx.step(p, s, g)
+    assert torch.equal(q["x"], p["x"]) and not torch.equal(q["y"], p["y"])
+    groups[1]["learning_rate"] = 0.0
+    groups[1]["weight_decay"] = 0.0
+    r, s = tx.step(q, s, g)
+    assert torch.equal(r["y"], q["y"])
+    frozen.clear()
+    r2, s = tx.step(r, s, g)
+    assert not torch.equal(r2["x"], r["x"]) and int(s.count) == 6
+
+
+def test_gradients_that_need_a_conversion():
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    tx, ref = fo.flash_lion(donate=True), fo.flash_lion()
+    p, q = {"w": torch.ones(64, 32, device="cuda", dtype=torch.bfloat16)}, {"w": torch.ones(64, 32, device="cuda", dtype=torch.bfloat16)}
+    s, t = tx.init(p), ref.init(q)
+    base = torch.randn(32, 64, device="cuda").bfloat16()
+    for g in (base.t().contiguous(), base.t(), base.t().double(), base.t().float(), base.t().contiguous()):
+        p, s = tx.step(p, s, {"w": g})
+        with _general_path():
+            q, t = ref.step(q, t, {"w": g.contiguous()})
+        _same((p, s.mu, s.ecc), (q, t.mu, t.ecc))
+    with pytest.raises(ValueError):
+        tx.step(p, s, {"v": base})
+
+
+def test_threads_share_an_optimizer():
+    import time
+
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    def schedule(count):
+        time.sleep(0.001)  # another thread steps meanwhile
+        return 1e-3
+
+    tx, ref = fo.flash_adamw(learning_rate=schedule, donate=True), fo.flash_adamw(learning_rate=1e-3)
+    results, errors = {}, []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                p = {"w": torch.full((3000,), 1.0 + k, device="cuda", dtype=torch.bfloat16)}
+                g = {"w": torch.full((3000,), 0.01 * (k + 1), device="cuda", dtype=torch.bfloat16)}
+                s = tx.init(p)
+                for _ in range(20):
+                    p, s = tx.step(p, s, g)
+                torch.cuda.current_stream().synchronize()
+                results[k] = (p, s)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not errors
+    for k in range(4):
+        p = {"w": torch.full((3000,), 1.0 + k, device="cuda", dtype=torch.bfloat16)}
+        g = {"w": torch.full((3000,), 0.01 * (k + 1), device="cuda", dtype=torch.bfloat16)}
+        s = ref.init(p)
+        for _ in range(20):
+            p, s = ref.step(p, s, g)
+        _same((results[k][0], results[k][1].mu, results[k][1].nu), (p, s.mu, s.nu))
+
+
+def test_trees_of_weights_through_the_codecs():
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from flashoptim_jax_b200 import tree
+
+    p = _params(3)
+    w = tree.tree_map(lambda x: torch.randn(x.shape, device="cuda"), p)
+    for bits in (None, 24, 32):
+        lp, ecc = fo.set_fp32_params(w, p, master_weight_bits=bits)
+        want = tree.tree_map(lambda a, b: fo.split_leaf(a, narrow_dtype=b.dtype, master_weight_bits=bits), w, p)
+        for a, b, (c, d) in zip(_leaves(lp), _leaves(ecc), tree.tree_leaves(want, is_leaf=lambda x: type(x) is tuple and isinstance(x[0], torch.Tensor))):
+            _same((a, b), (c, d))
+        back = fo.reconstruct_weights(lp, ecc)
+        _same(back, tree.tree_map(fo.reconstruct_leaf, lp, ecc))
+    with pytest.raises(ValueError):
+        fo.reconstruct_weights(lp, {"a": ecc["a"]})
+
+
+@pytest.mark.parametrize("group", [1, 8, 16, 32, 100, 256, 512])
+def test_codecs_at_edges(group):
+    import numpy as np
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from oracle import flashoptim_oracle as O
+
+    rng = np.random.default_rng(group)
+    for n in (1, 7, 8, 2047, 2048, 2049, 3 * 2048 + 5):
+        x = rng.normal(0, 1e-3, n).astype(np.float32)
+        x[: n // 5] = 0
+        for variance in (False, True):
+            v = x * x if variance else x
+            t = torch.from_numpy(np.concatenate([np.zeros(1, np.float32), v])).cuda()[1:]  # not 32-byte aligned
+            for a in (t, t.clone()):
+                q = (fo.quantize_variance if variance else fo.quantize_momentum)(a, group)
+                want_q = (O.quantize_variance if variance else O.quantize_momentum)(v, group)
+                assert np.array_equal(q.values.cpu().numpy(), want_q.values) and np.array_equal(q.scales.cpu().numpy(), want_q.scales)
+                d = (fo.dequantize_variance if variance else fo.dequantize_momentum)(q, group)
+                want = (O.dequantize_variance if variance else O.dequantize_momentum)(want_q, group)
+                assert np.array_equal(d.cpu().numpy(), want)
