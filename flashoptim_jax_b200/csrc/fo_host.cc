@@ -277,7 +277,10 @@ struct Plan {
   Ref member, paths, membership;   // member(path, leaf) -> index of the first matching group or -1; tuples
   Ref resolve;                     // learning rate of a schedule: resolve(lr, count tensor)
   bool busy = false;               // a selector or a schedule may run Python code, and that another step
-  std::vector<PyObject*> p, g, last;  // scratch (borrowed)
+  std::vector<PyObject*> p, g;     // scratch (borrowed)
+  // parameters of the last step.  A weak reference keeps no data alive, but its address is not given to another tensor while
+  // it is held: an equal address is the same tensor
+  std::vector<c10::weak_intrusive_ptr<at::TensorImpl>> last;
   std::vector<std::vector<PyObject*>> s;
 };
 constexpr const char* kPlanName = "flashoptim_b200.plan";
@@ -381,7 +384,7 @@ PyObject* make_plan(PyObject*, PyObject* args) {
   plan->paths = Ref::borrow(paths);
   plan->membership = Ref::borrow(membership);
   plan->resolve = Ref::borrow(resolve);
-  plan->p.resize(plan->n); plan->g.resize(plan->n); plan->last.assign(plan->n, nullptr);
+  plan->p.resize(plan->n); plan->g.resize(plan->n);
   plan->s.assign(plan->n_states, std::vector<PyObject*>(plan->n));
   for (Call& c : plan->calls) {  // moved into place: the tables' addresses are final now
     c.desc.n_leaves = (uint32_t)c.leaves.size();
@@ -456,6 +459,14 @@ bool fill_leaf(Plan& plan, const LeafSpec& l, int i) {
   return true;
 }
 
+// are the parameters (checked by fill_leaf) the very tensors of the last step?
+bool same_params(const Plan& plan) {
+  if (plan.last.size() != plan.p.size()) return false;
+  for (int i = 0; i < plan.n; ++i)
+    if (plan.last[i]._unsafe_get_target() != THPVariable_Unpack(plan.p[i]).unsafeGetTensorImpl()) return false;
+  return true;
+}
+
 // run(plan, params, count, states, grads, sq_norm address or 0, max_norm, whether the norm is the launch in front)
 //   -> None, or (params, states, count)
 PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -483,7 +494,8 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   for (int i = 0; i < plan->n; ++i)
     if (!fill_leaf(*plan, plan->leaves[i], i)) Py_RETURN_NONE;
   if (!groups_unchanged(*plan)) Py_RETURN_NONE;
-  if (plan->dynamic && (!plan->donate || plan->p != plan->last)) {  // ask the selectors again
+  const bool ask = plan->dynamic && !(plan->donate && same_params(*plan));
+  if (ask) {  // the selectors again
     for (int i = 0; i < plan->n; ++i) {
       Ref m(PyObject_CallFunctionObjArgs(plan->member.p, PyTuple_GET_ITEM(plan->paths.p, i), plan->p[i], nullptr));
       if (m.p == nullptr) return nullptr;
@@ -567,7 +579,10 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return true;
   });
   if (!launched) return nullptr;
-  plan->last = plan->p;
+  if (ask && plan->donate) {
+    plan->last.clear();
+    for (PyObject* p : plan->p) plan->last.emplace_back(THPVariable_Unpack(p).getIntrusivePtr());
+  }
 
   Ref count(host_int(old_count + 1));
   if (count.p == nullptr) return nullptr;

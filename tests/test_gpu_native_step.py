@@ -108,6 +108,30 @@ def test_edited_groups_and_selectors_are_honoured():
     assert not torch.equal(r2["x"], r["x"]) and int(s.count) == 6
 
 
+def test_selectors_see_every_new_tensor():
+    """Donated steps leave out the selectors only while the very same tensors come back, not tensors at a freed one's address."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    asked = []
+    tx = fo.flash_sgd(learning_rate=1e-2, donate=True, param_groups=[{"params": lambda path, leaf: asked.append(path) or False, "weight_decay": 0.0}])
+    p = {"w": torch.ones(64, device="cuda", dtype=torch.bfloat16)}
+    s, g = tx.init(p), {"w": torch.ones(64, device="cuda", dtype=torch.bfloat16)}
+    for _ in range(3):
+        p, s = tx.step(p, s, g)
+    asked.clear()
+    p, s = tx.step(p, s, g)
+    assert not asked
+    for _ in range(8):
+        host = p["w"].cpu()
+        del p["w"]  # the next tensor may get its address
+        p["w"] = host.cuda()
+        asked.clear()
+        p, s = tx.step(p, s, g)
+        assert asked
+
+
 def test_gradients_that_need_a_conversion():
     import torch
 
