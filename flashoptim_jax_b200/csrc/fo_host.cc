@@ -257,6 +257,7 @@ struct Call {
   std::vector<FoLeafOut> outs;
   std::vector<FoHyper> hypers;
   std::vector<int> slots;  // group of each hyper set
+  bool empty = true;       // no leaf has an element: nothing is launched
 };
 struct Watched {  // a param-group dict as it was when the plan was made
   Ref dict;
@@ -343,6 +344,7 @@ PyObject* make_plan(PyObject*, PyObject* args) {
     FoLeaf f;
     std::memset(&f, 0, sizeof(f));
     f.n = (uint64_t)l.n;
+    c.empty = c.empty && l.n == 0;
     f.hyper = (uint32_t)slot;
     c.leaves.push_back(f);
     c.outs.push_back(FoLeafOut{});
@@ -574,7 +576,7 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       c.desc.max_grad_norm = f32(max_norm);
       const FoStepMore more = {sizeof(FoStepMore), chain, plan->donate ? nullptr : c.outs.data()};
       if (!ok(api.step(&c.desc, &more, stream))) return false;
-      chain = FO_LAUNCH_CHAINED;
+      if (!c.empty) chain = FO_LAUNCH_CHAINED;  // (behind a call that launches nothing the stream holds what it held before)
     }
     return true;
   });

@@ -190,7 +190,7 @@ typedef struct FoStepMore {
   const FoLeafOut* outs;
 } FoStepMore;
 /* What the launch in front of this one on the stream is; the kernels then start before it has drained.
- * CHAINED: another fo_step* of the same pytree step (other leaves).  AFTER_NORM: the fo_sq_norm* call that forms
+ * CHAINED: another fo_step* of the same pytree step (other leaves), one that had elements to work on.  AFTER_NORM: the fo_sq_norm* call that forms
  * this step's grad_sq_norm (the kernels wait for its result). */
 #define FO_LAUNCH_CHAINED 1u
 #define FO_LAUNCH_AFTER_NORM 2u

@@ -132,6 +132,27 @@ def test_selectors_see_every_new_tensor():
         assert asked
 
 
+@pytest.mark.parametrize("donate", [False, True])
+def test_a_call_without_elements_in_front(donate):
+    """The launch table that comes first holds only leaves without elements; the clipped launches behind it still wait for the norm."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from flashoptim_jax_b200 import clipping
+
+    params = lambda: {"a": torch.ones(0, 3, device="cuda", dtype=torch.float16), "b": torch.ones(1 << 21, device="cuda"), "c": torch.ones(77, device="cuda", dtype=torch.bfloat16)}
+    tx = clipping.clip_by_global_norm(fo.flash_adamw(learning_rate=1e-2, donate=donate), 1.0)
+    ref = clipping.clip_by_global_norm(fo.flash_adamw(learning_rate=1e-2), 1.0)
+    p, q = params(), params()
+    s, t = tx.init(p), ref.init(q)
+    for k in range(4):
+        g = _grads(q, k)
+        p, s = tx.step(p, s, g)
+        with _general_path():
+            q, t = ref.step(q, t, g)
+        _same((p, tuple(s["opt"])), (q, tuple(t["opt"])))
+
+
 def test_gradients_that_need_a_conversion():
     import torch
 
