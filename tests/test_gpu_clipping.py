@@ -100,3 +100,23 @@ def test_wrapper_matches_reference_recipe_structure():
     for a, b in zip(tree.tree_leaves(new_state["opt"]), tree.tree_leaves(want_state)):
         assert torch.equal(torch.as_tensor(a), torch.as_tensor(b))
     assert int(new_state["opt"].count) == 1
+
+
+@pytest.mark.parametrize("dtype,chunk", [("bfloat16", 16384), ("float16", 16384), ("float32", 8192)])
+def test_sum_of_squares_at_the_edges_of_its_chunks(dtype, chunk):
+    """Sizes around the sweep's chunks (64 KB), aligned or not, alone and in one table.  Bound: eight squares are added in fp32
+    (8 roundings of 2^-24 each, all terms positive), everything beyond in fp64."""
+    import torch
+
+    from flashoptim_jax_b200 import clipping
+
+    g = torch.Generator(device="cuda").manual_seed(7)
+    sizes = (1, 7, 8, 9, chunk - 8, chunk - 1, chunk, chunk + 1, 2 * chunk, 700 * chunk + 13)
+    arrays = []
+    for n in sizes:
+        x = (torch.randn(n + 1, device="cuda", generator=g) * 1e-2).to(getattr(torch, dtype))
+        arrays += [x[1:], x[:n].clone()]
+    want = [float((a.double() ** 2).sum()) for a in arrays]
+    for a, w in zip(arrays, want):
+        assert abs(float(clipping.global_sq_norm({"a": a})) - w) <= 8 * 2.0**-24 * w
+    assert abs(float(clipping.global_sq_norm(arrays)) - sum(want)) <= 8 * 2.0**-24 * sum(want)
