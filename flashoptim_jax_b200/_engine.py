@@ -87,15 +87,14 @@ _clip = threading.local()
 
 
 @contextlib.contextmanager
-def grad_clip(sq_norm: torch.Tensor, max_norm: float, fresh: bool = False):
+def grad_clip(sq_norm: torch.Tensor, max_norm: float):
     """While active, every launch rescales its gradients as optax.clip_by_global_norm does
     (examples/train_gpt2_pretrain.py:56-70): `sq_norm` is a one-element float64 device tensor with the
-    sum of squares of all gradients of the step (see sq_norm_of).  `fresh`: the launch that forms it is the last thing
-    on the stream, so that the step's first launch may be chained to it."""
+    sum of squares of all gradients of the step (see sq_norm_of)."""
     if sq_norm.dtype != torch.float64 or sq_norm.numel() != 1 or not sq_norm.is_cuda:
         raise ValueError("sq_norm must be a one-element float64 CUDA tensor")
     previous = getattr(_clip, "value", None)
-    _clip.value = (sq_norm, float(max_norm), bool(fresh))
+    _clip.value = (sq_norm, float(max_norm))
     try:
         yield
     finally:
@@ -325,9 +324,9 @@ class NativeStep:
         if not self.plans or _observer is not None:
             return None
         clip = getattr(_clip, "value", None)
-        sq, max_norm, chained = (0, 0.0, False) if clip is None else (clip[0].data_ptr(), clip[1], clip[2])
+        sq, max_norm = (0, 0.0) if clip is None else (clip[0].data_ptr(), clip[1])
         for i, (host_run, plan) in enumerate(self.plans):
-            hit = host_run(plan, params, count, states, grads, sq, max_norm, chained)
+            hit = host_run(plan, params, count, states, grads, sq, max_norm)
             if hit is not None:
                 if i:
                     self.plans.insert(0, self.plans.pop(i))

@@ -38,7 +38,7 @@ def clip_by_global_norm(tx: FlashOptimizer, max_norm: float) -> FlashOptimizer:
 
     def step_fn(params: Any, state: Any, grads: Any):
         sq = global_sq_norm(grads)
-        with eng.grad_clip(sq, max_norm, fresh=True):
+        with eng.grad_clip(sq, max_norm):
             params, opt_state = tx.step(params, state["opt"], grads)
         return params, {"clip": (), "opt": opt_state}
 

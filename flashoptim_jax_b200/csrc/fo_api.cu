@@ -210,8 +210,10 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
   if (hs.sm_count <= 0) return fail(FO_ERR_CUDA, "fo_step: cannot query the current device");
   hs.sq_norm = d->grad_sq_norm; hs.max_norm = d->max_grad_norm;
   hs.peers = &peers;
-  bool chained = more != nullptr && (more->launch_flags & (FO_LAUNCH_CHAINED | FO_LAUNCH_AFTER_NORM)) != 0;
-  hs.after_norm = more != nullptr && (more->launch_flags & FO_LAUNCH_AFTER_NORM) != 0;
+  // Launches that touch peers' memory start in stream order, behind the exchange in front of them.
+  const bool same_step = more != nullptr && (more->launch_flags & FO_LAUNCH_CHAINED) != 0;
+  bool chained = same_step || !with_peers;
+  hs.wait = !same_step && !with_peers;
   const int most_leaves = (mode == kPlain || mode == kPeer) && !generic ? kMaxLeaves : kMaxLeavesFlex;
   const unsigned long long unit = generic ? generic_tile_elems(d->group_size) : kPieceElems;
   const unsigned long long kMaxBlocks = 0x7FFFFFFFull;

@@ -27,9 +27,11 @@ FO_DEVI void store8(float* p, const float (&v)[8]) {
 
 // Groups of 8 to 256 elements: 1 to 32 lanes.  (The maximum is taken over magnitude bits, so that a NaN survives.)
 template <bool VARIANCE>
-__global__ void __launch_bounds__(kCodecThreads) quantize_kernel(const float* __restrict__ x, void* __restrict__ values, __half* __restrict__ scales,
+__global__ void __launch_bounds__(kCodecThreads) quantize_kernel(const float* x, void* values, __half* scales,
                                                                  unsigned long long n, int gshift, int floor_mode, int aligned) {
   using namespace fast2;
+  chain_wait();
+  chain_release();
   const unsigned long long tiles = (n + kCodecTile - 1) / kCodecTile;
   const int lanes = 1 << (gshift - 3);
   for (unsigned long long t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -94,9 +96,9 @@ __global__ void __launch_bounds__(kCodecThreads) quantize_kernel(const float* __
 // Any other group size 1..1024: one block per tile of whole groups, group maxima through
 // shared-memory atomics on non-negative float bit patterns.
 template <bool VARIANCE>
-__global__ void __launch_bounds__(256) quantize_any_kernel(const float* __restrict__ x, void* __restrict__ values,
-                                                            __half* __restrict__ scales, unsigned long long n, int G,
-                                                            int floor_mode) {
+__global__ void __launch_bounds__(256) quantize_any_kernel(const float* x, void* values, __half* scales, unsigned long long n, int G, int floor_mode) {
+  chain_wait();
+  chain_release();
   __shared__ unsigned int smax[kGenericTile];
   const int groups_per_tile = max(1, kGenericTile / G);
   const int tile = groups_per_tile * G;
@@ -142,9 +144,11 @@ FO_DEVI float dequantize_one(unsigned int b, float sc) {
 
 // gshift >= 3: groups of 2^gshift, whole pieces lie in one group; else any group size G
 template <bool VARIANCE>
-__global__ void __launch_bounds__(kCodecThreads) dequantize_kernel(const void* __restrict__ values, const __half* __restrict__ scales,
-                                                                   float* __restrict__ out, unsigned long long n, int G, int gshift, int aligned) {
+__global__ void __launch_bounds__(kCodecThreads) dequantize_kernel(const void* values, const __half* scales, float* out, unsigned long long n, int G, int gshift,
+                                                                   int aligned) {
   using namespace fast2;
+  chain_wait();
+  chain_release();
   const unsigned long long tiles = (n + kCodecTile - 1) / kCodecTile;
   for (unsigned long long t = blockIdx.x; t < tiles; t += gridDim.x) {
     const unsigned long long i0 = t * kCodecTile + threadIdx.x * kPiece;
@@ -183,6 +187,8 @@ struct SplitParams {
 
 template <int PDT, int ECC_BITS>
 __global__ void __launch_bounds__(kCodecThreads) split_kernel(const __grid_constant__ SplitParams p) {
+  chain_wait();
+  chain_release();
   const uint32_t total = p.first_tile[p.n_leaves];
   for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const int l = leaf_of(p.first_tile, p.n_leaves, t);
@@ -229,6 +235,8 @@ __global__ void __launch_bounds__(kCodecThreads) split_kernel(const __grid_const
 
 template <int PDT, int ECC_BITS>
 __global__ void __launch_bounds__(kCodecThreads) reconstruct_kernel(const __grid_constant__ SplitParams p) {
+  chain_wait();
+  chain_release();
   const uint32_t total = p.first_tile[p.n_leaves];
   for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
     const int l = leaf_of(p.first_tile, p.n_leaves, t);
@@ -294,8 +302,12 @@ static int small_group_shift(int G) {
   return 0;
 }
 
-static int check_launch(const char* what) {
-  cudaError_t e = cudaGetLastError();
+// The kernels of this file begin with chain_wait().  (Their pointers are not __restrict__: loads through the read-only
+// path may be moved in front of it.)
+template <typename... P, typename... A>
+static int launch_codec(const char* what, void (*kernel)(P...), unsigned int grid, void* stream, const A&... args) {
+  bool chained = true;
+  const cudaError_t e = launch_chained<P...>(kernel, grid, (unsigned int)kCodecThreads, 0, chained, (cudaStream_t)stream, static_cast<P>(args)...);
   if (e != cudaSuccess) return fail(FO_ERR_CUDA, "%s: launch failed: %s", what, cudaGetErrorString(e));
   return FO_OK;
 }
@@ -309,14 +321,12 @@ static int quantize_entry(const float* x, void* values, void* scales, uint64_t n
   if (G > kGenericTile) return fail(FO_ERR_UNSUPPORTED, "%s: group_size %d > %d", what, G, kGenericTile);
   if (const int gshift = small_group_shift(G)) {
     const int aligned = aligned_to(x, 32) && aligned_to(values, 8);
-    quantize_kernel<VARIANCE><<<tile_grid((n + kCodecTile - 1) / kCodecTile), kCodecThreads, 0, (cudaStream_t)stream>>>(x, values, (__half*)scales, n, gshift, floor_mode, aligned);
-    return check_launch(what);
+    return launch_codec(what, quantize_kernel<VARIANCE>, tile_grid((n + kCodecTile - 1) / kCodecTile), stream, x, values, (__half*)scales, n, gshift, floor_mode, aligned);
   }
   const unsigned long long tile = (unsigned long long)(kGenericTile / G) * G;
   const unsigned long long blocks = (n + tile - 1) / tile;
   if (blocks > 0x7FFFFFFFull) return fail(FO_ERR_TOO_LARGE, "%s: %llu elements exceed one launch", what, (unsigned long long)n);
-  quantize_any_kernel<VARIANCE><<<(unsigned int)blocks, kCodecThreads, 0, (cudaStream_t)stream>>>(x, values, (__half*)scales, n, G, floor_mode);
-  return check_launch(what);
+  return launch_codec(what, quantize_any_kernel<VARIANCE>, (unsigned int)blocks, stream, x, values, (__half*)scales, n, G, floor_mode);
 }
 
 template <bool VARIANCE>
@@ -326,8 +336,7 @@ static int dequantize_entry(const void* values, const void* scales, float* out, 
   if (values == nullptr || scales == nullptr || out == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: null pointer", what);
   if (G < 1) return fail(FO_ERR_INVALID_ARG, "%s: group_size %d", what, G);
   const int aligned = aligned_to(out, 32) && aligned_to(values, 8);
-  dequantize_kernel<VARIANCE><<<tile_grid((n + kCodecTile - 1) / kCodecTile), kCodecThreads, 0, (cudaStream_t)stream>>>(values, (const __half*)scales, out, n, G, small_group_shift(G), aligned);
-  return check_launch(what);
+  return launch_codec(what, dequantize_kernel<VARIANCE>, tile_grid((n + kCodecTile - 1) / kCodecTile), stream, values, (const __half*)scales, out, n, G, small_group_shift(G), aligned);
 }
 
 using SplitKernel = void (*)(const SplitParams);
@@ -347,8 +356,7 @@ static int split_entry(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t pdt
     if (more > 0x7FFFFFFFull) return fail(FO_ERR_TOO_LARGE, "%s: leaf %u with %llu elements exceeds one launch", what, i, (unsigned long long)leaves[i].n);
     if (p.n_leaves > 0 && (i == n_leaves || p.n_leaves == kSplitLeaves || tiles + more > 0x7FFFFFFFull)) {
       p.first_tile[p.n_leaves] = (uint32_t)tiles;
-      kernel<<<tile_grid(tiles), kCodecThreads, 0, (cudaStream_t)stream>>>(p);
-      if (int rc = check_launch(what)) return rc;
+      if (int rc = launch_codec(what, kernel, tile_grid(tiles), stream, p)) return rc;
       p.n_leaves = 0;
       tiles = 0;
     }

@@ -469,10 +469,10 @@ bool same_params(const Plan& plan) {
   return true;
 }
 
-// run(plan, params, count, states, grads, sq_norm address or 0, max_norm, whether the norm is the launch in front)
+// run(plan, params, count, states, grads, sq_norm address or 0, max_norm)
 //   -> None, or (params, states, count)
 PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
-  if (nargs != 8) { PyErr_SetString(PyExc_TypeError, "run takes 8 arguments"); return nullptr; }
+  if (nargs != 7) { PyErr_SetString(PyExc_TypeError, "run takes 7 arguments"); return nullptr; }
   Plan* plan = (Plan*)PyCapsule_GetPointer(a[0], kPlanName);
   if (plan == nullptr) return nullptr;
   if (plan->busy) Py_RETURN_NONE;  // the tables are in use (another thread, or a step inside a callback)
@@ -567,7 +567,7 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   void* const sq = PyLong_AsVoidPtr(a[5]);
   const double max_norm = PyFloat_AsDouble(a[6]);
-  uint32_t chain = a[7] == Py_True ? FO_LAUNCH_AFTER_NORM : 0u;
+  uint32_t chain = 0u;
   if (PyErr_Occurred()) return nullptr;
   const bool launched = on_device(plan->device, [&](cudaStream_t stream) {
     for (Call& c : plan->calls) {

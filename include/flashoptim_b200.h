@@ -189,11 +189,9 @@ typedef struct FoStepMore {
    * Not together with peers. */
   const FoLeafOut* outs;
 } FoStepMore;
-/* What the launch in front of this one on the stream is; the kernels then start before it has drained.
- * CHAINED: another fo_step* of the same pytree step (other leaves), one that had elements to work on.  AFTER_NORM: the fo_sq_norm* call that forms
- * this step's grad_sq_norm (the kernels wait for its result). */
+/* CHAINED: the launch in front of this one on the stream is another fo_step* of the same pytree step (other leaves), one
+ * that had elements to work on; the kernels then do not wait for it. */
 #define FO_LAUNCH_CHAINED 1u
-#define FO_LAUNCH_AFTER_NORM 2u
 int fo_step_ex(const FoStepDesc* desc, const FoStepMore* more, void* cuda_stream);
 
 /* Per-step scalars formed on the device, so that a whole step can be captured in a CUDA graph
