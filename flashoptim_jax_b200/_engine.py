@@ -11,7 +11,9 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import functools
 import threading
+import types
 from typing import Any, Dict, List, NamedTuple, Optional, Tuple
 
 import numpy as np
@@ -25,6 +27,7 @@ from .utils import (
     GroupResolver,
     _group_config_for_path,
     _is_quantized_leaf,
+    _path_matches,
     _resolve_learning_rate,
     _tree_leaves_with_paths,
     _use_ecc_leaf,
@@ -300,6 +303,10 @@ def _static_selector(spec: Any) -> bool:
     return type(spec) is list and all(isinstance(x, (str, tuple)) for x in spec)
 
 
+def _spec_matches(spec: Any, path: Tuple[Any, ...], leaf: Any) -> bool:
+    return _path_matches(path, leaf, spec)
+
+
 class NativeStep:
     """tx.step without the per-leaf Python work: the general path runs once per kind of pytree (structure, shapes, dtypes,
     param-group membership) and leaves a compiled plan behind (csrc/fo_host.cc); a later call that fits it is one native call
@@ -307,9 +314,8 @@ class NativeStep:
     its operands, and launches.  Anything else (other dtypes, non-contiguous tensors, edited param groups, tensor subclasses, a
     launch observer) takes the general path.
 
-    Selectors that are functions are asked again whenever the parameters are not the very tensors of the last step,
-    which with donated buffers they are: a selector that reads a leaf's *values* is not re-evaluated while
-    the same tensors come back."""
+    Selectors that are functions are asked at every step, as the general path asks them: an answer may depend on anything (the
+    leaf's values, a set of frozen names, the epoch)."""
 
     MOST_PLANS = 4
 
@@ -375,12 +381,18 @@ class NativeStep:
         param_groups = self.param_groups
         watched = tuple(param_groups or ())
         member = GroupResolver(self.defaults, param_groups).member
+        selectors = []
+        for g in watched:
+            spec = g["params"]
+            if _static_selector(spec):
+                selectors.append(tuple(_path_matches(path, leaf, spec) for path, leaf in path_leaves))
+            else:  # a function is called as it is
+                selectors.append(spec if isinstance(spec, types.FunctionType) else functools.partial(_spec_matches, spec))
         host = _lib.host()
         plan = host.make_plan(
             self.opt, self.donate, work[0].bucket[0], params, n_states, tuple(leaves), tuple(hypers),
             tuple((*bucket[1:5], bucket[5], tuple(slots)) for bucket, slots in calls), param_groups, watched,
-            not all(_static_selector(g["params"]) for g in watched), member, tuple(path for path, _ in path_leaves),
-            tuple(member(path, leaf) for path, leaf in path_leaves), _resolve_learning_rate)
+            tuple(selectors), tuple(path for path, _ in path_leaves), tuple(member(path, leaf) for path, leaf in path_leaves), _resolve_learning_rate)
         if plan is not None:
             self.plans.insert(0, (host.run, plan))
             del self.plans[self.MOST_PLANS:]

@@ -274,14 +274,12 @@ struct Plan {
   std::vector<Call> calls;
   Ref param_groups;
   std::vector<Watched> watched;
-  bool dynamic = false;            // a selector that has to be asked again (a callable)
-  Ref member, paths, membership;   // member(path, leaf) -> index of the first matching group or -1; tuples
+  bool dynamic = false;            // a selector that has to be asked at every step (a callable)
+  Ref selectors, paths;            // per group: selector(path, leaf), or a tuple with its answer for every leaf; the leaves' paths
+  std::vector<int> membership;     // of each leaf: the first group that takes it, or -1
   Ref resolve;                     // learning rate of a schedule: resolve(lr, count tensor)
   bool busy = false;               // a selector or a schedule may run Python code, and that another step
   std::vector<PyObject*> p, g;     // scratch (borrowed)
-  // parameters of the last step.  A weak reference keeps no data alive, but its address is not given to another tensor while
-  // it is held: an equal address is the same tensor
-  std::vector<c10::weak_intrusive_ptr<at::TensorImpl>> last;
   std::vector<std::vector<PyObject*>> s;
 };
 constexpr const char* kPlanName = "flashoptim_b200.plan";
@@ -293,19 +291,18 @@ bool num(PyObject* t, Py_ssize_t i, double& out) {
   return !(out == -1.0 && PyErr_Occurred());
 }
 
-// make_plan(opt, donate, device, params, n_states, leaves, groups, calls, param_groups, watched, dynamic, member, paths, membership, resolve)
+// make_plan(opt, donate, device, params, n_states, leaves, groups, calls, param_groups, watched, selectors, paths, membership, resolve)
 //   leaves: tuples (shape, param dtype code, grad dtype code, ecc bits, state, group size, group, call, position)
 //   groups: tuples (lr, weight decay, b1, b2, 1 - b1, 1 - b2, eps, flags)
 //   calls:  tuples (param dtype code, grad dtype code, ecc bits, state, group size, (group of each hyper set))
 PyObject* make_plan(PyObject*, PyObject* args) {
-  PyObject *params, *leaves, *groups, *calls, *param_groups, *watched, *member, *paths, *membership, *resolve;
+  PyObject *params, *leaves, *groups, *calls, *param_groups, *watched, *selectors, *paths, *membership, *resolve;
   auto plan = std::make_unique<Plan>();
-  int donate, dynamic;
-  if (!PyArg_ParseTuple(args, "ipiOiO!O!O!OO!pOO!O!O", &plan->opt, &donate, &plan->device, &params, &plan->n_states, &PyTuple_Type, &leaves, &PyTuple_Type, &groups,
-                        &PyTuple_Type, &calls, &param_groups, &PyTuple_Type, &watched, &dynamic, &member, &PyTuple_Type, &paths, &PyTuple_Type, &membership, &resolve))
+  int donate;
+  if (!PyArg_ParseTuple(args, "ipiOiO!O!O!OO!O!O!O!O", &plan->opt, &donate, &plan->device, &params, &plan->n_states, &PyTuple_Type, &leaves, &PyTuple_Type, &groups,
+                        &PyTuple_Type, &calls, &param_groups, &PyTuple_Type, &watched, &PyTuple_Type, &selectors, &PyTuple_Type, &paths, &PyTuple_Type, &membership, &resolve))
     return nullptr;
   plan->donate = donate != 0;
-  plan->dynamic = dynamic != 0;
   if (!compile(params, plan->tree, plan->n)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
@@ -382,9 +379,16 @@ PyObject* make_plan(PyObject*, PyObject* args) {
   }
   if (PyErr_Occurred()) return nullptr;
   plan->param_groups = Ref::borrow(param_groups);
-  plan->member = Ref::borrow(member);
+  if (PyTuple_GET_SIZE(paths) != plan->n || PyTuple_GET_SIZE(membership) != plan->n || PyTuple_GET_SIZE(selectors) != (Py_ssize_t)plan->watched.size()) Py_RETURN_NONE;
+  for (Py_ssize_t k = 0; k < PyTuple_GET_SIZE(selectors); ++k) {
+    PyObject* sel = PyTuple_GET_ITEM(selectors, k);
+    if (!PyTuple_CheckExact(sel)) plan->dynamic = true;
+    else if (PyTuple_GET_SIZE(sel) != plan->n) Py_RETURN_NONE;
+  }
+  for (int i = 0; i < plan->n; ++i) plan->membership.push_back((int)PyLong_AsLong(PyTuple_GET_ITEM(membership, i)));
+  if (PyErr_Occurred()) return nullptr;
+  plan->selectors = Ref::borrow(selectors);
   plan->paths = Ref::borrow(paths);
-  plan->membership = Ref::borrow(membership);
   plan->resolve = Ref::borrow(resolve);
   plan->p.resize(plan->n); plan->g.resize(plan->n);
   plan->s.assign(plan->n_states, std::vector<PyObject*>(plan->n));
@@ -461,12 +465,27 @@ bool fill_leaf(Plan& plan, const LeafSpec& l, int i) {
   return true;
 }
 
-// are the parameters (checked by fill_leaf) the very tensors of the last step?
-bool same_params(const Plan& plan) {
-  if (plan.last.size() != plan.p.size()) return false;
-  for (int i = 0; i < plan.n; ++i)
-    if (plan.last[i]._unsafe_get_target() != THPVariable_Unpack(plan.p[i]).unsafeGetTensorImpl()) return false;
-  return true;
+// Is every leaf in the group it was in when the plan was made?  1, 0, or -1 with an exception set.  Selectors that are
+// functions are called, as the general path calls them: what they answer may depend on more than the leaf.
+int membership_unchanged(const Plan& plan) {
+  const Py_ssize_t groups = PyTuple_GET_SIZE(plan.selectors.p);
+  for (int i = 0; i < plan.n; ++i) {
+    int index = -1;
+    for (Py_ssize_t k = 0; k < groups && index < 0; ++k) {
+      PyObject* sel = PyTuple_GET_ITEM(plan.selectors.p, k);
+      if (PyTuple_CheckExact(sel)) {
+        if (PyTuple_GET_ITEM(sel, i) == Py_True) index = (int)k;
+        continue;
+      }
+      PyObject* const a[2] = {PyTuple_GET_ITEM(plan.paths.p, i), plan.p[i]};
+      Ref answer(PyObject_Vectorcall(sel, a, 2, nullptr));
+      const int yes = answer.p == nullptr ? -1 : PyObject_IsTrue(answer.p);
+      if (yes < 0) return -1;
+      if (yes) index = (int)k;
+    }
+    if (index != plan.membership[i]) return 0;
+  }
+  return 1;
 }
 
 // run(plan, params, count, states, grads, sq_norm address or 0, max_norm)
@@ -496,15 +515,10 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   for (int i = 0; i < plan->n; ++i)
     if (!fill_leaf(*plan, plan->leaves[i], i)) Py_RETURN_NONE;
   if (!groups_unchanged(*plan)) Py_RETURN_NONE;
-  const bool ask = plan->dynamic && !(plan->donate && same_params(*plan));
-  if (ask) {  // the selectors again
-    for (int i = 0; i < plan->n; ++i) {
-      Ref m(PyObject_CallFunctionObjArgs(plan->member.p, PyTuple_GET_ITEM(plan->paths.p, i), plan->p[i], nullptr));
-      if (m.p == nullptr) return nullptr;
-      const int same = PyObject_RichCompareBool(m.p, PyTuple_GET_ITEM(plan->membership.p, i), Py_EQ);
-      if (same < 0) return nullptr;
-      if (same == 0) Py_RETURN_NONE;
-    }
+  if (plan->dynamic) {
+    const int same = membership_unchanged(*plan);
+    if (same < 0) return nullptr;
+    if (same == 0) Py_RETURN_NONE;
   }
   const int32_t old_count = *count_t->const_data_ptr<int32_t>();
   const double step = (double)old_count + 1.0;
@@ -581,10 +595,6 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     return true;
   });
   if (!launched) return nullptr;
-  if (ask && plan->donate) {
-    plan->last.clear();
-    for (PyObject* p : plan->p) plan->last.emplace_back(THPVariable_Unpack(p).getIntrusivePtr());
-  }
 
   Ref count(host_int(old_count + 1));
   if (count.p == nullptr) return nullptr;
