@@ -66,6 +66,9 @@ FO_DEVI int log_half_ulp(uint32_t bits) {
 // ===========================================================================================
 namespace ieee {
 
+// x limited to [lo, hi]; a NaN stays one, and its code is 0, as XLA converts it
+FO_DEVI float clamp(float x, float lo, float hi) { return x < lo ? lo : (x > hi ? hi : x); }
+
 // flashoptim_jax/quantization.py:49-56 without the scale: (q/127) / (2 - |q/127|)
 FO_DEVI float deq_m_norm(int q) {
   float t = fdiv((float)q, 127.0f);
@@ -88,7 +91,7 @@ FO_DEVI void split(float theta, uint32_t& bits, int& ecc) {
   bits = Lp<PDT>::from_f32(theta);
   float err = fsub(theta, Lp<PDT>::to_f32(bits));
   float en = ldexpf(err, -log_half_ulp<PDT>(bits));
-  float c = fminf(fmaxf(en, -1.0f), 1.0f);
+  float c = clamp(en, -1.0f, 1.0f);
   float s = fmul(c, Ecc<ECC_BITS>::MAX);
   float r = floorf(fadd(fabsf(s), 0.5f));
   ecc = s > 0.0f ? (int)r : (s < 0.0f ? -(int)r : 0);
@@ -103,13 +106,13 @@ FO_DEVI int quant_m(float x, float safe) {
   float n = fdiv(x, safe);
   float t = fdiv(fmul(2.0f, n), fadd(1.0f, fabsf(n)));
   float q = floorf(fadd(fmul(t, 127.0f), 0.5f));
-  return (int)fminf(fmaxf(q, -127.0f), 127.0f);
+  return (int)clamp(q, -127.0f, 127.0f);
 }
 // flashoptim_jax/quantization.py:65-67 (root = sqrt(nu) already taken)
 FO_DEVI int quant_v(float root, float safe) {
   float t = fdiv(root, safe);
   float q = floorf(fadd(fmul(t, 255.0f), 0.5f));
-  return (int)fminf(fmaxf(q, 0.0f), 255.0f);
+  return (int)clamp(q, 0.0f, 255.0f);
 }
 
 }  // namespace ieee
@@ -194,7 +197,7 @@ FO_DEVI void split(float theta, uint32_t& bits, int& ecc) {
     // |theta| < 2^-118 (bf16 only): 2^(-ls) overflows a float, scale in two exact steps
     en = fmul(fmul(err, __uint_as_float(254u << 23)), __uint_as_float((uint32_t)(field - 127) << 23));
   }
-  float c = fminf(fmaxf(en, -1.0f), 1.0f);
+  float c = ieee::clamp(en, -1.0f, 1.0f);
   ecc = round_half_away(fmul(c, Ecc<ECC_BITS>::MAX));
 }
 

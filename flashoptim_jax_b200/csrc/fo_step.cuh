@@ -501,15 +501,38 @@ FO_DEVI uint32_t pack2(float lo, float hi) {
   }
 }
 
+// 2- and 3-input min / max (one instruction each on sm_100).  KEEP: a NaN among the operands is the result; otherwise it is left out.
+template <bool KEEP>
+FO_DEVI float max2(float a, float b) {
+  if constexpr (!KEEP) return fmaxf(a, b);
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+template <bool KEEP>
+FO_DEVI float min3(float a, float b, float c) {
+  float d;
+  if constexpr (KEEP) asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  else asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+template <bool KEEP>
+FO_DEVI float max3(float a, float b, float c) {
+  float d;
+  if constexpr (KEEP) asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  else asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // maximum over the lanes that share a quantization group: four for groups of 32, 2^(gshift - 3) in general
 template <bool ANY>
-FO_DEVI float group_max(float a, const int gshift) {
+FO_DEVI float group_max(float a, const int gshift, const bool keep_nan) {
+  auto larger = [&](float b) { return keep_nan ? max2<true>(a, b) : max2<false>(a, b); };
   if constexpr (ANY) {
-    for (int o = 1; o < (1 << (gshift - 3)); o <<= 1) a = fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, o));
+    for (int o = 1; o < (1 << (gshift - 3)); o <<= 1) a = larger(__shfl_xor_sync(0xFFFFFFFFu, a, o));
     return a;
   }
-  a = fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, 1));
-  return fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, 2));
+  a = larger(__shfl_xor_sync(0xFFFFFFFFu, a, 1));
+  return larger(__shfl_xor_sync(0xFFFFFFFFu, a, 2));
 }
 // low bytes of four words -> one word
 FO_DEVI uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -517,17 +540,6 @@ FO_DEVI uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
 }
 FO_DEVI uint32_t pack_halves(uint32_t lo, uint32_t hi) { return __byte_perm(lo, hi, 0x5410); }
 
-// 3-input min / max (one instruction on sm_100)
-FO_DEVI float min3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-FO_DEVI float max3(float a, float b, float c) {
-  float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
 // Per-lane repairs of the second-chance path (REPAIR = true below), kept out of line: they run only
 // for lanes that hold a value outside the range a shortcut is proven for (zeros, subnormals, huge
 // values) and redo that stage with IEEE operations.
@@ -757,19 +769,23 @@ FO_DEVI void pairs_of16(const uint4& w, float2 (&o)[4]) {
   unpack2<DT>(w.x, o[0].x, o[0].y); unpack2<DT>(w.y, o[1].x, o[1].y);
   unpack2<DT>(w.z, o[2].x, o[2].y); unpack2<DT>(w.w, o[3].x, o[3].y);
 }
+// Minima and maxima of a piece.  The range checks keep a NaN (the default): an infinity turns into a NaN in the packed
+// square root and divisions, and a NaN that a minimum leaves out would let the piece pass.
+template <bool KEEP = true>
 FO_DEVI float min8(const float2 (&x)[4]) {
-  return min3(min3(x[0].x, x[0].y, x[1].x), min3(x[1].y, x[2].x, x[2].y), fminf(x[3].x, x[3].y));
+  return min3<KEEP>(min3<KEEP>(x[0].x, x[0].y, x[1].x), min3<KEEP>(x[1].y, x[2].x, x[2].y), -max2<KEEP>(-x[3].x, -x[3].y));
 }
 FO_DEVI float max8(const float2 (&x)[4]) {
-  return max3(max3(x[0].x, x[0].y, x[1].x), max3(x[1].y, x[2].x, x[2].y), fmaxf(x[3].x, x[3].y));
+  return max3<true>(max3<true>(x[0].x, x[0].y, x[1].x), max3<true>(x[1].y, x[2].x, x[2].y), max2<true>(x[3].x, x[3].y));
 }
 FO_DEVI float minabs8(const float2 (&x)[4]) {
-  return min3(min3(fabsf(x[0].x), fabsf(x[0].y), fabsf(x[1].x)), min3(fabsf(x[1].y), fabsf(x[2].x), fabsf(x[2].y)),
-              fminf(fabsf(x[3].x), fabsf(x[3].y)));
+  return min3<true>(min3<true>(fabsf(x[0].x), fabsf(x[0].y), fabsf(x[1].x)), min3<true>(fabsf(x[1].y), fabsf(x[2].x), fabsf(x[2].y)),
+                    -max2<true>(-fabsf(x[3].x), -fabsf(x[3].y)));
 }
+template <bool KEEP = true>
 FO_DEVI float maxabs8(const float2 (&x)[4]) {
-  return max3(max3(fabsf(x[0].x), fabsf(x[0].y), fabsf(x[1].x)), max3(fabsf(x[1].y), fabsf(x[2].x), fabsf(x[2].y)),
-              fmaxf(fabsf(x[3].x), fabsf(x[3].y)));
+  return max3<KEEP>(max3<KEEP>(fabsf(x[0].x), fabsf(x[0].y), fabsf(x[1].x)), max3<KEEP>(fabsf(x[1].y), fabsf(x[2].x), fabsf(x[2].y)),
+                   max2<KEEP>(fabsf(x[3].x), fabsf(x[3].y)));
 }
 // byte k of a word as an index
 FO_DEVI uint32_t byte_of(uint32_t w, int k) { return __byte_perm(w, 0u, 0x4440u | (uint32_t)k); }
@@ -869,17 +885,19 @@ FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, 
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         theta[k] = reconstruct_ordinary2<PDT, ECC_BITS>(old_lp[k], mk(ef[2 * k], ef[2 * k + 1]));
-      if constexpr (PDT == FO_BF16) {
-        // a value too small for the exponent-field shortcut (zero included)
-        if (!(minabs8(old_lp) >= fast::Ordinary<PDT>::kMin)) {
-          rare = true;
-          if constexpr (REPAIR) {
-            const uint32_t w[4] = {p0.x, p0.y, p0.z, p0.w};
+      // a value too small for the exponent-field shortcut (zero included), or an infinity or NaN, which has no exponent to take (in
+      // the first pass it leaves a theta that is not finite either, and stored_form sees that)
+      bool odd = false;
+      if constexpr (PDT == FO_BF16) odd = !(minabs8(old_lp) >= fast::Ordinary<PDT>::kMin);
+      if constexpr (REPAIR) odd = odd || !(maxabs8(old_lp) <= 3.4e38f);
+      if (odd) {
+        rare = true;
+        if constexpr (REPAIR) {
+          const uint32_t w[4] = {p0.x, p0.y, p0.z, p0.w};
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              theta[k].x = repair_master<PDT, ECC_BITS>(w[k] & 0xFFFFu, e[2 * k]);
-              theta[k].y = repair_master<PDT, ECC_BITS>(w[k] >> 16, e[2 * k + 1]);
-            }
+          for (int k = 0; k < 4; ++k) {
+            theta[k].x = repair_master<PDT, ECC_BITS>(w[k] & 0xFFFFu, e[2 * k]);
+            theta[k].y = repair_master<PDT, ECC_BITS>(w[k] >> 16, e[2 * k + 1]);
           }
         }
       }
@@ -1255,7 +1273,7 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
     // (with quantized moments the largest square root is checked once per group below, after the
     // shuffles; the repairing pass needs the answer per lane)
     bool wild = !(max8(nv) <= -1.0e-30f) || !(minabs8(m) >= h.m_lo) || !(am_lane <= h.m_hi);
-    if constexpr (REPAIR || STATE != FO_STATE_QUANT) wild = wild || !(av_lane <= 1.0737418e9f);
+    if constexpr (REPAIR || STATE != FO_STATE_QUANT) wild = wild || !(av_lane <= 1.0737418e9f);  // (an overflown second moment: NaN here)
     if (wild) {
       rare = true;
       if constexpr (REPAIR) {
@@ -1266,7 +1284,6 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
           tn[k].y = repair_adam(-nv[k].y, m[k].y, theta[k].y, h.lr_bc1, h.sqrt_bc2, h.eps, ry);
           nroot[k] = mk(-rx, -ry);
         }
-        av_lane = -min8(nroot);
       }
     }
 #pragma unroll
@@ -1329,12 +1346,21 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
   float am = 0.0f, av = 0.0f;
   if constexpr (STATE == FO_STATE_QUANT) {
     const bool floor_mode = (h.flags & FO_FLAG_SCALE_FLOOR) != 0;
-    am = group_max<(MODE & kGroup) != 0>(am_lane, c.group_shift);
+    // A NaN makes its group's scale NaN, except in groups of 32, whose scale is that of the elements that are none.  (The first pass keeps it:
+    // the warp is redone.)
+    const bool keep_nan = !REPAIR || ((MODE & kGroup) != 0 && c.group_shift != 5);
+    if constexpr (REPAIR) {
+      am_lane = keep_nan ? maxabs8(m) : maxabs8<false>(m);
+      if constexpr (OPT == FO_OPT_ADAM) av_lane = keep_nan ? -min8(nroot) : -min8<false>(nroot);
+    }
+    am = group_max<(MODE & kGroup) != 0>(am_lane, c.group_shift, keep_nan);
     uint32_t q[8];
     const float2 nam = sp(-am), rm2 = sp(fast::rcp_rn(am));
 #pragma unroll
     for (int k = 0; k < 4; ++k) softsign_code_bits2(div_by_rcp2(m[k], nam, rm2), q[2 * k], q[2 * k + 1]);
-    if (!(am >= 1.0e-12f && am <= 1.0e30f)) {  // all-zero group, or a scale outside the reciprocal's range
+    bool odd = !(am >= 1.0e-12f && am <= 1.0e30f);  // all-zero group, or a scale outside the reciprocal's range
+    if constexpr (REPAIR) odd = odd || !(maxabs8(m) <= 1.0e30f);  // (a NaN that is not in the scale)
+    if (odd) {
       rare = true;
       if constexpr (REPAIR) {
         const float safe = ieee::safe_scale(am, floor_mode);
@@ -1348,11 +1374,13 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
     mq.x = pack_bytes(q[0], q[1], q[2], q[3]);
     mq.y = pack_bytes(q[4], q[5], q[6], q[7]);
     if constexpr (OPT == FO_OPT_ADAM) {
-      av = group_max<(MODE & kGroup) != 0>(av_lane, c.group_shift);
+      av = group_max<(MODE & kGroup) != 0>(av_lane, c.group_shift, keep_nan);
       const float2 av2 = sp(av), nrv2 = sp(-fast::rcp_rn(av));
 #pragma unroll
       for (int k = 0; k < 4; ++k) quant_v_bits2(nroot[k], av2, nrv2, q[2 * k], q[2 * k + 1]);
-      if (!(av >= 1.0e-12f && av <= 1.0737418e9f)) {  // 2^30: also the limit of the packed Adam division
+      odd = !(av >= 1.0e-12f && av <= 1.0737418e9f);  // 2^30: also the limit of the packed Adam division
+      if constexpr (REPAIR) odd = odd || !(min8(nroot) >= -1.0737418e9f);
+      if (odd) {
         rare = true;
         if constexpr (REPAIR) {
           const float safe = ieee::safe_scale(av, floor_mode);

@@ -122,3 +122,68 @@ def test_many_leaves_need_several_tables():
     sizes = [int(x) for x in rng.integers(1, 9000, 500)]
     _run(C.ADAM, 1, 8, C.STATE_QUANT, 32, O.FUSED, sizes, steps=2)
     _run(C.ADAM, 1, 8, C.STATE_QUANT, 64, O.FUSED, sizes, steps=1, elsewhere=True)
+
+
+@pytest.mark.parametrize("n", [1000, MAIN + 700])
+@pytest.mark.parametrize("pdt,ecc_bits,state,group,conv", [
+    (1, 16, C.STATE_QUANT, 32, O.FUSED), (0, 0, C.STATE_QUANT, 128, O.FUSED), (2, 8, C.STATE_QUANT, 16, O.UNFUSED), (1, 8, C.STATE_QUANT, 64, O.FUSED),
+    (1, 8, C.STATE_FULL, 32, O.UNFUSED), (0, 0, C.STATE_FULL, 32, O.FUSED), (2, 16, C.STATE_FULL, 32, O.FUSED)])
+def test_squares_that_overflow(pdt, ecc_bits, state, group, conv, n):
+    """Gradients of 1e20: the second moment is an infinity and the update zero, for those elements alone."""
+    rng = np.random.default_rng(n)
+    ref = H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), C.ADAM, state, ecc_bits, group)
+    dev = ref.copy().to_device()
+    g = H.make_grad(rng, n, 1e-2, np.float32)
+    g[rng.integers(0, n, n // 100)] *= np.float32(1e22)
+    hp = H.hyper_tuple(C.ADAM, conv, 1, lr=1e-3, wd=1e-2)
+    H.oracle_step(C.ADAM, g, ref, state, group, hp)
+    _step(C.ADAM, [H.to_torch(g)], [dev], None, state, group, hp, pdt, 0, ecc_bits)
+    assert np.isfinite(ref.param.astype(np.float32)).all()
+    H.assert_leaf_equal(dev.to_host(), ref, f"n={n}")
+
+
+@pytest.mark.parametrize("n", [1000, MAIN + 700])
+@pytest.mark.parametrize("opt,pdt,ecc_bits,group", [(C.ADAM, 2, 8, 16), (C.ADAM, 1, 16, 32), (C.LION, 2, 16, 128), (C.LION, 1, 8, 64), (C.SGD, 2, 8, 32)])
+def test_parameters_that_are_infinite(opt, pdt, ecc_bits, group, n):
+    """An infinity (an fp16 weight that left its range) stays one, with a code of zero, and its neighbours are stepped."""
+    rng = np.random.default_rng(n)
+    p = rng.normal(0, 0.02, n).astype(np.float32)
+    p[rng.integers(0, n, n // 100)] = np.inf
+    p[rng.integers(0, n, n // 100)] = -np.inf
+    ref = H.fresh_leaf(p.astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, group)
+    ref.ecc[:] = rng.integers(-100, 100, n)
+    dev = ref.copy().to_device()
+    g = H.make_grad(rng, n, 1e-2, H.BF16)
+    hp = H.hyper_tuple(opt, O.FUSED, 1, lr=1e-3, wd=1e-2)
+    H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+    _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 1, ecc_bits)
+    H.assert_leaf_equal(dev.to_host(), ref, f"n={n}")
+
+
+@pytest.mark.parametrize("n", [1000, MAIN + 700])
+@pytest.mark.parametrize("opt,pdt,ecc_bits", [(C.ADAM, 1, 8), (C.ADAM, 2, 16), (C.LION, 1, 16), (C.SGD, 0, 0)])
+def test_gradients_that_are_nan(opt, pdt, ecc_bits, n):
+    """Their parameters become NaN and their codes 0; the scale of a group of 32 is that of its other elements, any other
+    group's scale is NaN."""
+    rng = np.random.default_rng(n)
+    for group in (32, 128):
+        ref = H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, group)
+        dev = ref.copy().to_device()
+        g = H.make_grad(rng, n, 1e-2, H.BF16)
+        at = rng.integers(0, n, n // 100)
+        g[at] = np.nan
+        hp = H.hyper_tuple(opt, O.FUSED, 1, lr=1e-3, wd=1e-2)
+        H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+        _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 1, ecc_bits)
+        got = dev.to_host()
+        assert np.isnan(got.param[at].astype(np.float32)).all() and np.isnan(ref.param[at].astype(np.float32)).all()
+        got.param[at] = ref.param[at]  # (whichever NaN it is)
+        if group != 32:
+            for name, codes in (("mu_scales", "mu"), ("nu_scales", "nu")):
+                if getattr(ref, name) is not None:
+                    hit = np.unique(at // group)
+                    assert np.isnan(getattr(got, name)[hit]).all()
+                    getattr(got, name)[hit] = getattr(ref, name)[hit]
+                    inside = np.isin(np.arange(n) // group, hit)
+                    getattr(got, codes)[inside] = getattr(ref, codes)[inside]  # of a group whose scale is NaN
+        H.assert_leaf_equal(got, ref, f"n={n} group={group}")
