@@ -142,17 +142,16 @@ FO_DEVI float dequantize_one(unsigned int b, float sc) {
   return fmul(__ldg(&kDeqM.v[b]), sc);
 }
 
-// gshift >= 3: groups of 2^gshift, whole pieces lie in one group; else any group size G
+// Groups of 2^gshift = 8 to 256 elements, aligned arrays: whole pieces lie in one group.
 template <bool VARIANCE>
-__global__ void __launch_bounds__(kCodecThreads) dequantize_kernel(const void* values, const __half* scales, float* out, unsigned long long n, int G, int gshift,
-                                                                   int aligned) {
+__global__ void __launch_bounds__(kCodecThreads) dequantize_kernel(const void* values, const __half* scales, float* out, unsigned long long n, int gshift) {
   using namespace fast2;
   chain_wait();
   chain_release();
   const unsigned long long tiles = (n + kCodecTile - 1) / kCodecTile;
   for (unsigned long long t = blockIdx.x; t < tiles; t += gridDim.x) {
     const unsigned long long i0 = t * kCodecTile + threadIdx.x * kPiece;
-    if (i0 + kPiece <= n && aligned && gshift >= 3) {
+    if (i0 + kPiece <= n) {
       const uint2 w = *(const uint2*)((const unsigned char*)values + i0);
       const uint32_t word[2] = {w.x, w.y};
       const f2 sc = sp(__half2float(scales[i0 >> gshift]));
@@ -171,22 +170,114 @@ __global__ void __launch_bounds__(kCodecThreads) dequantize_kernel(const void* v
       store8(out + i0, v);
     } else {
       for (int j = 0; j < 8; ++j)
-        if (i0 + j < n) out[i0 + j] = dequantize_one<VARIANCE>(((const unsigned char*)values)[i0 + j], __half2float(scales[(i0 + j) / G]));
+        if (i0 + j < n) out[i0 + j] = dequantize_one<VARIANCE>(((const unsigned char*)values)[i0 + j], __half2float(scales[(i0 + j) >> gshift]));
+    }
+  }
+}
+
+// Any other group size, and arrays that are not aligned: one element per thread at a time, neighbours side by side; a shift for
+// powers of two (gshift >= 0), else one wide division per tile and a narrow one per element.  A kernel of its own, so that the one above keeps its registers.  (Eight elements in a row per thread took twice
+// as long: 16.8 M elements in groups of 48 69 us, this 36; unaligned in groups of 32 69 and 21.)
+template <bool VARIANCE>
+__global__ void __launch_bounds__(kCodecThreads) dequantize_any_kernel(const void* values, const __half* scales, float* out, unsigned long long n, unsigned int G, int gshift) {
+  chain_wait();
+  chain_release();
+  const unsigned long long tiles = (n + kCodecTile - 1) / kCodecTile;
+  for (unsigned long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const unsigned long long base = t * kCodecTile, group = gshift >= 0 ? base >> gshift : base / G;
+    const uint32_t rest = (uint32_t)(base - group * G) + threadIdx.x;  // below 2^31 + 2^8: the group size is an int
+    unsigned int code[8];
+    float sc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const unsigned long long i = base + j * kCodecThreads + threadIdx.x;
+      if (i < n) {
+        code[j] = ((const unsigned char*)values)[i];
+        const uint32_t r = rest + j * kCodecThreads;
+        sc[j] = __half2float(scales[group + (gshift >= 0 ? r >> gshift : r / G)]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const unsigned long long i = base + j * kCodecThreads + threadIdx.x;
+      if (i < n) out[i] = dequantize_one<VARIANCE>(code[j], sc[j]);
     }
   }
 }
 
 // ---- fp32 <-> (16-bit parameter, ECC), a table of leaves per launch --------------------------------------------
-constexpr int kSplitLeaves = 256;
+// Two table sizes: a launch copies its whole parameter block (9.5 KB of the large one), which shows on a call for a leaf or two:
+// 100 000 elements 5.9 us with the large table, 4.2 with the small one.
+constexpr int kSplitLeavesSmall = 8, kSplitLeaves = 256;
+template <int N>
 struct SplitParams {
-  FoSplitLeaf leaf[kSplitLeaves];
-  uint32_t first_tile[kSplitLeaves + 1];
-  uint8_t aligned[kSplitLeaves];
+  FoSplitLeaf leaf[N];
+  uint32_t first_tile[N + 1];
   int32_t n_leaves;
 };
 
 template <int PDT, int ECC_BITS>
-__global__ void __launch_bounds__(kCodecThreads) split_kernel(const __grid_constant__ SplitParams p) {
+FO_DEVI void split_one(const FoSplitLeaf& L, const unsigned long long i, const float theta) {
+  uint32_t nb;
+  int e = 0;
+  if constexpr (ECC_BITS != 0) fast::split<PDT, ECC_BITS>(theta, nb, e);
+  else nb = Lp<PDT>::from_f32(theta);
+  ((unsigned short*)L.lp)[i] = (unsigned short)nb;
+  if constexpr (ECC_BITS == 16) ((short*)L.ecc)[i] = (short)e;
+  if constexpr (ECC_BITS == 8) ((signed char*)L.ecc)[i] = (signed char)e;
+}
+template <int PDT, int ECC_BITS>
+FO_DEVI float reconstruct_one(const uint32_t bits, const int e) {
+  if constexpr (ECC_BITS != 0) return fast::reconstruct<PDT, ECC_BITS>(bits, e);
+  else return Lp<PDT>::to_f32(bits);
+}
+template <int ECC_BITS>
+FO_DEVI int code_at(const void* ecc, const unsigned long long i) {
+  if constexpr (ECC_BITS == 16) return ((const short*)ecc)[i];
+  if constexpr (ECC_BITS == 8) return ((const signed char*)ecc)[i];
+  return 0;
+}
+
+// A leaf that is not aligned: one element per thread at a time, neighbours side by side, eight loads in flight.  A launch per
+// leaf, in kernels of their own, so that those below keep their registers.  (Eight elements in a row per thread took twice as
+// long: 16.8 M elements with 16-bit codes 87 us split and 71 reconstructed, this 25 and 26.)
+template <int PDT, int ECC_BITS>
+__global__ void __launch_bounds__(kCodecThreads) split_unaligned_kernel(const FoSplitLeaf L) {
+  chain_wait();
+  chain_release();
+  for (unsigned long long base = blockIdx.x * kCodecTile + threadIdx.x; base < L.n; base += gridDim.x * kCodecTile) {
+    float theta[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (base + j * kCodecThreads < L.n) theta[j] = L.theta[base + j * kCodecThreads];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (base + j * kCodecThreads < L.n) split_one<PDT, ECC_BITS>(L, base + j * kCodecThreads, theta[j]);
+  }
+}
+template <int PDT, int ECC_BITS>
+__global__ void __launch_bounds__(kCodecThreads) reconstruct_unaligned_kernel(const FoSplitLeaf L) {
+  chain_wait();
+  chain_release();
+  for (unsigned long long base = blockIdx.x * kCodecTile + threadIdx.x; base < L.n; base += gridDim.x * kCodecTile) {
+    uint32_t bits[8];
+    int e[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const unsigned long long i = base + j * kCodecThreads;
+      if (i < L.n) {
+        bits[j] = ((const unsigned short*)L.lp)[i];
+        e[j] = code_at<ECC_BITS>(L.ecc, i);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (base + j * kCodecThreads < L.n) L.theta[base + j * kCodecThreads] = reconstruct_one<PDT, ECC_BITS>(bits[j], e[j]);
+  }
+}
+
+template <int PDT, int ECC_BITS, int N>
+__global__ void __launch_bounds__(kCodecThreads) split_kernel(const __grid_constant__ SplitParams<N> p) {
   chain_wait();
   chain_release();
   const uint32_t total = p.first_tile[p.n_leaves];
@@ -194,7 +285,7 @@ __global__ void __launch_bounds__(kCodecThreads) split_kernel(const __grid_const
     const int l = leaf_of(p.first_tile, p.n_leaves, t);
     const FoSplitLeaf& L = p.leaf[l];
     const unsigned long long i0 = (unsigned long long)(t - p.first_tile[l]) * kCodecTile + threadIdx.x * kPiece;
-    if (i0 + kPiece <= L.n && p.aligned[l]) {
+    if (i0 + kPiece <= L.n) {
       float v[8];
       load8(L.theta + i0, v);
       uint32_t nw[4];
@@ -218,23 +309,13 @@ __global__ void __launch_bounds__(kCodecThreads) split_kernel(const __grid_const
       if constexpr (ECC_BITS == 16) *(uint4*)((short*)L.ecc + i0) = e;
       if constexpr (ECC_BITS == 8) *(uint2*)((signed char*)L.ecc + i0) = make_uint2(e.x, e.y);
     } else {
-      for (int j = 0; j < 8; ++j) {
-        const unsigned long long i = i0 + j;
-        if (i >= L.n) break;
-        uint32_t nb;
-        int e = 0;
-        if constexpr (ECC_BITS != 0) fast::split<PDT, ECC_BITS>(L.theta[i], nb, e);
-        else nb = Lp<PDT>::from_f32(L.theta[i]);
-        ((unsigned short*)L.lp)[i] = (unsigned short)nb;
-        if constexpr (ECC_BITS == 16) ((short*)L.ecc)[i] = (short)e;
-        if constexpr (ECC_BITS == 8) ((signed char*)L.ecc)[i] = (signed char)e;
-      }
+      for (unsigned long long i = i0; i < L.n && i < i0 + kPiece; ++i) split_one<PDT, ECC_BITS>(L, i, L.theta[i]);
     }
   }
 }
 
-template <int PDT, int ECC_BITS>
-__global__ void __launch_bounds__(kCodecThreads) reconstruct_kernel(const __grid_constant__ SplitParams p) {
+template <int PDT, int ECC_BITS, int N>
+__global__ void __launch_bounds__(kCodecThreads) reconstruct_kernel(const __grid_constant__ SplitParams<N> p) {
   chain_wait();
   chain_release();
   const uint32_t total = p.first_tile[p.n_leaves];
@@ -242,11 +323,7 @@ __global__ void __launch_bounds__(kCodecThreads) reconstruct_kernel(const __grid
     const int l = leaf_of(p.first_tile, p.n_leaves, t);
     const FoSplitLeaf& L = p.leaf[l];
     const unsigned long long i0 = (unsigned long long)(t - p.first_tile[l]) * kCodecTile + threadIdx.x * kPiece;
-    auto one = [&](uint32_t bits, int e) {
-      if constexpr (ECC_BITS != 0) return fast::reconstruct<PDT, ECC_BITS>(bits, e);
-      else return Lp<PDT>::to_f32(bits);
-    };
-    if (i0 + kPiece <= L.n && p.aligned[l]) {
+    if (i0 + kPiece <= L.n) {
       const uint4 w = *(const uint4*)((const unsigned short*)L.lp + i0);
       uint4 e = make_uint4(0u, 0u, 0u, 0u);
       if constexpr (ECC_BITS == 16) e = *(const uint4*)((const short*)L.ecc + i0);
@@ -259,32 +336,10 @@ __global__ void __launch_bounds__(kCodecThreads) reconstruct_kernel(const __grid
       float v[8];
 #pragma unroll
       for (int k = 0; k < 4; ++k) { v[2 * k] = theta[k].x; v[2 * k + 1] = theta[k].y; }
-      if constexpr (ECC_BITS != 0) {
-        constexpr uint32_t kInf = PDT == FO_BF16 ? 0x7F80u : 0x7C00u;
-        const uint32_t words[4] = {w.x, w.y, w.z, w.w}, ecc_words[4] = {e.x, e.y, e.z, e.w};
-        uint32_t top = 0u;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) top = max(top, max(words[k] & 0x7FFFu, (words[k] >> 16) & 0x7FFFu));
-        if (top >= kInf) {  // infinities and NaNs have no exponent the shortcut could use
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            int ej;
-            if constexpr (ECC_BITS == 16) ej = (int)(short)(ecc_words[j >> 1] >> (16 * (j & 1)));
-            else ej = (int)(signed char)(ecc_words[j >> 2] >> (8 * (j & 3)));
-            v[j] = one((words[j >> 1] >> (16 * (j & 1))) & 0xFFFFu, ej);
-          }
-        }
-      }
       store8((float*)L.theta + i0, v);
     } else {
-      for (int j = 0; j < 8; ++j) {
-        const unsigned long long i = i0 + j;
-        if (i >= L.n) break;
-        int e = 0;
-        if constexpr (ECC_BITS == 16) e = ((const short*)L.ecc)[i];
-        if constexpr (ECC_BITS == 8) e = ((const signed char*)L.ecc)[i];
-        ((float*)L.theta)[i] = one(((const unsigned short*)L.lp)[i], e);
-      }
+      for (unsigned long long i = i0; i < L.n && i < i0 + kPiece; ++i)
+        L.theta[i] = reconstruct_one<PDT, ECC_BITS>(((const unsigned short*)L.lp)[i], code_at<ECC_BITS>(L.ecc, i));
     }
   }
 }
@@ -307,7 +362,7 @@ static int small_group_shift(int G) {
 template <typename... P, typename... A>
 static int launch_codec(const char* what, void (*kernel)(P...), unsigned int grid, void* stream, const A&... args) {
   bool chained = true;
-  const cudaError_t e = launch_chained<P...>(kernel, grid, (unsigned int)kCodecThreads, 0, chained, (cudaStream_t)stream, static_cast<P>(args)...);
+  const cudaError_t e = launch_chained<P...>(kernel, grid, (unsigned int)kCodecThreads, 0, chained, (cudaStream_t)stream, static_cast<const P&>(args)...);
   if (e != cudaSuccess) return fail(FO_ERR_CUDA, "%s: launch failed: %s", what, cudaGetErrorString(e));
   return FO_OK;
 }
@@ -335,26 +390,34 @@ static int dequantize_entry(const void* values, const void* scales, float* out, 
   if (n == 0) return FO_OK;
   if (values == nullptr || scales == nullptr || out == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: null pointer", what);
   if (G < 1) return fail(FO_ERR_INVALID_ARG, "%s: group_size %d", what, G);
-  const int aligned = aligned_to(out, 32) && aligned_to(values, 8);
-  return launch_codec(what, dequantize_kernel<VARIANCE>, tile_grid((n + kCodecTile - 1) / kCodecTile), stream, values, (const __half*)scales, out, n, G, small_group_shift(G), aligned);
+  const unsigned int grid = tile_grid((n + kCodecTile - 1) / kCodecTile);
+  const int gshift = small_group_shift(G);
+  if (gshift != 0 && aligned_to(out, 32) && aligned_to(values, 8))
+    return launch_codec(what, dequantize_kernel<VARIANCE>, grid, stream, values, (const __half*)scales, out, n, gshift);
+  int power = 30;
+  while (power >= 0 && G != 1 << power) --power;
+  return launch_codec(what, dequantize_any_kernel<VARIANCE>, grid, stream, values, (const __half*)scales, out, n, (unsigned int)G, power);
 }
 
-using SplitKernel = void (*)(const SplitParams);
-static int split_entry(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t pdt, int32_t ecc_bits, void* stream, bool split, const char* what) {
-  SplitKernel kernel = nullptr;
-#define X(P, E) \
-  if (pdt == P && ecc_bits == E) kernel = split ? split_kernel<P, E> : reconstruct_kernel<P, E>;
+template <int N>
+static int split_table(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t pdt, int32_t ecc_bits, void* stream, bool split, const char* what) {
+  void (*kernel)(const SplitParams<N>) = nullptr;
+  void (*unaligned)(const FoSplitLeaf) = nullptr;
+#define X(P, E)                                                                            \
+  if (pdt == P && ecc_bits == E) {                                                         \
+    kernel = split ? split_kernel<P, E, N> : reconstruct_kernel<P, E, N>;                  \
+    unaligned = split ? split_unaligned_kernel<P, E> : reconstruct_unaligned_kernel<P, E>; \
+  }
   X(FO_BF16, 0) X(FO_BF16, 8) X(FO_BF16, 16) X(FO_F16, 0) X(FO_F16, 8) X(FO_F16, 16)
 #undef X
   if (kernel == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: param_dtype %d with ecc_bits %d", what, pdt, ecc_bits);
-  if (n_leaves > 0 && leaves == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: null table", what);
-  SplitParams p;  // filled as far as it is used
+  SplitParams<N> p;  // filled as far as it is used
   p.n_leaves = 0;
   unsigned long long tiles = 0;
   for (uint32_t i = 0; i <= n_leaves; ++i) {
     const unsigned long long more = i < n_leaves ? (leaves[i].n + kCodecTile - 1) / kCodecTile : 0ull;
     if (more > 0x7FFFFFFFull) return fail(FO_ERR_TOO_LARGE, "%s: leaf %u with %llu elements exceeds one launch", what, i, (unsigned long long)leaves[i].n);
-    if (p.n_leaves > 0 && (i == n_leaves || p.n_leaves == kSplitLeaves || tiles + more > 0x7FFFFFFFull)) {
+    if (p.n_leaves > 0 && (i == n_leaves || p.n_leaves == N || tiles + more > 0x7FFFFFFFull)) {
       p.first_tile[p.n_leaves] = (uint32_t)tiles;
       if (int rc = launch_codec(what, kernel, tile_grid(tiles), stream, p)) return rc;
       p.n_leaves = 0;
@@ -363,13 +426,21 @@ static int split_entry(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t pdt
     if (i == n_leaves || leaves[i].n == 0) continue;
     const FoSplitLeaf& L = leaves[i];
     if (L.theta == nullptr || L.lp == nullptr || (ecc_bits != 0 && L.ecc == nullptr)) return fail(FO_ERR_INVALID_ARG, "%s: null pointer", what);
+    if (!(aligned_to(L.theta, 32) && aligned_to(L.lp, 16) && aligned_to(L.ecc, 16))) {
+      if (int rc = launch_codec(what, unaligned, tile_grid(more), stream, L)) return rc;
+      continue;
+    }
     p.leaf[p.n_leaves] = L;
     p.first_tile[p.n_leaves] = (uint32_t)tiles;
-    p.aligned[p.n_leaves] = aligned_to(L.theta, 32) && aligned_to(L.lp, 16) && aligned_to(L.ecc, 16);
     tiles += more;
     ++p.n_leaves;
   }
   return FO_OK;
+}
+static int split_entry(const FoSplitLeaf* leaves, uint32_t n_leaves, int32_t pdt, int32_t ecc_bits, void* stream, bool split, const char* what) {
+  if (n_leaves > 0 && leaves == nullptr) return fail(FO_ERR_INVALID_ARG, "%s: null table", what);
+  return n_leaves <= kSplitLeavesSmall ? split_table<kSplitLeavesSmall>(leaves, n_leaves, pdt, ecc_bits, stream, split, what)
+                                       : split_table<kSplitLeaves>(leaves, n_leaves, pdt, ecc_bits, stream, split, what);
 }
 
 }  // namespace fo

@@ -115,3 +115,32 @@ def test_set_fp32_params_round_trip():
     with pytest.raises(ValueError, match="matching tree structure"):
         fo.set_fp32_params({"w": fp32["w"]}, param_template=params)
     assert fo.cast_tree_bf16({"a": torch.ones(2)})["a"].dtype == torch.bfloat16
+
+
+@pytest.mark.parametrize("bits", [None, 24, 32])
+@pytest.mark.parametrize("leaves", [1, 8, 9, 300])  # one table of either size, several tables
+def test_trees_with_unaligned_leaves(leaves, bits):
+    """Every third leaf starts off the boundary of the wide accesses; sizes around the tile of 2048 elements."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    rng = np.random.default_rng(leaves)
+    like, weights, want = [], [], []
+    for i in range(leaves):
+        n = (1, 7, 2047, 2048, 2049, 5 * 2048 + 3)[i % 6]
+        x = (rng.normal(0, 1, n) * np.exp2(rng.integers(-20, 5, n))).astype(np.float32)
+        tdt, ndt = ((torch.bfloat16, H.BF16), (torch.float16, np.dtype(np.float16)))[i % 2]
+        like.append(torch.empty(n, dtype=tdt, device="cuda"))
+        weights.append(torch.cat([torch.zeros(1, device="cuda"), H.to_torch(x)])[1:] if i % 3 == 0 else H.to_torch(x))
+        want.append(O.split_leaf(x, ndt, bits))
+    lp, ecc = fo.set_fp32_params(weights, like, master_weight_bits=bits)
+    if bits is None:
+        for a, (b, _) in zip(lp, want):
+            assert np.array_equal(H.bits(H.to_numpy(a)), H.bits(b))
+        return
+    off = lambda t: torch.cat([t[:1], t])[1:]
+    lp2, ecc2 = [off(t) if i % 3 == 1 else t for i, t in enumerate(lp)], [off(t) if i % 3 == 2 else t for i, t in enumerate(ecc)]
+    for a, e, back, (b, c) in zip(lp, ecc, fo.reconstruct_weights(lp2, ecc2), want):
+        assert np.array_equal(H.bits(H.to_numpy(a)), H.bits(b)) and np.array_equal(H.to_numpy(e), c)
+        assert np.array_equal(H.bits(H.to_numpy(back)), H.bits(O.reconstruct_leaf(b, c)))
