@@ -1582,6 +1582,15 @@ FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut& o
   Unpacked u;
   hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, LutGlobal{}, u);
   if (clip.active) clip_grads<true>(u.g, gdt, clip);
+  if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT) {
+    // a whole warp at rest, as in step_kernel (one million elements at rest: 23.0 us with every element repaired, 5.8 so)
+    const bool codes_zero = n_valid == kPiece && (raw.mq.x | raw.mq.y | raw.vq.x | raw.vq.y) == 0u;
+    const bool plain = (h.flags & FO_FLAG_LP_DELTA) == 0 && (out.param | out.ecc | out.mu | out.mu_scales | out.nu | out.nu_scales) == 0;
+    if (__all_sync(0xFFFFFFFFu, codes_zero && plain)) {
+      const bool rest = maxabs8(u.g) == 0.0f && maxabs8(u.m) == 0.0f && maxabs8(u.v) == 0.0f;
+      if (__all_sync(0xFFFFFFFFu, rest) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
+    }
+  }
   hot_finish<true, OPT, PDT, ECC_BITS, STATE, kAll, true>(c, L, &out, dh, h, gdt, i0, at, false, u, OutAt{&out},
                                                            [&](uint4& w0, uint4& w1) { w0 = raw.p0; w1 = raw.p1; }, nullptr, n_valid, group_valid);
 }

@@ -187,3 +187,41 @@ def test_gradients_that_are_nan(opt, pdt, ecc_bits, n):
                     inside = np.isin(np.arange(n) // group, hit)
                     getattr(got, codes)[inside] = getattr(ref, codes)[inside]  # of a group whose scale is NaN
         H.assert_leaf_equal(got, ref, f"n={n} group={group}")
+
+
+@pytest.mark.parametrize("n", [1024, 20 * 1024 + 300, MAIN + 700])
+@pytest.mark.parametrize("pdt,ecc_bits,group,conv,max_norm,elsewhere", [
+    (1, 16, 32, O.FUSED, None, False), (2, 8, 32, O.FUSED, 0.5, False), (1, 8, 128, O.FUSED, None, False), (0, 0, 16, O.FUSED, 0.5, False),
+    (1, 16, 32, O.UNFUSED, None, False), (1, 8, 32, O.FUSED, None, True)])
+def test_rows_at_rest(pdt, ecc_bits, group, conv, max_norm, elsewhere, n):
+    """AdamW on a leaf most of whose rows never see a gradient: only weight decay, in whole warps and in parts of them."""
+    import torch
+
+    from flashoptim_jax_b200 import _engine as eng
+
+    rng = np.random.default_rng(n + group)
+    ref = H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), C.ADAM, C.STATE_QUANT, ecc_bits, group)
+    ref.param[600:700] = 0
+    dev = ref.copy().to_device()
+    for t in (1, 2):
+        g = H.make_grad(rng, n, 1e-2, H.BF16)
+        g[: n // 4] = 0
+        g[n // 2 + 100 :] = -H.BF16.type(0)
+        dev_g, sq, step_g = H.to_torch(g), None, g
+        if max_norm is not None:
+            sq = eng.sq_norm_of([dev_g])
+            step_g = O.clip_by_global_norm([g], max_norm, sq_norm=float(sq.cpu()))[0]
+        hp = H.hyper_tuple(C.ADAM, conv, t, lr=1e-3, wd=1e-2)
+        H.oracle_step(C.ADAM, step_g, ref, C.STATE_QUANT, group, hp)
+        outs = [H.LeafArrays(*[None if getattr(dev, f) is None else torch.empty_like(getattr(dev, f)) for f in dev.fields()])] if elsewhere else None
+        _step(C.ADAM, [dev_g], [dev], outs, C.STATE_QUANT, group, hp, pdt, 1, ecc_bits, sq, max_norm or 0.0)
+        dev = outs[0] if elsewhere else dev
+        H.assert_leaf_equal(dev.to_host(), ref, f"step {t}")
+    # codes of zero under an infinite scale are no rest: 0 * inf
+    dev.mu_scales[:] = float("inf")
+    dev.mu.zero_()
+    ref.mu_scales[:] = np.inf
+    ref.mu[:] = 0
+    dev_g = torch.zeros(n, dtype=torch.bfloat16, device="cuda")
+    _step(C.ADAM, [dev_g], [dev], None, C.STATE_QUANT, group, hp, pdt, 1, ecc_bits)
+    assert bool(torch.isnan(dev.param.float()).all())
