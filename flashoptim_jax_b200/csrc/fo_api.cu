@@ -47,7 +47,7 @@ static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool ge
     if (state == FO_STATE_NONE) { FO_PICK(lookup_sgd_none) }
   }
 #undef FO_PICK
-  return Launcher{nullptr, 0u};
+  return Launcher{nullptr, 0u, 0};
 }
 static PieceFn find_pieces(int opt, int pdt, int ecc_bits, int state) {
   if (opt == FO_OPT_ADAM) return state == FO_STATE_QUANT ? lookup_adam_quant_piece(pdt, ecc_bits) : lookup_adam_full_piece(pdt, ecc_bits);
@@ -210,11 +210,12 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
   if (hs.sm_count <= 0) return fail(FO_ERR_CUDA, "fo_step: cannot query the current device");
   hs.sq_norm = d->grad_sq_norm; hs.max_norm = d->max_grad_norm;
   hs.peers = &peers;
+  hs.outs = outs != nullptr;
   // Launches that touch peers' memory start in stream order, behind the exchange in front of them.
   const bool same_step = more != nullptr && (more->launch_flags & FO_LAUNCH_CHAINED) != 0;
   bool chained = same_step || !with_peers;
   hs.wait = !same_step && !with_peers;
-  const int most_leaves = (mode == kPlain || mode == kPeer) && !generic ? kMaxLeaves : kMaxLeavesFlex;
+  const int most_leaves = outs != nullptr ? kMaxLeavesFlex : launcher.most_leaves;
   const unsigned long long unit = generic ? generic_tile_elems(d->group_size) : kPieceElems;
   const unsigned long long kMaxBlocks = 0x7FFFFFFFull;
   unsigned long long blocks = 0, whole = 0;
@@ -276,7 +277,7 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
       D.mu_scales = advance(L.mu_scales, done >> group_shift, 2);
       D.nu_scales = advance(L.nu_scales, done >> group_shift, 2);
       D.n = n;
-      H.out = out;
+      if (outs != nullptr) H.out = out;
       H.hyper = (uint8_t)L.hyper;
       const DevHyper& dh = hyper[L.hyper];
       bool hot = aligned && !(mode == kPeer && (dh.flags & FO_FLAG_LP_DELTA) != 0);

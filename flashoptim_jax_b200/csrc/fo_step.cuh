@@ -34,8 +34,8 @@
 
 namespace fo {
 
-constexpr int kMaxLeaves = 320;      // leaves per launch of the plain and the peers' kernel (kernel-parameter table)
-constexpr int kMaxLeavesFlex = 240;  // of the kernel that can also write elsewhere: its table entries are larger
+constexpr int kMaxLeaves = 320;      // leaves per launch (kernel-parameter table)
+constexpr int kMaxLeavesFlex = 240;  // of the kernels that can also write elsewhere: their table entries are larger
 constexpr int kMaxPeers = 7;
 constexpr int kGenericTile = 1024;   // slots per block of the any-group-size kernel
 constexpr int kPieceThreads = 128, kPieceElems = kPieceThreads * 8;
@@ -179,20 +179,27 @@ struct StepTables<false, true> : StepCommon {
 };
 template <int MODE>
 using StepParams = StepTables<(MODE & kOut) != 0, MODE == kPeer>;
-// Kernel parameters of piece_kernel.  Two table sizes: a launch copies its whole parameter block, and 2 KB
-// instead of 31 saves about 1.5 us of host time on a call for a leaf or two.
-template <int N>
-struct PieceParams : StepCommon {
-  DevLeaf leaf[N];
+template <int N, bool OUT>
+struct OutTable {
   DevOut out[N];
+};
+template <int N>
+struct OutTable<N, false> {};
+// Kernel parameters of piece_kernel.  Two table sizes: a launch copies its whole parameter block, and 2 KB
+// instead of 31 saves about 1.5 us of host time on a call for a leaf or two.  Without separate outputs an entry is 74 bytes
+// instead of 122.
+template <int N, bool OUT>
+struct PieceParams : StepCommon, OutTable<N, OUT> {
+  DevLeaf leaf[N];
   uint32_t first_piece[N + 1];
   uint32_t start[N];    // first piece of the leaf this launch takes (the ones before went through step_kernel)
   uint8_t hyper_of[N];
   uint8_t hot[N];       // the vector path may take the leaf (alignment; hyper-parameters known on the host)
   Peers peers;
 };
-constexpr int kPieceLeavesSmall = 12, kPieceLeavesLarge = 236;
-static_assert(sizeof(PieceParams<kPieceLeavesLarge>) <= 32764 && sizeof(StepParams<kOut>) <= 32764 && sizeof(StepParams<kPeer>) <= 32764,
+constexpr int kPieceLeavesSmall = 12;
+__host__ __device__ constexpr int piece_leaves(bool out) { return out ? 236 : kMaxLeaves; }
+static_assert(sizeof(PieceParams<piece_leaves(true), true>) <= 32764 && sizeof(PieceParams<piece_leaves(false), false>) <= 32764 && sizeof(StepParams<kOut>) <= 32764 && sizeof(StepParams<kPeer>) <= 32764,
               "kernel parameters");
 
 inline namespace FO_SHAPE_NS {
@@ -1559,8 +1566,8 @@ FO_DEVI void masked_load(const Piece& at, const int gdt, const int last, Raw<OPT
 // lanes here compute with the last element instead, which changes none either.  (With zeros every padded element took the
 // scalar repairs for a second moment of zero: 9 of the 15 us of an AdamW step on a leaf of 700 x 700 and its bias.)
 // A warp that lies wholly beyond the end returns at once.
-template <int OPT, int PDT, int ECC_BITS, int STATE>
-FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut& out, const DevHyper& dh, const Hyp& h, const Clip& clip,
+template <int OPT, int PDT, int ECC_BITS, int STATE, bool OUT>
+FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const Clip& clip,
                           const uint32_t i0, const uint32_t n_limit) {
   if ((i0 & ~255u) >= n_limit) return;  // the warp's first element: the same answer in all its lanes
   const int gdt = c.grad_dtype, gshift = c.group_shift;
@@ -1582,16 +1589,16 @@ FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut& o
   Unpacked u;
   hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, LutGlobal{}, u);
   if (clip.active) clip_grads<true>(u.g, gdt, clip);
-  if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT) {
+  if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && !OUT) {
     // a whole warp at rest, as in step_kernel (one million elements at rest: 23.0 us with every element repaired, 5.8 so)
     const bool codes_zero = n_valid == kPiece && (raw.mq.x | raw.mq.y | raw.vq.x | raw.vq.y) == 0u;
-    const bool plain = (h.flags & FO_FLAG_LP_DELTA) == 0 && (out.param | out.ecc | out.mu | out.mu_scales | out.nu | out.nu_scales) == 0;
-    if (__all_sync(0xFFFFFFFFu, codes_zero && plain)) {
+    if (__all_sync(0xFFFFFFFFu, codes_zero && (h.flags & FO_FLAG_LP_DELTA) == 0)) {
       const bool rest = maxabs8(u.g) == 0.0f && maxabs8(u.m) == 0.0f && maxabs8(u.v) == 0.0f;
       if (__all_sync(0xFFFFFFFFu, rest) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
     }
   }
-  hot_finish<true, OPT, PDT, ECC_BITS, STATE, kAll, true>(c, L, &out, dh, h, gdt, i0, at, false, u, OutAt{&out},
+  constexpr int kMode = OUT ? kAll : kAll & ~kOut;
+  hot_finish<true, OPT, PDT, ECC_BITS, STATE, kMode, true>(c, L, out, dh, h, gdt, i0, at, false, u, OutAt{out},
                                                            [&](uint4& w0, uint4& w1) { w0 = raw.p0; w1 = raw.p1; }, nullptr, n_valid, group_valid);
 }
 
@@ -1979,8 +1986,8 @@ __global__ void __launch_bounds__(kThreads, min_blocks(OPT)) step_kernel(const _
 // Latency bound (a piece is one load, one pass of arithmetic, one store), hence many small blocks; measured
 // against the same work on step_kernel's grid of 512- and 768-thread blocks, which took 10 to 17 us for a single
 // ragged end, see launch_pieces.
-template <int OPT, int PDT, int ECC_BITS, int STATE, int N>
-__global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_constant__ PieceParams<N> p) {
+template <int OPT, int PDT, int ECC_BITS, int STATE, int N, bool OUT>
+__global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_constant__ PieceParams<N, OUT> p) {
   if (p.wait) chain_wait();
   chain_release();
   const bool with_peers = p.peers.n > 0 || p.peers.ng > 0 || p.peers.mc_pdelta != 0 || p.peers.mc_gdelta != 0;
@@ -1994,10 +2001,12 @@ __global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_const
     bool vector_ok = p.hot[l] != 0 && !with_peers;
     const Hyp h = load_hyper<OPT>(dh);
     if constexpr (OPT == FO_OPT_ADAM) vector_ok = vector_ok && (h.flags & kFlagTameAdam) != 0;
+    const DevOut* out = nullptr;
+    if constexpr (OUT) out = &p.out[l];
     if (vector_ok)
-      ragged_piece<OPT, PDT, ECC_BITS, STATE>(p, L, p.out[l], dh, h, clip, i0, (uint32_t)L.n);
+      ragged_piece<OPT, PDT, ECC_BITS, STATE, OUT>(p, L, out, dh, h, clip, i0, (uint32_t)L.n);
     else
-      cold_piece<OPT, PDT, ECC_BITS, STATE>(L, &p.out[l], dh, p.grad_dtype, p.group_shift, i0, with_peers ? &p.peers : nullptr, p.sq_norm, p.max_norm);
+      cold_piece<OPT, PDT, ECC_BITS, STATE>(L, out, dh, p.grad_dtype, p.group_shift, i0, with_peers ? &p.peers : nullptr, p.sq_norm, p.max_norm);
   }
   chain_end();
 }
@@ -2005,15 +2014,16 @@ __global__ void __launch_bounds__(kPieceThreads) piece_kernel(const __grid_const
 // ---- any group size (1..1024): one block per tile of whole groups, group maxima through
 // shared-memory atomics on the (non-negative) float bit patterns; IEEE arithmetic only.  For group sizes that
 // are not 8, 16, ..., 256 (those run step_kernel and piece_kernel) ------------------------------------------
-template <int OPT, int PDT, int ECC_BITS>
-__global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant__ StepParams<kOut> p) {
+template <int OPT, int PDT, int ECC_BITS, int MODE>
+__global__ void __launch_bounds__(256) step_kernel_generic(const __grid_constant__ StepParams<MODE> p) {
   if (p.wait) chain_wait();
   chain_release();
   __shared__ unsigned int smax_m[kGenericTile], smax_v[kGenericTile];
   const Clip clip = load_clip(p.sq_norm, p.max_norm, p.grad_dtype);
   const int l = leaf_of(p.t.first_block, p.n_leaves, blockIdx.x);
   const DevLeaf& L = p.t.leaf[l];
-  const DevOut& out = p.out[l];
+  DevOut out = {};
+  if constexpr (MODE == kOut) out = p.out[l];
   const Hyp h = load_hyper<OPT>(p.hyper[p.t.hyper_of[l]]);
   const int G = p.group_size;
   const int groups_per_tile = max(1, kGenericTile / G);
@@ -2119,17 +2129,19 @@ struct HostStep {
   const double* sq_norm;
   float max_norm;
   const Peers* peers;
+  bool outs;  // results go where HostLeaf::out says
   bool wait;  // of the next launch
 };
 // `chained`: the launch in front of this one on the stream is one of this library's and works on other leaves,
 // or the kernel begins with chain_wait(); set to true by a launch.
 using MainFn = cudaError_t (*)(HostStep&, bool& chained, cudaStream_t);
 using PieceFn = cudaError_t (*)(HostStep&, unsigned int main_chunk, bool& chained, cudaStream_t);
-// A slice of step_kernel and the elements one of its chunks covers.  Block size, and with it the chunk, is a
-// property of the slice (the slices are compiled with their own FO_THREADS).
+// A slice of step_kernel, the elements one of its chunks covers and the leaves its table holds (of a call without separate
+// outputs).  Block size, and with it the chunk, is a property of the slice (the slices are compiled with their own FO_THREADS).
 struct Launcher {
   MainFn launch;
   unsigned int chunk;
+  int most_leaves;
 };
 
 template <typename... P>
@@ -2257,9 +2269,9 @@ cudaError_t launch_main(HostStep& hs, bool& chained, cudaStream_t s) {
 }
 
 // The pieces that the whole chunks (of main_chunk elements; 0: step_kernel is not used) of the hot leaves leave over.
-template <int OPT, int PDT, int ECC_BITS, int STATE, int N>
+template <int OPT, int PDT, int ECC_BITS, int STATE, int N, bool OUT>
 cudaError_t launch_piece_table(HostStep& hs, const int* which, int n, unsigned int main_chunk, bool& chained, cudaStream_t s) {
-  PieceParams<N> p;  // filled as far as it is used
+  PieceParams<N, OUT> p;  // filled as far as it is used
   fill_common(p, hs);
   p.peers = *hs.peers;
   uint32_t total = 0;
@@ -2267,7 +2279,7 @@ cudaError_t launch_piece_table(HostStep& hs, const int* which, int n, unsigned i
     const HostLeaf& l = hs.leaf[which[k]];
     const unsigned long long done = l.hot && main_chunk != 0 ? l.src.n / main_chunk * main_chunk : 0ull;
     p.leaf[k] = l.src;
-    p.out[k] = l.out;
+    if constexpr (OUT) p.out[k] = l.out;
     p.hyper_of[k] = l.hyper;
     p.hot[k] = l.hot;
     p.start[k] = (uint32_t)(done / kPieceElems);
@@ -2277,11 +2289,12 @@ cudaError_t launch_piece_table(HostStep& hs, const int* which, int n, unsigned i
   p.n_leaves = n;
   p.first_piece[n] = total;
   const unsigned int most = (unsigned int)hs.sm_count * 64u;  // a misaligned leaf can be large: blocks then take several pieces
-  return launch_chained(piece_kernel<OPT, PDT, ECC_BITS, STATE, N>, total < most ? total : most, kPieceThreads, 0, chained, s, p);
+  return launch_chained(piece_kernel<OPT, PDT, ECC_BITS, STATE, N, OUT>, total < most ? total : most, kPieceThreads, 0, chained, s, p);
 }
-template <int OPT, int PDT, int ECC_BITS, int STATE>
-cudaError_t launch_pieces(HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
-  int which[kPieceLeavesLarge];
+template <int OPT, int PDT, int ECC_BITS, int STATE, bool OUT>
+cudaError_t launch_piece_tables(HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
+  constexpr int kLarge = piece_leaves(OUT);
+  int which[kLarge];
   int n = 0;
   for (int i = 0; i <= hs.n_leaves; ++i) {
     if (i < hs.n_leaves) {
@@ -2289,31 +2302,40 @@ cudaError_t launch_pieces(HostStep& hs, unsigned int main_chunk, bool& chained, 
       if (l.src.n == 0 || (l.hot && main_chunk != 0 && l.src.n % main_chunk == 0)) continue;
       which[n++] = i;
     }
-    if (n == kPieceLeavesLarge || (i == hs.n_leaves && n > 0)) {
-      const cudaError_t e = n <= kPieceLeavesSmall ? launch_piece_table<OPT, PDT, ECC_BITS, STATE, kPieceLeavesSmall>(hs, which, n, main_chunk, chained, s)
-                                                   : launch_piece_table<OPT, PDT, ECC_BITS, STATE, kPieceLeavesLarge>(hs, which, n, main_chunk, chained, s);
+    if (n == kLarge || (i == hs.n_leaves && n > 0)) {
+      const cudaError_t e = n <= kPieceLeavesSmall ? launch_piece_table<OPT, PDT, ECC_BITS, STATE, kPieceLeavesSmall, OUT>(hs, which, n, main_chunk, chained, s)
+                                                   : launch_piece_table<OPT, PDT, ECC_BITS, STATE, kLarge, OUT>(hs, which, n, main_chunk, chained, s);
       if (e != cudaSuccess) return e;
       n = 0;
     }
   }
   return cudaSuccess;
 }
-template <int OPT, int PDT, int ECC_BITS>
-cudaError_t launch_generic(HostStep& hs, bool& chained, cudaStream_t s) {
-  StepParams<kOut> p;
+template <int OPT, int PDT, int ECC_BITS, int STATE>
+cudaError_t launch_pieces(HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
+  return hs.outs ? launch_piece_tables<OPT, PDT, ECC_BITS, STATE, true>(hs, main_chunk, chained, s)
+                 : launch_piece_tables<OPT, PDT, ECC_BITS, STATE, false>(hs, main_chunk, chained, s);
+}
+template <int OPT, int PDT, int ECC_BITS, int MODE>
+cudaError_t launch_generic_table(HostStep& hs, bool& chained, cudaStream_t s) {
+  StepParams<MODE> p;
   fill_common(p, hs);
   const unsigned int tile = generic_tile_elems(hs.group_size);
   uint32_t total = 0;
   for (int i = 0; i < hs.n_leaves; ++i) {
     p.t.leaf[i] = hs.leaf[i].src;
-    p.out[i] = hs.leaf[i].out;
+    if constexpr (MODE == kOut) p.out[i] = hs.leaf[i].out;
     p.t.hyper_of[i] = hs.leaf[i].hyper;
     p.t.first_block[i] = total;
     total += (uint32_t)((hs.leaf[i].src.n + tile - 1) / tile);
   }
   p.n_leaves = hs.n_leaves;
   p.t.first_block[hs.n_leaves] = total;
-  return launch_chained(step_kernel_generic<OPT, PDT, ECC_BITS>, total, 256u, 0, chained, s, p);
+  return launch_chained(step_kernel_generic<OPT, PDT, ECC_BITS, MODE>, total, 256u, 0, chained, s, p);
+}
+template <int OPT, int PDT, int ECC_BITS>
+cudaError_t launch_generic(HostStep& hs, bool& chained, cudaStream_t s) {
+  return hs.outs ? launch_generic_table<OPT, PDT, ECC_BITS, kOut>(hs, chained, s) : launch_generic_table<OPT, PDT, ECC_BITS, kPlain>(hs, chained, s);
 }
 
 }  // namespace FO_SHAPE_NS

@@ -26,14 +26,14 @@ PieceFn FO_INST_NAME(int pdt, int ecc_bits) {
 Launcher FO_INST_NAME(int pdt, int ecc_bits) {
 #if FO_INST_KIND == 3
 #define X(P, E) \
-  if (pdt == P && ecc_bits == E) return Launcher{&launch_generic<FO_INST_OPT, P, E>, 0u};
+  if (pdt == P && ecc_bits == E) return Launcher{&launch_generic<FO_INST_OPT, P, E>, 0u, kMaxLeaves};
 #else
 #define X(P, E) \
-  if (pdt == P && ecc_bits == E) return Launcher{&launch_main<FO_INST_OPT, P, E, FO_INST_KIND, FO_INST_MODE>, (unsigned int)kChunk};
+  if (pdt == P && ecc_bits == E) return Launcher{&launch_main<FO_INST_OPT, P, E, FO_INST_KIND, FO_INST_MODE>, (unsigned int)kChunk, (FO_INST_MODE & kOut) != 0 ? kMaxLeavesFlex : kMaxLeaves};
 #endif
   FO_COMBOS(X)
 #undef X
-  return Launcher{nullptr, 0u};
+  return Launcher{nullptr, 0u, 0};
 }
 #endif
 

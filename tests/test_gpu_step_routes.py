@@ -225,3 +225,12 @@ def test_rows_at_rest(pdt, ecc_bits, group, conv, max_norm, elsewhere, n):
     dev_g = torch.zeros(n, dtype=torch.bfloat16, device="cuda")
     _step(C.ADAM, [dev_g], [dev], None, C.STATE_QUANT, group, hp, pdt, 1, ecc_bits)
     assert bool(torch.isnan(dev.param.float()).all())
+
+
+@pytest.mark.parametrize("opt,group,conv,elsewhere", [(C.ADAM, 32, O.FUSED, False), (C.ADAM, 128, O.UNFUSED, False), (C.SGD, 40, O.FUSED, False),
+                                                      (C.LION, 40, O.FUSED, True), (C.LION, 32, O.FUSED, True)])
+def test_leaf_counts_around_the_table_sizes(opt, group, conv, elsewhere):
+    """Kernel-parameter tables of 12, 236, 240 and 320 leaves, full, one over, and behind whole chunks."""
+    for count in (12, 13, 236, 237, 240, 241, 320, 321, 700):
+        _run(opt, 1, 8, C.STATE_QUANT, group, conv, [1 + i % 61 for i in range(count)], steps=1, elsewhere=elsewhere)
+    _run(opt, 1, 8, C.STATE_QUANT, group, conv, [6000 + i for i in range(330)], steps=1, elsewhere=elsewhere)
