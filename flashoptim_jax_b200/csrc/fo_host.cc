@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <memory>
@@ -279,7 +280,7 @@ struct Plan {
   std::vector<int> membership;     // of each leaf: the first group that takes it, or -1
   Ref resolve;                     // learning rate of a schedule: resolve(lr, count tensor)
   bool busy = false;               // a selector or a schedule may run Python code, and that another step
-  std::vector<PyObject*> p, g;     // scratch (borrowed)
+  std::vector<PyObject*> p, g;     // scratch (borrowed; run() holds references for as long as it needs them)
   std::vector<std::vector<PyObject*>> s;
 };
 constexpr const char* kPlanName = "flashoptim_b200.plan";
@@ -465,6 +466,54 @@ bool fill_leaf(Plan& plan, const LeafSpec& l, int i) {
   return true;
 }
 
+// The leaves of the trees into the plan's scratch.  False: not what the plan describes (or, with an exception set, an error).
+bool walk_trees(Plan& plan, PyObject* params, PyObject* states, PyObject* grads) {
+  if (!walk(plan.tree, params, plan.p.data()) || !walk(plan.tree, grads, plan.g.data())) return false;
+  for (int k = 0; k < plan.n_states; ++k)
+    if (!walk(plan.tree, PyTuple_GET_ITEM(states, k), plan.s[k].data())) return false;
+  return true;
+}
+// Do parameters and gradients look like the plan's?  (What tells plans apart, asked before the user's selectors and schedules
+// are called for a plan; fill_leaf checks everything.)
+bool plausible(const Plan& plan) {
+  for (int i = 0; i < plan.n; ++i) {
+    const LeafSpec& l = plan.leaves[i];
+    const at::Tensor *p = plain_tensor(plan.p[i]), *g = plain_tensor(plan.g[i]);
+    if (p == nullptr || g == nullptr || p->scalar_type() != l.param || g->scalar_type() != l.grad || p->sizes() != l.sizes || g->sizes() != l.sizes || !g->is_contiguous()) return false;
+  }
+  return true;
+}
+
+// owning references to the leaves
+class Held {
+  std::vector<PyObject*> v_;
+
+ public:
+  explicit Held(const Plan& plan) {
+    v_.reserve((size_t)plan.n * (2 + plan.n_states));
+    v_.insert(v_.end(), plan.p.begin(), plan.p.end());
+    v_.insert(v_.end(), plan.g.begin(), plan.g.end());
+    for (int k = 0; k < plan.n_states; ++k) v_.insert(v_.end(), plan.s[k].begin(), plan.s[k].end());
+    for (PyObject* x : v_) Py_INCREF(x);
+  }
+  Held(const Held&) = delete;
+  ~Held() {
+    for (PyObject* x : v_) Py_DECREF(x);
+  }
+  // are the plan's leaves still these?
+  bool same(const Plan& plan) const {
+    auto at = v_.begin();
+    auto next = [&](const std::vector<PyObject*>& x) {
+      const bool eq = std::equal(x.begin(), x.end(), at);
+      at += (ptrdiff_t)x.size();
+      return eq;
+    };
+    bool eq = next(plan.p) && next(plan.g);
+    for (int k = 0; eq && k < plan.n_states; ++k) eq = next(plan.s[k]);
+    return eq;
+  }
+};
+
 // Is every leaf in the group it was in when the plan was made?  1, 0, or -1 with an exception set.  Selectors that are
 // functions are called, as the general path calls them: what they answer may depend on more than the leaf.
 int membership_unchanged(const Plan& plan) {
@@ -503,25 +552,42 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   PyObject *params = a[1], *states = a[3], *grads = a[4];
   const at::Tensor* count_t = plain_tensor(a[2]);
   if (count_t == nullptr || !count_t->is_cpu() || count_t->scalar_type() != at::kInt || count_t->dim() != 0) Py_RETURN_NONE;
-  if (!walk(plan->tree, params, plan->p.data()) || !walk(plan->tree, grads, plan->g.data())) {
+  if (!walk_trees(*plan, params, states, grads) || !groups_unchanged(*plan)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
-  for (int k = 0; k < plan->n_states; ++k)
-    if (!walk(plan->tree, PyTuple_GET_ITEM(states, k), plan->s[k].data())) {
-      if (PyErr_Occurred()) return nullptr;
-      Py_RETURN_NONE;
-    }
-  for (int i = 0; i < plan->n; ++i)
-    if (!fill_leaf(*plan, plan->leaves[i], i)) Py_RETURN_NONE;
-  if (!groups_unchanged(*plan)) Py_RETURN_NONE;
+  const int32_t old_count = *count_t->const_data_ptr<int32_t>();
+  const double step = (double)old_count + 1.0;
+  const Held held(*plan);  // the leaves stay alive, whatever happens to the trees meanwhile
+
+  std::vector<double> lr(plan->groups.size());
+  bool call = plan->dynamic;  // code of the user's
+  for (const Group& gr : plan->groups) call = call || !PyFloat_CheckExact(gr.lr.p);
+  if (call && !plausible(*plan)) Py_RETURN_NONE;
   if (plan->dynamic) {
     const int same = membership_unchanged(*plan);
     if (same < 0) return nullptr;
     if (same == 0) Py_RETURN_NONE;
   }
-  const int32_t old_count = *count_t->const_data_ptr<int32_t>();
-  const double step = (double)old_count + 1.0;
+  for (size_t i = 0; i < lr.size(); ++i) {
+    PyObject* const value = plan->groups[i].lr.p;
+    if (PyFloat_CheckExact(value)) {
+      lr[i] = PyFloat_AS_DOUBLE(value);
+      continue;
+    }
+    Ref v(PyObject_CallFunctionObjArgs(plan->resolve.p, value, a[2], nullptr));  // zero-based count (adamw.py:526)
+    if (v.p == nullptr) return nullptr;
+    lr[i] = PyFloat_AsDouble(v.p);
+    if (lr[i] == -1.0 && PyErr_Occurred()) return nullptr;
+  }
+  // A selector or a schedule, or another thread that ran meanwhile, may have put other tensors into the trees or other storage
+  // under a tensor: addresses are taken now, and nothing is called between here and the launches.
+  if (call && (!walk_trees(*plan, params, states, grads) || !held.same(*plan))) {
+    if (PyErr_Occurred()) return nullptr;
+    Py_RETURN_NONE;
+  }
+  for (int i = 0; i < plan->n; ++i)
+    if (!fill_leaf(*plan, plan->leaves[i], i)) Py_RETURN_NONE;
 
   // from here on the step is taken
   std::vector<Ref> out_p, out_s[3];
@@ -560,18 +626,9 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   std::vector<FoHyper> hyper(plan->groups.size());
   for (size_t i = 0; i < plan->groups.size(); ++i) {
     const Group& gr = plan->groups[i];
-    double lr;
-    if (PyFloat_CheckExact(gr.lr.p)) {
-      lr = PyFloat_AS_DOUBLE(gr.lr.p);
-    } else {
-      Ref v(PyObject_CallFunctionObjArgs(plan->resolve.p, gr.lr.p, a[2], nullptr));  // zero-based count (adamw.py:526)
-      if (v.p == nullptr) return nullptr;
-      lr = PyFloat_AsDouble(v.p);
-      if (lr == -1.0 && PyErr_Occurred()) return nullptr;
-    }
     FoHyper& h = hyper[i];
     std::memset(&h, 0, sizeof(h));
-    h.lr = f32(lr); h.wd = gr.wd; h.b1 = gr.b1; h.b2 = gr.b2; h.one_minus_b1 = gr.omb1; h.one_minus_b2 = gr.omb2; h.eps = gr.eps;
+    h.lr = f32(lr[i]); h.wd = gr.wd; h.b1 = gr.b1; h.b2 = gr.b2; h.one_minus_b1 = gr.omb1; h.one_minus_b2 = gr.omb2; h.eps = gr.eps;
     h.bc1 = h.bc2 = 1.0f;
     if (plan->opt == FO_OPT_ADAM) {  // as _engine.bias_correction
       h.bc1 = 1.0f - f32(std::pow(gr.beta1, step));

@@ -256,3 +256,41 @@ def test_codecs_at_edges(group):
                 d = (fo.dequantize_variance if variance else fo.dequantize_momentum)(q, group)
                 want = (O.dequantize_variance if variance else O.dequantize_momentum)(want_q, group)
                 assert np.array_equal(d.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("donate", [False, True])
+@pytest.mark.parametrize("where", ["schedule", "selector"])
+def test_callbacks_that_touch_the_trees(where, donate):
+    """A schedule or a selector puts other storage under a parameter, or another tensor into the tree, while the step is being prepared: what
+    is in the tree when the step is launched is stepped."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    trees = {}
+
+    def touch(leaf_of):
+        p = trees["params"]
+        p["w"].data = p["w"].data.clone()
+        if leaf_of == "b":
+            p["b"] = p["b"].clone()
+        del p
+
+    kw = {}
+    if where == "schedule":
+        kw["learning_rate"] = lambda count: (touch("b"), 1e-2)[1]
+    else:
+        kw.update(learning_rate=1e-2, param_groups=[{"params": lambda path, leaf: (touch(path[0]), False)[1], "weight_decay": 0.5}])
+    tx, ref = fo.flash_adamw(donate=donate, **kw), fo.flash_adamw(learning_rate=1e-2)
+    make = lambda: {"b": torch.ones(33, device="cuda"), "w": torch.full((3000,), 0.5, device="cuda", dtype=torch.bfloat16)}
+    p, q = make(), make()
+    trees["params"] = p
+    s, t = tx.init(p), ref.init(q)
+    for k in range(5):
+        g = _grads(q, k)
+        trees["params"] = p
+        p, s = tx.step(p, s, g)
+        q, t = ref.step(q, t, g)
+        if donate:
+            p = dict(p)  # a container of its own for the next callback
+        _same((p, s.mu, s.nu, s.ecc), (q, t.mu, t.nu, t.ecc))
