@@ -277,7 +277,7 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
       D.mu_scales = advance(L.mu_scales, done >> group_shift, 2);
       D.nu_scales = advance(L.nu_scales, done >> group_shift, 2);
       D.n = n;
-      if (outs != nullptr) H.out = out;
+      H.out = out;  // (zeros without outs: the kernel that carries all features adds them)
       H.hyper = (uint8_t)L.hyper;
       const DevHyper& dh = hyper[L.hyper];
       bool hot = aligned && !(mode == kPeer && (dh.flags & FO_FLAG_LP_DELTA) != 0);
