@@ -231,9 +231,14 @@ PyObject* host_int(int32_t v) {
   return THPVariable_Wrap(t);
 }
 
-// runs f on the device and its current stream
+// Runs f (an allocation or a launch may block: no Python in it) on the device and its current stream, with the GIL released; returns f's
+// status, for ok().  The caller holds references to the tensors whose addresses f uses.
 template <typename F>
-bool on_device(int device, F f) {
+int on_device(int device, F f) {
+  struct Released {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Released() { PyEval_RestoreThread(state); }
+  } released;
   c10::cuda::OptionalCUDAGuard guard;
   if (c10::cuda::current_device() != device) guard.set_index((c10::DeviceIndex)device);
   return f(c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream());
@@ -537,6 +542,68 @@ int membership_unchanged(const Plan& plan) {
   return 1;
 }
 
+// f(leaf, output table entry of its array k, size of that array, dtype): the arrays of a leaf that a step writes.
+// (0 parameter; 1 code; 2, 3 moment 1 and its scales; 4, 5 moment 2 and its scales)
+template <typename F>
+void each_result(Plan& plan, F f) {
+  for (int i = 0; i < plan.n; ++i) {
+    const LeafSpec& l = plan.leaves[i];
+    FoLeafOut& o = plan.calls[l.call].outs[l.at];
+    const at::IntArrayRef sizes = l.sizes;
+    f(i, 0, o.param, sizes, l.param);
+    if (l.ecc_bits != 0) f(i, 1, o.ecc, sizes, l.ecc);
+    for (int k = 1; k < plan.n_states; ++k) {
+      void *&values = k == 1 ? o.mu : o.nu, *&scales = k == 1 ? o.mu_scales : o.nu_scales;
+      if (l.state == FO_STATE_QUANT) {
+        f(i, 2 * k, values, sizes, k == 1 ? at::kChar : at::kByte);
+        f(i, 2 * k + 1, scales, at::IntArrayRef(l.n_scales), at::kHalf);
+      } else if (l.state == FO_STATE_FULL) {
+        f(i, 2 * k, values, sizes, at::kFloat);
+      }
+    }
+  }
+}
+void allocate_results(Plan& plan, std::vector<at::Tensor>& made) {
+  made.reserve((size_t)plan.n * 6);
+  each_result(plan, [&](int, int, void*& address, at::IntArrayRef sizes, at::ScalarType dtype) {
+    made.push_back(empty_like_on(sizes, dtype, plan.device));
+    address = made.back().data_ptr();
+  });
+}
+// the same arrays as Python objects, with the markers of the absent ones handed on
+bool wrap_results(Plan& plan, std::vector<at::Tensor>& made, std::vector<Ref>& params, std::vector<Ref> (&states)[3]) {
+  params.resize(plan.n);
+  for (int k = 0; k < plan.n_states; ++k) {
+    states[k].resize(plan.n);
+    for (int i = 0; i < plan.n; ++i)
+      if (k == 0 ? plan.leaves[i].ecc_bits == 0 : plan.leaves[i].state == FO_STATE_NONE) states[k][i] = Ref::borrow(plan.s[k][i]);
+  }
+  size_t at = 0;
+  Ref pending;  // values, until their scales come
+  bool good = true;
+  each_result(plan, [&](int i, int array, void*&, at::IntArrayRef, at::ScalarType) {
+    Ref t(good ? THPVariable_Wrap(std::move(made[at++])) : nullptr);
+    good = good && t.p != nullptr;
+    if (!good) return;
+    if (array <= 1) {
+      (array == 0 ? params : states[0])[i] = std::move(t);
+    } else if (array & 1) {
+      PyObject* pair = PyTuple_New(2);
+      if (pair != nullptr) {
+        PyTuple_SET_ITEM(pair, 0, pending.release());
+        PyTuple_SET_ITEM(pair, 1, t.release());
+      }
+      states[array / 2][i] = Ref(tuple_of_type((PyTypeObject*)quantized_type, pair));
+      good = states[array / 2][i].p != nullptr;
+    } else if (plan.leaves[i].state == FO_STATE_QUANT) {
+      pending = std::move(t);
+    } else {
+      states[array / 2][i] = std::move(t);
+    }
+  });
+  return good;
+}
+
 // run(plan, params, count, states, grads, sq_norm address or 0, max_norm)
 //   -> None, or (params, states, count)
 PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
@@ -590,39 +657,6 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!fill_leaf(*plan, plan->leaves[i], i)) Py_RETURN_NONE;
 
   // from here on the step is taken
-  std::vector<Ref> out_p, out_s[3];
-  if (!plan->donate) {
-    out_p.resize(plan->n);
-    for (int k = 0; k < plan->n_states; ++k) out_s[k].resize(plan->n);
-    for (int i = 0; i < plan->n; ++i) {
-      const LeafSpec& l = plan->leaves[i];
-      FoLeafOut& o = plan->calls[l.call].outs[l.at];
-      auto make = [&](at::IntArrayRef sizes, at::ScalarType dt, void*& address) {
-        at::Tensor t = empty_like_on(sizes, dt, plan->device);
-        address = t.data_ptr();
-        return Ref(THPVariable_Wrap(std::move(t)));
-      };
-      out_p[i] = make(l.sizes, l.param, o.param);
-      if (l.ecc_bits != 0) out_s[0][i] = make(l.sizes, l.ecc, o.ecc);
-      else out_s[0][i] = Ref::borrow(plan->s[0][i]);
-      for (int k = 1; k < plan->n_states; ++k) {
-        void*& values = k == 1 ? o.mu : o.nu;
-        void*& scales = k == 1 ? o.mu_scales : o.nu_scales;
-        if (l.state == FO_STATE_QUANT) {
-          PyObject* t = PyTuple_New(2);
-          if (t == nullptr) return nullptr;
-          PyTuple_SET_ITEM(t, 0, make(l.sizes, k == 1 ? at::kChar : at::kByte, values).release());
-          PyTuple_SET_ITEM(t, 1, make({l.n_scales}, at::kHalf, scales).release());
-          out_s[k][i] = Ref(tuple_of_type((PyTypeObject*)quantized_type, t));
-          if (out_s[k][i].p == nullptr) return nullptr;
-        } else if (l.state == FO_STATE_FULL) {
-          out_s[k][i] = make(l.sizes, at::kFloat, values);
-        } else {
-          out_s[k][i] = Ref::borrow(plan->s[k][i]);
-        }
-      }
-    }
-  }
   std::vector<FoHyper> hyper(plan->groups.size());
   for (size_t i = 0; i < plan->groups.size(); ++i) {
     const Group& gr = plan->groups[i];
@@ -638,26 +672,31 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   void* const sq = PyLong_AsVoidPtr(a[5]);
   const double max_norm = PyFloat_AsDouble(a[6]);
-  uint32_t chain = 0u;
   if (PyErr_Occurred()) return nullptr;
-  const bool launched = on_device(plan->device, [&](cudaStream_t stream) {
+  std::vector<at::Tensor> made;  // results that must not overwrite their operands, in the order of leaf, array
+  const int status = on_device(plan->device, [&](cudaStream_t stream) {
+    if (!plan->donate) allocate_results(*plan, made);
+    uint32_t chain = 0u;
     for (Call& c : plan->calls) {
       for (size_t k = 0; k < c.slots.size(); ++k) c.hypers[k] = hyper[c.slots[k]];
       c.desc.grad_sq_norm = (const double*)sq;
       c.desc.max_grad_norm = f32(max_norm);
       const FoStepMore more = {sizeof(FoStepMore), chain, plan->donate ? nullptr : c.outs.data()};
-      if (!ok(api.step(&c.desc, &more, stream))) return false;
+      const int rc = api.step(&c.desc, &more, stream);
+      if (rc != FO_OK) return rc;
       if (!c.empty) chain = FO_LAUNCH_CHAINED;  // (behind a call that launches nothing the stream holds what it held before)
     }
-    return true;
+    return (int)FO_OK;
   });
-  if (!launched) return nullptr;
+  if (!ok(status)) return nullptr;
 
   Ref count(host_int(old_count + 1));
   if (count.p == nullptr) return nullptr;
   if (plan->donate) {  // every array was updated in place
     return PyTuple_Pack(3, params, states, count.p);
   }
+  std::vector<Ref> out_p, out_s[3];
+  if (!wrap_results(*plan, made, out_p, out_s)) return nullptr;
   Ref new_params(build(plan->tree, out_p));
   Ref new_states(PyTuple_New(plan->n_states));
   if (new_params.p == nullptr || new_states.p == nullptr) return nullptr;
@@ -670,7 +709,7 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 }
 
 // ---- gradient norm -------------------------------------------------------------------------------------------------
-bool collect(PyObject* x, std::vector<const at::Tensor*>& out) {
+bool collect(PyObject* x, std::vector<at::Tensor>& out) {
   if (x == Py_None) return true;
   if (PyDict_CheckExact(x)) {
     // the order of the sum is that of the flattened tree
@@ -702,28 +741,29 @@ bool collect(PyObject* x, std::vector<const at::Tensor*>& out) {
   }
   const at::Tensor* t = plain_tensor(x);
   if (t == nullptr || !t->is_cuda() || dtype_code(t->scalar_type()) < 0 || !t->is_contiguous()) return false;
-  if (!out.empty() && t->device() != out[0]->device()) return false;
-  out.push_back(t);
+  if (!out.empty() && t->device() != out[0].device()) return false;
+  out.push_back(*t);
   return true;
 }
 
 // sq_norm(tree) -> one-element float64 tensor, or None
 PyObject* sq_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 1) { PyErr_SetString(PyExc_TypeError, "sq_norm takes 1 argument"); return nullptr; }
-  std::vector<const at::Tensor*> t;
+  std::vector<at::Tensor> t;  // (references: the GIL is released below)
   if (!collect(a[0], t) || t.empty()) Py_RETURN_NONE;
-  const int device = t[0]->device().index();
+  const int device = t[0].device().index();
   std::vector<FoArray> arrays(t.size());
   std::vector<int32_t> dtypes(t.size());
   for (size_t i = 0; i < t.size(); ++i) {
-    arrays[i] = FoArray{t[i]->const_data_ptr(), (uint64_t)t[i]->numel()};
-    dtypes[i] = dtype_code(t[i]->scalar_type());
+    arrays[i] = FoArray{t[i].const_data_ptr(), (uint64_t)t[i].numel()};
+    dtypes[i] = dtype_code(t[i].scalar_type());
   }
-  at::Tensor out = empty_like_on({1}, at::kDouble, device);
-  at::Tensor workspace = empty_like_on({FO_SQ_NORM_WORKSPACE_BYTES}, at::kByte, device);  // its own: streams do not share one
-  if (!on_device(device, [&](cudaStream_t s) {
-        return ok(api.sq_norm(arrays.data(), dtypes.data(), (uint32_t)arrays.size(), 0, (double*)out.data_ptr(), workspace.data_ptr(), s));
-      }))
+  at::Tensor out;
+  if (!ok(on_device(device, [&](cudaStream_t s) {
+        out = empty_like_on({1}, at::kDouble, device);
+        const at::Tensor workspace = empty_like_on({FO_SQ_NORM_WORKSPACE_BYTES}, at::kByte, device);  // its own: streams do not share one
+        return api.sq_norm(arrays.data(), dtypes.data(), (uint32_t)arrays.size(), 0, (double*)out.data_ptr(), workspace.data_ptr(), s);
+      })))
     return nullptr;
   return THPVariable_Wrap(std::move(out));
 }
@@ -731,13 +771,13 @@ PyObject* sq_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // ---- fp32 weights <-> (parameters, ECC) ------------------------------------------------------------------------------
 struct SplitTables {  // by (dtype, ECC width)
   std::vector<FoSplitLeaf> t[3][3];
-  bool launch(int device, decltype(&fo_split_many) fn) {
-    return on_device(device, [&](cudaStream_t s) {
-      for (int d = 0; d < 3; ++d)
-        for (int e = 0; e < 3; ++e)
-          if (!t[d][e].empty() && !ok(fn(t[d][e].data(), (uint32_t)t[d][e].size(), d, e * 8, s))) return false;
-      return true;
-    });
+  std::vector<at::Tensor> in;  // what the tables point to
+  int launch(cudaStream_t s, decltype(&fo_split_many) fn) {
+    for (int d = 0; d < 3; ++d)
+      for (int e = 0; e < 3; ++e)
+        if (!t[d][e].empty())
+          if (const int rc = fn(t[d][e].data(), (uint32_t)t[d][e].size(), d, e * 8, s)) return rc;
+    return FO_OK;
   }
 };
 int one_device(const std::vector<PyObject*>& xs, int device) {  // index of the CUDA device all tensors are on, or -1
@@ -775,19 +815,24 @@ PyObject* reconstruct(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!et->is_cuda() || et->device().index() != device || et->sizes() != pt->sizes() || !et->is_contiguous()) Py_RETURN_NONE;
   }
   SplitTables tables;
-  std::vector<Ref> out(n);
   for (int i = 0; i < n; ++i) {
-    const at::Tensor *pt = plain_tensor(p[i]), *et = plain_tensor(e[i]);
-    const int code = dtype_code(pt->scalar_type());
-    if (code == FO_F32) {
-      out[i] = Ref::borrow(p[i]);
-      continue;
-    }
-    at::Tensor t = empty_like_on(pt->sizes(), at::kFloat, device);
-    tables.t[code][et->scalar_type() == at::kChar ? 1 : 2].push_back(FoSplitLeaf{(float*)t.data_ptr(), const_cast<void*>(pt->const_data_ptr()), const_cast<void*>(et->const_data_ptr()), (uint64_t)pt->numel()});
-    out[i] = Ref(THPVariable_Wrap(std::move(t)));
+    tables.in.push_back(*plain_tensor(p[i]));
+    tables.in.push_back(*plain_tensor(e[i]));
   }
-  if (!tables.launch(device, api.reconstruct)) return nullptr;
+  std::vector<at::Tensor> made(n);
+  if (!ok(on_device(device, [&](cudaStream_t s) {
+        for (int i = 0; i < n; ++i) {
+          const at::Tensor &pt = tables.in[2 * i], &et = tables.in[2 * i + 1];
+          const int code = dtype_code(pt.scalar_type());
+          if (code == FO_F32) continue;
+          made[i] = empty_like_on(pt.sizes(), at::kFloat, device);
+          tables.t[code][et.scalar_type() == at::kChar ? 1 : 2].push_back(FoSplitLeaf{(float*)made[i].data_ptr(), const_cast<void*>(pt.const_data_ptr()), const_cast<void*>(et.const_data_ptr()), (uint64_t)pt.numel()});
+        }
+        return tables.launch(s, api.reconstruct);
+      })))
+    return nullptr;
+  std::vector<Ref> out(n);
+  for (int i = 0; i < n; ++i) out[i] = made[i].defined() ? Ref(THPVariable_Wrap(std::move(made[i]))) : Ref(THPVariable_Wrap(tables.in[2 * i]));
   return build(tree, out);
 }
 
@@ -817,27 +862,35 @@ PyObject* split(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (code < 0) Py_RETURN_NONE;
     if (code == FO_F32 || ecc_bits == 0) ++markers;
   }
-  at::Tensor zeros;  // the 0-d markers of leaves without ECC, cleared at once
-  if (markers > 0) zeros = at::zeros({markers}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, (c10::DeviceIndex)device)));
   SplitTables tables;
-  std::vector<Ref> lp(n), ecc(n);
-  int used = 0;
+  std::vector<at::ScalarType> dtype(n);
   for (int i = 0; i < n; ++i) {
-    const at::Tensor *wt = plain_tensor(w[i]), *lt = plain_tensor(like[i]);
-    const int code = dtype_code(lt->scalar_type());
-    if (code == FO_F32 || ecc_bits == 0) ecc[i] = Ref(THPVariable_Wrap(zeros.select(0, used++)));
-    if (code == FO_F32) {
-      lp[i] = Ref::borrow(w[i]);
-      continue;
-    }
-    at::Tensor t = empty_like_on(wt->sizes(), lt->scalar_type(), device), e;
-    if (ecc_bits != 0) e = empty_like_on(wt->sizes(), ecc_bits == 8 ? at::kChar : at::kShort, device);
-    tables.t[code][ecc_bits / 8].push_back(FoSplitLeaf{(float*)const_cast<void*>(wt->const_data_ptr()), t.data_ptr(), ecc_bits != 0 ? e.data_ptr() : nullptr, (uint64_t)wt->numel()});
-    lp[i] = Ref(THPVariable_Wrap(std::move(t)));
-    if (ecc_bits != 0) ecc[i] = Ref(THPVariable_Wrap(std::move(e)));
+    tables.in.push_back(*plain_tensor(w[i]));
+    dtype[i] = plain_tensor(like[i])->scalar_type();
   }
-  if (!tables.launch(device, api.split)) return nullptr;
-  Ref x(build(tree, lp)), y(build(tree, ecc));
+  std::vector<at::Tensor> lp(n), ecc(n);
+  if (!ok(on_device(device, [&](cudaStream_t s) {
+        at::Tensor zeros;  // the 0-d markers of leaves without ECC, cleared at once
+        if (markers > 0) zeros = at::zeros({markers}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, (c10::DeviceIndex)device)));
+        int used = 0;
+        for (int i = 0; i < n; ++i) {
+          const at::Tensor& wt = tables.in[i];
+          const int code = dtype_code(dtype[i]);
+          if (code == FO_F32 || ecc_bits == 0) ecc[i] = zeros.select(0, used++);
+          if (code == FO_F32) continue;
+          lp[i] = empty_like_on(wt.sizes(), dtype[i], device);
+          if (ecc_bits != 0) ecc[i] = empty_like_on(wt.sizes(), ecc_bits == 8 ? at::kChar : at::kShort, device);
+          tables.t[code][ecc_bits / 8].push_back(FoSplitLeaf{(float*)const_cast<void*>(wt.const_data_ptr()), lp[i].data_ptr(), ecc_bits != 0 ? ecc[i].data_ptr() : nullptr, (uint64_t)wt.numel()});
+        }
+        return tables.launch(s, api.split);
+      })))
+    return nullptr;
+  std::vector<Ref> new_p(n), new_e(n);
+  for (int i = 0; i < n; ++i) {
+    new_p[i] = lp[i].defined() ? Ref(THPVariable_Wrap(std::move(lp[i]))) : Ref(THPVariable_Wrap(tables.in[i]));
+    new_e[i] = Ref(THPVariable_Wrap(std::move(ecc[i])));
+  }
+  Ref x(build(tree, new_p)), y(build(tree, new_e));
   return x.p == nullptr || y.p == nullptr ? nullptr : PyTuple_Pack(2, x.p, y.p);
 }
 
@@ -845,18 +898,21 @@ PyObject* split(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 // quantize(x, group size, variance) -> QuantizedArray, or None
 PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "quantize takes 3 arguments"); return nullptr; }
-  const at::Tensor* x = plain_tensor(a[0]);
-  if (x == nullptr || !x->is_cuda() || x->scalar_type() != at::kFloat || !x->is_contiguous() || !PyLong_CheckExact(a[1])) Py_RETURN_NONE;
+  const at::Tensor* given = plain_tensor(a[0]);
+  if (given == nullptr || !given->is_cuda() || given->scalar_type() != at::kFloat || !given->is_contiguous() || !PyLong_CheckExact(a[1])) Py_RETURN_NONE;
   const long g = PyLong_AsLong(a[1]);
   if (g < 1 || g > 1024) Py_RETURN_NONE;
   const bool variance = a[2] == Py_True;
-  const int device = x->device().index();
-  const int64_t n = x->numel();
-  at::Tensor values = empty_like_on(x->sizes(), variance ? at::kByte : at::kChar, device), scales = empty_like_on({(n + g - 1) / g}, at::kHalf, device);
-  if (!on_device(device, [&](cudaStream_t s) {
-        return ok(variance ? api.quantize_v((const float*)x->const_data_ptr(), (uint8_t*)values.data_ptr(), scales.data_ptr(), (uint64_t)n, (int32_t)g, 0, s)
-                           : api.quantize_m((const float*)x->const_data_ptr(), (int8_t*)values.data_ptr(), scales.data_ptr(), (uint64_t)n, (int32_t)g, 0, s));
-      }))
+  const at::Tensor x = *given;  // (a reference: the GIL is released below)
+  const int device = x.device().index();
+  const int64_t n = x.numel();
+  at::Tensor values, scales;
+  if (!ok(on_device(device, [&](cudaStream_t s) {
+        values = empty_like_on(x.sizes(), variance ? at::kByte : at::kChar, device);
+        scales = empty_like_on({(n + g - 1) / g}, at::kHalf, device);
+        return variance ? api.quantize_v((const float*)x.const_data_ptr(), (uint8_t*)values.data_ptr(), scales.data_ptr(), (uint64_t)n, (int32_t)g, 0, s)
+                        : api.quantize_m((const float*)x.const_data_ptr(), (int8_t*)values.data_ptr(), scales.data_ptr(), (uint64_t)n, (int32_t)g, 0, s);
+      })))
     return nullptr;
   PyObject* t = PyTuple_New(2);
   if (t == nullptr) return nullptr;
@@ -875,12 +931,14 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (v == nullptr || sc == nullptr || g < 1 || !v->is_cuda() || !sc->is_cuda() || v->device() != sc->device() || v->element_size() != 1 || sc->scalar_type() != at::kHalf ||
       !v->is_contiguous() || !sc->is_contiguous() || sc->numel() < (v->numel() + g - 1) / g)
     Py_RETURN_NONE;
-  const int device = v->device().index();
-  at::Tensor out = empty_like_on(v->sizes(), at::kFloat, device);
-  if (!on_device(device, [&](cudaStream_t s) {
-        return ok(variance ? api.dequantize_v((const uint8_t*)v->const_data_ptr(), sc->const_data_ptr(), (float*)out.data_ptr(), (uint64_t)v->numel(), (int32_t)g, s)
-                           : api.dequantize_m((const int8_t*)v->const_data_ptr(), sc->const_data_ptr(), (float*)out.data_ptr(), (uint64_t)v->numel(), (int32_t)g, s));
-      }))
+  const at::Tensor codes = *v, scales = *sc;  // (references: the GIL is released below)
+  const int device = codes.device().index();
+  at::Tensor out;
+  if (!ok(on_device(device, [&](cudaStream_t s) {
+        out = empty_like_on(codes.sizes(), at::kFloat, device);
+        return variance ? api.dequantize_v((const uint8_t*)codes.const_data_ptr(), scales.const_data_ptr(), (float*)out.data_ptr(), (uint64_t)codes.numel(), (int32_t)g, s)
+                        : api.dequantize_m((const int8_t*)codes.const_data_ptr(), scales.const_data_ptr(), (float*)out.data_ptr(), (uint64_t)codes.numel(), (int32_t)g, s);
+      })))
     return nullptr;
   return THPVariable_Wrap(std::move(out));
 }

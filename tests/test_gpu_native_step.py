@@ -294,3 +294,41 @@ def test_callbacks_that_touch_the_trees(where, donate):
         if donate:
             p = dict(p)  # a container of its own for the next callback
         _same((p, s.mu, s.nu, s.ecc), (q, t.mu, t.nu, t.ecc))
+
+
+def test_the_gil_is_released_around_launches():
+    """Every call of the host extension into the library, with the library's function replaced by PyGILState_Check: 1, which reads as an
+    invalid argument, where the calling thread holds the GIL."""
+    import ctypes
+
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from flashoptim_jax_b200 import _lib, clipping
+
+    host, lib = _lib.host(), _lib.lib()
+    names = ("fo_step_ex", "fo_sq_norm_mixed", "fo_split_many", "fo_reconstruct_many", "fo_quantize_momentum", "fo_quantize_variance",
+             "fo_dequantize_momentum", "fo_dequantize_variance", "fo_status_string", "fo_last_error")
+    table = {name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in names}
+    check = ctypes.cast(ctypes.pythonapi.PyGILState_Check, ctypes.c_void_p).value
+    p = {"w": torch.ones(64, device="cuda", dtype=torch.bfloat16)}
+    steps = []
+    for donate in (False, True):
+        tx = fo.flash_adamw(donate=donate)
+        q, s = p, tx.init(p)
+        for _ in range(2):
+            q, s = tx.step(q, s, p)
+        steps.append((tx, q, s))
+    x = torch.ones(64, device="cuda")
+    codes = fo.quantize_momentum(x)
+    lp, ecc = fo.set_fp32_params({"w": x}, p)
+    host.bind({**table, **{name: check for name in names[:8]}}, fo.QuantizedArray)
+    try:
+        for tx, q, s in steps:
+            tx.step(q, s, p)
+        clipping.global_sq_norm(p)
+        fo.set_fp32_params({"w": x}, p)
+        fo.reconstruct_weights(lp, ecc)
+        fo.quantize_momentum(x), fo.quantize_variance(x), fo.dequantize_momentum(codes), fo.dequantize_variance(codes)
+    finally:
+        host.bind(table, fo.QuantizedArray)
