@@ -340,14 +340,14 @@ class NativeStep:
                 return hit
         return None
 
-    def remember(self, params: Any, path_leaves, work: List[LeafWork], configs: List[Dict[str, Any]], n_states: int) -> None:
-        """Compile the step the general path has just taken."""
+    def remember(self, params: Any, path_leaves, work: List[LeafWork], configs: List[Dict[str, Any]], n_states: int, resolver: GroupResolver) -> None:
+        """Compile the step the general path has just taken; `resolver` is where its configs came from."""
         if _observer is not None:
             return
         if self.wait:  # steps of this kind keep missing their plans: making them is not free
             self.wait -= 1
             return
-        self.backoff = min(2 * self.backoff + 1, 1023)
+        self.backoff = min(2 * self.backoff + 1, 31)
         self.wait = self.backoff - 1
         if not work or any(w.bucket[0] != work[0].bucket[0] for w in work):
             return
@@ -358,11 +358,12 @@ class NativeStep:
                 group_of[id(c)] = len(groups)
                 groups.append(c)
         hypers = []
+        index_of = resolver.index_of()
         for c in groups:
             if not all(type(c[k]) in (float, int) for k in ("weight_decay", "b1", "b2", "eps", "momentum", "dampening") if k in c):
                 return
             _, wd, b1, b2, omb1, omb2, eps, _, _, flags = self.hyper_of_config(c)
-            hypers.append((c["learning_rate"], float(wd), float(b1), float(b2), float(omb1), float(omb2), float(eps), int(flags)))
+            hypers.append((c["learning_rate"], float(wd), float(b1), float(b2), float(omb1), float(omb2), float(eps), int(flags), index_of[id(c)]))
         calls: List[Tuple[Tuple[Any, ...], List[int]]] = []
         open_call: Dict[Tuple[Any, ...], int] = {}
         leaves = []

@@ -112,7 +112,7 @@ def _make_adam_transform(learning_rate, b1, b2, eps, weight_decay, quantize, mas
         new_state = FlashAdamState(count=torch.tensor(count, dtype=torch.int32), mu=treedef.unflatten(new_m),
                                    nu=treedef.unflatten(new_v), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        native.remember(params, param_pl, work, configs, 3)
+        native.remember(params, param_pl, work, configs, 3, resolve)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

@@ -252,7 +252,8 @@ struct LeafSpec {
   int ecc_bits = 0, state = 0, group = 0, call = 0, at = 0;
 };
 struct Group {
-  Ref lr;
+  Ref lr;      // the learning rate, unless the watched dict has one
+  int dict;    // which of the watched dicts the group comes from, or -1
   float wd, b1, b2, omb1, omb2, eps;
   double beta1, beta2;  // as fp32, for the bias corrections
   uint32_t flags;
@@ -269,6 +270,7 @@ struct Watched {  // a param-group dict as it was when the plan was made
   Ref dict;
   std::vector<Ref> keys, values;
   Ref items;        // a list of selectors: its items then
+  int lr = -1;      // position of the learning rate, if it has one
 };
 struct Plan {
   int opt = 0, device = 0, n_states = 0;
@@ -288,6 +290,7 @@ struct Plan {
   std::vector<PyObject*> p, g;     // scratch (borrowed; run() holds references for as long as it needs them)
   std::vector<std::vector<PyObject*>> s;
 };
+bool is_lr(PyObject* key) { return PyUnicode_CheckExact(key) && PyUnicode_CompareWithASCIIString(key, "learning_rate") == 0; }
 constexpr const char* kPlanName = "flashoptim_b200.plan";
 
 float f32(double x) { return (float)x; }
@@ -299,7 +302,7 @@ bool num(PyObject* t, Py_ssize_t i, double& out) {
 
 // make_plan(opt, donate, device, params, n_states, leaves, groups, calls, param_groups, watched, selectors, paths, membership, resolve)
 //   leaves: tuples (shape, param dtype code, grad dtype code, ecc bits, state, group size, group, call, position)
-//   groups: tuples (lr, weight decay, b1, b2, 1 - b1, 1 - b2, eps, flags)
+//   groups: tuples (default lr, weight decay, b1, b2, 1 - b1, 1 - b2, eps, flags, position of its dict in watched or -1)
 //   calls:  tuples (param dtype code, grad dtype code, ecc bits, state, group size, (group of each hyper set))
 PyObject* make_plan(PyObject*, PyObject* args) {
   PyObject *params, *leaves, *groups, *calls, *param_groups, *watched, *selectors, *paths, *membership, *resolve;
@@ -364,6 +367,8 @@ PyObject* make_plan(PyObject*, PyObject* args) {
     gr.wd = f32(v[0]); gr.b1 = f32(v[1]); gr.b2 = f32(v[2]); gr.omb1 = f32(v[3]); gr.omb2 = f32(v[4]); gr.eps = f32(v[5]);
     gr.beta1 = (double)gr.b1; gr.beta2 = (double)gr.b2;
     gr.flags = (uint32_t)PyLong_AsUnsignedLong(PyTuple_GET_ITEM(t, 7));
+    gr.dict = (int)PyLong_AsLong(PyTuple_GET_ITEM(t, 8));
+    if (gr.dict >= (int)PyTuple_GET_SIZE(watched)) Py_RETURN_NONE;
     plan->groups.push_back(std::move(gr));
   }
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(watched); ++i) {
@@ -374,8 +379,10 @@ PyObject* make_plan(PyObject*, PyObject* args) {
     Py_ssize_t pos = 0;
     PyObject *k, *v;
     while (PyDict_Next(d, &pos, &k, &v)) {
+      if (is_lr(k)) w.lr = (int)w.keys.size();
       w.keys.push_back(Ref::borrow(k));
       w.values.push_back(Ref::borrow(v));
+      if ((int)w.keys.size() - 1 == w.lr) continue;
       if (PyList_CheckExact(v)) {
         if (w.items.p != nullptr) Py_RETURN_NONE;
         w.items = Ref(PyList_AsTuple(v));
@@ -407,7 +414,8 @@ PyObject* make_plan(PyObject*, PyObject* args) {
   return PyCapsule_New(plan.release(), kPlanName, [](PyObject* c) { delete (Plan*)PyCapsule_GetPointer(c, kPlanName); });
 }
 
-// are the optimizer's param_groups what they were?
+// Are the optimizer's param_groups what they were?  (Learning rates aside: a program may write one before every step, and the
+// step reads it.)
 bool groups_unchanged(const Plan& plan) {
   PyObject* pg = plan.param_groups.p;
   const Py_ssize_t size = pg == Py_None ? 0 : PyList_CheckExact(pg) ? PyList_GET_SIZE(pg) : PyTuple_CheckExact(pg) ? PyTuple_GET_SIZE(pg) : -1;
@@ -420,7 +428,12 @@ bool groups_unchanged(const Plan& plan) {
     PyObject *k, *v;
     size_t j = 0;
     while (PyDict_Next(w.dict.p, &pos, &k, &v)) {
-      if (j >= w.keys.size() || k != w.keys[j].p || v != w.values[j].p) return false;
+      if (j >= w.keys.size() || k != w.keys[j].p) return false;
+      if ((int)j == w.lr) {
+        ++j;
+        continue;
+      }
+      if (v != w.values[j].p) return false;
       if (PyList_CheckExact(v)) {
         if (PyList_GET_SIZE(v) != PyTuple_GET_SIZE(w.items.p)) return false;
         for (Py_ssize_t q = 0; q < PyList_GET_SIZE(v); ++q)
@@ -628,8 +641,18 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const Held held(*plan);  // the leaves stay alive, whatever happens to the trees meanwhile
 
   std::vector<double> lr(plan->groups.size());
+  std::vector<Ref> lr_now;
   bool call = plan->dynamic;  // code of the user's
-  for (const Group& gr : plan->groups) call = call || !PyFloat_CheckExact(gr.lr.p);
+  for (const Group& gr : plan->groups) {
+    const Watched* w = gr.dict < 0 ? nullptr : &plan->watched[gr.dict];
+    PyObject* value = w == nullptr || w->lr < 0 ? gr.lr.p : PyDict_GetItemWithError(w->dict.p, w->keys[w->lr].p);
+    if (value == nullptr) {
+      if (PyErr_Occurred()) return nullptr;
+      Py_RETURN_NONE;
+    }
+    lr_now.push_back(Ref::borrow(value));
+    call = call || !PyFloat_CheckExact(value);
+  }
   if (call && !plausible(*plan)) Py_RETURN_NONE;
   if (plan->dynamic) {
     const int same = membership_unchanged(*plan);
@@ -637,7 +660,7 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (same == 0) Py_RETURN_NONE;
   }
   for (size_t i = 0; i < lr.size(); ++i) {
-    PyObject* const value = plan->groups[i].lr.p;
+    PyObject* const value = lr_now[i].p;
     if (PyFloat_CheckExact(value)) {
       lr[i] = PyFloat_AS_DOUBLE(value);
       continue;

@@ -94,7 +94,7 @@ def flash_lion(learning_rate=1e-4, b1: float = 0.9, b2: float = 0.99, weight_dec
         new_state = FlashLionState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32),
                                    mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        native.remember(params, param_pl, work, configs, 2)
+        native.remember(params, param_pl, work, configs, 2, resolve)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

@@ -118,7 +118,7 @@ def _make_sgd_transform(learning_rate, momentum, dampening, weight_decay, nester
         new_state = FlashSGDState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32),
                                   mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        native.remember(params, param_pl, work, configs, 2)
+        native.remember(params, param_pl, work, configs, 2, resolve)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

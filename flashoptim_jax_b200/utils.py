@@ -111,6 +111,10 @@ class GroupResolver:
             self._configs[index] = config
         return config
 
+    def index_of(self) -> Dict[int, int]:
+        """Group index (-1: the defaults) of each config handed out, by the config's id."""
+        return {id(config): index for index, config in self._configs.items()}
+
 
 # ---- validation (utils.py:157-266) ----------------------------------------------------------
 

@@ -332,3 +332,40 @@ def test_the_gil_is_released_around_launches():
         fo.quantize_momentum(x), fo.quantize_variance(x), fo.dequantize_momentum(codes), fo.dequantize_variance(codes)
     finally:
         host.bind(table, fo.QuantizedArray)
+
+
+@contextlib.contextmanager
+def _only_planned_steps(monkeypatch):
+    from flashoptim_jax_b200 import _engine as eng
+
+    def refuse(*a, **k):
+        raise AssertionError("the general path took a step")
+
+    with monkeypatch.context() as m:
+        m.setattr(eng, "launch", refuse)
+        yield
+
+
+@pytest.mark.parametrize("donate", [False, True])
+def test_learning_rates_written_before_every_step(donate, monkeypatch):
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    groups, plain = [[{"params": "bias", "learning_rate": 1e-2, "weight_decay": 0.0}, {"params": "a/w", "learning_rate": lambda c: 1e-3}] for _ in range(2)]
+    tx, ref = fo.flash_lion(learning_rate=1e-4, param_groups=groups, donate=donate), fo.flash_lion(learning_rate=1e-4, param_groups=plain)
+    p, q = _params(), _params()
+    s, t = tx.init(p), ref.init(q)
+    p, s = tx.step(p, s, _grads(q, 9))
+    q, t = ref.step(q, t, _grads(q, 9))
+    rates = [3e-2, 1, torch.tensor(2e-2), lambda c: 1e-2 * int(c), 0.0, 5e-3]
+    grads = [_grads(_params(), k) for k in range(len(rates))]
+    with _only_planned_steps(monkeypatch):
+        for k, rate in enumerate(rates):
+            groups[0]["learning_rate"], groups[1]["learning_rate"] = rate, rates[-1 - k]
+            p, s = tx.step(p, s, grads[k])
+    for k, rate in enumerate(rates):
+        plain[0]["learning_rate"], plain[1]["learning_rate"] = rate, rates[-1 - k]
+        with _general_path():
+            q, t = ref.step(q, t, grads[k])
+    _same((p, s.mu, s.ecc), (q, t.mu, t.ecc))
