@@ -22,6 +22,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/flashoptim_b200.h"
@@ -99,15 +100,16 @@ bool compile(PyObject* x, Node& n, int& leaves) {
       return false;  // (left to the Python walk)
     }
     n.children.resize(size);
-    n.seen.resize(size);
+    std::unordered_map<PyObject*, int> place;
+    place.reserve(size);
     for (Py_ssize_t i = 0; i < size; ++i) {
       PyObject* k = PyList_GET_ITEM(keys.p, i);
       n.keys.push_back(Ref::borrow(k));
       PyObject* v = PyDict_GetItemWithError(x, k);
       if (v == nullptr || !compile(v, n.children[i], leaves)) return false;
-      for (Py_ssize_t j = 0; j < size; ++j)
-        if (n.seen_keys[j].p == k) n.seen[j] = (int)i;
+      place[k] = (int)i;
     }
+    for (const Ref& k : n.seen_keys) n.seen.push_back(place[k.p]);
   } else if (PyList_CheckExact(x) || PyTuple_CheckExact(x) || is_named(x)) {
     n.kind = PyList_CheckExact(x) ? Node::kList : PyTuple_CheckExact(x) ? Node::kTuple : Node::kNamed;
     if (n.kind == Node::kNamed) n.type = Py_TYPE(x);

@@ -1,0 +1,28 @@
+"""The host extension (csrc/fo_host.cc) where it needs no GPU: walks over trees that it hands back to the Python walk (their
+leaves are no CUDA tensors) or that it has to refuse, and the bookkeeping of compiled step plans around it."""
+
+import time
+
+import pytest
+import torch
+
+from flashoptim_jax_b200 import _engine as eng
+from flashoptim_jax_b200 import _lib
+
+
+def test_trees_are_compiled_in_linear_time():
+    """set_fp32_params compiles the tree on every call: 16 times the keys may take 16 times as long (64 allows for the sort and the
+    cache), not 256 times."""
+    host = _lib.host()
+
+    def best(n):
+        tree = {f"{i * 7919 % n:06d}": None for i in range(n)}  # inserted out of order
+        times = []
+        for _ in range(5):
+            t = time.perf_counter()
+            assert host.split(tree, tree, 8) is None
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    best(100)
+    assert best(32000) < 64 * best(2000)
