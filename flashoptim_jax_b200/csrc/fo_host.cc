@@ -879,13 +879,10 @@ PyObject* split(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   const int device = one_device(w, -1);
   if (device < 0) Py_RETURN_NONE;
-  int markers = 0;
   for (int i = 0; i < n; ++i) {
     const at::Tensor *wt = plain_tensor(w[i]), *lt = plain_tensor(like[i]);
     if (lt == nullptr || wt->scalar_type() != at::kFloat || !wt->is_contiguous()) Py_RETURN_NONE;
-    const int code = dtype_code(lt->scalar_type());
-    if (code < 0) Py_RETURN_NONE;
-    if (code == FO_F32 || ecc_bits == 0) ++markers;
+    if (dtype_code(lt->scalar_type()) < 0) Py_RETURN_NONE;
   }
   SplitTables tables;
   std::vector<at::ScalarType> dtype(n);
@@ -895,18 +892,17 @@ PyObject* split(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   std::vector<at::Tensor> lp(n), ecc(n);
   if (!ok(on_device(device, [&](cudaStream_t s) {
-        at::Tensor zeros;  // the 0-d markers of leaves without ECC, cleared at once
-        if (markers > 0) zeros = at::zeros({markers}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, (c10::DeviceIndex)device)));
-        int used = 0;
+        std::vector<at::Tensor> markers;  // 0-d zeros in the place of an absent ECC, each with storage of its own
         for (int i = 0; i < n; ++i) {
           const at::Tensor& wt = tables.in[i];
           const int code = dtype_code(dtype[i]);
-          if (code == FO_F32 || ecc_bits == 0) ecc[i] = zeros.select(0, used++);
+          if (code == FO_F32 || ecc_bits == 0) markers.push_back(ecc[i] = empty_like_on({}, at::kInt, device));
           if (code == FO_F32) continue;
           lp[i] = empty_like_on(wt.sizes(), dtype[i], device);
           if (ecc_bits != 0) ecc[i] = empty_like_on(wt.sizes(), ecc_bits == 8 ? at::kChar : at::kShort, device);
           tables.t[code][ecc_bits / 8].push_back(FoSplitLeaf{(float*)const_cast<void*>(wt.const_data_ptr()), lp[i].data_ptr(), ecc_bits != 0 ? ecc[i].data_ptr() : nullptr, (uint64_t)wt.numel()});
         }
+        if (!markers.empty()) at::_foreach_zero_(markers);  // (one launch)
         return tables.launch(s, api.split);
       })))
     return nullptr;

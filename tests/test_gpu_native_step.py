@@ -369,3 +369,18 @@ def test_learning_rates_written_before_every_step(donate, monkeypatch):
         with _general_path():
             q, t = ref.step(q, t, grads[k])
     _same((p, s.mu, s.ecc), (q, t.mu, t.ecc))
+
+
+def test_markers_have_storage_of_their_own():
+    """The 0-d zeros of leaves without an error-correction code: none shares memory, or a saved file, with another."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    w = {k: torch.ones(5, device="cuda") for k in "abc"}
+    like = {"a": w["a"], "b": w["b"], "c": torch.empty(5, device="cuda", dtype=torch.bfloat16)}
+    for bits, count in ((24, 2), (None, 3)):
+        ecc = fo.set_fp32_params(w, like, master_weight_bits=bits)[1]
+        markers = [e for e in ecc.values() if e.dim() == 0]
+        assert len(markers) == count and all(e.dtype == torch.int32 and int(e) == 0 and e.untyped_storage().nbytes() == 4 for e in markers)
+        assert len({e.data_ptr() for e in markers}) == count
