@@ -322,7 +322,7 @@ class NativeStep:
     def __init__(self, opt: int, donate: bool, defaults: Dict[str, Any], param_groups: Any, hyper_of_config):
         self.opt, self.donate, self.defaults, self.param_groups = opt, bool(donate), defaults, param_groups
         self.hyper_of_config = hyper_of_config  # config -> hyper-parameter tuple (lr and bias corrections are filled in per step)
-        self.plans: List[Any] = []
+        self.plans: Tuple[Any, ...] = ()  # (run, plan), the last one used in front
         self.wait = self.backoff = 0
 
     def run(self, params: Any, count: Any, states: Tuple[Any, ...], grads: Any):
@@ -331,11 +331,12 @@ class NativeStep:
             return None
         clip = getattr(_clip, "value", None)
         sq, max_norm = (0, 0.0) if clip is None else (clip[0].data_ptr(), clip[1])
-        for i, (host_run, plan) in enumerate(self.plans):
-            hit = host_run(plan, params, count, states, grads, sq, max_norm)
+        plans = self.plans  # (replaced as a whole, never changed: several threads may step)
+        for entry in plans:
+            hit = entry[0](entry[1], params, count, states, grads, sq, max_norm)
             if hit is not None:
-                if i:
-                    self.plans.insert(0, self.plans.pop(i))
+                if entry is not plans[0]:
+                    self.plans = (entry, *(e for e in self.plans if e is not entry))[:self.MOST_PLANS]
                 self.backoff = 0
                 return hit
         return None
@@ -395,8 +396,7 @@ class NativeStep:
             tuple((*bucket[1:5], bucket[5], tuple(slots)) for bucket, slots in calls), param_groups, watched,
             tuple(selectors), tuple(path for path, _ in path_leaves), tuple(member(path, leaf) for path, leaf in path_leaves), _resolve_learning_rate)
         if plan is not None:
-            self.plans.insert(0, (host.run, plan))
-            del self.plans[self.MOST_PLANS:]
+            self.plans = ((host.run, plan), *self.plans)[:self.MOST_PLANS]
 
 
 def launch(opt: int, work: List[LeafWork], peer_param_offsets: Optional[List[int]] = None,

@@ -26,3 +26,17 @@ def test_trees_are_compiled_in_linear_time():
 
     best(100)
     assert best(32000) < 64 * best(2000)
+
+
+def test_plans_reordered_by_another_thread_do_not_lose_a_step():
+    """While one thread's step runs on the second plan, another moves that plan to the front or drops plans."""
+    native = eng.NativeStep(_lib.FO_OPT_ADAM, True, {}, None, None)
+    miss = lambda *a: None
+
+    def run(*a):
+        native.plans = type(native.plans)(native.plans[1:2])  # what the other thread does meanwhile
+        return "the step"
+
+    native.plans = type(native.plans)([(miss, 0), (miss, 1), (run, 2)])
+    assert native.run(None, None, (), None) == "the step"
+    assert (run, 2) in native.plans
