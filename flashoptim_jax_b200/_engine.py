@@ -342,7 +342,8 @@ class NativeStep:
         return None
 
     def remember(self, params: Any, path_leaves, work: List[LeafWork], configs: List[Dict[str, Any]], n_states: int, resolver: GroupResolver) -> None:
-        """Compile the step the general path has just taken; `resolver` is where its configs came from."""
+        """Compile the step that the general path is about to launch; `resolver` is where its configs came from.  Before the launch, and
+        without calling anything of the user's: what fails here fails while nothing has happened yet."""
         if _observer is not None:
             return
         if self.wait:  # steps of this kind keep missing their plans: making them is not free
@@ -382,7 +383,6 @@ class NativeStep:
             return
         param_groups = self.param_groups
         watched = tuple(param_groups or ())
-        member = GroupResolver(self.defaults, param_groups).member
         selectors = []
         for g in watched:
             spec = g["params"]
@@ -394,7 +394,7 @@ class NativeStep:
         plan = host.make_plan(
             self.opt, self.donate, work[0].bucket[0], params, n_states, tuple(leaves), tuple(hypers),
             tuple((*bucket[1:5], bucket[5], tuple(slots)) for bucket, slots in calls), param_groups, watched,
-            tuple(selectors), tuple(path for path, _ in path_leaves), tuple(member(path, leaf) for path, leaf in path_leaves), _resolve_learning_rate)
+            tuple(selectors), tuple(path for path, _ in path_leaves), tuple(index_of[id(c)] for c in configs), _resolve_learning_rate)
         if plan is not None:
             self.plans = ((host.run, plan), *self.plans)[:self.MOST_PLANS]
 

@@ -108,11 +108,11 @@ def _make_adam_transform(learning_rate, b1, b2, eps, weight_decay, quantize, mas
             work.append(w)
             configs.append(config)
             new_p.append(p_out); new_e.append(e_out); new_m.append(m_out); new_v.append(v_out)
+        native.remember(params, param_pl, work, configs, 3, resolve)
         eng.launch(_lib.FO_OPT_ADAM, work)
         new_state = FlashAdamState(count=torch.tensor(count, dtype=torch.int32), mu=treedef.unflatten(new_m),
                                    nu=treedef.unflatten(new_v), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        native.remember(params, param_pl, work, configs, 3, resolve)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

@@ -3,7 +3,7 @@
 The step-kernel family is split into instantiation slices (optimizer x state kind x kernel)
 compiled from one source with different -D switches, so the build runs in parallel.
 Objects go to csrc/build/, the library to lib/.  Nothing is compiled at import time:
-call build_native() (or `python -m flashoptim_jax_b200.build`).
+call build_native() and build_host() (or `python -m flashoptim_jax_b200.build`, which does both).
 """
 
 from __future__ import annotations

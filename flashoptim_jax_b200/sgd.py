@@ -114,11 +114,11 @@ def _make_sgd_transform(learning_rate, momentum, dampening, weight_decay, nester
             work.append(w)
             configs.append(config)
             new_p.append(p_out); new_e.append(e_out); new_m.append(m_out)
+        native.remember(params, param_pl, work, configs, 2, resolve)
         eng.launch(_lib.FO_OPT_SGD, work)
         new_state = FlashSGDState(count=torch.tensor(int(old_count) + 1, dtype=torch.int32),
                                   mu=treedef.unflatten(new_m), ecc=treedef.unflatten(new_e))
         new_params = treedef.unflatten(new_p)
-        native.remember(params, param_pl, work, configs, 2, resolve)
         return new_params, new_state
 
     return utils.FlashOptimizer(init=init_fn, step=capturable_step_fn if capturable else step_fn)

@@ -384,3 +384,52 @@ def test_markers_have_storage_of_their_own():
         markers = [e for e in ecc.values() if e.dim() == 0]
         assert len(markers) == count and all(e.dtype == torch.int32 and int(e) == 0 and e.untyped_storage().nbytes() == 4 for e in markers)
         assert len({e.data_ptr() for e in markers}) == count
+
+
+def test_selectors_that_read_values():
+    """Asked before the step and not after it; a donated step that changes the answer does not change what it used."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    asked = []
+
+    def large(path, leaf):
+        asked.append(path)
+        return bool((leaf > 0.995).all())
+
+    make = lambda: {"w": torch.ones(64, device="cuda", dtype=torch.bfloat16), "x": torch.ones(64, device="cuda")}
+    results = []
+    for donate in (False, True):
+        tx = fo.flash_sgd(learning_rate=1e-2, momentum=0.0, donate=donate, param_groups=[{"params": large, "learning_rate": 2e-2}])
+        p = make()
+        s = tx.init(p)
+        for _ in range(4):
+            asked.clear()
+            p, s = tx.step(p, s, {k: torch.ones_like(v) for k, v in p.items()})
+            assert asked[-2:] == [("w",), ("x",)]  # (before them perhaps for a plan that did not fit)
+        results.append(p)
+    _same(*results)
+
+
+@pytest.mark.parametrize("name", ["flash_adamw", "flash_lion", "flash_sgd"])
+def test_a_step_that_cannot_be_planned_has_no_effect(name, monkeypatch):
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from flashoptim_jax_b200 import _lib
+
+    def missing():
+        raise _lib.NativeLibraryError("no extension")
+
+    tx = getattr(fo, name)(donate=True)
+    p = {"w": torch.ones(64, device="cuda", dtype=torch.bfloat16)}
+    s = tx.init(p)
+    before = [x.clone() for x in _leaves((p, s.mu))]
+    with monkeypatch.context() as m:
+        m.setattr(_lib, "host", missing)
+        with pytest.raises(_lib.NativeLibraryError):
+            tx.step(p, s, p)
+    _same((p, s.mu), before)
+    p, s = tx.step(p, s, {"w": torch.ones_like(p["w"])})
+    assert int(s.count) == 1
