@@ -775,7 +775,7 @@ bool collect(PyObject* x, std::vector<at::Tensor>& out) {
 PyObject* sq_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 1) { PyErr_SetString(PyExc_TypeError, "sq_norm takes 1 argument"); return nullptr; }
   std::vector<at::Tensor> t;  // (references: the GIL is released below)
-  if (!collect(a[0], t) || t.empty()) Py_RETURN_NONE;
+  if (!collect(a[0], t) || std::all_of(t.begin(), t.end(), [](const at::Tensor& x) { return x.numel() == 0; })) Py_RETURN_NONE;  // (an error, reported there)
   const int device = t[0].device().index();
   std::vector<FoArray> arrays(t.size());
   std::vector<int32_t> dtypes(t.size());

@@ -120,3 +120,15 @@ def test_sum_of_squares_at_the_edges_of_its_chunks(dtype, chunk):
     for a, w in zip(arrays, want):
         assert abs(float(clipping.global_sq_norm({"a": a})) - w) <= 8 * 2.0**-24 * w
     assert abs(float(clipping.global_sq_norm(arrays)) - sum(want)) <= 8 * 2.0**-24 * sum(want)
+
+
+def test_a_norm_of_nothing_is_an_error():
+    """No gradients, or none with an element: there is nothing to tell the device by, and no norm."""
+    import torch
+
+    from flashoptim_jax_b200 import clipping
+
+    for grads in ({}, {"a": torch.zeros(0, 3, device="cuda")}, [torch.zeros(0, device="cuda"), torch.zeros(0, device="cuda", dtype=torch.bfloat16)]):
+        with pytest.raises(ValueError):
+            clipping.global_sq_norm(grads)
+    assert float(clipping.global_sq_norm([torch.zeros(0, device="cuda"), torch.full((2,), 3.0, device="cuda")])) == 18.0
