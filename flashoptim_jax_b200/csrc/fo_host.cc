@@ -916,12 +916,18 @@ PyObject* split(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 }
 
 // ---- moment codecs ---------------------------------------------------------------------------------------------------
+long group_size(PyObject* x) {  // 0: not one the library's int32_t holds
+  int beyond = 0;
+  const long g = PyLong_AsLongAndOverflow(x, &beyond);
+  return beyond != 0 || g < 0 || g > INT32_MAX ? 0 : g;
+}
+
 // quantize(x, group size, variance) -> QuantizedArray, or None
 PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "quantize takes 3 arguments"); return nullptr; }
   const at::Tensor* given = plain_tensor(a[0]);
   if (given == nullptr || !given->is_cuda() || given->scalar_type() != at::kFloat || !given->is_contiguous() || !PyLong_CheckExact(a[1])) Py_RETURN_NONE;
-  const long g = PyLong_AsLong(a[1]);
+  const long g = group_size(a[1]);
   if (g < 1 || g > 1024) Py_RETURN_NONE;
   const bool variance = a[2] == Py_True;
   const at::Tensor x = *given;  // (a reference: the GIL is released below)
@@ -947,7 +953,7 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 3) { PyErr_SetString(PyExc_TypeError, "dequantize takes 3 arguments"); return nullptr; }
   if ((PyObject*)Py_TYPE(a[0]) != quantized_type || PyTuple_GET_SIZE(a[0]) != 2 || !PyLong_CheckExact(a[1])) Py_RETURN_NONE;
   const at::Tensor *v = plain_tensor(PyTuple_GET_ITEM(a[0], 0)), *sc = plain_tensor(PyTuple_GET_ITEM(a[0], 1));
-  const long g = PyLong_AsLong(a[1]);
+  const long g = group_size(a[1]);
   const bool variance = a[2] == Py_True;
   if (v == nullptr || sc == nullptr || g < 1 || !v->is_cuda() || !sc->is_cuda() || v->device() != sc->device() || v->element_size() != 1 || sc->scalar_type() != at::kHalf ||
       !v->is_contiguous() || !sc->is_contiguous() || sc->numel() < (v->numel() + g - 1) / g)

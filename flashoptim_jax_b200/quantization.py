@@ -26,12 +26,21 @@ def _num_groups(n: int, group_size: int) -> int:
     return (n + group_size - 1) // group_size
 
 
+def _checked(group_size) -> int:
+    """A size the library's 32-bit argument holds (it refuses the ones it has no kernel for)."""
+    g = int(group_size)
+    if not 0 < g < 2**31:
+        raise ValueError(f"group_size {g}")
+    return g
+
+
 def _quantize(x, group_size: int, variance: bool) -> QuantizedArray:
     q = _lib.host().quantize(x, group_size, variance)  # None: something to convert first, or an error to report
     if q is not None:
         return q
     x = as_tensor(x)
     require_cuda(x, "x")
+    group_size = _checked(group_size)
     xf = x.to(torch.float32).contiguous()
     n = xf.numel()
     values = torch.empty(x.shape, dtype=torch.uint8 if variance else torch.int8, device=x.device)
@@ -48,6 +57,7 @@ def _dequantize(q: QuantizedArray, group_size: int, variance: bool) -> torch.Ten
         return out
     values, scales = q.values, q.scales
     require_cuda(values, "values")
+    group_size = _checked(group_size)
     values = values.contiguous()
     scales = scales.to(torch.float16).contiguous()
     out = torch.empty(values.shape, dtype=torch.float32, device=values.device)

@@ -144,3 +144,18 @@ def test_trees_with_unaligned_leaves(leaves, bits):
     for a, e, back, (b, c) in zip(lp, ecc, fo.reconstruct_weights(lp2, ecc2), want):
         assert np.array_equal(H.bits(H.to_numpy(a)), H.bits(b)) and np.array_equal(H.to_numpy(e), c)
         assert np.array_equal(H.bits(H.to_numpy(back)), H.bits(O.reconstruct_leaf(b, c)))
+
+
+@pytest.mark.parametrize("group_size", [0, -1, 2**32 + 32, -(2**32) + 32, 2**70, -(2**70)])
+def test_group_sizes_beyond_the_library_s_integer_are_refused(group_size):
+    """(2**32 + 32 would arrive as 32: scales for one group, codes for thousands.)"""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    x = torch.ones(4096, device="cuda")
+    q = fo.quantize_momentum(x, 4096 // 4)
+    for call in (lambda: fo.quantize_momentum(x, group_size), lambda: fo.quantize_variance(x, group_size),
+                 lambda: fo.dequantize_momentum(q, group_size), lambda: fo.dequantize_variance(q, group_size)):
+        with pytest.raises(ValueError):
+            call()
