@@ -159,3 +159,15 @@ def test_group_sizes_beyond_the_library_s_integer_are_refused(group_size):
                  lambda: fo.dequantize_momentum(q, group_size), lambda: fo.dequantize_variance(q, group_size)):
         with pytest.raises(ValueError):
             call()
+
+
+def test_scales_of_another_group_size_are_refused():
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    q = fo.quantize_momentum(torch.ones(4096, device="cuda"), 128)
+    for bad in (q, q._replace(scales=q.scales.cpu()), q._replace(values=q.values.float())):
+        with pytest.raises(ValueError):
+            fo.dequantize_momentum(bad, 32)
+    assert torch.equal(fo.dequantize_momentum(q, 128), torch.ones(4096, device="cuda"))
