@@ -83,8 +83,19 @@ bool is_named(PyObject* x) {
   return has == 1;
 }
 
+// A container inside itself, or nested too deeply for the stack, is a RecursionError, as in the Python walk.  (The other walks follow
+// a compiled tree and go no deeper than that.)
+struct Deeper {
+  const bool ok = Py_EnterRecursiveCall(" while walking a pytree") == 0;
+  ~Deeper() {
+    if (ok) Py_LeaveRecursiveCall();
+  }
+};
+
 // false: a container this walk does not take (or, with an exception set, an error)
 bool compile(PyObject* x, Node& n, int& leaves) {
+  const Deeper deeper;
+  if (!deeper.ok) return false;
   n.first = leaves;
   if (x == Py_None) {
     n.kind = Node::kNone;
@@ -735,6 +746,8 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
 // ---- gradient norm -------------------------------------------------------------------------------------------------
 bool collect(PyObject* x, std::vector<at::Tensor>& out) {
+  const Deeper deeper;
+  if (!deeper.ok) return false;
   if (x == Py_None) return true;
   if (PyDict_CheckExact(x)) {
     // the order of the sum is that of the flattened tree
@@ -775,7 +788,9 @@ bool collect(PyObject* x, std::vector<at::Tensor>& out) {
 PyObject* sq_norm(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   if (nargs != 1) { PyErr_SetString(PyExc_TypeError, "sq_norm takes 1 argument"); return nullptr; }
   std::vector<at::Tensor> t;  // (references: the GIL is released below)
-  if (!collect(a[0], t) || std::all_of(t.begin(), t.end(), [](const at::Tensor& x) { return x.numel() == 0; })) Py_RETURN_NONE;  // (an error, reported there)
+  const bool taken = collect(a[0], t);
+  if (PyErr_Occurred()) return nullptr;
+  if (!taken || std::all_of(t.begin(), t.end(), [](const at::Tensor& x) { return x.numel() == 0; })) Py_RETURN_NONE;  // (an error, reported there)
   const int device = t[0].device().index();
   std::vector<FoArray> arrays(t.size());
   std::vector<int32_t> dtypes(t.size());

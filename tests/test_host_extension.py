@@ -40,3 +40,31 @@ def test_plans_reordered_by_another_thread_do_not_lose_a_step():
     native.plans = type(native.plans)([(miss, 0), (miss, 1), (run, 2)])
     assert native.run(None, None, (), None) == "the step"
     assert (run, 2) in native.plans
+
+
+def test_trees_without_an_end_are_a_recursion_error():
+    """In a process of its own: without the check the stack runs out."""
+    import os
+    import subprocess
+    import sys
+
+    code = """
+from flashoptim_jax_b200 import _lib
+h = _lib.host()
+a = []; a.append(a)
+b = {}; b["x"] = (b,)
+deep = None
+for _ in range(200000): deep = [deep]
+for tree in (a, b, deep):
+    for call in (lambda: h.sq_norm(tree), lambda: h.reconstruct(tree, tree), lambda: h.split(tree, tree, 8)):
+        try:
+            call()
+            raise SystemExit("accepted")
+        except RecursionError:
+            pass
+while deep is not None: deep = deep[0]
+print("refused")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "refused", (r.returncode, r.stderr[-500:])
