@@ -73,6 +73,7 @@ struct Node {
   std::vector<Ref> keys;             // kDict: flattening order
   std::vector<int> seen;             // kDict: position in flattening order of the k-th item in insertion order
   std::vector<Ref> seen_keys;        // kDict: keys in insertion order
+  PyTypeObject* key_type = nullptr;  // kDict: type of all its keys, if it is one
   std::vector<Node> children;
   int first = 0, count = 1;          // leaves
 };
@@ -121,6 +122,9 @@ bool compile(PyObject* x, Node& n, int& leaves) {
       place[k] = (int)i;
     }
     for (const Ref& k : n.seen_keys) n.seen.push_back(place[k.p]);
+    if (size > 0) n.key_type = Py_TYPE(n.keys[0].p);
+    for (const Ref& k : n.keys)
+      if (Py_TYPE(k.p) != n.key_type) n.key_type = nullptr;
   } else if (PyList_CheckExact(x) || PyTuple_CheckExact(x) || is_named(x)) {
     n.kind = PyList_CheckExact(x) ? Node::kList : PyTuple_CheckExact(x) ? Node::kTuple : Node::kNamed;
     if (n.kind == Node::kNamed) n.type = Py_TYPE(x);
@@ -159,6 +163,10 @@ bool walk(const Node& n, PyObject* x, PyObject** out) {
         ++j;
       }
       if (same) return true;
+      // Equal keys then, of the same type: 1 and True are equal, and selectors see different paths.
+      pos = 0;
+      while (PyDict_Next(x, &pos, &k, &v))
+        if (Py_TYPE(k) != n.key_type) return false;
       for (size_t i = 0; i < n.keys.size(); ++i) {
         v = PyDict_GetItemWithError(x, n.keys[i].p);
         if (v == nullptr || !walk(n.children[i], v, out)) return false;
@@ -765,10 +773,14 @@ bool collect(PyObject* x, std::vector<at::Tensor>& out) {
         if (!collect(v, out)) return false;
       return true;
     }
+    while (PyDict_Next(x, &pos, &k, &v))
+      if (!PyUnicode_CheckExact(k)) return false;
     Ref keys(PyDict_Keys(x));
-    if (keys.p == nullptr || PyList_Sort(keys.p) != 0) { PyErr_Clear(); return false; }
-    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(keys.p); ++i)
-      if (!collect(PyDict_GetItem(x, PyList_GET_ITEM(keys.p, i)), out)) return false;
+    if (keys.p == nullptr || PyList_Sort(keys.p) != 0) return false;
+    for (Py_ssize_t i = 0; i < PyList_GET_SIZE(keys.p); ++i) {
+      v = PyDict_GetItemWithError(x, PyList_GET_ITEM(keys.p, i));
+      if (v == nullptr || !collect(v, out)) return false;
+    }
     return true;
   }
   if (PyList_CheckExact(x) || PyTuple_Check(x)) {

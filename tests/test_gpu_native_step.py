@@ -433,3 +433,20 @@ def test_a_step_that_cannot_be_planned_has_no_effect(name, monkeypatch):
     _same((p, s.mu), before)
     p, s = tx.step(p, s, {"w": torch.ones_like(p["w"])})
     assert int(s.count) == 1
+
+
+def test_equal_keys_of_another_type_are_another_tree():
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    tx = fo.flash_lion(learning_rate=1e-2, param_groups=[{"params": "1", "learning_rate": 0.0}])
+    w, g = torch.ones(64, device="cuda"), torch.ones(64, device="cuda")
+    p = {1: w}
+    s = tx.init(p)
+    for _ in range(2):
+        p, s = tx.step(p, s, {1: g})
+    assert torch.equal(p[1], w)
+    t = type(s)(s.count, *({True: x[1]} for x in (s.mu, s.ecc)))
+    q, t = tx.step({True: p[1]}, t, {True: g})  # its path reads "True"
+    assert type(next(iter(q))) is bool and not torch.equal(q[True], w)

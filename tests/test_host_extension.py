@@ -68,3 +68,18 @@ print("refused")
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip() == "refused", (r.returncode, r.stderr[-500:])
+
+
+def test_keys_of_mixed_types_go_to_the_python_walk():
+    """Keys whose comparison is code of the user's, behind a key that is out of order."""
+
+    class Key:
+        def __lt__(self, other):
+            tree.clear()
+            return True
+
+        __gt__ = __lt__
+
+    tree = {"b": None, "a": None, Key(): None}
+    assert _lib.host().sq_norm(tree) is None
+    assert len(tree) == 3
