@@ -78,10 +78,18 @@ struct Node {
   int first = 0, count = 1;          // leaves
 };
 
+// A NamedTuple that is made of its items and nothing else: no __new__ or __init__ of its own (build() calls tuple.__new__), no metaclass,
+// no iteration of its own.  A subclass that adds one is left to the Python walk.
 bool is_named(PyObject* x) {
   if (!PyTuple_Check(x) || PyTuple_CheckExact(x)) return false;
-  const int has = PyObject_HasAttrString((PyObject*)Py_TYPE(x), "_fields");
-  return has == 1;
+  PyTypeObject* const type = Py_TYPE(x);
+  if (!Py_IS_TYPE((PyObject*)type, &PyType_Type) || type->tp_init != PyTuple_Type.tp_init || type->tp_iter != PyTuple_Type.tp_iter || type->tp_mro == nullptr) return false;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(type->tp_mro); ++i) {
+    PyObject* const d = ((PyTypeObject*)PyTuple_GET_ITEM(type->tp_mro, i))->tp_dict;
+    if (d == nullptr) return false;  // (tuple itself: nothing in front of it has _fields)
+    if (PyDict_GetItemString(d, "__new__") != nullptr) return PyDict_GetItemString(d, "_fields") != nullptr;
+  }
+  return false;
 }
 
 // A container inside itself, or nested too deeply for the stack, is a RecursionError, as in the Python walk.  (The other walks follow
@@ -783,7 +791,7 @@ bool collect(PyObject* x, std::vector<at::Tensor>& out) {
     }
     return true;
   }
-  if (PyList_CheckExact(x) || PyTuple_Check(x)) {
+  if (PyList_CheckExact(x) || PyTuple_CheckExact(x) || is_named(x)) {
     const Py_ssize_t size = PySequence_Fast_GET_SIZE(x);
     for (Py_ssize_t i = 0; i < size; ++i)
       if (!collect(PySequence_Fast_GET_ITEM(x, i), out)) return false;

@@ -58,7 +58,6 @@ def _dequantize(q: QuantizedArray, group_size: int, variance: bool) -> torch.Ten
     values, scales = q.values, q.scales
     require_cuda(values, "values")
     group_size = _checked(group_size)
-    require_cuda(scales, "scales")
     if scales.numel() < _num_groups(values.numel(), group_size) or scales.device != values.device or values.element_size() != 1:
         raise ValueError(f"{tuple(scales.shape)} scales do not fit codes of shape {tuple(values.shape)} in groups of {group_size}")
     values = values.contiguous()

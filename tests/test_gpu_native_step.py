@@ -450,3 +450,42 @@ def test_equal_keys_of_another_type_are_another_tree():
     t = type(s)(s.count, *({True: x[1]} for x in (s.mu, s.ecc)))
     q, t = tx.step({True: p[1]}, t, {True: g})  # its path reads "True"
     assert type(next(iter(q))) is bool and not torch.equal(q[True], w)
+
+
+class Checked(Pair):
+    """A NamedTuple with a constructor of its own."""
+
+    made = 0
+
+    def __new__(cls, kernel, bias):
+        Checked.made += 1
+        return super().__new__(cls, kernel, bias)
+
+
+class Plain(Pair):
+    pass
+
+
+def test_named_tuples_are_made_by_their_constructors():
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from flashoptim_jax_b200 import clipping
+
+    for kind in (Checked, Plain):
+        make = lambda: kind(torch.ones(64, device="cuda", dtype=torch.bfloat16), torch.ones(5, device="cuda"))
+        tx, ref = fo.flash_lion(learning_rate=1e-2), fo.flash_lion(learning_rate=1e-2)
+        p, q = make(), make()
+        s, t = tx.init(p), ref.init(q)
+        for k in range(3):
+            g = kind(*(0.1 * (k + 1) * torch.ones_like(x) for x in q))
+            Checked.made = 0
+            p, s = tx.step(p, s, g)
+            assert type(p) is kind and type(s.mu) is kind and (kind is Plain or Checked.made == 3)
+            with _general_path():
+                q, t = ref.step(q, t, g)
+            _same((p, s.mu, s.ecc), (q, t.mu, t.ecc))
+        sq = float(clipping.global_sq_norm(g))
+        assert abs(sq - sum(float((x.double() ** 2).sum()) for x in g)) <= 1e-6 * sq
+        w, ecc = fo.set_fp32_params(kind(*(x.float() for x in p)), p)
+        assert type(w) is kind and type(ecc) is kind and type(fo.reconstruct_weights(w, ecc)) is kind
