@@ -64,9 +64,15 @@ struct Ref {  // owning reference
 };
 
 PyObject* quantized_type = nullptr;  // QuantizedArray
+PyObject *ordered_type = nullptr, *default_type = nullptr;  // collections.OrderedDict and defaultdict
 
 // ---- pytrees -----------------------------------------------------------------------------------------------------
-// The containers of tree.py, exact types only (a subclass may redefine item access: the Python walk takes those).
+// The containers of tree.py, exact types and the two dicts of the standard library that keep dict's item access (another subclass may
+// redefine it: the Python walk takes those).
+bool is_dict(PyObject* x) {
+  PyObject* const type = (PyObject*)Py_TYPE(x);
+  return PyDict_CheckExact(x) || type == ordered_type || type == default_type;
+}
 struct Node {
   enum Kind { kLeaf, kNone, kDict, kList, kTuple, kNamed } kind = kLeaf;
   PyTypeObject* type = nullptr;      // kNamed
@@ -75,6 +81,7 @@ struct Node {
   std::vector<Ref> seen_keys;        // kDict: keys in insertion order
   PyTypeObject* key_type = nullptr;  // kDict: type of all its keys, if it is one
   std::vector<Node> children;
+  bool nested = false;               // a child is no leaf
   int first = 0, count = 1;          // leaves
 };
 
@@ -108,7 +115,7 @@ bool compile(PyObject* x, Node& n, int& leaves) {
   n.first = leaves;
   if (x == Py_None) {
     n.kind = Node::kNone;
-  } else if (PyDict_CheckExact(x)) {
+  } else if (is_dict(x)) {
     n.kind = Node::kDict;
     Ref keys(PyDict_Keys(x));
     if (keys.p == nullptr) return false;
@@ -146,6 +153,7 @@ bool compile(PyObject* x, Node& n, int& leaves) {
     ++leaves;
   }
   n.count = leaves - n.first;
+  for (const Node& c : n.children) n.nested = n.nested || c.kind != Node::kLeaf;
   return true;
 }
 
@@ -159,7 +167,7 @@ bool walk(const Node& n, PyObject* x, PyObject** out) {
     case Node::kNone:
       return x == Py_None;
     case Node::kDict: {
-      if (!PyDict_CheckExact(x) || PyDict_GET_SIZE(x) != (Py_ssize_t)n.keys.size()) return false;
+      if (!is_dict(x) || PyDict_GET_SIZE(x) != (Py_ssize_t)n.keys.size()) return false;
       // usually the very key objects in the very order: no look-up by hash
       Py_ssize_t pos = 0;
       PyObject *k, *v;
@@ -195,6 +203,21 @@ bool walk(const Node& n, PyObject* x, PyObject** out) {
       return true;
   }
   return false;
+}
+
+// is every dict of x, which walk() has taken, a dict and no subclass?
+bool plain(const Node& n, PyObject* x) {
+  if (n.kind == Node::kLeaf || n.kind == Node::kNone) return true;
+  if (n.kind != Node::kDict) {
+    for (size_t i = 0; i < n.children.size(); ++i)
+      if (!plain(n.children[i], n.kind == Node::kList ? PyList_GET_ITEM(x, i) : PyTuple_GET_ITEM(x, i))) return false;
+    return true;
+  }
+  if (!PyDict_CheckExact(x)) return false;
+  if (!n.nested) return true;
+  for (size_t i = 0; i < n.keys.size(); ++i)
+    if (!plain(n.children[i], PyDict_GetItem(x, n.keys[i].p))) return false;
+  return true;
 }
 
 PyObject* tuple_of_type(PyTypeObject* type, PyObject* items) {  // items: a tuple, stolen
@@ -742,13 +765,24 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   });
   if (!ok(status)) return nullptr;
 
+  std::vector<Ref> out_p, out_s[3];
   Ref count(host_int(old_count + 1));
   if (count.p == nullptr) return nullptr;
   if (plan->donate) {  // every array was updated in place
-    return PyTuple_Pack(3, params, states, count.p);
+    bool as_they_are = plain(plan->tree, params);
+    for (int k = 0; k < plan->n_states; ++k) as_they_are = as_they_are && plain(plan->tree, PyTuple_GET_ITEM(states, k));
+    if (as_they_are) return PyTuple_Pack(3, params, states, count.p);
+    // plain dicts come back, as from the general path
+    auto leaves = [](const std::vector<PyObject*>& x) {
+      std::vector<Ref> out;
+      for (PyObject* leaf : x) out.push_back(Ref::borrow(leaf));
+      return out;
+    };
+    out_p = leaves(plan->p);
+    for (int k = 0; k < plan->n_states; ++k) out_s[k] = leaves(plan->s[k]);
+  } else if (!wrap_results(*plan, made, out_p, out_s)) {
+    return nullptr;
   }
-  std::vector<Ref> out_p, out_s[3];
-  if (!wrap_results(*plan, made, out_p, out_s)) return nullptr;
   Ref new_params(build(plan->tree, out_p));
   Ref new_states(PyTuple_New(plan->n_states));
   if (new_params.p == nullptr || new_states.p == nullptr) return nullptr;
@@ -765,7 +799,7 @@ bool collect(PyObject* x, std::vector<at::Tensor>& out) {
   const Deeper deeper;
   if (!deeper.ok) return false;
   if (x == Py_None) return true;
-  if (PyDict_CheckExact(x)) {
+  if (is_dict(x)) {
     // the order of the sum is that of the flattened tree
     bool sorted = true;
     Py_ssize_t pos = 0;
@@ -1019,9 +1053,18 @@ PyObject* bind(PyObject*, PyObject* args) {
       !get("fo_quantize_momentum", api.quantize_m) || !get("fo_quantize_variance", api.quantize_v) || !get("fo_dequantize_momentum", api.dequantize_m) ||
       !get("fo_dequantize_variance", api.dequantize_v) || !get("fo_status_string", api.status_string) || !get("fo_last_error", api.last_error))
     return nullptr;
-  Py_INCREF(type);
-  Py_XDECREF(quantized_type);
-  quantized_type = type;
+  Ref collections(PyImport_ImportModule("collections"));
+  Ref ordered(collections.p == nullptr ? nullptr : PyObject_GetAttrString(collections.p, "OrderedDict"));
+  Ref with_default(ordered.p == nullptr ? nullptr : PyObject_GetAttrString(collections.p, "defaultdict"));
+  if (with_default.p == nullptr) return nullptr;
+  auto keep = [](PyObject*& slot, PyObject* x) {
+    Py_INCREF(x);
+    Py_XDECREF(slot);
+    slot = x;
+  };
+  keep(quantized_type, type);
+  keep(ordered_type, ordered.p);
+  keep(default_type, with_default.p);
   Py_RETURN_NONE;
 }
 

@@ -441,8 +441,8 @@ def test_equal_keys_of_another_type_are_another_tree():
     import flashoptim_jax_b200 as fo
 
     tx = fo.flash_lion(learning_rate=1e-2, param_groups=[{"params": "1", "learning_rate": 0.0}])
-    w, g = torch.ones(64, device="cuda"), torch.ones(64, device="cuda")
-    p = {1: w}
+    w = torch.ones(64, device="cuda", dtype=torch.bfloat16)
+    g, p = torch.ones_like(w), {1: w}
     s = tx.init(p)
     for _ in range(2):
         p, s = tx.step(p, s, {1: g})
@@ -489,3 +489,27 @@ def test_named_tuples_are_made_by_their_constructors():
         assert abs(sq - sum(float((x.double() ** 2).sum()) for x in g)) <= 1e-6 * sq
         w, ecc = fo.set_fp32_params(kind(*(x.float() for x in p)), p)
         assert type(w) is kind and type(ecc) is kind and type(fo.reconstruct_weights(w, ecc)) is kind
+
+
+@pytest.mark.parametrize("donate", [False, True])
+def test_ordered_and_default_dicts_are_planned(donate, monkeypatch):
+    """Their order does not matter, and plain dicts come back, as from the general path."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    ordered = lambda x: collections.OrderedDict((k, collections.defaultdict(list, v) if isinstance(v, dict) else v) for k, v in reversed(x.items()))
+    make = lambda: {"a": {"w": torch.ones(64, device="cuda", dtype=torch.bfloat16), "v": torch.ones(7, device="cuda")}, "b": torch.ones(5, device="cuda")}
+    tx, ref = fo.flash_adamw(donate=donate), fo.flash_adamw()
+    p, q = make(), make()
+    s, t = tx.init(p), ref.init(q)
+    grads = [_grads(make(), k) for k in range(4)]
+    p, s = tx.step(p, s, grads[0])
+    with _only_planned_steps(monkeypatch):
+        for g in grads[1:]:
+            p, s = tx.step(ordered(p), s, ordered(g))
+            assert type(p) is dict and type(p["a"]) is dict and list(p) == ["a", "b"]
+    with _general_path():
+        for g in grads:
+            q, t = ref.step(q, t, g)
+    _same((p, s.mu, s.nu, s.ecc), (q, t.mu, t.nu, t.ecc))
