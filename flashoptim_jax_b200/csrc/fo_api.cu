@@ -236,8 +236,8 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
     return FO_OK;
   };
   // The 32-group kernels address elements with 32-bit offsets: a longer leaf goes in as several
-  // leaves of 2^31 elements (a multiple of the chunk and of the group, so every piece keeps
-  // its alignment and its own whole groups).
+  // leaves of 2^31 elements (a multiple of the pieces of 1024 and of the group, so every piece keeps
+  // its alignment and its own whole groups; what the chunks leave over goes to piece_kernel).
   const unsigned long long kMaxLeafElems = generic ? ~0ull : (1ull << 31);
   const size_t grad_size = d->grad_dtype == FO_F32 ? 4 : 2, param_size = d->param_dtype == FO_F32 ? 4 : 2;
   const size_t ecc_size = (size_t)d->ecc_bits / 8, moment_size = d->state == FO_STATE_FULL ? 4 : 1;

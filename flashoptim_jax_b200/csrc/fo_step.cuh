@@ -209,6 +209,9 @@ constexpr int min_blocks(int opt) { return opt == FO_OPT_ADAM ? FO_MIN_BLOCKS_AD
 constexpr int kPiece = 8;
 constexpr int kLutCopies = FO_LUT_COPIES;                 // copies of the momentum dequantization table in shared memory
 constexpr int kChunk = kThreads * kPiece;      // elements per chunk
+// launch_pieces continues where the whole chunks end, counted in pieces: with a chunk that is no multiple of one, both kernels
+// would update the elements in between, in place and at the same time
+static_assert(kChunk % kPieceElems == 0, "a chunk is a whole number of pieces");
 
 // true when the quotient sqrt(nu)/sqrt(bc2) may be formed as div_by_rcp without changing
 // (quotient + eps): for sqrt(nu) >= 2^-100 the shortcut is exact, below it the quotient is

@@ -240,3 +240,16 @@ def test_warmup_cosine_schedule_host_formula():
     assert abs(s(100)) < 1e-10 and s(1000) == s(100)                                      # clipped at the end
     assert warmup_cosine(50, 0, 2e-3)(0) == float(np.float32(np.float32(1e-3) * np.float32(2.0)))  # no warm-up: straight to the cosine
     assert all(s(t) >= s(t + 1) for t in range(10, 100))
+
+
+def test_every_block_shape_covers_whole_pieces():
+    """The chunk of a step-kernel slice, 8 elements per thread, has to be a multiple of piece_kernel's 1024 elements: the header
+    refuses any other at compile time, and the shapes of the build are none."""
+    from flashoptim_jax_b200 import build
+
+    text = open(os.path.join(build.CSRC, "fo_step.cuh")).read()
+    assert 'static_assert(kChunk % kPieceElems == 0' in text and "kPieceThreads = 128, kPieceElems = kPieceThreads * 8" in text
+    for name, _source, flags in build._units():
+        for flag in flags:
+            if flag.startswith("-DFO_THREADS="):
+                assert int(flag.split("=")[1]) * 8 % 1024 == 0, name
