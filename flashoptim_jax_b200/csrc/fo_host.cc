@@ -168,14 +168,15 @@ bool walk(const Node& n, PyObject* x, PyObject** out) {
       return x == Py_None;
     case Node::kDict: {
       if (!is_dict(x) || PyDict_GET_SIZE(x) != (Py_ssize_t)n.keys.size()) return false;
-      // usually the very key objects in the very order: no look-up by hash
+      // usually the very key objects, in the order of the parameters or (trees that were rebuilt: states, results) sorted: no look-up by hash
       Py_ssize_t pos = 0;
       PyObject *k, *v;
       size_t j = 0;
-      bool same = true;
+      bool same = true, sorted = false;
       while (PyDict_Next(x, &pos, &k, &v)) {
-        if (k != n.seen_keys[j].p) { same = false; break; }
-        if (!walk(n.children[n.seen[j]], v, out)) return false;
+        if (j == 0) sorted = k != n.seen_keys[0].p;
+        if (k != (sorted ? n.keys : n.seen_keys)[j].p) { same = false; break; }
+        if (!walk(n.children[sorted ? (int)j : n.seen[j]], v, out)) return false;
         ++j;
       }
       if (same) return true;
@@ -537,8 +538,10 @@ bool fill_leaf(Plan& plan, const LeafSpec& l, int i) {
 }
 
 // The leaves of the trees into the plan's scratch.  False: not what the plan describes (or, with an exception set, an error).
-bool walk_trees(Plan& plan, PyObject* params, PyObject* states, PyObject* grads) {
-  if (!walk(plan.tree, params, plan.p.data()) || !walk(plan.tree, grads, plan.g.data())) return false;
+bool walk_params(Plan& plan, PyObject* params, PyObject* grads) {
+  return walk(plan.tree, params, plan.p.data()) && walk(plan.tree, grads, plan.g.data());
+}
+bool walk_states(Plan& plan, PyObject* states) {
   for (int k = 0; k < plan.n_states; ++k)
     if (!walk(plan.tree, PyTuple_GET_ITEM(states, k), plan.s[k].data())) return false;
   return true;
@@ -554,33 +557,23 @@ bool plausible(const Plan& plan) {
   return true;
 }
 
-// owning references to the leaves
+// owning references to leaves
 class Held {
   std::vector<PyObject*> v_;
 
  public:
-  explicit Held(const Plan& plan) {
-    v_.reserve((size_t)plan.n * (2 + plan.n_states));
-    v_.insert(v_.end(), plan.p.begin(), plan.p.end());
-    v_.insert(v_.end(), plan.g.begin(), plan.g.end());
-    for (int k = 0; k < plan.n_states; ++k) v_.insert(v_.end(), plan.s[k].begin(), plan.s[k].end());
-    for (PyObject* x : v_) Py_INCREF(x);
-  }
+  explicit Held(const Plan& plan) { v_.reserve((size_t)plan.n * (2 + plan.n_states)); }
   Held(const Held&) = delete;
   ~Held() {
     for (PyObject* x : v_) Py_DECREF(x);
   }
-  // are the plan's leaves still these?
-  bool same(const Plan& plan) const {
-    auto at = v_.begin();
-    auto next = [&](const std::vector<PyObject*>& x) {
-      const bool eq = std::equal(x.begin(), x.end(), at);
-      at += (ptrdiff_t)x.size();
-      return eq;
-    };
-    bool eq = next(plan.p) && next(plan.g);
-    for (int k = 0; eq && k < plan.n_states; ++k) eq = next(plan.s[k]);
-    return eq;
+  void take(const std::vector<PyObject*>& leaves) {
+    for (PyObject* x : leaves) Py_INCREF(x);
+    v_.insert(v_.end(), leaves.begin(), leaves.end());
+  }
+  // are these the leaves taken first and second?
+  bool are(const std::vector<PyObject*>& a, const std::vector<PyObject*>& b) const {
+    return std::equal(a.begin(), a.end(), v_.begin()) && std::equal(b.begin(), b.end(), v_.begin() + (ptrdiff_t)a.size());
   }
 };
 
@@ -684,13 +677,15 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   PyObject *params = a[1], *states = a[3], *grads = a[4];
   const at::Tensor* count_t = plain_tensor(a[2]);
   if (count_t == nullptr || !count_t->is_cpu() || count_t->scalar_type() != at::kInt || count_t->dim() != 0) Py_RETURN_NONE;
-  if (!walk_trees(*plan, params, states, grads) || !groups_unchanged(*plan)) {
+  if (!walk_params(*plan, params, grads) || !groups_unchanged(*plan)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
   const int32_t old_count = *count_t->const_data_ptr<int32_t>();
   const double step = (double)old_count + 1.0;
-  const Held held(*plan);  // the leaves stay alive, whatever happens to the trees meanwhile
+  Held held(*plan);  // the leaves stay alive, whatever happens to the trees meanwhile
+  held.take(plan->p);
+  held.take(plan->g);
 
   std::vector<double> lr(plan->groups.size());
   std::vector<Ref> lr_now;
@@ -724,10 +719,11 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   }
   // A selector or a schedule, or another thread that ran meanwhile, may have put other tensors into the trees or other storage
   // under a tensor: addresses are taken now, and nothing is called between here and the launches.
-  if (call && (!walk_trees(*plan, params, states, grads) || !held.same(*plan))) {
+  if ((call && (!walk_params(*plan, params, grads) || !held.are(plan->p, plan->g))) || !walk_states(*plan, states)) {
     if (PyErr_Occurred()) return nullptr;
     Py_RETURN_NONE;
   }
+  for (int k = 0; k < plan->n_states; ++k) held.take(plan->s[k]);
   for (int i = 0; i < plan->n; ++i)
     if (!fill_leaf(*plan, plan->leaves[i], i)) Py_RETURN_NONE;
 
