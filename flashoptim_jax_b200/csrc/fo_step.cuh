@@ -2163,7 +2163,7 @@ cudaError_t launch_chained(void (*kernel)(P...), unsigned int grid, unsigned int
   return cudaLaunchKernelEx(&c, kernel, p...);
 }
 
-inline void fill_common(StepCommon& p, HostStep& s) {
+inline void fill_common(StepCommon& p, const HostStep& s) {
   for (int i = 0; i < s.n_hypers; ++i) p.hyper[i] = s.hyper[i];
   p.n_leaves = 0;
   p.grad_dtype = s.grad_dtype;
@@ -2175,7 +2175,12 @@ inline void fill_common(StepCommon& p, HostStep& s) {
   p.sq_norm = s.sq_norm;
   p.max_norm = s.max_norm;
   p.wait = s.wait ? 1 : 0;
-  s.wait = false;
+}
+// The result of a launch of the step: behind one that was made, the next need not wait.  (Not where the parameters are filled: a launcher
+// that finds nothing to launch leaves the waiting to the next.)
+inline cudaError_t launched(HostStep& s, cudaError_t e) {
+  if (e == cudaSuccess) s.wait = false;
+  return e;
 }
 
 inline namespace FO_SHAPE_NS {
@@ -2268,7 +2273,7 @@ cudaError_t launch_main(HostStep& hs, bool& chained, cudaStream_t s) {
   const unsigned int share = (total + grid - 1u) / grid;
   if (share <= FO_RUN_WHOLE) run = share;
   p.run_chunks = run < 1u ? 1u : (run > FO_RUN_MAX ? FO_RUN_MAX : run);
-  return launch_chained(kernel, grid, kThreads, dynamic_smem, chained, s, p);
+  return launched(hs, launch_chained(kernel, grid, kThreads, dynamic_smem, chained, s, p));
 }
 
 // The pieces that the whole chunks (of main_chunk elements; 0: step_kernel is not used) of the hot leaves leave over.
@@ -2292,7 +2297,7 @@ cudaError_t launch_piece_table(HostStep& hs, const int* which, int n, unsigned i
   p.n_leaves = n;
   p.first_piece[n] = total;
   const unsigned int most = (unsigned int)hs.sm_count * 64u;  // a misaligned leaf can be large: blocks then take several pieces
-  return launch_chained(piece_kernel<OPT, PDT, ECC_BITS, STATE, N, OUT>, total < most ? total : most, kPieceThreads, 0, chained, s, p);
+  return launched(hs, launch_chained(piece_kernel<OPT, PDT, ECC_BITS, STATE, N, OUT>, total < most ? total : most, kPieceThreads, 0, chained, s, p));
 }
 template <int OPT, int PDT, int ECC_BITS, int STATE, bool OUT>
 cudaError_t launch_piece_tables(HostStep& hs, unsigned int main_chunk, bool& chained, cudaStream_t s) {
@@ -2334,7 +2339,7 @@ cudaError_t launch_generic_table(HostStep& hs, bool& chained, cudaStream_t s) {
   }
   p.n_leaves = hs.n_leaves;
   p.t.first_block[hs.n_leaves] = total;
-  return launch_chained(step_kernel_generic<OPT, PDT, ECC_BITS, MODE>, total, 256u, 0, chained, s, p);
+  return launched(hs, launch_chained(step_kernel_generic<OPT, PDT, ECC_BITS, MODE>, total, 256u, 0, chained, s, p));
 }
 template <int OPT, int PDT, int ECC_BITS>
 cudaError_t launch_generic(HostStep& hs, bool& chained, cudaStream_t s) {
