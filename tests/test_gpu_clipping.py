@@ -23,7 +23,7 @@ def test_sum_of_squares_many_arrays_dtypes_alignments():
     import torch
 
     rng = np.random.default_rng(0)
-    sizes = [1, 7, 2048, 2049, 4096 * 3 + 5, 100003, 33] * 30  # 210 arrays: more than one launch holds
+    sizes = [1, 7, 2048, 2049, 4096 * 3 + 5, 100003, 33] * 100  # 700 arrays: a launch holds 320
     for np_dt in (np.float32, ml_dtypes.bfloat16, np.float16):
         arrays = [rng.normal(0, 0.3, n).astype(np.float32).astype(np_dt) for n in sizes]
         want = O.global_sq_norm(arrays)

@@ -63,7 +63,7 @@ FACTORIES = [("flash_adamw", dict(learning_rate=1e-3)), ("flash_adam", dict(lear
 
 @pytest.mark.parametrize("donate", [False, True])
 @pytest.mark.parametrize("name,kw", FACTORIES)
-def test_planned_steps_equal_general_steps(name, kw, donate):
+def test_planned_steps_equal_general_steps(name, kw, donate, monkeypatch):
     import flashoptim_jax_b200 as fo
 
     groups = [{"params": ["bias", "a/z/1"], "weight_decay": 0.0, "learning_rate": 5e-3}, {"params": lambda p, leaf: leaf.dim() == 1, "weight_decay": 0.1}]
@@ -75,7 +75,8 @@ def test_planned_steps_equal_general_steps(name, kw, donate):
         g = _grads(q, k)
         before = [x.clone() for x in _leaves((p, s))]
         old = (p, s)
-        p, s = tx.step(p, s, g)
+        with _only_planned_steps(monkeypatch) if k else contextlib.nullcontext():
+            p, s = tx.step(p, s, g)
         with _general_path():
             q, t = ref.step(q, t, g)
         _same((p, tuple(s)), (q, tuple(t)))
@@ -137,7 +138,7 @@ def test_selectors_are_asked_at_every_step():
 
 
 @pytest.mark.parametrize("donate", [False, True])
-def test_a_call_without_elements_in_front(donate):
+def test_a_call_without_elements_in_front(donate, monkeypatch):
     """The launch table that comes first holds only leaves without elements; the clipped launches behind it still wait for the norm."""
     import torch
 
@@ -151,7 +152,8 @@ def test_a_call_without_elements_in_front(donate):
     s, t = tx.init(p), ref.init(q)
     for k in range(4):
         g = _grads(q, k)
-        p, s = tx.step(p, s, g)
+        with _only_planned_steps(monkeypatch) if k else contextlib.nullcontext():
+            p, s = tx.step(p, s, g)
         with _general_path():
             q, t = ref.step(q, t, g)
         _same((p, tuple(s["opt"])), (q, tuple(t["opt"])))
@@ -513,3 +515,26 @@ def test_ordered_and_default_dicts_are_planned(donate, monkeypatch):
         for g in grads:
             q, t = ref.step(q, t, g)
     _same((p, s.mu, s.nu, s.ecc), (q, t.mu, t.nu, t.ecc))
+
+
+@pytest.mark.parametrize("donate", [False, True])
+def test_plans_of_several_tables_and_hyper_sets(donate, monkeypatch):
+    """More leaves than a launch holds, and more hyper-parameter sets than a call takes, through a compiled plan."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    names = [f"{i:03d}" for i in range(700)]
+    groups = [{"params": names[i::40], "learning_rate": 1e-3 * (i + 1), "weight_decay": 0.01 * i} for i in range(20)]
+    rng = torch.Generator(device="cuda").manual_seed(0)
+    make = lambda: {k: torch.full((1 + 37 * i % 2500,), 0.02 * (1 + i % 7), device="cuda", dtype=torch.bfloat16 if i % 5 else torch.float32) for i, k in enumerate(names)}
+    tx, ref = fo.flash_adamw(param_groups=groups, donate=donate), fo.flash_adamw(param_groups=groups)
+    p, q = make(), make()
+    s, t = tx.init(p), ref.init(q)
+    for k in range(3):
+        g = {n: (torch.randn(x.shape, device="cuda", generator=rng) * 1e-2).to(x.dtype) for n, x in q.items()}
+        with _only_planned_steps(monkeypatch) if k else contextlib.nullcontext():
+            p, s = tx.step(p, s, g)
+        with _general_path():
+            q, t = ref.step(q, t, g)
+        _same((p, s.mu, s.nu, s.ecc), (q, t.mu, t.nu, t.ecc))

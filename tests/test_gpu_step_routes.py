@@ -234,3 +234,82 @@ def test_leaf_counts_around_the_table_sizes(opt, group, conv, elsewhere):
     for count in (12, 13, 236, 237, 240, 241, 320, 321, 700):
         _run(opt, 1, 8, C.STATE_QUANT, group, conv, [1 + i % 61 for i in range(count)], steps=1, elsewhere=elsewhere)
     _run(opt, 1, 8, C.STATE_QUANT, group, conv, [6000 + i for i in range(330)], steps=1, elsewhere=elsewhere)
+
+
+@pytest.mark.parametrize("opt,pdt,ecc_bits,group,conv", [
+    (C.ADAM, 1, 8, 32, O.FUSED), (C.ADAM, 2, 16, 32, O.FUSED), (C.ADAM, 0, 0, 64, O.FUSED), (C.ADAM, 1, 16, 32, O.UNFUSED),
+    (C.LION, 1, 16, 32, O.FUSED), (C.LION, 1, 8, 32, O.UNFUSED), (C.SGD, 1, 8, 128, O.FUSED), (C.SGD, 2, 16, 32, O.FUSED)])
+@pytest.mark.parametrize("elsewhere", [False, True])
+def test_extreme_values_in_whole_chunks(opt, pdt, ecc_bits, group, conv, elsewhere):
+    """Zeros, subnormals, huge and tiny values scattered and in whole groups through step_kernel: nearly every warp takes the
+    repairing pass."""
+    import torch
+
+    rng = np.random.default_rng(11)
+    n = MAIN + 300
+    p32 = np.ldexp(rng.normal(0, 1, n), np.clip(rng.integers(-140, 60, n), -140, 30)).astype(np.float32)
+    p32[::7] = 0
+    ref = H.fresh_leaf((np.clip(p32, -1e3, 1e3) if pdt == 2 else p32).astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, group)
+    dev = ref.copy().to_device()
+    for t in (1, 2):
+        g = np.ldexp(rng.normal(0, 1, n), rng.integers(-140, 12, n)).astype(np.float32)
+        g[::5] = 0
+        g[5000:9000] = 0
+        hp = H.hyper_tuple(opt, conv, t, lr=1e-3, wd=1e-2)
+        H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+        outs = [H.LeafArrays(*[None if getattr(dev, f) is None else torch.empty_like(getattr(dev, f)) for f in dev.fields()])] if elsewhere else None
+        _step(opt, [H.to_torch(g)], [dev], outs, C.STATE_QUANT, group, hp, pdt, 0, ecc_bits)
+        dev = outs[0] if elsewhere else dev
+        H.assert_leaf_equal(dev.to_host(), ref, f"step {t}")
+
+
+@pytest.mark.parametrize("pdt,ecc_bits,state,group,max_norm", [(1, 8, C.STATE_QUANT, 32, None), (1, 16, C.STATE_QUANT, 128, 0.5), (2, 8, C.STATE_FULL, 32, None)])
+@pytest.mark.parametrize("bc2", [0.5, 1e-12])
+def test_device_scalars_in_whole_chunks(pdt, ecc_bits, state, group, max_norm, bc2):
+    """Learning rate and bias corrections read from the device: a correction in the range of the reciprocal shortcut, and one outside it,
+    which step_kernel only sees once it runs (its chunks then go element by element)."""
+    import torch
+
+    from flashoptim_jax_b200 import _engine as eng
+
+    rng = np.random.default_rng(5)
+    n = MAIN + 77
+    ref = H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), C.ADAM, state, ecc_bits, group)
+    dev = ref.copy().to_device()
+    g = H.make_grad(rng, n, 1e-2, H.BF16)
+    dev_g, sq, step_g = H.to_torch(g), None, g
+    if max_norm is not None:
+        sq = eng.sq_norm_of([dev_g])
+        step_g = O.clip_by_global_norm([g], max_norm, sq_norm=float(sq.cpu()))[0]
+    lr, bc1, bc2 = np.float32(2e-3), np.float32(0.25), np.float32(bc2)
+    hp = list(H.hyper_tuple(C.ADAM, O.FUSED, 3, lr=lr, wd=1e-2))
+    hp[7], hp[8] = bc1, bc2
+    H.oracle_step(C.ADAM, step_g, ref, state, group, hp)
+    scalars = torch.tensor([lr, bc1, bc2], device="cuda")
+    host = list(H.hyper_tuple(C.ADAM, O.FUSED, 1, lr=0.5, wd=1e-2))  # what the host says about these three does not count
+    H.abi_step(C.ADAM, [dev_g], [dev], state, group, [tuple(host) + (scalars.data_ptr(),)], [0], pdt, 1, ecc_bits, grad_sq_norm=sq,
+               max_grad_norm=max_norm or 0.0)
+    H.assert_leaf_equal(dev.to_host(), ref)
+
+
+def test_nothing_is_written_beside_a_leaf_of_whole_chunks():
+    """Guard bytes on both sides of every array of a leaf that step_kernel and piece_kernel share."""
+    import torch
+
+    rng = np.random.default_rng(2)
+    n = MAIN + 333
+    ref = H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.BF16), C.ADAM, C.STATE_QUANT, 16)
+    inner, framed = ref.copy().to_device(), {}
+    for f in inner.fields():
+        t = getattr(inner, f)
+        framed[f] = torch.full((t.numel() * t.element_size() + 512,), 0xA5, dtype=torch.uint8, device="cuda")
+        view = framed[f][256 : 256 + t.numel() * t.element_size()].view(t.dtype)
+        view.copy_(t)
+        setattr(inner, f, view)
+    g = H.make_grad(rng, n, 1e-2, H.BF16)
+    hp = H.hyper_tuple(C.ADAM, O.FUSED, 1, lr=1e-3, wd=1e-2)
+    H.oracle_step(C.ADAM, g, ref, C.STATE_QUANT, 32, hp)
+    _step(C.ADAM, [H.to_torch(g)], [inner], None, C.STATE_QUANT, 32, hp, 1, 1, 16)
+    H.assert_leaf_equal(inner.to_host(), ref)
+    for f, whole in framed.items():
+        assert bool((whole[:256] == 0xA5).all()) and bool((whole[-256:] == 0xA5).all()), f
