@@ -237,8 +237,8 @@ class PreparedLaunch:
             raise ValueError("peer_param_offsets and peer_grad_offsets must name the same peers")
         n_peers = max(len(self.peers), len(self.grad_peers))
         buckets: Dict[Tuple[Any, ...], List[Tuple[LeafWork, int]]] = {}
-        for i, (w, gid) in enumerate(zip(work, group_ids)):
-            buckets.setdefault(w.bucket, []).append((w, gid, i))
+        for w, gid in zip(work, group_ids):
+            buckets.setdefault(w.bucket, []).append((w, gid))
         self.calls: List[Dict[str, Any]] = []
         for key, items in buckets.items():
             dev_index, pdt, gdt, ecc_bits, state, group_size = key
@@ -246,18 +246,18 @@ class PreparedLaunch:
             while start < len(items):
                 slots: Dict[int, int] = {}
                 end = start
-                while end < len(items) and (items[end][1] in slots or len(slots) < _lib.FO_MAX_HYPERS):  # noqa: E501
+                while end < len(items) and (items[end][1] in slots or len(slots) < _lib.FO_MAX_HYPERS):
                     slots.setdefault(items[end][1], len(slots))
                     end += 1
                 part = items[start:end]
-                ws = [w for w, _, _ in part]
+                ws = [w for w, _ in part]
                 leaves = np.zeros(len(part), dtype=LEAF_DTYPE)
                 leaves["grad"] = [w.grad.data_ptr() for w in ws]
                 leaves["param"] = [w.param.data_ptr() for w in ws]
                 for name in ("ecc", "mu", "mu_scales", "nu", "nu_scales"):
                     leaves[name] = [_ptr(getattr(w, name)) for w in ws]
                 leaves["n"] = [w.param.numel() for w in ws]
-                leaves["hyper"] = [slots[gid] for _, gid, _ in part]
+                leaves["hyper"] = [slots[gid] for _, gid in part]
                 hypers = np.zeros(len(slots), dtype=HYPER_DTYPE)
                 desc = _lib.FoStepDesc(
                     struct_size=ctypes.sizeof(_lib.FoStepDesc), opt=opt, param_dtype=pdt, grad_dtype=gdt, ecc_bits=ecc_bits,
@@ -269,7 +269,6 @@ class PreparedLaunch:
                 desc.mc_param_offset, desc.mc_grad_offset = int(mc_param_offset), int(mc_grad_offset)
                 self.calls.append({"key": key, "desc": desc, "leaves": leaves, "hypers": hypers, "slots": list(slots.items()),
                                    "device": torch.device("cuda", dev_index), "n_params": int(leaves["n"].sum()),
-                                   "index": np.asarray([i for _, _, i in part], dtype=np.int64),
                                    "keep": ws})  # the tensors stay alive as long as their addresses are in the tables
                 start = end
 

@@ -1133,7 +1133,9 @@ FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const CLIP& source) {
   if (gdt == FO_BF16) {
     // g and n_g have 8-bit mantissas, so g / n_g is never halfway between two bf16 values and no closer to
     // that than 2^-17 of itself: the product with the fp32 reciprocal (off by 2^-23 at most) rounds to the same
-    // bf16 value as the quotient, and the second product is one bf16 instruction.  Holds while the quotient is
+    // bf16 value as the quotient.  The second product, of two 8-bit mantissas, is exact in fp32 down to 2^-134, and
+    // below that rounds to zero either way (half of the smallest bf16 is 2^-134): the bf16 instruction, which rounds once, gives
+    // what an fp32 product rounded to bf16 does for every max_norm.  The first holds while the quotient is
     // normal: |g| >= 2^-100 (n_g <= 2^20), or zero.  Twice the magnitude bits minus one, as unsigned: zero wraps
     // to the top and passes.  (With the exact division and both conversions the same took 11 instructions per
     // element instead of 4.)
