@@ -158,6 +158,38 @@ __global__ void selftest_group_div(const float one, unsigned long long pairs, un
   tally(bad, out);
 }
 
+// The update division on the quotients nearest to a rounding boundary: X / Y with 2^s X - M Y = k, |k| <= 16, for every 24-bit Y
+// and every odd 25-bit M (M / 2^s lies halfway between two floats; s = 24 for X >= Y, 25 below).  M follows from
+// Y and k modulo 2^s: with Y = 2^t Z, Z odd, it is -(k / 2^t) / Z modulo 2^(s - t).
+__global__ void selftest_hard_divisions(unsigned long long* out) {
+  unsigned long long bad = 0;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t Y = (1u << 23) + blockIdx.x * blockDim.x + threadIdx.x; Y < (1u << 24); Y += stride) {
+    const int t = __ffs((int)Y) - 1;
+    const uint32_t Z = Y >> t;
+    uint32_t inv = Z;  // 1 / Z modulo 2^32: right to 3 bits, and each step doubles them
+#pragma unroll
+    for (int i = 0; i < 4; ++i) inv *= 2u - Z * inv;
+    const float d = (float)Y;
+    for (int s = 24; s <= 25; ++s) {
+      const uint32_t period = 1u << (s - t);
+      for (int k = -16; k <= 16; ++k) {
+        if (k % (1 << t) != 0) continue;
+        const uint32_t M0 = ((uint32_t)(-(k / (1 << t))) * inv) & (period - 1u);
+        for (uint32_t M = (1u << 24) + ((M0 - (1u << 24)) & (period - 1u)); M < (1u << 25); M += period) {
+          const long long num = (long long)M * Y + k;
+          const long long X = num >> s;
+          if ((M & 1u) == 0u || (num & ((1ll << s) - 1)) != 0 || X < (1 << 23) || X >= (1 << 24) || (X >= (long long)Y) != (s == 24)) continue;
+          const float a = (float)X;
+          const float2 q = fast2::neg_div2(make_float2(a, -a), make_float2(d, d));
+          bad += !same_float(q.x, fdiv(-a, d)) || !same_float(q.y, fdiv(a, d));
+        }
+      }
+    }
+  }
+  tally(bad, out);
+}
+
 // every float in [1e-30, 1e30]: reciprocal by MUFU.RCP + k correction steps vs the IEEE one.
 // out[0] counts mismatches of the variant the kernels use, out[1] of one step, out[2] of two.
 __global__ void selftest_rcp(unsigned long long* out) {
@@ -251,6 +283,7 @@ static void launch_sweep(int32_t which, int64_t arg, unsigned long long* d, cuda
     case FO_SELFTEST_SOFTSIGN: selftest_softsign<<<grid, block, 0, s>>>(one, d); return;
     case FO_SELFTEST_GROUP_DIV:
       selftest_group_div<<<grid, block, 0, s>>>(one, (unsigned long long)(arg > 0 ? arg : 1) * 1000000ull, d);
+      selftest_hard_divisions<<<grid, block, 0, s>>>(d);
       return;
     case FO_SELFTEST_CODE_TABLES: selftest_code_tables<<<64, block, 0, s>>>(d); return;
     case FO_SELFTEST_RCP: selftest_rcp<<<grid, block, 0, s>>>(d); return;
