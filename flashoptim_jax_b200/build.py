@@ -36,15 +36,19 @@ _OPTS = (("adam", "FO_OPT_ADAM"), ("lion", "FO_OPT_LION"), ("sgd", "FO_OPT_SGD")
 _KINDS = (("quant", 0), ("full", 1), ("generic", 3))
 
 
-# block shape of a slice: (threads per block, resident blocks per SM).  Measured on B200: the
+# Block shape of a slice that runs step_kernel: (threads per block, resident blocks per SM).  Measured on B200: the
 # Adam kernels run best as one 512-thread block per SM (all warps of an SM share one instruction
 # stream and one set of tables); the kernels that also read peers' gradients keep 256-thread blocks,
-# whose smaller stages leave room for a deeper copy pipeline.  Lion gains 2 % from one 768-thread block
-# over three of 256; SGD measures the same either way and keeps the default (256 x 3).
-_SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1), ("adam", "group"): (512, 1),
+# whose smaller stages leave room for a deeper copy pipeline.
+_SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1),
            ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1),
-           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "group"): (512, 1), ("lion", "all"): (512, 1),
-           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "group"): (512, 1), ("sgd", "all"): (512, 1)}
+           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1),
+           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "all"): (512, 1)}
+# Threads of the one block per SM that runs tile_kernel (quantized moments, one feature at most).  AdamW wants 150 to 168 registers
+# for the 16 elements of a lane (2^28 elements, 24-bit masters: 588 us with 384 threads, 623 with 512; with the power cap reached
+# 672 and 704); Lion and SGD need fewer (with the cap reached 477 us with 512 threads and 485 with 384, and 445 against 464).
+_TILE_THREADS = {"adam": 384, "lion": 512, "sgd": 512}
+_TILE_MODES = ("plain", "clip", "out", "group", "delta")
 # name and feature mask (fo_step.cuh) of the kernels of a slice
 _MODES = (("plain", 0), ("clip", 1), ("out", 2), ("group", 4), ("delta", 8), ("all", 15), ("peer", 16), ("piece", -1))
 
@@ -64,7 +68,7 @@ def _units(shapes=None, ffi_dir: str | None = None) -> List[Tuple[str, str, List
         suffix = f"_{mname}" if mname else ""
         flags = [f"-DFO_INST_OPT={omacro}", f"-DFO_INST_KIND={kind}", f"-DFO_INST_MODE={mode}",
                  f"-DFO_INST_NAME=lookup_{oname}_{kname}{suffix}"]
-        shape = shapes.get((oname, mname))
+        shape = (_TILE_THREADS[oname], 1) if kind == 0 and mname in _TILE_MODES else shapes.get((oname, mname))
         if shape is not None and kind != 3:
             flags += [f"-DFO_THREADS={shape[0]}", f"-DFO_MIN_BLOCKS_ADAM={shape[1]}", f"-DFO_MIN_BLOCKS_MOMENTUM={shape[1]}"]
             if len(shape) > 2:

@@ -388,8 +388,8 @@ FO_DEVI f2 neg_rcp2(f2 d) {
 // error before its rounding of less than 8 * 2^-50 (mantissas scaled to [1, 2)): d y is 1 up to 2^-25 d, q is a/d up to
 // a 2^-25 + 2^-24, and their product is what the correction misses.  A quotient that near a rounding boundary M / 2^s is one of the
 // pairs with |2^s a - M d| <= 3 in units of the last places, and all pairs up to 16 (93 million) are
-// compared with the IEEE division by the self-test.  (A second correction, two of 29 packed operations per
-// element, changed nothing: 2^28 elements 717 -> 712 us, 2^24 49.7 -> 46.7, spills of the AdamW kernels 28 / 40 -> 8 / 16 bytes.)
+// compared with the IEEE division by the self-test.  (A second correction, two packed operations
+// of 57 per pair of elements, changed nothing: 2^28 elements 717 -> 712 us, 2^24 49.7 -> 46.7, spills of the AdamW kernels 28 / 40 -> 8 / 16 bytes.)
 FO_DEVI f2 neg_div2(f2 a, f2 d) {
   f2 ny = neg_rcp2(d);
   f2 q = mul2(a, ny);        // -a*y

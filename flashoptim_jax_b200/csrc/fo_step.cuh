@@ -1,7 +1,8 @@
 // Multi-tensor fused optimizer step for sm_100a.
 //
-// A call walks a table of pytree leaves.  Two kernels share the work:
-//   step_kernel   the whole chunks of the leaves (a chunk: threads per block x 8 elements), a persistent
+// A call walks a table of pytree leaves.  Three kernels share the work:
+//   tile_kernel   (fo_tile.cuh) quantized moments with at most one feature beyond the plain step, beyond the smallest problems;
+//   step_kernel   the other kinds of state, mixtures of features and peers: the whole chunks of the leaves (a chunk: threads per block x 8 elements), a persistent
 //                 grid with a copy pipeline through shared memory, one block (or a few) per SM;
 //   piece_kernel  everything else in pieces of 1024 elements, one 128-thread block each: the ragged ends,
 //                 leaves shorter than a chunk, leaves the vector path cannot take, and whole small problems.
@@ -51,6 +52,7 @@ constexpr int kOut = 2;    // results written elsewhere
 constexpr int kGroup = 4;  // quantization groups of 8, 16, 64, 128 or 256
 constexpr int kDelta = 8;  // FO_FLAG_LP_DELTA
 constexpr int kAll = 15;
+constexpr int kCoupled = 32;  // weight decay added to the gradient (not zero, not decoupled); quantized moments
 constexpr int kPeer = 16;  // peers' gradients and parameter replicas, clipping; groups of 32, in place
 
 // Names below depend on the block shape of the translation unit (FO_THREADS): each shape has its own.
@@ -1222,35 +1224,25 @@ FO_DEVI void hand_back_delta(const uint4& o0, const uint4& o1, uint32_t (&nw)[4]
   }
 }
 
-// Second half of a hot chunk: update, split, requantize, store.  Each stage runs its packed
-// shortcut unconditionally.
-// REPAIR = false (first pass): a value outside the range a shortcut is proven for only raises
-// `rare`; nothing is stored until the end, and if any lane of the warp saw such a value the warp's
-// 256 elements are redone from memory by warm_chunk, otherwise the results are written.
-// REPAIR = true (warm_chunk, pieces): the lane that holds such a value (exact zeros are the common case:
-// untouched rows, padding, zero gradients) redoes that stage with IEEE operations, then stores.
-// The stored bits are those of the IEEE path in every case.
-// `at` is the piece the operands came from, `distance` (kOut) tells how far away the results go;
-// old_param(w0, w1) delivers the words of the old parameter.
-template <bool REPAIR, int OPT, int PDT, int ECC_BITS, int STATE, int MODE, bool MASKED = false, typename OUT, typename OLD>
-FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const int gdt, const uint32_t i0,
-                        const Piece& at, bool rare, Unpacked& u, const OUT& distance, OLD old_param, const Peers* peers,
-                        const int n_valid = kPiece, const bool group_valid = true) {
-  const float one = c.one;
+// One step of eight elements: u.theta becomes the new master weight, u.m (and, kept in full, u.v) the new moments, nroot the negated
+// square root of the new second moment; am_lane and av_lane the largest magnitude of the first moment and of that root.
+// Same contract for REPAIR as hot_unpack.  COUPLED = false leaves out the weight decay that is added to the gradient: for calls in which
+// it is zero or decoupled.
+template <bool REPAIR, int OPT, int STATE, bool COUPLED>
+FO_DEVI bool update_pairs(const Hyp& h, const float one, Unpacked& u, float2 (&nroot)[4], float& am_lane, float& av_lane) {
   using namespace fast2;
   const float2 one2 = sp(one);
   float2 (&g)[4] = u.g;
   float2 (&theta)[4] = u.theta;
   float2 (&m)[4] = u.m;
   float2 (&v)[4] = u.v;
-  float2 nroot[4];  // Adam: -sqrt(second moment)
-
-  // ---- update --------------------------------------------------------------------------------------
-  const bool decoupled = (h.flags & FO_FLAG_DECOUPLED_WD) != 0;
-  float am_lane = 0.0f, av_lane = 1.0f;
+  const bool coupled = COUPLED && (h.flags & FO_FLAG_DECOUPLED_WD) == 0;
+  bool rare = false;
+  am_lane = 0.0f;
+  av_lane = 1.0f;
   if constexpr (OPT == FO_OPT_ADAM) {
     // flashoptim_jax/adamw.py:95-106
-    if (!decoupled) {
+    if (coupled) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) g[k] = sum2(mul2(sp(h.wd), theta[k]), g[k], one2);
     }
@@ -1266,7 +1258,7 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
 #pragma unroll
       for (int k = 0; k < 4; ++k) v[k] = mul2(nv[k], sp(-1.0f));  // stored as it is
     }
-    if (decoupled) {
+    if (!coupled) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) theta[k] = mul2(theta[k], sp(h.decay));
     }
@@ -1324,7 +1316,7 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
     am_lane = maxabs8(m);
   } else {
     // flashoptim_jax/momentum_kernel.py:74-75,80-86; flashoptim_jax/sgd.py:45-63
-    if (!decoupled) {
+    if (coupled) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) g[k] = sum2(mul2(sp(h.wd), theta[k]), g[k], one2);
     }
@@ -1340,13 +1332,38 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
       }
       am_lane = maxabs8(m);
     }
-    if (decoupled) {
+    if (!coupled) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) theta[k] = mul2(theta[k], sp(h.decay));
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) theta[k] = sum2(mul2(sp(-h.lr), g[k]), theta[k], one2);  // theta - lr*dir
   }
+  return rare;
+}
+
+// Second half of a hot chunk: update, split, requantize, store.  Each stage runs its packed
+// shortcut unconditionally.
+// REPAIR = false (first pass): a value outside the range a shortcut is proven for only raises
+// `rare`; nothing is stored until the end, and if any lane of the warp saw such a value the warp's
+// 256 elements are redone from memory by warm_chunk, otherwise the results are written.
+// REPAIR = true (warm_chunk, pieces): the lane that holds such a value (exact zeros are the common case:
+// untouched rows, padding, zero gradients) redoes that stage with IEEE operations, then stores.
+// The stored bits are those of the IEEE path in every case.
+// `at` is the piece the operands came from, `distance` (kOut) tells how far away the results go;
+// old_param(w0, w1) delivers the words of the old parameter.
+template <bool REPAIR, int OPT, int PDT, int ECC_BITS, int STATE, int MODE, bool MASKED = false, typename OUT, typename OLD>
+FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const int gdt, const uint32_t i0,
+                        const Piece& at, bool rare, Unpacked& u, const OUT& distance, OLD old_param, const Peers* peers,
+                        const int n_valid = kPiece, const bool group_valid = true) {
+  using namespace fast2;
+  float2 (&theta)[4] = u.theta;
+  float2 (&m)[4] = u.m;
+  float2 (&v)[4] = u.v;
+  float2 nroot[4];  // Adam: -sqrt(second moment)
+
+  float am_lane, av_lane;
+  rare = update_pairs<REPAIR, OPT, STATE, true>(h, c.one, u, nroot, am_lane, av_lane) || rare;
 
   // ---- parameter (+ECC) in stored form --------------------------------------------------------------
   uint32_t nw[4];
@@ -1911,7 +1928,8 @@ FO_DEVI void chain_end() {
 }
 
 // the leaf of a table that holds position c of the common sequence
-FO_DEVI int leaf_of(const uint32_t* first, const int n_leaves, const uint32_t c) {
+template <typename T>
+FO_DEVI int leaf_of(const T* first, const int n_leaves, const T c) {
   int lo = 0;
   for (int hi = n_leaves; hi - lo > 1;) {
     const int mid = (lo + hi) >> 1;
@@ -2141,8 +2159,8 @@ struct HostStep {
 // or the kernel begins with chain_wait(); set to true by a launch.
 using MainFn = cudaError_t (*)(HostStep&, bool& chained, cudaStream_t);
 using PieceFn = cudaError_t (*)(HostStep&, unsigned int main_chunk, bool& chained, cudaStream_t);
-// A slice of step_kernel, the elements one of its chunks covers and the leaves its table holds (of a call without separate
-// outputs).  Block size, and with it the chunk, is a property of the slice (the slices are compiled with their own FO_THREADS).
+// A slice of step_kernel or tile_kernel, the elements one of its chunks covers (1: it takes the leaves whole) and the leaves its table holds
+// (of a call without separate outputs).  Block size, and with it the chunk, is a property of the slice (the slices are compiled with their own FO_THREADS).
 struct Launcher {
   MainFn launch;
   unsigned int chunk;
@@ -2353,23 +2371,25 @@ cudaError_t launch_generic(HostStep& hs, bool& chained, cudaStream_t s) {
 // lookups implemented by the instantiation units (fo_step_inst.cu, one per slice: optimizer x state
 // kind x kernel); each returns null for a (param dtype, ecc width) pair that does not exist
 #define FO_DECLARE_SLICE(stem)                       \
-  Launcher stem##_plain(int pdt, int ecc_bits);      \
-  Launcher stem##_clip(int pdt, int ecc_bits);       \
-  Launcher stem##_out(int pdt, int ecc_bits);        \
-  Launcher stem##_all(int pdt, int ecc_bits);        \
-  Launcher stem##_peer(int pdt, int ecc_bits);       \
+  Launcher stem##_plain(int pdt, int ecc_bits, int gdt);      \
+  Launcher stem##_clip(int pdt, int ecc_bits, int gdt);       \
+  Launcher stem##_out(int pdt, int ecc_bits, int gdt);        \
+  Launcher stem##_all(int pdt, int ecc_bits, int gdt);        \
+  Launcher stem##_peer(int pdt, int ecc_bits, int gdt);       \
   PieceFn stem##_piece(int pdt, int ecc_bits);
 FO_DECLARE_SLICE(lookup_adam_quant) FO_DECLARE_SLICE(lookup_adam_full)
 FO_DECLARE_SLICE(lookup_lion_quant) FO_DECLARE_SLICE(lookup_lion_full)
 FO_DECLARE_SLICE(lookup_sgd_quant) FO_DECLARE_SLICE(lookup_sgd_full) FO_DECLARE_SLICE(lookup_sgd_none)
-Launcher lookup_adam_quant_group(int pdt, int ecc_bits);
-Launcher lookup_lion_quant_group(int pdt, int ecc_bits);
-Launcher lookup_sgd_quant_group(int pdt, int ecc_bits);
-Launcher lookup_adam_quant_delta(int pdt, int ecc_bits);
-Launcher lookup_adam_full_delta(int pdt, int ecc_bits);
-Launcher lookup_adam_generic(int pdt, int ecc_bits);
-Launcher lookup_lion_generic(int pdt, int ecc_bits);
-Launcher lookup_sgd_generic(int pdt, int ecc_bits);
+Launcher lookup_adam_quant_group(int pdt, int ecc_bits, int gdt);
+Launcher lookup_lion_quant_group(int pdt, int ecc_bits, int gdt);
+Launcher lookup_sgd_quant_group(int pdt, int ecc_bits, int gdt);
+Launcher lookup_adam_quant_delta(int pdt, int ecc_bits, int gdt);
+Launcher lookup_adam_full_delta(int pdt, int ecc_bits, int gdt);
+Launcher lookup_adam_generic(int pdt, int ecc_bits, int gdt);
+Launcher lookup_lion_generic(int pdt, int ecc_bits, int gdt);
+Launcher lookup_sgd_generic(int pdt, int ecc_bits, int gdt);
 #undef FO_DECLARE_SLICE
 
 }  // namespace fo
+
+#include "fo_tile.cuh"

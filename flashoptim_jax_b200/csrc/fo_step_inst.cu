@@ -23,13 +23,23 @@ PieceFn FO_INST_NAME(int pdt, int ecc_bits) {
   return nullptr;
 }
 #else
-Launcher FO_INST_NAME(int pdt, int ecc_bits) {
+Launcher FO_INST_NAME(int pdt, int ecc_bits, int gdt) {
+  constexpr int most_leaves = (FO_INST_MODE & kOut) != 0 ? kMaxLeavesFlex : kMaxLeaves;
+  (void)gdt;
 #if FO_INST_KIND == 3
 #define X(P, E) \
   if (pdt == P && ecc_bits == E) return Launcher{&launch_generic<FO_INST_OPT, P, E>, 0u, kMaxLeaves};
+#elif FO_INST_KIND == 0 && FO_INST_MODE != 15 && FO_INST_MODE != 16
+  // tiles: gradients of the parameter's dtype or fp32, which is what steps have, by kernels of their own
+#define X(P, E)                                                                                                       \
+  if (pdt == P && ecc_bits == E) {                                                                                    \
+    if (gdt == P) return Launcher{&launch_tiles<FO_INST_OPT, P, E, P, FO_INST_MODE>, 1u, most_leaves};                \
+    if (gdt == FO_F32) return Launcher{&launch_tiles<FO_INST_OPT, P, E, FO_F32, FO_INST_MODE>, 1u, most_leaves};      \
+    return Launcher{&launch_tiles<FO_INST_OPT, P, E, kAnyGrad, FO_INST_MODE>, 1u, most_leaves};                       \
+  }
 #else
 #define X(P, E) \
-  if (pdt == P && ecc_bits == E) return Launcher{&launch_main<FO_INST_OPT, P, E, FO_INST_KIND, FO_INST_MODE>, (unsigned int)kChunk, (FO_INST_MODE & kOut) != 0 ? kMaxLeavesFlex : kMaxLeaves};
+  if (pdt == P && ecc_bits == E) return Launcher{&launch_main<FO_INST_OPT, P, E, FO_INST_KIND, FO_INST_MODE>, (unsigned int)kChunk, most_leaves};
 #endif
   FO_COMBOS(X)
 #undef X

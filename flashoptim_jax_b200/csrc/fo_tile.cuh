@@ -1,0 +1,469 @@
+// The step on quantized moments, in tiles of 512 elements per warp: what step_kernel (fo_step.cuh) is for the other kinds of state.
+//
+// Bound: a sweep over 10 to 19 bytes per element whose arithmetic takes about as long as its memory traffic, under the chip's
+// power cap.  A warp works for itself: it copies its next tile into a slot of shared memory of its own (cp.async, 16 bytes per
+// lane, no block barrier), and a lane owns 16 consecutive elements of it.  Against 8 elements per lane that halves
+// everything that is per lane and not per element (group maxima and their shuffles, reciprocals, range checks, votes, address
+// steps; a 32-element group is two lanes), makes every copy 16 bytes wide, also of the one-byte streams, and lets a lane store whole
+// 32-byte sectors.
+//
+//   * Dequantization tables: row b holds 32 copies of the momentum value of code b, one per lane and bank, and 32
+//     copies of b / 255 for the second moment.  A row is 256 bytes, so one byte permutation of (codes, lane * 4) is the address, and no
+//     look-up has a bank conflict.  64 KB of the SM's 227.
+//   * Slots: 16-byte units are stored at positions permuted inside 128 bytes (see Units), so that both the coalesced copies and
+//     the reads of a lane's 32 or 64 consecutive bytes fall on all banks.
+//   * All range checks are known once the group maxima are: one vote, then the stores of parameter and ECC, then the codes.
+//   * Two slots per warp and a loop body that is not unrolled: three slots and an unrolled body measured the same.
+//
+// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 627 now, 0.94 of the copy rate; with
+// the power cap reached 798 -> 717.  52 to 55 instructions per element instead of 63.
+#pragma once
+
+namespace fo {
+
+inline namespace FO_SHAPE_NS {
+
+constexpr int kTileElems = 512;   // of a warp
+constexpr int kEnd = 256;         // elements of the warp's pieces that a leaf's ragged end is taken in
+constexpr int kWarps = kThreads / 32;
+constexpr int kTableBytes = 256 * 256;
+constexpr int kAnyGrad = -1;      // gradient dtype known at run time only
+
+template <int MODE>
+struct TileParams : StepParams<MODE> {
+  uint16_t first_end[((MODE & kOut) != 0 ? kMaxLeavesFlex : kMaxLeaves) + 1];  // first piece of each leaf's ragged end
+};
+static_assert(sizeof(TileParams<kOut>) <= 32764 && sizeof(TileParams<kPlain>) <= 32764, "kernel parameters");
+
+template <int OPT, int PDT, int ECC_BITS, int GDT>
+struct TileSlot {
+  static constexpr int kParamUnits = PDT == FO_F32 ? 4 : 2;  // 16-byte units per lane
+  static constexpr int kEccUnits = ECC_BITS / 8;
+  static constexpr int kGradUnits = (GDT == FO_F32 || GDT == kAnyGrad) ? 4 : 2;
+  static constexpr int kEcc = kParamUnits * 512;  // byte offsets
+  static constexpr int kMu = kEcc + kEccUnits * 512;
+  static constexpr int kNu = kMu + 512;
+  static constexpr int kGrad = kNu + (OPT == FO_OPT_ADAM ? 512 : 0);
+  static constexpr int kScales = kGrad + kGradUnits * 512;  // up to 32 of the first moment, then as many of the second
+  static constexpr int kBytes = kScales + 128;
+};
+constexpr int kTileStages = 2;
+constexpr int kSmemPerBlock = 227 * 1024 - 64;  // (the clipping constants are static)
+template <int OPT, int PDT, int ECC_BITS, int GDT>
+__host__ __device__ constexpr int tile_smem() {
+  return kTableBytes + kTileStages * kWarps * TileSlot<OPT, PDT, ECC_BITS, GDT>::kBytes;
+}
+
+// Streams of U 16-byte units per lane (U x 512 bytes per tile).  Unit u goes to position u ^ (u >> 3 & (U - 1)): lane l copies units
+// l + 32 i, which stay eight to a row of 128 bytes, and the eight lanes of a quarter warp that read their j-th units U l + j
+// find them in eight different places of a row.
+template <int U>
+struct Units {
+  static FO_DEVI uint32_t copy_to(uint32_t lane) { return (lane ^ ((lane >> 3) & (U - 1))) * 16u; }
+  static FO_DEVI uint32_t read_at(uint32_t lane) { return (lane * U + (((lane * U) >> 3) & (U - 1))) * 16u; }  // unit j: ^ (j * 16)
+};
+template <int U>
+FO_DEVI void copy_units(const uint32_t at, const char* src) {
+#pragma unroll
+  for (int i = 0; i < U; ++i) copy_async16(at + 512u * i, src + 512 * i);
+}
+FO_DEVI void copy_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+FO_DEVI float lds_half(uint32_t a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
+  return __half2float(__ushort_as_half(v));
+}
+
+// 32 bytes of a lane.  An array that starts on a 16-byte boundary only takes two stores.
+FO_DEVI void store32(void* p, const uint4& a, const uint4& b, const bool wide) {
+  if (wide) {
+    asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x),
+                 "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+  } else {
+    __stcs((uint4*)p, a);
+    __stcs((uint4*)p + 1, b);
+  }
+}
+FO_DEVI uint4 bits_of(const float2& a, const float2& b) {
+  return make_uint4(__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y));
+}
+
+// The tables: thread t makes the values of one code and stores eight copies at a time, rotated by its lane, so that the lanes of
+// a store fall on different banks.
+template <int OPT>
+FO_DEVI void build_tables(char* table) {
+  for (int i = threadIdx.x; i < (OPT == FO_OPT_ADAM ? 512 : 256); i += kThreads) {
+    const int code = i & 255;
+    const float x = i < 256 ? kDeqM.v[code] : fdiv((float)code, 255.0f);
+    float4* row = reinterpret_cast<float4*>(table + code * 256 + (i < 256 ? 0 : 128));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) row[(k + threadIdx.x) & 7] = make_float4(x, x, x, x);
+  }
+  __syncthreads();
+}
+// the values of the codes in bytes b and b + 1 of w; lane4: four times the lane
+FO_DEVI float2 table_pair(const char* table, const uint32_t w, const int b, const uint32_t lane4) {
+  return make_float2(*reinterpret_cast<const float*>(table + __byte_perm(w, lane4, 0x5504u | (uint32_t)(b << 4))),
+                     *reinterpret_cast<const float*>(table + __byte_perm(w, lane4, 0x5504u | (uint32_t)((b + 1) << 4))));
+}
+
+// A tile that holds a value outside the shortcuts' ranges: again from memory, in the two halves of 256 elements (sixteen lanes' worth) that
+// zero_chunk and warm_chunk take.  `rest`: bit k for a half k in which no new first moment differs from zero.  (Storing a half
+// that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28 elements.)
+template <int OPT, int PDT, int ECC_BITS, int MODE>
+__device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, const uint32_t rest,
+                                       const uint32_t flags, const float wd, const float decay) {
+#pragma unroll 1
+  for (uint32_t half = 0; half < 2u; ++half) {
+    const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
+    if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
+      if ((rest >> half) & 1u) {
+        const Piece at = piece_at<PDT, ECC_BITS, FO_STATE_QUANT>(L, c.grad_dtype, (MODE & kGroup) != 0 ? c.group_shift : 5, i0);
+        if (zero_chunk<OPT, PDT, ECC_BITS>(flags, wd, decay, c.grad_dtype, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) continue;
+      }
+    }
+    warm_chunk<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE>(c, L, out, dh, i0, nullptr);
+  }
+}
+
+// 256 elements from i0 - 8 * lane on of a leaf's ragged end: the code of piece_kernel.
+template <int OPT, int PDT, int ECC_BITS, bool OUT>
+__device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t i0) {
+  const Hyp h = load_hyper<OPT>(dh);
+  if (OPT != FO_OPT_ADAM || (h.flags & kFlagTameAdam) != 0) {
+    const Clip clip = load_clip(c.sq_norm, c.max_norm, c.grad_dtype);
+    ragged_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT, OUT>(c, L, out, dh, h, clip, i0, (uint32_t)L.n);
+  } else {
+    cold_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT>(L, out, dh, c.grad_dtype, c.group_shift, i0, nullptr, c.sq_norm, c.max_norm);
+  }
+}
+
+// One warp's tiles t, t + kWarps, ... below t1 of a leaf.
+template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE, typename OUT>
+FO_DEVI void tile_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const SharedClip& clip, uint32_t t,
+                      const uint32_t t1, const uint32_t slots, const char* table, const OUT& distance) {
+  using namespace fast2;
+  using S = TileSlot<OPT, PDT, ECC_BITS, GDT>;
+  constexpr bool kAdam = OPT == FO_OPT_ADAM;
+  constexpr int kStep = kWarps * kTileElems;  // elements from one of the warp's tiles to the next
+  constexpr int kPsz = PDT == FO_F32 ? 4 : 2, kEsz = ECC_BITS / 8;
+  const int gdt = GDT == kAnyGrad ? c.grad_dtype : GDT;
+  const int gsz = gdt == FO_F32 ? 4 : 2;
+  const int gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;  // 4 to 8 here
+  uint32_t tid;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));  // read once: otherwise re-read at every use
+  const uint32_t lane = tid & 31u, lane4 = lane * 4u, lane16 = lane * 16u;
+  // where the lane's copies come from
+  const size_t e0 = (size_t)t * kTileElems;
+  const char* s_grad = (const char*)L.grad + e0 * (size_t)gsz + lane16;
+  char* s_param = (char*)L.param + e0 * kPsz + lane16;
+  char* s_ecc = (char*)L.ecc + e0 * kEsz + lane16;
+  char* s_mu = (char*)L.mu + e0 + lane16;
+  char* s_nu = (char*)L.nu + e0 + lane16;
+  char* s_msc = (char*)L.mu_scales + ((e0 + lane16) >> gshift) * 2u;  // the scale of the lane's group
+  char* s_vsc = (char*)L.nu_scales + ((e0 + lane16) >> gshift) * 2u;
+  const int sc_step = (kStep >> gshift) * 2;
+  // The group scales travel with the tile in words of four bytes, the first moment's by lanes 0 to 15, the second's by the others.  (Loaded
+  // into registers one tile ahead, they shared a scoreboard with the loads from shared memory, which then waited for DRAM: 615 to
+  // 750 us per 2^28 elements, as the compiler happened to assign it.)  Arrays that begin in the middle of a word still do that.
+  const bool sc_words = ((reinterpret_cast<uintptr_t>(L.mu_scales) | (kAdam ? reinterpret_cast<uintptr_t>(L.nu_scales) : 0)) & 3u) == 0;
+  const bool sc_mine = sc_words && (lane & 15u) < (256u >> gshift) && (kAdam || lane < 16u);
+  const char* s_sc = (const char*)(kAdam && lane >= 16u ? L.nu_scales : L.mu_scales) + (e0 >> gshift) * 2u + (lane & 15u) * 4u;
+  // copies of the lane's units of the tile `ahead` steps on
+  auto fill = [&](const uint32_t slot, const int ahead) {
+    copy_units<S::kParamUnits>(slot + Units<S::kParamUnits>::copy_to(lane), s_param + ahead * (kStep * kPsz));
+    if constexpr (ECC_BITS != 0) copy_units<S::kEccUnits>(slot + S::kEcc + Units<S::kEccUnits>::copy_to(lane), s_ecc + ahead * (kStep * kEsz));
+    copy_units<1>(slot + S::kMu + lane16, s_mu + ahead * kStep);
+    if constexpr (kAdam) copy_units<1>(slot + S::kNu + lane16, s_nu + ahead * kStep);
+    if (gdt == FO_F32) copy_units<4>(slot + S::kGrad + Units<4>::copy_to(lane), s_grad + ahead * (kStep * 4));
+    else copy_units<2>(slot + S::kGrad + Units<2>::copy_to(lane), s_grad + ahead * (kStep * 2));
+    if (sc_mine) copy_async4(slot + S::kScales + lane4, s_sc + ahead * sc_step);
+  };
+  bool wide = ((reinterpret_cast<uintptr_t>(L.param) | (ECC_BITS == 16 ? reinterpret_cast<uintptr_t>(L.ecc) : 0)) & 31u) == 0;
+  if constexpr ((MODE & kOut) != 0) wide = wide && ((distance(&DevOut::param) | (ECC_BITS == 16 ? distance(&DevOut::ecc) : 0)) & 31) == 0;
+  uint32_t slot = slots;
+  __syncwarp();
+  fill(slot, 0);
+  copy_commit();
+  __half msc = __float2half(0.0f), vsc = msc;
+  if (!sc_words) {
+    msc = *(const __half*)s_msc;
+    if constexpr (kAdam) vsc = *(const __half*)s_vsc;
+  }
+  while (true) {
+    const bool more = t + kWarps < t1;
+    __syncwarp();
+    if (more) fill(2u * slots + S::kBytes - slot, 1);
+    copy_commit();
+    copy_wait<1>();
+    __syncwarp();
+    float2 msc2, vsc2 = sp(0.0f);
+    if (sc_words) {
+      const uint32_t sc_at = slot + S::kScales + ((lane16 >> gshift) << 1);
+      msc2 = sp(lds_half(sc_at));
+      if constexpr (kAdam) vsc2 = sp(lds_half(sc_at + 64u));
+    } else {
+      msc2 = sp(__half2float(msc));
+      if constexpr (kAdam) vsc2 = sp(__half2float(vsc));
+      if (more) {
+        msc = *(const __half*)(s_msc + sc_step);
+        if constexpr (kAdam) vsc = *(const __half*)(s_vsc + sc_step);
+      }
+    }
+    const uint4 mq = lds128(slot + S::kMu + lane16);
+    uint4 vq = make_uint4(0, 0, 0, 0), eq = vq;
+    if constexpr (kAdam) vq = lds128(slot + S::kNu + lane16);
+    if constexpr (ECC_BITS == 8) eq = lds128(slot + S::kEcc + lane16);
+    bool rare = false;
+    float2 m[2][4], nroot[2][4], theta[2][4];
+    uint32_t nw[2][4];
+    uint4 ecc_out[2];
+    float am = 0.0f, av = 0.0f;
+    const uint32_t p_at = slot + Units<S::kParamUnits>::read_at(lane);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {  // the lane's first and second eight elements
+      Unpacked u;
+      if (gdt == FO_F32) {
+        const uint32_t g_at = slot + S::kGrad + Units<4>::read_at(lane);
+        pairs_of(lds128(g_at ^ (32u * k)), lds128(g_at ^ (32u * k + 16u)), u.g);
+      } else {
+        const uint4 w = lds128((slot + S::kGrad + Units<2>::read_at(lane)) ^ (16u * k));
+        if (gdt == FO_BF16) pairs_of16<FO_BF16>(w, u.g);
+        else pairs_of16<FO_F16>(w, u.g);
+      }
+      uint4 p0, p1 = make_uint4(0, 0, 0, 0), e = p1;
+      if constexpr (PDT == FO_F32) { p0 = lds128(p_at ^ (32u * k)); p1 = lds128(p_at ^ (32u * k + 16u)); }
+      else p0 = lds128(p_at ^ (16u * k));
+      if constexpr (ECC_BITS == 16) e = lds128((slot + S::kEcc + Units<2>::read_at(lane)) ^ (16u * k));
+      if constexpr (ECC_BITS == 8) { e.x = k ? eq.z : eq.x; e.y = k ? eq.w : eq.y; }
+      bool odd = unpack_master<false, PDT, ECC_BITS>(p0, p1, e, u.theta);
+      const uint32_t mw[2] = {k ? mq.z : mq.x, k ? mq.w : mq.y}, vw[2] = {k ? vq.z : vq.x, k ? vq.w : vq.y};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        u.m[j] = mul2(table_pair(table, mw[j >> 1], 2 * (j & 1), lane4), msc2);  // quantization.py:52-55
+        if constexpr (kAdam) {                                                   // quantization.py:74-77
+          const float2 s = mul2(table_pair(table + 128, vw[j >> 1], 2 * (j & 1), lane4), vsc2);
+          u.v[j] = mul2(s, s);
+        }
+      }
+      if constexpr ((MODE & kClip) != 0) {
+        if (clip.active) odd = clip_grads<false>(u.g, gdt, clip) || odd;
+      }
+      float am_lane, av_lane;
+      odd = update_pairs<false, OPT, FO_STATE_QUANT, false>(h, c.one, u, nroot[k], am_lane, av_lane) || odd;
+      // (an infinite fp32 parameter takes part in a weight decay of zero too)
+      if constexpr (PDT == FO_F32) odd = odd || !(maxabs8(u.theta) <= 3.4e38f);
+      odd = stored_form<false, PDT, ECC_BITS>(u.theta, nw[k], ecc_out[k]) || odd;
+      rare = rare || odd;
+      am = k ? max2<true>(am, am_lane) : am_lane;
+      av = k ? max2<true>(av, av_lane) : av_lane;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { m[k][j] = u.m[j]; theta[k][j] = u.theta[j]; }
+    }
+    // ---- group maxima, and one decision per warp ------------------------------------------------------------
+    const bool rest = am == 0.0f;
+    if constexpr ((MODE & kGroup) != 0) {
+      for (int o = 1; o < (1 << (gshift - 4)); o <<= 1) {
+        am = max2<true>(am, __shfl_xor_sync(0xFFFFFFFFu, am, o));
+        if constexpr (kAdam) av = max2<true>(av, __shfl_xor_sync(0xFFFFFFFFu, av, o));
+      }
+    } else {
+      am = max2<true>(am, __shfl_xor_sync(0xFFFFFFFFu, am, 1));
+      if constexpr (kAdam) av = max2<true>(av, __shfl_xor_sync(0xFFFFFFFFu, av, 1));
+    }
+    rare = rare || !(am >= 1.0e-12f && am <= 1.0e30f);                           // an all-zero group, or beyond the reciprocal's range
+    if constexpr (kAdam) rare = rare || !(av >= 1.0e-12f && av <= 1.0737418e9f);  // 2^30: also the limit of the packed division
+    if (__any_sync(0xFFFFFFFFu, rare)) {
+      uint32_t still = 0u;
+      if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
+        // (Lion, SGD: with a learning rate and momentum of the other sign a parameter of -0 becomes +0.  An infinite fp32 parameter
+        // under a decay of zero that is added to the gradient is no row at rest.)
+        if ((kAdam || (h.lr >= 0.0f && h.lr <= 1.0e30f && h.b1 >= 0.0f)) && (PDT != FO_F32 || OPT == FO_OPT_LION || (h.flags & FO_FLAG_DECOUPLED_WD) != 0)) {
+          const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
+          still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
+        }
+      }
+      redo_tile<OPT, PDT, ECC_BITS, MODE>(c, L, out, dh, t * (uint32_t)kTileElems, still, h.flags, h.wd, h.decay);
+    } else {
+      // ---- stores: parameter and ECC, scales, codes -------------------------------------------------------------
+      auto to = [&](char* base, long long DevOut::*d) {
+        if constexpr ((MODE & kOut) != 0) return base + distance(d);
+        else return base;
+      };
+      if constexpr ((MODE & kDelta) != 0) {
+        if (h.flags & FO_FLAG_LP_DELTA) {  // (the old parameter is still in the slot)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            if constexpr (PDT == FO_F32) hand_back_delta<PDT>(lds128(p_at ^ (32u * k)), lds128(p_at ^ (32u * k + 16u)), nw[k], theta[k]);
+            else hand_back_delta<PDT>(lds128(p_at ^ (16u * k)), make_uint4(0, 0, 0, 0), nw[k], theta[k]);
+          }
+        }
+      }
+      char* const o_param = to(s_param, &DevOut::param) + lane16 * (S::kParamUnits - 1);
+      if constexpr (PDT == FO_F32) {
+        store32(o_param, bits_of(theta[0][0], theta[0][1]), bits_of(theta[0][2], theta[0][3]), wide);
+        store32(o_param + 32, bits_of(theta[1][0], theta[1][1]), bits_of(theta[1][2], theta[1][3]), wide);
+      } else {
+        store32(o_param, make_uint4(nw[0][0], nw[0][1], nw[0][2], nw[0][3]), make_uint4(nw[1][0], nw[1][1], nw[1][2], nw[1][3]), wide);
+      }
+      if constexpr (ECC_BITS == 16) store32(to(s_ecc, &DevOut::ecc) + lane16, ecc_out[0], ecc_out[1], wide);
+      if constexpr (ECC_BITS == 8) __stcs((uint4*)to(s_ecc, &DevOut::ecc), make_uint4(ecc_out[0].x, ecc_out[0].y, ecc_out[1].x, ecc_out[1].y));
+      // all lanes of a group store its scale: same value to the same address, one unpredicated instruction
+      *(__half*)to(s_msc, &DevOut::mu_scales) = __float2half_rn(am);
+      if constexpr (kAdam) *(__half*)to(s_vsc, &DevOut::nu_scales) = __float2half_rn(av);
+      uint32_t q[2][8];
+      {
+        const float2 nam = sp(-am), rm2 = sp(fast::rcp_rn(am));
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) softsign_code_bits2(div_by_rcp2(m[k][j], nam, rm2), q[k][2 * j], q[k][2 * j + 1]);
+        __stcs((uint4*)to(s_mu, &DevOut::mu), make_uint4(pack_bytes(q[0][0], q[0][1], q[0][2], q[0][3]), pack_bytes(q[0][4], q[0][5], q[0][6], q[0][7]),
+                                                         pack_bytes(q[1][0], q[1][1], q[1][2], q[1][3]), pack_bytes(q[1][4], q[1][5], q[1][6], q[1][7])));
+      }
+      if constexpr (kAdam) {
+        const float2 av2 = sp(av), nrv2 = sp(-fast::rcp_rn(av));
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) quant_v_bits2(nroot[k][j], av2, nrv2, q[k][2 * j], q[k][2 * j + 1]);
+        __stcs((uint4*)to(s_nu, &DevOut::nu), make_uint4(pack_bytes(q[0][0], q[0][1], q[0][2], q[0][3]), pack_bytes(q[0][4], q[0][5], q[0][6], q[0][7]),
+                                                         pack_bytes(q[1][0], q[1][1], q[1][2], q[1][3]), pack_bytes(q[1][4], q[1][5], q[1][6], q[1][7])));
+      }
+    }
+    if (!more) return;
+    t += kWarps;
+    slot = 2u * slots + S::kBytes - slot;
+    s_grad += kStep * gsz;
+    s_param += kStep * kPsz;
+    if constexpr (ECC_BITS != 0) s_ecc += kStep * kEsz;
+    s_mu += kStep;
+    s_sc += sc_step;
+    s_msc += sc_step;
+    if constexpr (kAdam) { s_nu += kStep; s_vsc += sc_step; }
+  }
+}
+
+// Persistent grid, one block per SM.  The tiles of all leaves form one sequence, cut into runs of p.run_chunks tiles; block b takes
+// runs b, b + grid, ..., and tile i of a run belongs to warp i modulo the number of warps, so the work of an SM is even to a tile.
+template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE>
+__global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant__ TileParams<MODE> p) {
+  extern __shared__ __align__(128) unsigned char tile_mem[];  // the tables, then every warp's slots
+  char* const table = reinterpret_cast<char*>(tile_mem);
+  build_tables<OPT>(table);
+  if (p.wait) chain_wait();
+  chain_release();
+  using S = TileSlot<OPT, PDT, ECC_BITS, GDT>;
+  const uint32_t warp = threadIdx.x / 32u;
+  const uint32_t slots = (uint32_t)__cvta_generic_to_shared(tile_mem) + (uint32_t)kTableBytes + warp * (uint32_t)(kTileStages * S::kBytes);
+  SharedClip clip{false, 0u};
+  if constexpr ((MODE & kClip) != 0) {
+    __shared__ float4 clip_constants;
+    const Clip k = load_clip(p.sq_norm, p.max_norm, p.grad_dtype);
+    if (threadIdx.x == 0) clip_constants = make_float4(k.n_g, k.rcp_n, k.m_g, __uint_as_float(k.div_ok ? 1u : 0u));
+    __syncthreads();
+    clip.active = k.active;
+    clip.at = (uint32_t)__cvta_generic_to_shared(&clip_constants);
+  }
+  // Ragged ends first, one piece to a block at a time, beginning with the last blocks and warps, which have the fewest tiles: their
+  // latency then passes behind the other warps' work.  (As a launch of piece_kernel they came behind the last tile, and
+  // cost the host a launch: Lion on 2999 x 1777 and its bias 13.2 us, now 12.2.)
+  for (uint32_t q = (kWarps - 1u - warp) * gridDim.x + (gridDim.x - 1u - blockIdx.x); q < p.first_end[p.n_leaves]; q += kWarps * gridDim.x) {
+    const int l = leaf_of(p.first_end, p.n_leaves, (uint16_t)q);
+    const DevLeaf& L = p.t.leaf[l];
+    const DevOut* out = nullptr;
+    if constexpr ((MODE & kOut) != 0) out = &p.out[l];
+    const uint32_t i0 = (uint32_t)(L.n / kTileElems) * kTileElems + (q - p.first_end[l]) * kEnd + (threadIdx.x & 31u) * kPiece;
+    end_piece<OPT, PDT, ECC_BITS, (MODE & kOut) != 0>(p, L, out, p.hyper[p.t.hyper_of[l]], i0);
+  }
+  const uint32_t total = p.t.first_block[p.n_leaves];
+  for (uint32_t run0 = blockIdx.x * p.run_chunks; run0 < total; run0 += gridDim.x * p.run_chunks) {
+    uint32_t at = run0;  // this block's next position in the sequence
+    const uint32_t run1 = min(total, run0 + p.run_chunks);
+    for (int l = leaf_of(p.t.first_block, p.n_leaves, at); l < p.n_leaves; ++l) {
+      if (at >= run1) break;
+      const uint32_t first = p.t.first_block[l];
+      const uint32_t next = min(p.t.first_block[l + 1], run1);
+      if (at >= next) continue;
+      uint32_t t = at - first + (warp + kWarps - (at - run0) % kWarps) % kWarps;  // the warp's first tile of the leaf in this run
+      const uint32_t t1 = next - first;
+      at = next;
+      if (t >= t1) continue;
+      const DevLeaf& L = p.t.leaf[l];
+      const DevHyper& dh = p.hyper[p.t.hyper_of[l]];
+      const DevOut* out = nullptr;
+      if constexpr ((MODE & kOut) != 0) out = &p.out[l];
+      const Hyp h = load_hyper<OPT>(dh);
+      if constexpr (OPT == FO_OPT_ADAM) {
+        // device-resident scalars can leave the range the reciprocal shortcut in the denominator is proven for
+        if ((h.flags & kFlagTameAdam) == 0) {
+          for (; t < t1; t += kWarps)
+            for (uint32_t half = 0; half < 2u; ++half)
+              cold_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT>(L, out, dh, p.grad_dtype, (MODE & kGroup) != 0 ? p.group_shift : 5,
+                                                             (unsigned long long)t * kTileElems + half * 256u + (threadIdx.x & 31u) * 8u, nullptr,
+                                                             (MODE & kClip) != 0 ? p.sq_norm : nullptr, p.max_norm);
+          continue;
+        }
+      }
+      if constexpr ((MODE & kOut) != 0)
+        tile_run<OPT, PDT, ECC_BITS, GDT, MODE>(p, L, out, dh, h, clip, t, t1, slots, table, OutOf{p, l});
+      else
+        tile_run<OPT, PDT, ECC_BITS, GDT, MODE>(p, L, out, dh, h, clip, t, t1, slots, table, OutAt{nullptr});
+    }
+  }
+  chain_end();
+}
+
+template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE>
+cudaError_t launch_tiles(HostStep& hs, bool& chained, cudaStream_t s) {
+  auto kernel = tile_kernel<OPT, PDT, ECC_BITS, GDT, MODE>;
+  constexpr int smem = tile_smem<OPT, PDT, ECC_BITS, GDT>();
+  static_assert(smem <= kSmemPerBlock, "the slots fit a block");
+  // whether a device's copy of the function has been opted in above 48 KB (per instantiation; concurrent first calls may both set it)
+  static std::atomic<bool> opted_in[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64 || !opted_in[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) opted_in[dev].store(true, std::memory_order_release);
+  }
+  TileParams<MODE> p;  // filled as far as it is used
+  fill_common(p, hs);
+  uint32_t total = 0, ends = 0;
+  int n = 0;
+  for (int i = 0; i < hs.n_leaves; ++i) {
+    const HostLeaf& l = hs.leaf[i];
+    if (!l.hot || l.src.n == 0) continue;
+    p.t.leaf[n] = l.src;
+    p.t.hyper_of[n] = l.hyper;
+    p.t.first_block[n] = total;
+    p.first_end[n] = (uint16_t)ends;
+    if constexpr ((MODE & kOut) != 0) p.out[n] = l.out;
+    total += (uint32_t)(l.src.n / kTileElems);
+    ends += (uint32_t)((l.src.n % kTileElems + kEnd - 1) / kEnd);
+    ++n;
+  }
+  if (n == 0) return cudaSuccess;
+  p.n_leaves = n;
+  p.t.first_block[n] = total;
+  p.first_end[n] = (uint16_t)ends;
+  const unsigned int grid = (unsigned int)hs.sm_count;
+  // Run length: a launch of at most 256 tiles per block (it lasts tens of microseconds) goes out as one run per block, to within a
+  // tile; a larger one in runs of a quarter of a block's share, at most 1536 tiles, so that regions that cost more (rows at rest, values
+  // outside the shortcuts' ranges) are spread over all blocks.
+  const unsigned int share = (total + grid - 1u) / grid;
+  unsigned int run = share;
+  if (share > 256u) run = (total + grid * 4u - 1u) / (grid * 4u);
+  p.run_chunks = run < 1u ? 1u : (run > 1536u ? 1536u : run);
+  return launched(hs, launch_chained(kernel, grid, kThreads, smem, chained, s, p));
+}
+
+}  // namespace FO_SHAPE_NS
+
+}  // namespace fo

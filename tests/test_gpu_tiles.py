@@ -1,0 +1,109 @@
+"""tile_kernel, bit for bit against the CPU oracle, where its tiles of 512 elements, its leaf tables and its copies can go wrong:
+leaves that end around a tile or shorter than one, runs that begin inside a leaf, arrays that start off 32 bytes (parameters and
+ECC then leave in two stores) or in the middle of a four-byte word (scales), every gradient dtype, weight decay added to the gradient."""
+
+import numpy as np
+import pytest
+
+from oracle import c_oracle as C
+from oracle import flashoptim_oracle as O
+from tests import helpers as H
+from tests.test_gpu_step_routes import G_NP, _step
+
+pytestmark = pytest.mark.gpu
+
+MANY = 148 * 8192 + 1  # a call of more than 148 * 8192 elements is not left to piece_kernel alone
+SIZES = (512, 511, 513, 255, 256, 257, 767, 768, 769, 1, 1023, 1025, 1536, 2047, 2048, 3072 + 511, 16 * 1024, 16 * 1024 + 512, 33 * 1024, 5)
+
+
+def _moved(t, elems):
+    """The same values `elems` elements further into an allocation."""
+    import torch
+
+    return None if t is None else torch.cat([t[:1].expand(elems), t])[elems:]
+
+
+def _check(opt, pdt, ecc_bits, group, conv, gdt, sizes, *, max_norm=None, elsewhere=False, moved=None, **hyper):
+    import torch
+
+    from flashoptim_jax_b200 import _engine as eng
+
+    rng = np.random.default_rng(sum(sizes) + group + gdt)
+    refs = [H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, group) for n in sizes]
+    refs[0].param[::97] = 0  # values outside the shortcuts' ranges
+    place = (lambda leaf: H.LeafArrays(*[_moved(getattr(leaf, f), moved[f]) for f in leaf.fields()])) if moved else lambda leaf: leaf
+    devs = [place(r.copy().to_device()) for r in refs]
+    for t in (1, 2):
+        grads = [H.make_grad(rng, n, 1e-2, G_NP[gdt], outliers=1e-3) for n in sizes]
+        hp = H.hyper_tuple(opt, conv, t, lr=1e-3, wd=1e-2, **hyper)
+        dev_g = [H.to_torch(g) for g in grads]
+        sq = None
+        if max_norm is not None:
+            sq = eng.sq_norm_of(dev_g)
+            grads = O.clip_by_global_norm(grads, max_norm, sq_norm=float(sq.cpu()))
+        for g, r in zip(grads, refs):
+            H.oracle_step(opt, g, r, C.STATE_QUANT, group, hp)
+        outs = [place(H.LeafArrays(*[None if getattr(d, f) is None else torch.empty_like(getattr(d, f)) for f in d.fields()])) for d in devs] if elsewhere else None
+        _step(opt, dev_g, devs, outs, C.STATE_QUANT, group, hp, pdt, gdt, ecc_bits, sq, max_norm or 0.0)
+        torch.cuda.synchronize()
+        devs = outs if elsewhere else devs
+        for i, (d, r) in enumerate(zip(devs, refs)):
+            H.assert_leaf_equal(d.to_host(), r, f"step {t} leaf {i} n={sizes[i]}")
+
+
+@pytest.mark.parametrize("gdt", [0, 1, 2])
+@pytest.mark.parametrize("opt,pdt,ecc_bits,group,conv,more", [
+    (C.ADAM, 1, 16, 32, O.FUSED, {}), (C.ADAM, 2, 8, 256, O.FUSED, {}), (C.ADAM, 1, 8, 32, O.UNFUSED, {}), (C.ADAM, 0, 0, 16, O.FUSED, {}),
+    (C.ADAM, 1, 0, 32, O.FUSED, dict(max_norm=0.5)), (C.ADAM, 2, 16, 32, O.FUSED, dict(elsewhere=True)), (C.ADAM, 1, 8, 8, O.FUSED, {}),
+    (C.ADAM, 1, 16, 32, O.FUSED, dict(decoupled=False)), (C.LION, 1, 8, 32, O.FUSED, {}), (C.LION, 2, 16, 64, O.UNFUSED, {}),
+    (C.LION, 0, 0, 32, O.FUSED, dict(max_norm=0.5)), (C.SGD, 1, 16, 32, O.FUSED, dict(nesterov=True)), (C.SGD, 2, 8, 128, O.FUSED, {}),
+    (C.SGD, 0, 0, 32, O.FUSED, dict(decoupled=False)), (C.SGD, 1, 8, 32, O.FUSED, dict(elsewhere=True))])
+def test_leaves_that_end_around_a_tile(opt, pdt, ecc_bits, group, conv, more, gdt):
+    _check(opt, pdt, ecc_bits, group, conv, gdt, (MANY + 700,) + SIZES, **more)
+
+
+@pytest.mark.parametrize("offset,scale_offset", [(8, 1), (16, 2), (8, 2), (24, 3)])
+@pytest.mark.parametrize("opt,pdt,ecc_bits,elsewhere", [(C.ADAM, 1, 16, False), (C.ADAM, 2, 8, True), (C.LION, 1, 16, True), (C.SGD, 0, 0, False)])
+def test_arrays_off_the_alignment_of_the_wide_accesses(opt, pdt, ecc_bits, elsewhere, offset, scale_offset):
+    moved = {"param": offset // (2 if pdt == 0 else 1), "ecc": offset * 2 if ecc_bits == 8 else offset, "mu": 16, "nu": 48, "mu_scales": scale_offset,
+             "nu_scales": 2}
+    _check(opt, pdt, ecc_bits, 32, O.FUSED, 0, (MANY + 700, 4096, 1536), elsewhere=elsewhere, moved=moved)
+
+
+def test_tables_of_many_leaves_and_several_runs_per_block():
+    rng = np.random.default_rng(5)
+    _check(C.ADAM, 1, 8, 32, O.FUSED, 1, tuple(int(x) for x in rng.integers(500, 30000, 330)))
+    _check(C.LION, 1, 8, 32, O.FUSED, 1, (148 * 512 * 300 + 1024, 700 * 1024 + 512, 3 * 1024))  # more than 256 tiles per block
+
+
+@pytest.mark.parametrize("opt,pdt,ecc_bits,group,more", [
+    (C.ADAM, 1, 16, 32, {}), (C.ADAM, 0, 0, 32, dict(decoupled=False, wd=0.0)), (C.LION, 1, 16, 32, {}), (C.LION, 2, 8, 128, {}), (C.LION, 0, 0, 32, {}),
+    (C.SGD, 1, 8, 32, {}), (C.SGD, 2, 16, 256, dict(nesterov=True)), (C.SGD, 0, 0, 32, {}), (C.SGD, 0, 0, 32, dict(decoupled=False, wd=0.0)),
+    (C.SGD, 1, 8, 32, dict(lr=-1e-3, momentum=-0.9)), (C.LION, 2, 8, 32, dict(lr=-1e-3))])
+def test_rows_at_rest_in_parts_of_tiles(opt, pdt, ecc_bits, group, more):
+    """Rows without gradients that begin and end inside tiles and halves of tiles, with zeros of both signs and infinities among
+    their parameters."""
+    import torch
+
+    rng = np.random.default_rng(opt * 10 + pdt)
+    n = MANY + 5000
+    p = rng.normal(0, 0.02, n).astype(np.float32)
+    p[::301], p[7::401] = 0.0, -0.0
+    if pdt != 1:
+        p[5::70001] = np.inf
+    ref = H.fresh_leaf(p.astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, group)
+    dev = ref.copy().to_device()
+    kw = dict(dict(lr=1e-3, wd=1e-2), **more)
+    for t in (1, 2):
+        g = H.make_grad(rng, n, 1e-2, H.BF16)
+        for start, length in ((0, 512), (5 * 512 + 256, 256), (9000, 700), (20000, 1408), (30001, 4099), (n - 3000, 3000)):
+            g[start:start + length] = 0
+            g[start:start + length:3] = -0.0
+        hp = H.hyper_tuple(opt, O.FUSED, t, **kw)
+        H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+        _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 1, ecc_bits)
+        torch.cuda.synchronize()
+        got = dev.to_host()
+        both = np.isnan(got.param.astype(np.float32)) & np.isnan(ref.param.astype(np.float32))
+        got.param[both] = ref.param[both]  # (whichever NaN it is)
+        H.assert_leaf_equal(got, ref, f"step {t}")
