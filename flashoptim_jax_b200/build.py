@@ -44,10 +44,11 @@ _SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "ou
            ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1),
            ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1),
            ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "all"): (512, 1)}
-# Threads of the one block per SM that runs tile_kernel (quantized moments, one feature at most).  AdamW wants 150 to 168 registers
-# for the 16 elements of a lane (2^28 elements, 24-bit masters: 588 us with 384 threads, 623 with 512; with the power cap reached
-# 672 and 704); Lion and SGD need fewer (with the cap reached 477 us with 512 threads and 485 with 384, and 445 against 464).
-_TILE_THREADS = {"adam": 384, "lion": 512, "sgd": 512}
+# Threads of the one block per SM that runs tile_kernel (quantized moments, one feature at most).  The 16 elements of a lane want 150 to
+# 168 registers under AdamW (2^28 elements, 24-bit masters: 588 us with 384 threads, 623 with 512; with the power cap reached
+# 672 and 704) and 138 under SGD (65 M elements, 32-bit masters, results elsewhere: 129 us with 384 threads, 143 with 512, 132 with 256);
+# Lion fits 512 (fp16, 2^28 elements: 435 us, 455 with 384).
+_TILE_THREADS = {"adam": 384, "lion": 512, "sgd": 384}
 _TILE_MODES = ("plain", "clip", "out", "group", "delta")
 # name and feature mask (fo_step.cuh) of the kernels of a slice
 _MODES = (("plain", 0), ("clip", 1), ("out", 2), ("group", 4), ("delta", 8), ("all", 15), ("peer", 16), ("piece", -1))

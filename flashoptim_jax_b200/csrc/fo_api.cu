@@ -62,6 +62,9 @@ static PieceFn find_pieces(int opt, int pdt, int ecc_bits, int state) {
 #ifndef FO_SMALL_ELEMS
 #define FO_SMALL_ELEMS (148ull * 8192ull)
 #endif
+// The same where tile_kernel takes over, whose warps spread tiles of 512 elements (AdamW, 24-bit masters, in us with pieces and with tiles:
+// 2^19 elements 4.5 / 4.7, 2^20 6.8 / 5.5, 2^21 12.8 / 8.2).
+constexpr unsigned long long kSmallElemsTiles = 148ull * 4096ull;
 
 static DevHyper make_dev_hyper(const FoHyper& h, int opt) {
   DevHyper d;
@@ -229,7 +232,8 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
       e = launcher.launch(hs, chained, stream);
     } else {
       // with peers the whole chunks always take the kernel that knows them (the pieces' path is scalar there)
-      const unsigned int main_chunk = (with_peers ? whole > 0 : whole > FO_SMALL_ELEMS) ? launcher.chunk : 0u;
+      const unsigned long long small = launcher.chunk == 1u ? kSmallElemsTiles : FO_SMALL_ELEMS;
+      const unsigned int main_chunk = (with_peers ? whole > 0 : whole > small) ? launcher.chunk : 0u;
       if (main_chunk != 0) e = launcher.launch(hs, chained, stream);
       if (e == cudaSuccess) e = pieces(hs, main_chunk, chained, stream);
     }

@@ -12,7 +12,7 @@ from tests.test_gpu_step_routes import G_NP, _step
 
 pytestmark = pytest.mark.gpu
 
-MANY = 148 * 8192 + 1  # a call of more than 148 * 8192 elements is not left to piece_kernel alone
+MANY = 148 * 8192 + 1  # more elements than go through piece_kernel alone (148 * 4096 here)
 SIZES = (512, 511, 513, 255, 256, 257, 767, 768, 769, 1, 1023, 1025, 1536, 2047, 2048, 3072 + 511, 16 * 1024, 16 * 1024 + 512, 33 * 1024, 5)
 
 
