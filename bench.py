@@ -597,7 +597,7 @@ def run_ours(args):
         captured = NCU_DRAM_BYTES_PER_PARAM.get((optimizer, bucket[3])) if bucket[1] == 1 and bucket[2] == 1 else None
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "traffic": captured * n_par if captured is not None else None,
-                    "kernel": f"step_kernel<{optimizer}, {'f32' if bucket[1] == 0 else ('bf16' if bucket[1] == 1 else 'f16')}, ecc{bucket[3]}, quant>",
+                    "kernel": f"tile_kernel<{optimizer}, {'f32' if bucket[1] == 0 else ('bf16' if bucket[1] == 1 else 'f16')}, ecc{bucket[3]}, quant>",
                     "params_per_launch": n_par, "avg_launch_ms": avg_ms, "launches_timed": len(pool[top]),
                     "algorithmic_bytes_per_param": bpp, "peak_source": peak_src}
         if world > 1:
@@ -805,7 +805,7 @@ def run_square_sweep(args):
                    "l2": "cases marked l2_resident touch less than the 126 MB L2 per step and run from it (no flush): their GB/s is "
                          "not an HBM figure; the others exceed L2"},
         "roofline": {"bound": "hbm", "achieved": head["gb_per_s"], "peak": peak, "unit": "GB/s", "frac": head["frac_of_peak"],
-                     "traffic": NCU_DRAM_BYTES_PER_PARAM[("adamw", 16)] * head["params"], "kernel": "step_kernel<adamw, bf16, ecc16, quant>",
+                     "traffic": NCU_DRAM_BYTES_PER_PARAM[("adamw", 16)] * head["params"], "kernel": "tile_kernel<adamw, bf16, ecc16, quant>",
                      "params_per_launch": head["params"], "avg_launch_ms": head["ms_per_step"], "peak_source": peak_src,
                      "algorithmic_bytes_per_param": bytes_per_param("adamw", 2, 16, 2)},
         "cpu_baseline": None, "e2e": None, "gpu_launches": launches, "clocks": clocks,
