@@ -15,8 +15,8 @@
 //   * All range checks are known once the group maxima are: one vote, then the stores of parameter and ECC, then the codes.
 //   * Two slots per warp and a loop body that is not unrolled: three slots and an unrolled body measured the same.
 //
-// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 627 now, 0.94 of the copy rate; with
-// the power cap reached 798 -> 717.  52 to 55 instructions per element instead of 63.
+// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 632 now, 0.93 of the copy rate; with
+// the power cap reached 798 -> 705.  52 to 55 instructions per element instead of 63.
 #pragma once
 
 namespace fo {
@@ -140,9 +140,49 @@ __device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, co
   }
 }
 
-// One warp's tiles t, t + kWarps, ... below t1 of a leaf.
+// Where a lane's copies of a tile come from, and the copies.
+template <int OPT, int PDT, int ECC_BITS, int GDT>
+struct TileSource {
+  using S = TileSlot<OPT, PDT, ECC_BITS, GDT>;
+  static constexpr bool kAdam = OPT == FO_OPT_ADAM;
+  static constexpr int kPsz = PDT == FO_F32 ? 4 : 2, kEsz = ECC_BITS / 8;
+  const char* grad;
+  char* param;
+  char* ecc;
+  char* mu;
+  char* nu;
+  // The group scales travel with the tile in words of four bytes, the first moment's by lanes 0 to 15, the second's by the others.  (Loaded
+  // into registers one tile ahead, they shared a scoreboard with the loads from shared memory, which then waited for DRAM: 615 to
+  // 750 us per 2^28 elements, as the compiler happened to assign it.)  Arrays that begin in the middle of a word still do that.
+  const char* sc;
+  bool sc_words, sc_mine;
+  FO_DEVI TileSource(const DevLeaf& L, const uint32_t t, const int gsz, const int gshift, const uint32_t lane) {
+    const size_t e0 = (size_t)t * kTileElems;
+    grad = (const char*)L.grad + e0 * (size_t)gsz + lane * 16u;
+    param = (char*)L.param + e0 * kPsz + lane * 16u;
+    ecc = (char*)L.ecc + e0 * kEsz + lane * 16u;
+    mu = (char*)L.mu + e0 + lane * 16u;
+    nu = (char*)L.nu + e0 + lane * 16u;
+    sc = (const char*)(kAdam && lane >= 16u ? L.nu_scales : L.mu_scales) + (e0 >> gshift) * 2u + (lane & 15u) * 4u;
+    sc_words = ((reinterpret_cast<uintptr_t>(L.mu_scales) | (kAdam ? reinterpret_cast<uintptr_t>(L.nu_scales) : 0)) & 3u) == 0;
+    sc_mine = sc_words && (lane & 15u) < (256u >> gshift) && (kAdam || lane < 16u);
+  }
+  // the lane's units of the tile `ahead` steps on
+  FO_DEVI void fill(const uint32_t slot, const int ahead, const int gdt, const int gshift, const uint32_t lane) const {
+    constexpr int kStep = kWarps * kTileElems;
+    copy_units<S::kParamUnits>(slot + Units<S::kParamUnits>::copy_to(lane), param + ahead * (kStep * kPsz));
+    if constexpr (ECC_BITS != 0) copy_units<S::kEccUnits>(slot + S::kEcc + Units<S::kEccUnits>::copy_to(lane), ecc + ahead * (kStep * kEsz));
+    copy_units<1>(slot + S::kMu + lane * 16u, mu + ahead * kStep);
+    if constexpr (kAdam) copy_units<1>(slot + S::kNu + lane * 16u, nu + ahead * kStep);
+    if (gdt == FO_F32) copy_units<4>(slot + S::kGrad + Units<4>::copy_to(lane), grad + ahead * (kStep * 4));
+    else copy_units<2>(slot + S::kGrad + Units<2>::copy_to(lane), grad + ahead * (kStep * 2));
+    if (sc_mine) copy_async4(slot + S::kScales + lane * 4u, sc + ahead * ((kStep >> gshift) * 2));
+  }
+};
+
+// One warp's tiles t, t + kWarps, ... below t1 of a leaf.  `primed`: the first one's copies are under way, in the first slot.
 template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE, typename OUT>
-FO_DEVI void tile_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const SharedClip& clip, uint32_t t,
+FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const SharedClip& clip, uint32_t t,
                       const uint32_t t1, const uint32_t slots, const char* table, const OUT& distance) {
   using namespace fast2;
   using S = TileSlot<OPT, PDT, ECC_BITS, GDT>;
@@ -155,52 +195,33 @@ FO_DEVI void tile_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, 
   uint32_t tid;
   asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));  // read once: otherwise re-read at every use
   const uint32_t lane = tid & 31u, lane4 = lane * 4u, lane16 = lane * 16u;
-  // where the lane's copies come from
   const size_t e0 = (size_t)t * kTileElems;
-  const char* s_grad = (const char*)L.grad + e0 * (size_t)gsz + lane16;
-  char* s_param = (char*)L.param + e0 * kPsz + lane16;
-  char* s_ecc = (char*)L.ecc + e0 * kEsz + lane16;
-  char* s_mu = (char*)L.mu + e0 + lane16;
-  char* s_nu = (char*)L.nu + e0 + lane16;
+  TileSource<OPT, PDT, ECC_BITS, GDT> s(L, t, gsz, gshift, lane);
   char* s_msc = (char*)L.mu_scales + ((e0 + lane16) >> gshift) * 2u;  // the scale of the lane's group
   char* s_vsc = (char*)L.nu_scales + ((e0 + lane16) >> gshift) * 2u;
   const int sc_step = (kStep >> gshift) * 2;
-  // The group scales travel with the tile in words of four bytes, the first moment's by lanes 0 to 15, the second's by the others.  (Loaded
-  // into registers one tile ahead, they shared a scoreboard with the loads from shared memory, which then waited for DRAM: 615 to
-  // 750 us per 2^28 elements, as the compiler happened to assign it.)  Arrays that begin in the middle of a word still do that.
-  const bool sc_words = ((reinterpret_cast<uintptr_t>(L.mu_scales) | (kAdam ? reinterpret_cast<uintptr_t>(L.nu_scales) : 0)) & 3u) == 0;
-  const bool sc_mine = sc_words && (lane & 15u) < (256u >> gshift) && (kAdam || lane < 16u);
-  const char* s_sc = (const char*)(kAdam && lane >= 16u ? L.nu_scales : L.mu_scales) + (e0 >> gshift) * 2u + (lane & 15u) * 4u;
-  // copies of the lane's units of the tile `ahead` steps on
-  auto fill = [&](const uint32_t slot, const int ahead) {
-    copy_units<S::kParamUnits>(slot + Units<S::kParamUnits>::copy_to(lane), s_param + ahead * (kStep * kPsz));
-    if constexpr (ECC_BITS != 0) copy_units<S::kEccUnits>(slot + S::kEcc + Units<S::kEccUnits>::copy_to(lane), s_ecc + ahead * (kStep * kEsz));
-    copy_units<1>(slot + S::kMu + lane16, s_mu + ahead * kStep);
-    if constexpr (kAdam) copy_units<1>(slot + S::kNu + lane16, s_nu + ahead * kStep);
-    if (gdt == FO_F32) copy_units<4>(slot + S::kGrad + Units<4>::copy_to(lane), s_grad + ahead * (kStep * 4));
-    else copy_units<2>(slot + S::kGrad + Units<2>::copy_to(lane), s_grad + ahead * (kStep * 2));
-    if (sc_mine) copy_async4(slot + S::kScales + lane4, s_sc + ahead * sc_step);
-  };
   bool wide = ((reinterpret_cast<uintptr_t>(L.param) | (ECC_BITS == 16 ? reinterpret_cast<uintptr_t>(L.ecc) : 0)) & 31u) == 0;
   if constexpr ((MODE & kOut) != 0) wide = wide && ((distance(&DevOut::param) | (ECC_BITS == 16 ? distance(&DevOut::ecc) : 0)) & 31) == 0;
   uint32_t slot = slots;
-  __syncwarp();
-  fill(slot, 0);
-  copy_commit();
+  if (!primed) {
+    __syncwarp();
+    s.fill(slot, 0, gdt, gshift, lane);
+    copy_commit();
+  }
   __half msc = __float2half(0.0f), vsc = msc;
-  if (!sc_words) {
+  if (!s.sc_words) {
     msc = *(const __half*)s_msc;
     if constexpr (kAdam) vsc = *(const __half*)s_vsc;
   }
   while (true) {
     const bool more = t + kWarps < t1;
     __syncwarp();
-    if (more) fill(2u * slots + S::kBytes - slot, 1);
+    if (more) s.fill(2u * slots + S::kBytes - slot, 1, gdt, gshift, lane);
     copy_commit();
     copy_wait<1>();
     __syncwarp();
     float2 msc2, vsc2 = sp(0.0f);
-    if (sc_words) {
+    if (s.sc_words) {
       const uint32_t sc_at = slot + S::kScales + ((lane16 >> gshift) << 1);
       msc2 = sp(lds_half(sc_at));
       if constexpr (kAdam) vsc2 = sp(lds_half(sc_at + 64u));
@@ -301,15 +322,15 @@ FO_DEVI void tile_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, 
           }
         }
       }
-      char* const o_param = to(s_param, &DevOut::param) + lane16 * (S::kParamUnits - 1);
+      char* const o_param = to(s.param, &DevOut::param) + lane16 * (S::kParamUnits - 1);
       if constexpr (PDT == FO_F32) {
         store32(o_param, bits_of(theta[0][0], theta[0][1]), bits_of(theta[0][2], theta[0][3]), wide);
         store32(o_param + 32, bits_of(theta[1][0], theta[1][1]), bits_of(theta[1][2], theta[1][3]), wide);
       } else {
         store32(o_param, make_uint4(nw[0][0], nw[0][1], nw[0][2], nw[0][3]), make_uint4(nw[1][0], nw[1][1], nw[1][2], nw[1][3]), wide);
       }
-      if constexpr (ECC_BITS == 16) store32(to(s_ecc, &DevOut::ecc) + lane16, ecc_out[0], ecc_out[1], wide);
-      if constexpr (ECC_BITS == 8) __stcs((uint4*)to(s_ecc, &DevOut::ecc), make_uint4(ecc_out[0].x, ecc_out[0].y, ecc_out[1].x, ecc_out[1].y));
+      if constexpr (ECC_BITS == 16) store32(to(s.ecc, &DevOut::ecc) + lane16, ecc_out[0], ecc_out[1], wide);
+      if constexpr (ECC_BITS == 8) __stcs((uint4*)to(s.ecc, &DevOut::ecc), make_uint4(ecc_out[0].x, ecc_out[0].y, ecc_out[1].x, ecc_out[1].y));
       // all lanes of a group store its scale: same value to the same address, one unpredicated instruction
       *(__half*)to(s_msc, &DevOut::mu_scales) = __float2half_rn(am);
       if constexpr (kAdam) *(__half*)to(s_vsc, &DevOut::nu_scales) = __float2half_rn(av);
@@ -320,7 +341,7 @@ FO_DEVI void tile_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, 
         for (int k = 0; k < 2; ++k)
 #pragma unroll
           for (int j = 0; j < 4; ++j) softsign_code_bits2(div_by_rcp2(m[k][j], nam, rm2), q[k][2 * j], q[k][2 * j + 1]);
-        __stcs((uint4*)to(s_mu, &DevOut::mu), make_uint4(pack_bytes(q[0][0], q[0][1], q[0][2], q[0][3]), pack_bytes(q[0][4], q[0][5], q[0][6], q[0][7]),
+        __stcs((uint4*)to(s.mu, &DevOut::mu), make_uint4(pack_bytes(q[0][0], q[0][1], q[0][2], q[0][3]), pack_bytes(q[0][4], q[0][5], q[0][6], q[0][7]),
                                                          pack_bytes(q[1][0], q[1][1], q[1][2], q[1][3]), pack_bytes(q[1][4], q[1][5], q[1][6], q[1][7])));
       }
       if constexpr (kAdam) {
@@ -329,20 +350,20 @@ FO_DEVI void tile_run(const StepCommon& c, const DevLeaf& L, const DevOut* out, 
         for (int k = 0; k < 2; ++k)
 #pragma unroll
           for (int j = 0; j < 4; ++j) quant_v_bits2(nroot[k][j], av2, nrv2, q[k][2 * j], q[k][2 * j + 1]);
-        __stcs((uint4*)to(s_nu, &DevOut::nu), make_uint4(pack_bytes(q[0][0], q[0][1], q[0][2], q[0][3]), pack_bytes(q[0][4], q[0][5], q[0][6], q[0][7]),
+        __stcs((uint4*)to(s.nu, &DevOut::nu), make_uint4(pack_bytes(q[0][0], q[0][1], q[0][2], q[0][3]), pack_bytes(q[0][4], q[0][5], q[0][6], q[0][7]),
                                                          pack_bytes(q[1][0], q[1][1], q[1][2], q[1][3]), pack_bytes(q[1][4], q[1][5], q[1][6], q[1][7])));
       }
     }
     if (!more) return;
     t += kWarps;
     slot = 2u * slots + S::kBytes - slot;
-    s_grad += kStep * gsz;
-    s_param += kStep * kPsz;
-    if constexpr (ECC_BITS != 0) s_ecc += kStep * kEsz;
-    s_mu += kStep;
-    s_sc += sc_step;
+    s.grad += kStep * gsz;
+    s.param += kStep * kPsz;
+    if constexpr (ECC_BITS != 0) s.ecc += kStep * kEsz;
+    s.mu += kStep;
+    s.sc += sc_step;
     s_msc += sc_step;
-    if constexpr (kAdam) { s_nu += kStep; s_vsc += sc_step; }
+    if constexpr (kAdam) { s.nu += kStep; s_vsc += sc_step; }
   }
 }
 
@@ -352,12 +373,25 @@ template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE>
 __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant__ TileParams<MODE> p) {
   extern __shared__ __align__(128) unsigned char tile_mem[];  // the tables, then every warp's slots
   char* const table = reinterpret_cast<char*>(tile_mem);
-  build_tables<OPT>(table);
-  if (p.wait) chain_wait();
-  chain_release();
   using S = TileSlot<OPT, PDT, ECC_BITS, GDT>;
   const uint32_t warp = threadIdx.x / 32u;
   const uint32_t slots = (uint32_t)__cvta_generic_to_shared(tile_mem) + (uint32_t)kTableBytes + warp * (uint32_t)(kTileStages * S::kBytes);
+  const uint32_t total = p.t.first_block[p.n_leaves];
+  // The block's first run, and its first leaf, are known before the wait: a warp that has a tile there asks for it right behind.
+  // (The hyper-parameters, clipping constants and ends then pass under the latency of the copies.  AdamW, 24-bit masters, cold arrays of 2^21,
+  // 2^22, 2^24 elements: 8.4, 14.5, 43.7 us without, 7.5, 13.5, 41.6 so; Lion on 5.3 M 12.7, 12.4.  Asking for the first tile
+  // of every later run or leaf ahead as well gave nothing more.)
+  const int l0 = leaf_of(p.t.first_block, p.n_leaves, blockIdx.x * p.run_chunks);
+  const uint32_t t0 = blockIdx.x * p.run_chunks - p.t.first_block[l0] + warp;
+  const bool primed0 = blockIdx.x * p.run_chunks < total &&
+                       t0 < min(p.t.first_block[l0 + 1], min(total, (blockIdx.x + 1u) * p.run_chunks)) - p.t.first_block[l0];
+  const int gdt0 = GDT == kAnyGrad ? p.grad_dtype : GDT, gshift0 = (MODE & kGroup) != 0 ? p.group_shift : 5;
+  const TileSource<OPT, PDT, ECC_BITS, GDT> source0(p.t.leaf[l0], t0, gdt0 == FO_F32 ? 4 : 2, gshift0, threadIdx.x & 31u);
+  build_tables<OPT>(table);
+  if (p.wait) chain_wait();
+  chain_release();
+  if (primed0) source0.fill(slots, 0, gdt0, gshift0, threadIdx.x & 31u);
+  copy_commit();
   SharedClip clip{false, 0u};
   if constexpr ((MODE & kClip) != 0) {
     __shared__ float4 clip_constants;
@@ -378,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
     const uint32_t i0 = (uint32_t)(L.n / kTileElems) * kTileElems + (q - p.first_end[l]) * kEnd + (threadIdx.x & 31u) * kPiece;
     end_piece<OPT, PDT, ECC_BITS, (MODE & kOut) != 0>(p, L, out, p.hyper[p.t.hyper_of[l]], i0);
   }
-  const uint32_t total = p.t.first_block[p.n_leaves];
+  bool primed = primed0;
   for (uint32_t run0 = blockIdx.x * p.run_chunks; run0 < total; run0 += gridDim.x * p.run_chunks) {
     uint32_t at = run0;  // this block's next position in the sequence
     const uint32_t run1 = min(total, run0 + p.run_chunks);
@@ -399,6 +433,8 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
       if constexpr (OPT == FO_OPT_ADAM) {
         // device-resident scalars can leave the range the reciprocal shortcut in the denominator is proven for
         if ((h.flags & kFlagTameAdam) == 0) {
+          copy_wait<0>();
+          primed = false;
           for (; t < t1; t += kWarps)
             for (uint32_t half = 0; half < 2u; ++half)
               cold_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT>(L, out, dh, p.grad_dtype, (MODE & kGroup) != 0 ? p.group_shift : 5,
@@ -408,9 +444,10 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
         }
       }
       if constexpr ((MODE & kOut) != 0)
-        tile_run<OPT, PDT, ECC_BITS, GDT, MODE>(p, L, out, dh, h, clip, t, t1, slots, table, OutOf{p, l});
+        tile_run<OPT, PDT, ECC_BITS, GDT, MODE>(primed, p, L, out, dh, h, clip, t, t1, slots, table, OutOf{p, l});
       else
-        tile_run<OPT, PDT, ECC_BITS, GDT, MODE>(p, L, out, dh, h, clip, t, t1, slots, table, OutAt{nullptr});
+        tile_run<OPT, PDT, ECC_BITS, GDT, MODE>(primed, p, L, out, dh, h, clip, t, t1, slots, table, OutAt{nullptr});
+      primed = false;
     }
   }
   chain_end();
