@@ -274,8 +274,9 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
       }
       float am_lane, av_lane;
       odd = update_pairs<false, OPT, FO_STATE_QUANT, false>(h, c.one, u, nroot[k], am_lane, av_lane) || odd;
-      // (an infinite fp32 parameter takes part in a weight decay of zero too)
-      if constexpr (PDT == FO_F32) odd = odd || !(maxabs8(u.theta) <= 3.4e38f);
+      // (Infinite parameters and NaNs take part in a weight decay of zero that is added to the gradient, which this pass leaves out.  Where there
+      // is an error-correction code stored_form sees them.)
+      if constexpr (ECC_BITS == 0 && OPT != FO_OPT_LION) odd = odd || !(maxabs8(u.theta) <= 3.4e38f);
       odd = stored_form<false, PDT, ECC_BITS>(u.theta, nw[k], ecc_out[k]) || odd;
       rare = rare || odd;
       am = k ? max2<true>(am, am_lane) : am_lane;
@@ -299,9 +300,9 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
     if (__any_sync(0xFFFFFFFFu, rare)) {
       uint32_t still = 0u;
       if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
-        // (Lion, SGD: with a learning rate and momentum of the other sign a parameter of -0 becomes +0.  An infinite fp32 parameter
-        // under a decay of zero that is added to the gradient is no row at rest.)
-        if ((kAdam || (h.lr >= 0.0f && h.lr <= 1.0e30f && h.b1 >= 0.0f)) && (PDT != FO_F32 || OPT == FO_OPT_LION || (h.flags & FO_FLAG_DECOUPLED_WD) != 0)) {
+        // (Lion, SGD: with a learning rate and momentum of the other sign a parameter of -0 becomes +0.  A parameter without a code that is
+        // infinite under a decay of zero that is added to the gradient is no row at rest.)
+        if ((kAdam || (h.lr >= 0.0f && h.lr <= 1.0e30f && h.b1 >= 0.0f)) && (ECC_BITS != 0 || OPT == FO_OPT_LION || (h.flags & FO_FLAG_DECOUPLED_WD) != 0)) {
           const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
           still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
         }

@@ -107,3 +107,40 @@ def test_rows_at_rest_in_parts_of_tiles(opt, pdt, ecc_bits, group, more):
         both = np.isnan(got.param.astype(np.float32)) & np.isnan(ref.param.astype(np.float32))
         got.param[both] = ref.param[both]  # (whichever NaN it is)
         H.assert_leaf_equal(got, ref, f"step {t}")
+
+
+def _but_for_nans(got, ref, group, at):
+    """`got` with what NaNs leave open made that of `ref`: which NaN a parameter is, and, where the elements `at` have NaN moments, the scales of
+    their groups (any size but 32: NaN, which is checked here; of 32 elements that of the others) and the codes beside them."""
+    both = np.isnan(got.param.astype(np.float32)) & np.isnan(ref.param.astype(np.float32))
+    got.param[both] = ref.param[both]
+    if group != 32:
+        hit = np.unique(at // group)
+        for scales, codes in (("mu_scales", "mu"), ("nu_scales", "nu")):
+            if getattr(ref, scales) is not None:
+                assert np.isnan(getattr(got, scales)[hit]).all()
+                getattr(got, scales)[hit] = getattr(ref, scales)[hit]
+                inside = np.isin(np.arange(ref.param.size) // group, hit)
+                getattr(got, codes)[inside] = getattr(ref, codes)[inside]
+    return got
+
+
+@pytest.mark.parametrize("n", [1000, MANY + 700])
+@pytest.mark.parametrize("decay", [dict(decoupled=False, wd=0.0), dict(decoupled=False, wd=1e-2), dict(wd=1e-2)])
+@pytest.mark.parametrize("opt,pdt,group", [(C.ADAM, 1, 32), (C.ADAM, 2, 64), (C.ADAM, 0, 32), (C.SGD, 1, 16), (C.SGD, 2, 32), (C.SGD, 0, 128), (C.LION, 2, 32)])
+def test_parameters_without_codes_that_are_not_finite(opt, pdt, group, decay, n):
+    """Infinities and NaNs among parameters without error-correction codes: a decay that is added to the gradient makes the element's
+    moments NaN, a decay of zero too."""
+    rng = np.random.default_rng(n + opt)
+    p = rng.normal(0, 0.02, n).astype(np.float32)
+    for value in (np.inf, -np.inf, np.nan):
+        p[rng.integers(0, n, 1 + n // 3000)] = value
+    ref = H.fresh_leaf(p.astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, 0, group)
+    dev = ref.copy().to_device()
+    g = H.make_grad(rng, n, 1e-2, H.BF16)
+    hp = H.hyper_tuple(opt, O.FUSED, 1, **dict(dict(lr=1e-3), **decay))
+    H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+    _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 1, 0)
+    odd = np.isnan(p) if decay["wd"] != 0.0 else ~np.isfinite(p)  # (a decay of infinity that is not zero is an infinity)
+    at = np.flatnonzero(odd) if opt != C.LION and "decoupled" in decay else np.empty(0, dtype=np.int64)
+    H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, group, at), ref, f"n={n}")
