@@ -1009,6 +1009,8 @@ __device__ __noinline__ bool zero_chunk(const uint32_t flags, const float wd, co
   }
   float2 theta[4];
   bool rare = unpack_master<false, PDT, ECC_BITS>(p0, p1, e, theta);
+  // (0 * inf and 0 * NaN are NaN in a gradient that takes a decay of zero; with a code stored_form sees such a parameter)
+  if constexpr (ECC_BITS == 0 && OPT != FO_OPT_LION) rare = rare || ((h.flags & FO_FLAG_DECOUPLED_WD) == 0 && !(maxabs8(theta) <= 3.4e38f));
   if (OPT == FO_OPT_LION || (h.flags & FO_FLAG_DECOUPLED_WD) != 0) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) theta[k] = mul2(theta[k], sp(h.decay));

@@ -300,9 +300,8 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
     if (__any_sync(0xFFFFFFFFu, rare)) {
       uint32_t still = 0u;
       if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
-        // (Lion, SGD: with a learning rate and momentum of the other sign a parameter of -0 becomes +0.  A parameter without a code that is
-        // infinite under a decay of zero that is added to the gradient is no row at rest.)
-        if ((kAdam || (h.lr >= 0.0f && h.lr <= 1.0e30f && h.b1 >= 0.0f)) && (ECC_BITS != 0 || OPT == FO_OPT_LION || (h.flags & FO_FLAG_DECOUPLED_WD) != 0)) {
+        // (Lion, SGD: with a learning rate and momentum of the other sign a parameter of -0 becomes +0)
+        if (kAdam || (h.lr >= 0.0f && h.lr <= 1.0e30f && h.b1 >= 0.0f)) {
           const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
           still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
         }

@@ -144,3 +144,22 @@ def test_parameters_without_codes_that_are_not_finite(opt, pdt, group, decay, n)
     odd = np.isnan(p) if decay["wd"] != 0.0 else ~np.isfinite(p)  # (a decay of infinity that is not zero is an infinity)
     at = np.flatnonzero(odd) if opt != C.LION and "decoupled" in decay else np.empty(0, dtype=np.int64)
     H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, group, at), ref, f"n={n}")
+
+
+@pytest.mark.parametrize("n", [1024, 3000, MANY + 700])
+@pytest.mark.parametrize("opt,pdt,ecc_bits", [(C.ADAM, 1, 0), (C.ADAM, 2, 0), (C.ADAM, 0, 0), (C.SGD, 1, 0), (C.SGD, 2, 0), (C.SGD, 0, 0), (C.ADAM, 1, 8), (C.SGD, 2, 16)])
+def test_parameters_at_rest_that_are_not_finite(opt, pdt, ecc_bits, n):
+    """The same in rows without gradients, under a decay of zero that is added to the gradient: no rows at rest, in pieces and in tiles."""
+    rng = np.random.default_rng(n + opt)
+    p = rng.normal(0, 0.02, n).astype(np.float32)
+    at = np.unique(rng.integers(0, n, 3 + n // 3000))
+    p[at] = rng.choice([np.inf, -np.inf], at.size) if ecc_bits else rng.choice([np.inf, -np.inf, np.nan], at.size)
+    ref = H.fresh_leaf(p.astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, 32)
+    dev = ref.copy().to_device()
+    g = np.zeros(n, dtype=H.BF16)
+    g[::3] = -0.0
+    hp = H.hyper_tuple(opt, O.FUSED, 1, lr=1e-3, decoupled=False, wd=0.0)
+    for t in (1, 2):
+        H.oracle_step(opt, g, ref, C.STATE_QUANT, 32, hp)
+        _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, 32, hp, pdt, 1, ecc_bits)
+        H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, 32, at), ref, f"n={n} step {t}")
