@@ -257,6 +257,14 @@ FO_DEVI Hyp load_hyper(const DevHyper& d) {
   return h;
 }
 
+// Whether a step without gradients on moments of zero is the weight decay alone.  Its update term is the learning rate times +0 then: a NaN under
+// an infinite one, and -0, which turns a parameter of -0 into +0, under a learning rate or momentum with a sign.
+template <int OPT>
+FO_DEVI bool rest_is_decay(const Hyp& h) {
+  const float lr = OPT == FO_OPT_ADAM ? h.lr_bc1 : h.lr;
+  return __float_as_int(lr) >= 0 && lr <= 1.0e30f && __float_as_int(h.b1) >= 0;
+}
+
 FO_DEVI float sign_of(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : x); }
 
 // ============================================================================================
@@ -1433,7 +1441,7 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
     if (__any_sync(0xFFFFFFFFu, rare)) {
       if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && (MODE & ~(kClip | kGroup)) == 0) {
         // no new first moment of the warp differs from zero: look whether the whole piece is at rest
-        if (__all_sync(0xFFFFFFFFu, am_lane == 0.0f) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
+        if (__all_sync(0xFFFFFFFFu, am_lane == 0.0f) && rest_is_decay<OPT>(h) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
       }
       warm_chunk<OPT, PDT, ECC_BITS, STATE, MODE>(c, L, out, dh, i0, peers);
       return;
@@ -1616,7 +1624,7 @@ FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut* o
   if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && !OUT) {
     // a whole warp at rest, as in step_kernel (one million elements at rest: 23.0 us with every element repaired, 5.8 so)
     const bool codes_zero = n_valid == kPiece && (raw.mq.x | raw.mq.y | raw.vq.x | raw.vq.y) == 0u;
-    if (__all_sync(0xFFFFFFFFu, codes_zero && (h.flags & FO_FLAG_LP_DELTA) == 0)) {
+    if (__all_sync(0xFFFFFFFFu, codes_zero && (h.flags & FO_FLAG_LP_DELTA) == 0) && rest_is_decay<OPT>(h)) {
       const bool rest = maxabs8(u.g) == 0.0f && maxabs8(u.m) == 0.0f && maxabs8(u.v) == 0.0f;
       if (__all_sync(0xFFFFFFFFu, rest) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
     }

@@ -113,8 +113,9 @@ FO_DEVI float2 table_pair(const char* table, const uint32_t w, const int b, cons
 // zero_chunk and warm_chunk take.  `rest`: bit k for a half k in which no new first moment differs from zero.  (Storing a half
 // that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28 elements.)
 template <int OPT, int PDT, int ECC_BITS, int MODE>
-__device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, const uint32_t rest,
+__device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, uint32_t rest,
                                        const uint32_t flags, const float wd, const float decay) {
+  if (rest != 0u && !rest_is_decay<OPT>(load_hyper<OPT>(dh))) rest = 0u;  // (asked here: in the loop it costs AdamW's kernels up to 5 %)
 #pragma unroll 1
   for (uint32_t half = 0; half < 2u; ++half) {
     const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
@@ -300,11 +301,8 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
     if (__any_sync(0xFFFFFFFFu, rare)) {
       uint32_t still = 0u;
       if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
-        // (Lion, SGD: with a learning rate and momentum of the other sign a parameter of -0 becomes +0)
-        if (kAdam || (h.lr >= 0.0f && h.lr <= 1.0e30f && h.b1 >= 0.0f)) {
-          const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
-          still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
-        }
+        const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
+        still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
       }
       redo_tile<OPT, PDT, ECC_BITS, MODE>(c, L, out, dh, t * (uint32_t)kTileElems, still, h.flags, h.wd, h.decay);
     } else {

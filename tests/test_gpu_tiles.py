@@ -163,3 +163,17 @@ def test_parameters_at_rest_that_are_not_finite(opt, pdt, ecc_bits, n):
         H.oracle_step(opt, g, ref, C.STATE_QUANT, 32, hp)
         _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, 32, hp, pdt, 1, ecc_bits)
         H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, 32, at), ref, f"n={n} step {t}")
+
+
+@pytest.mark.parametrize("n", [1024, MANY + 700])
+@pytest.mark.parametrize("lr", [-0.0, -1e-3, np.inf])
+@pytest.mark.parametrize("opt", [C.ADAM, C.LION, C.SGD])
+def test_rows_at_rest_under_learning_rates_that_change_them(opt, lr, n):
+    """A parameter of -0 becomes +0 under a learning rate with a sign, every parameter a NaN under an infinite one."""
+    ref = H.fresh_leaf(np.where(np.arange(n) % 3 == 0, -0.0, 0.5).astype(np.float32), opt, C.STATE_QUANT, 0, 32)
+    dev = ref.copy().to_device()
+    g = np.zeros(n, dtype=np.float32)
+    hp = H.hyper_tuple(opt, O.FUSED, 1, lr=lr, wd=1e-2)
+    H.oracle_step(opt, g, ref, C.STATE_QUANT, 32, hp)
+    _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, 32, hp, 0, 0, 0)
+    H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, 32, np.empty(0, dtype=np.int64)), ref, f"n={n} lr={lr}")
