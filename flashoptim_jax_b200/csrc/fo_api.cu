@@ -199,8 +199,7 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
   }
   const bool with_peers = peers.n > 0 || peers.ng > 0;
   const int features = (d->grad_sq_norm != nullptr ? kClip : 0) | (outs != nullptr ? kOut : 0) |
-                       (d->state == FO_STATE_QUANT && d->group_size != 32 ? kGroup : 0) | (lp_delta ? kDelta : 0) |
-                       (d->state == FO_STATE_QUANT && coupled ? kCoupled : 0);
+                       (d->state == FO_STATE_QUANT && d->group_size != 32 ? kGroup : 0) | (lp_delta ? kDelta : 0);
   // (a tile's lane holds two groups of 8: those go through the kernel that carries all features)
   const int mode = with_peers ? kPeer : (features & kGroup) != 0 && d->group_size < 16 ? kAll : features;
   const Launcher launcher = find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, mode, d->grad_dtype);
@@ -217,6 +216,7 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
   hs.sq_norm = d->grad_sq_norm; hs.max_norm = d->max_grad_norm;
   hs.peers = &peers;
   hs.outs = outs != nullptr;
+  hs.coupled = coupled;
   // Launches that touch peers' memory start in stream order, behind the exchange in front of them.
   const bool same_step = more != nullptr && (more->launch_flags & FO_LAUNCH_CHAINED) != 0;
   bool chained = same_step || !with_peers;

@@ -52,8 +52,8 @@ constexpr int kOut = 2;    // results written elsewhere
 constexpr int kGroup = 4;  // quantization groups of 8, 16, 64, 128 or 256
 constexpr int kDelta = 8;  // FO_FLAG_LP_DELTA
 constexpr int kAll = 15;
-constexpr int kCoupled = 32;  // weight decay added to the gradient (not zero, not decoupled); quantized moments
 constexpr int kPeer = 16;  // peers' gradients and parameter replicas, clipping; groups of 32, in place
+constexpr int kCoupled = 32;  // beside any one of tile_kernel's: weight decay added to the gradient, not zero (step_kernel always knows it)
 
 // Names below depend on the block shape of the translation unit (FO_THREADS): each shape has its own.
 #ifndef FO_SHAPE_NS
@@ -2164,6 +2164,7 @@ struct HostStep {
   const Peers* peers;
   bool outs;  // results go where HostLeaf::out says
   bool wait;  // of the next launch
+  bool coupled;  // some leaf's weight decay is added to its gradient and not zero
 };
 // `chained`: the launch in front of this one on the stream is one of this library's and works on other leaves,
 // or the kernel begins with chain_wait(); set to true by a launch.

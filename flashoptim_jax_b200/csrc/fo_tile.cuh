@@ -119,13 +119,13 @@ __device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, co
 #pragma unroll 1
   for (uint32_t half = 0; half < 2u; ++half) {
     const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
-    if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
+    if constexpr ((MODE & ~(kClip | kGroup | kCoupled)) == 0) {
       if ((rest >> half) & 1u) {
         const Piece at = piece_at<PDT, ECC_BITS, FO_STATE_QUANT>(L, c.grad_dtype, (MODE & kGroup) != 0 ? c.group_shift : 5, i0);
         if (zero_chunk<OPT, PDT, ECC_BITS>(flags, wd, decay, c.grad_dtype, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) continue;
       }
     }
-    warm_chunk<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE>(c, L, out, dh, i0, nullptr);
+    warm_chunk<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE & ~kCoupled>(c, L, out, dh, i0, nullptr);
   }
 }
 
@@ -274,10 +274,10 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
         if (clip.active) odd = clip_grads<false>(u.g, gdt, clip) || odd;
       }
       float am_lane, av_lane;
-      odd = update_pairs<false, OPT, FO_STATE_QUANT, false>(h, c.one, u, nroot[k], am_lane, av_lane) || odd;
+      odd = update_pairs<false, OPT, FO_STATE_QUANT, (MODE & kCoupled) != 0>(h, c.one, u, nroot[k], am_lane, av_lane) || odd;
       // (Infinite parameters and NaNs take part in a weight decay of zero that is added to the gradient, which this pass leaves out.  Where there
       // is an error-correction code stored_form sees them.)
-      if constexpr (ECC_BITS == 0 && OPT != FO_OPT_LION) odd = odd || !(maxabs8(u.theta) <= 3.4e38f);
+      if constexpr (ECC_BITS == 0 && OPT != FO_OPT_LION && (MODE & kCoupled) == 0) odd = odd || !(maxabs8(u.theta) <= 3.4e38f);
       odd = stored_form<false, PDT, ECC_BITS>(u.theta, nw[k], ecc_out[k]) || odd;
       rare = rare || odd;
       am = k ? max2<true>(am, am_lane) : am_lane;
@@ -300,7 +300,7 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
     if constexpr (kAdam) rare = rare || !(av >= 1.0e-12f && av <= 1.0737418e9f);  // 2^30: also the limit of the packed division
     if (__any_sync(0xFFFFFFFFu, rare)) {
       uint32_t still = 0u;
-      if constexpr ((MODE & ~(kClip | kGroup)) == 0) {
+      if constexpr ((MODE & ~(kClip | kGroup | kCoupled)) == 0) {
         const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
         still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
       }
@@ -453,6 +453,9 @@ __global__ void __launch_bounds__(kThreads, 1) tile_kernel(const __grid_constant
 
 template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE>
 cudaError_t launch_tiles(HostStep& hs, bool& chained, cudaStream_t s) {
+  if constexpr (OPT != FO_OPT_LION && (MODE & kCoupled) == 0) {
+    if (hs.coupled) return launch_tiles<OPT, PDT, ECC_BITS, GDT, MODE | kCoupled>(hs, chained, s);
+  }
   auto kernel = tile_kernel<OPT, PDT, ECC_BITS, GDT, MODE>;
   constexpr int smem = tile_smem<OPT, PDT, ECC_BITS, GDT>();
   static_assert(smem <= kSmemPerBlock, "the slots fit a block");

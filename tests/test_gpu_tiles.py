@@ -62,6 +62,22 @@ def test_leaves_that_end_around_a_tile(opt, pdt, ecc_bits, group, conv, more, gd
     _check(opt, pdt, ecc_bits, group, conv, gdt, (MANY + 700,) + SIZES, **more)
 
 
+@pytest.mark.parametrize("more", [{}, dict(max_norm=0.5), dict(elsewhere=True), dict(group=128), dict(conv=O.UNFUSED)])
+@pytest.mark.parametrize("opt,pdt,ecc_bits,gdt", [(C.ADAM, 1, 16, 1), (C.ADAM, 2, 8, 0), (C.ADAM, 0, 0, 0), (C.SGD, 1, 8, 1), (C.SGD, 2, 0, 1)])
+def test_decay_added_to_the_gradient(opt, pdt, ecc_bits, gdt, more):
+    """A weight decay that is added to the gradient beside every feature, by tile_kernel as without it."""
+    import torch
+
+    more = dict(dict(group=32, conv=O.FUSED), **more)
+    group, conv = more.pop("group"), more.pop("conv")
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        _check(opt, pdt, ecc_bits, group, conv, gdt, (MANY + 700,) + SIZES, decoupled=False, **more)
+    kernels = {e.key for e in prof.key_averages()}
+    if not any("kernel" in k for k in kernels):
+        pytest.skip("the profiler records no kernels here")
+    assert any("tile_kernel" in k for k in kernels) and not any("step_kernel" in k for k in kernels), kernels
+
+
 @pytest.mark.parametrize("offset,scale_offset", [(8, 1), (16, 2), (8, 2), (24, 3)])
 @pytest.mark.parametrize("opt,pdt,ecc_bits,elsewhere", [(C.ADAM, 1, 16, False), (C.ADAM, 2, 8, True), (C.LION, 1, 16, True), (C.SGD, 0, 0, False)])
 def test_arrays_off_the_alignment_of_the_wide_accesses(opt, pdt, ecc_bits, elsewhere, offset, scale_offset):
