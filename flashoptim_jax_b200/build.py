@@ -41,22 +41,23 @@ _KINDS = (("quant", 0), ("full", 1), ("generic", 3))
 # stream and one set of tables); the kernels that also read peers' gradients keep 256-thread blocks,
 # whose smaller stages leave room for a deeper copy pipeline.
 _SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1),
-           ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1),
-           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1),
-           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "all"): (512, 1)}
+           ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1), ("adam", "group8"): (512, 1),
+           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1), ("lion", "group8"): (512, 1),
+           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "all"): (512, 1), ("sgd", "group8"): (512, 1)}
 # Threads of the one block per SM that runs tile_kernel (quantized moments, one feature at most).  The 16 elements of a lane want 150 to
 # 168 registers under AdamW (2^28 elements, 24-bit masters: 588 us with 384 threads, 623 with 512; with the power cap reached
 # 672 and 704) and 138 under SGD (65 M elements, 32-bit masters, results elsewhere: 129 us with 384 threads, 143 with 512, 132 with 256);
 # Lion fits 512 (fp16, 2^28 elements: 435 us, 455 with 384).
 _TILE_THREADS = {"adam": 384, "lion": 512, "sgd": 384}
 _TILE_MODES = ("plain", "clip", "out", "group", "delta")
-# name and feature mask (fo_step.cuh) of the kernels of a slice
-_MODES = (("plain", 0), ("clip", 1), ("out", 2), ("group", 4), ("delta", 8), ("all", 15), ("peer", 16), ("piece", -1))
+# Name and feature mask (fo_step.cuh) of the kernels of a slice.  Groups of 8, two to a tile's lane, go through step_kernel (one of their own: AdamW
+# 4096 x 4096 49 us, through the kernel that carries all features 59; Lion 32.9 and 34.8, SGDW 31.9 and 33.3).
+_MODES = (("plain", 0), ("clip", 1), ("out", 2), ("group", 4), ("group8", 4), ("delta", 8), ("all", 15), ("peer", 16), ("piece", -1))
 
 
 def _has_kernel(oname: str, kname: str, mname: str) -> bool:
     """Group sizes concern quantized moments only, the parameter hand-back Adam only."""
-    return not (mname == "group" and kname != "quant") and not (mname == "delta" and oname != "adam")
+    return not (mname.startswith("group") and kname != "quant") and not (mname == "delta" and oname != "adam")
 
 
 def _units(shapes=None, ffi_dir: str | None = None) -> List[Tuple[str, str, List[str]]]:
@@ -69,7 +70,10 @@ def _units(shapes=None, ffi_dir: str | None = None) -> List[Tuple[str, str, List
         suffix = f"_{mname}" if mname else ""
         flags = [f"-DFO_INST_OPT={omacro}", f"-DFO_INST_KIND={kind}", f"-DFO_INST_MODE={mode}",
                  f"-DFO_INST_NAME=lookup_{oname}_{kname}{suffix}"]
-        shape = (_TILE_THREADS[oname], 1) if kind == 0 and mname in _TILE_MODES else shapes.get((oname, mname))
+        tiles = kind == 0 and mname in _TILE_MODES
+        if tiles:
+            flags.append("-DFO_INST_TILES")
+        shape = (_TILE_THREADS[oname], 1) if tiles else shapes.get((oname, mname))
         if shape is not None and kind != 3:
             flags += [f"-DFO_THREADS={shape[0]}", f"-DFO_MIN_BLOCKS_ADAM={shape[1]}", f"-DFO_MIN_BLOCKS_MOMENTUM={shape[1]}"]
             if len(shape) > 2:

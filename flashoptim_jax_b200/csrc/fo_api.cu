@@ -19,7 +19,7 @@ int fail(int code, const char* fmt, ...) {
 }
 
 // the kernel with the asked features: one of its own for one feature, else the one that carries them all
-static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool generic, int mode, int gdt) {
+static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool generic, int mode, int group_size, int gdt) {
 #define FO_PICK(stem)                                                    \
   switch (mode) {                                                        \
     case kPlain: return stem##_plain(pdt, ecc_bits, gdt);                     \
@@ -30,18 +30,18 @@ static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool ge
   }
   if (opt == FO_OPT_ADAM) {
     if (generic) return lookup_adam_generic(pdt, ecc_bits, gdt);
-    if (mode == kGroup) return lookup_adam_quant_group(pdt, ecc_bits, gdt);
+    if (mode == kGroup) return group_size < 16 ? lookup_adam_quant_group8(pdt, ecc_bits, gdt) : lookup_adam_quant_group(pdt, ecc_bits, gdt);
     if (mode == kDelta) return state == FO_STATE_QUANT ? lookup_adam_quant_delta(pdt, ecc_bits, gdt) : lookup_adam_full_delta(pdt, ecc_bits, gdt);
     if (state == FO_STATE_QUANT) { FO_PICK(lookup_adam_quant) }
     if (state == FO_STATE_FULL) { FO_PICK(lookup_adam_full) }
   } else if (opt == FO_OPT_LION) {
     if (generic) return lookup_lion_generic(pdt, ecc_bits, gdt);
-    if (mode == kGroup) return lookup_lion_quant_group(pdt, ecc_bits, gdt);
+    if (mode == kGroup) return group_size < 16 ? lookup_lion_quant_group8(pdt, ecc_bits, gdt) : lookup_lion_quant_group(pdt, ecc_bits, gdt);
     if (state == FO_STATE_QUANT) { FO_PICK(lookup_lion_quant) }
     if (state == FO_STATE_FULL) { FO_PICK(lookup_lion_full) }
   } else if (opt == FO_OPT_SGD) {
     if (generic) return lookup_sgd_generic(pdt, ecc_bits, gdt);
-    if (mode == kGroup) return lookup_sgd_quant_group(pdt, ecc_bits, gdt);
+    if (mode == kGroup) return group_size < 16 ? lookup_sgd_quant_group8(pdt, ecc_bits, gdt) : lookup_sgd_quant_group(pdt, ecc_bits, gdt);
     if (state == FO_STATE_QUANT) { FO_PICK(lookup_sgd_quant) }
     if (state == FO_STATE_FULL) { FO_PICK(lookup_sgd_full) }
     if (state == FO_STATE_NONE) { FO_PICK(lookup_sgd_none) }
@@ -141,7 +141,7 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
   if (d->n_peers > 0 && d->peer_param_offsets == nullptr && d->peer_grad_offsets == nullptr)
     return fail(FO_ERR_INVALID_ARG, "fo_step: n_peers without peer_param_offsets or peer_grad_offsets");
   if (d->n_peers > 0 && d->state == FO_STATE_QUANT && d->group_size != 32) return fail(FO_ERR_UNSUPPORTED, "fo_step: peer replicas need group_size 32");
-  if (find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, kPlain, d->grad_dtype).launch == nullptr)
+  if (find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, kPlain, 32, d->grad_dtype).launch == nullptr)
     return fail(FO_ERR_UNSUPPORTED, "fo_step: no kernel for this combination");
 
   const bool need_mu = d->state != FO_STATE_NONE;
@@ -200,9 +200,8 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
   const bool with_peers = peers.n > 0 || peers.ng > 0;
   const int features = (d->grad_sq_norm != nullptr ? kClip : 0) | (outs != nullptr ? kOut : 0) |
                        (d->state == FO_STATE_QUANT && d->group_size != 32 ? kGroup : 0) | (lp_delta ? kDelta : 0);
-  // (a tile's lane holds two groups of 8: those go through the kernel that carries all features)
-  const int mode = with_peers ? kPeer : (features & kGroup) != 0 && d->group_size < 16 ? kAll : features;
-  const Launcher launcher = find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, mode, d->grad_dtype);
+  const int mode = with_peers ? kPeer : features;
+  const Launcher launcher = find_launcher(d->opt, d->param_dtype, d->ecc_bits, d->state, generic, mode, d->group_size, d->grad_dtype);
   const PieceFn pieces = generic ? nullptr : find_pieces(d->opt, d->param_dtype, d->ecc_bits, d->state);
   if (launcher.launch == nullptr || (!generic && pieces == nullptr)) return fail(FO_ERR_UNSUPPORTED, "fo_step: no kernel for this combination");
 

@@ -2392,8 +2392,11 @@ FO_DECLARE_SLICE(lookup_adam_quant) FO_DECLARE_SLICE(lookup_adam_full)
 FO_DECLARE_SLICE(lookup_lion_quant) FO_DECLARE_SLICE(lookup_lion_full)
 FO_DECLARE_SLICE(lookup_sgd_quant) FO_DECLARE_SLICE(lookup_sgd_full) FO_DECLARE_SLICE(lookup_sgd_none)
 Launcher lookup_adam_quant_group(int pdt, int ecc_bits, int gdt);
+Launcher lookup_adam_quant_group8(int pdt, int ecc_bits, int gdt);
 Launcher lookup_lion_quant_group(int pdt, int ecc_bits, int gdt);
+Launcher lookup_lion_quant_group8(int pdt, int ecc_bits, int gdt);
 Launcher lookup_sgd_quant_group(int pdt, int ecc_bits, int gdt);
+Launcher lookup_sgd_quant_group8(int pdt, int ecc_bits, int gdt);
 Launcher lookup_adam_quant_delta(int pdt, int ecc_bits, int gdt);
 Launcher lookup_adam_full_delta(int pdt, int ecc_bits, int gdt);
 Launcher lookup_adam_generic(int pdt, int ecc_bits, int gdt);

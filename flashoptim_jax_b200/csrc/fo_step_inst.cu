@@ -1,7 +1,7 @@
 // Instantiates one slice of the step-kernel family.  Compiled once per (optimizer, state kind,
 // kernel) with -DFO_INST_OPT=<FO_OPT_*> -DFO_INST_KIND=<0 quantized | 1 full | 2 none | 3 any group size>
-// -DFO_INST_MODE=<the kernel's features, fo_step.cuh; -1 pieces> -DFO_INST_NAME=<lookup function name>, so the slices
-// build in parallel and each can have its own block size (-DFO_THREADS, -DFO_MIN_BLOCKS_*, and a namespace
+// -DFO_INST_MODE=<the kernel's features, fo_step.cuh; -1 pieces> -DFO_INST_NAME=<lookup function name>, and -DFO_INST_TILES for
+// tile_kernel in place of step_kernel, so the slices build in parallel and each can have its own block size (-DFO_THREADS, -DFO_MIN_BLOCKS_*, and a namespace
 // -DFO_SHAPE_NS of its own for what depends on it).
 #include "fo_step.cuh"
 
@@ -29,8 +29,8 @@ Launcher FO_INST_NAME(int pdt, int ecc_bits, int gdt) {
 #if FO_INST_KIND == 3
 #define X(P, E) \
   if (pdt == P && ecc_bits == E) return Launcher{&launch_generic<FO_INST_OPT, P, E>, 0u, kMaxLeaves};
-#elif FO_INST_KIND == 0 && FO_INST_MODE != 15 && FO_INST_MODE != 16
-  // tiles: gradients of the parameter's dtype or fp32, which is what steps have, by kernels of their own
+#elif defined(FO_INST_TILES)
+  // gradients of the parameter's dtype or fp32, which is what steps have, by kernels of their own
 #define X(P, E)                                                                                                       \
   if (pdt == P && ecc_bits == E) {                                                                                    \
     if (gdt == P) return Launcher{&launch_tiles<FO_INST_OPT, P, E, P, FO_INST_MODE>, 1u, most_leaves};                \

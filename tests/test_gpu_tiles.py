@@ -51,6 +51,18 @@ def _check(opt, pdt, ecc_bits, group, conv, gdt, sizes, *, max_norm=None, elsewh
             H.assert_leaf_equal(d.to_host(), r, f"step {t} leaf {i} n={sizes[i]}")
 
 
+def _kernels_of(call):
+    """Names of the kernels that `call` launches."""
+    import torch
+
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+    kernels = {e.key for e in prof.key_averages()}
+    if not any("kernel" in k for k in kernels):
+        pytest.skip("the profiler records no kernels here")
+    return kernels
+
+
 @pytest.mark.parametrize("gdt", [0, 1, 2])
 @pytest.mark.parametrize("opt,pdt,ecc_bits,group,conv,more", [
     (C.ADAM, 1, 16, 32, O.FUSED, {}), (C.ADAM, 2, 8, 256, O.FUSED, {}), (C.ADAM, 1, 8, 32, O.UNFUSED, {}), (C.ADAM, 0, 0, 16, O.FUSED, {}),
@@ -66,16 +78,17 @@ def test_leaves_that_end_around_a_tile(opt, pdt, ecc_bits, group, conv, more, gd
 @pytest.mark.parametrize("opt,pdt,ecc_bits,gdt", [(C.ADAM, 1, 16, 1), (C.ADAM, 2, 8, 0), (C.ADAM, 0, 0, 0), (C.SGD, 1, 8, 1), (C.SGD, 2, 0, 1)])
 def test_decay_added_to_the_gradient(opt, pdt, ecc_bits, gdt, more):
     """A weight decay that is added to the gradient beside every feature, by tile_kernel as without it."""
-    import torch
-
     more = dict(dict(group=32, conv=O.FUSED), **more)
     group, conv = more.pop("group"), more.pop("conv")
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        _check(opt, pdt, ecc_bits, group, conv, gdt, (MANY + 700,) + SIZES, decoupled=False, **more)
-    kernels = {e.key for e in prof.key_averages()}
-    if not any("kernel" in k for k in kernels):
-        pytest.skip("the profiler records no kernels here")
+    kernels = _kernels_of(lambda: _check(opt, pdt, ecc_bits, group, conv, gdt, (MANY + 700,) + SIZES, decoupled=False, **more))
     assert any("tile_kernel" in k for k in kernels) and not any("step_kernel" in k for k in kernels), kernels
+
+
+@pytest.mark.parametrize("opt,pdt,ecc_bits", [(C.ADAM, 1, 16), (C.LION, 2, 8), (C.SGD, 0, 0)])
+def test_groups_of_8_have_a_kernel_of_their_own(opt, pdt, ecc_bits):
+    kernels = _kernels_of(lambda: _check(opt, pdt, ecc_bits, 8, O.FUSED, 1, (MANY + 6143 * 3, 8 * 6144, 7)))
+    main = {k for k in kernels if "step_kernel" in k or "tile_kernel" in k}
+    assert len(main) == 1 and f"step_kernel<{opt}, {pdt}, {ecc_bits}, 0, 4>" in main.pop(), kernels
 
 
 @pytest.mark.parametrize("offset,scale_offset", [(8, 1), (16, 2), (8, 2), (24, 3)])
