@@ -36,19 +36,19 @@ _OPTS = (("adam", "FO_OPT_ADAM"), ("lion", "FO_OPT_LION"), ("sgd", "FO_OPT_SGD")
 _KINDS = (("quant", 0), ("full", 1), ("generic", 3))
 
 
-# Block shape of a slice that runs step_kernel: (threads per block, resident blocks per SM).  Measured on B200: the
+# Block shape of a slice: (threads per block, resident blocks per SM).  Measured on B200: the
 # Adam kernels run best as one 512-thread block per SM (all warps of an SM share one instruction
 # stream and one set of tables); the kernels that also read peers' gradients keep 256-thread blocks,
 # whose smaller stages leave room for a deeper copy pipeline.
-_SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1),
-           ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1), ("adam", "group8"): (512, 1),
-           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1), ("lion", "group8"): (512, 1),
-           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "all"): (512, 1), ("sgd", "group8"): (512, 1)}
-# Threads of the one block per SM that runs tile_kernel (quantized moments, one feature at most).  The 16 elements of a lane want 150 to
+# "tile": the slices that run tile_kernel (quantized moments, one feature at most), one block per SM.  The 16 elements of a lane want 150 to
 # 168 registers under AdamW (2^28 elements, 24-bit masters: 588 us with 384 threads, 623 with 512; with the power cap reached
 # 672 and 704) and 138 under SGD (65 M elements, 32-bit masters, results elsewhere: 129 us with 384 threads, 143 with 512, 132 with 256);
 # Lion fits 512 (fp16, 2^28 elements: 435 us, 455 with 384).
-_TILE_THREADS = {"adam": 384, "lion": 512, "sgd": 384}
+_SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1),
+           ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1), ("adam", "group8"): (512, 1), ("adam", "tile"): (384, 1),
+           ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1), ("lion", "group8"): (512, 1),
+           ("lion", "tile"): (512, 1),
+           ("sgd", "clip"): (512, 1), ("sgd", "out"): (512, 1), ("sgd", "all"): (512, 1), ("sgd", "group8"): (512, 1), ("sgd", "tile"): (384, 1)}
 _TILE_MODES = ("plain", "clip", "out", "group", "delta")
 # Name and feature mask (fo_step.cuh) of the kernels of a slice.  Groups of 8, two to a tile's lane, go through step_kernel (one of their own: AdamW
 # 4096 x 4096 49 us, through the kernel that carries all features 59; Lion 32.9 and 34.8, SGDW 31.9 and 33.3).
@@ -73,7 +73,7 @@ def _units(shapes=None, ffi_dir: str | None = None) -> List[Tuple[str, str, List
         tiles = kind == 0 and mname in _TILE_MODES
         if tiles:
             flags.append("-DFO_INST_TILES")
-        shape = (_TILE_THREADS[oname], 1) if tiles else shapes.get((oname, mname))
+        shape = shapes.get((oname, "tile" if tiles else mname))
         if shape is not None and kind != 3:
             flags += [f"-DFO_THREADS={shape[0]}", f"-DFO_MIN_BLOCKS_ADAM={shape[1]}", f"-DFO_MIN_BLOCKS_MOMENTUM={shape[1]}"]
             if len(shape) > 2:
@@ -130,7 +130,7 @@ def _sources_digest(extra: List[str], units=None) -> str:
 def build_native(force: bool = False, jobs: int | None = None, extra_flags: List[str] | None = None,
                  lib_path: str = LIB_PATH, verbose: bool = False, shapes=None) -> str:
     """Compile every CUDA source for sm_100a and link the shared object; returns its path.
-    `shapes` overrides the block shapes of the step slices ({(optimizer, kernel): (threads, blocks per SM)})."""
+    `shapes` takes the place of _SHAPES, the block shapes of the step slices; where it names none the default of fo_step.cuh holds."""
     extra = list(extra_flags or [])
     units = _units(shapes, ffi_include_dir())
     os.makedirs(OBJ_DIR, exist_ok=True)
