@@ -47,7 +47,7 @@ static Launcher find_launcher(int opt, int pdt, int ecc_bits, int state, bool ge
     if (state == FO_STATE_NONE) { FO_PICK(lookup_sgd_none) }
   }
 #undef FO_PICK
-  return Launcher{nullptr, 0u, 0};
+  return Launcher{nullptr, 0u, 0, false};
 }
 static PieceFn find_pieces(int opt, int pdt, int ecc_bits, int state) {
   if (opt == FO_OPT_ADAM) return state == FO_STATE_QUANT ? lookup_adam_quant_piece(pdt, ecc_bits) : lookup_adam_full_piece(pdt, ecc_bits);
@@ -231,7 +231,7 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
       e = launcher.launch(hs, chained, stream);
     } else {
       // with peers the whole chunks always take the kernel that knows them (the pieces' path is scalar there)
-      const unsigned long long small = launcher.chunk == 1u ? kSmallElemsTiles : FO_SMALL_ELEMS;
+      const unsigned long long small = launcher.tiles ? kSmallElemsTiles : FO_SMALL_ELEMS;
       const unsigned int main_chunk = (with_peers ? whole > 0 : whole > small) ? launcher.chunk : 0u;
       if (main_chunk != 0) e = launcher.launch(hs, chained, stream);
       if (e == cudaSuccess) e = pieces(hs, main_chunk, chained, stream);

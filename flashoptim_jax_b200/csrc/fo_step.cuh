@@ -2170,12 +2170,13 @@ struct HostStep {
 // or the kernel begins with chain_wait(); set to true by a launch.
 using MainFn = cudaError_t (*)(HostStep&, bool& chained, cudaStream_t);
 using PieceFn = cudaError_t (*)(HostStep&, unsigned int main_chunk, bool& chained, cudaStream_t);
-// A slice of step_kernel or tile_kernel, the elements one of its chunks covers (1: it takes the leaves whole) and the leaves its table holds
-// (of a call without separate outputs).  Block size, and with it the chunk, is a property of the slice (the slices are compiled with their own FO_THREADS).
+// A slice of step_kernel or tile_kernel, the elements one of its chunks covers (1: it takes the leaves whole), the leaves its table holds
+// (of a call without separate outputs) and whether it is tile_kernel's.  Block size, and with it the chunk, is a property of the slice (the slices are compiled with their own FO_THREADS).
 struct Launcher {
   MainFn launch;
   unsigned int chunk;
   int most_leaves;
+  bool tiles;
 };
 
 template <typename... P>

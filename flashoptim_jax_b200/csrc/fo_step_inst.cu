@@ -28,22 +28,22 @@ Launcher FO_INST_NAME(int pdt, int ecc_bits, int gdt) {
   (void)gdt;
 #if FO_INST_KIND == 3
 #define X(P, E) \
-  if (pdt == P && ecc_bits == E) return Launcher{&launch_generic<FO_INST_OPT, P, E>, 0u, kMaxLeaves};
+  if (pdt == P && ecc_bits == E) return Launcher{&launch_generic<FO_INST_OPT, P, E>, 0u, kMaxLeaves, false};
 #elif defined(FO_INST_TILES)
   // gradients of the parameter's dtype or fp32, which is what steps have, by kernels of their own
 #define X(P, E)                                                                                                       \
   if (pdt == P && ecc_bits == E) {                                                                                    \
-    if (gdt == P) return Launcher{&launch_tiles<FO_INST_OPT, P, E, P, FO_INST_MODE>, 1u, most_leaves};                \
-    if (gdt == FO_F32) return Launcher{&launch_tiles<FO_INST_OPT, P, E, FO_F32, FO_INST_MODE>, 1u, most_leaves};      \
-    return Launcher{&launch_tiles<FO_INST_OPT, P, E, kAnyGrad, FO_INST_MODE>, 1u, most_leaves};                       \
+    if (gdt == P) return Launcher{&launch_tiles<FO_INST_OPT, P, E, P, FO_INST_MODE>, 1u, most_leaves, true};              \
+    if (gdt == FO_F32) return Launcher{&launch_tiles<FO_INST_OPT, P, E, FO_F32, FO_INST_MODE>, 1u, most_leaves, true};    \
+    return Launcher{&launch_tiles<FO_INST_OPT, P, E, kAnyGrad, FO_INST_MODE>, 1u, most_leaves, true};                     \
   }
 #else
 #define X(P, E) \
-  if (pdt == P && ecc_bits == E) return Launcher{&launch_main<FO_INST_OPT, P, E, FO_INST_KIND, FO_INST_MODE>, (unsigned int)kChunk, most_leaves};
+  if (pdt == P && ecc_bits == E) return Launcher{&launch_main<FO_INST_OPT, P, E, FO_INST_KIND, FO_INST_MODE>, (unsigned int)kChunk, most_leaves, false};
 #endif
   FO_COMBOS(X)
 #undef X
-  return Launcher{nullptr, 0u, 0};
+  return Launcher{nullptr, 0u, 0, false};
 }
 #endif
 
