@@ -258,7 +258,7 @@ def test_every_block_shape_covers_whole_pieces():
 def test_block_shapes_handed_to_the_build_reach_every_slice():
     from flashoptim_jax_b200 import build
 
-    shapes = dict(build._SHAPES, **{("adam", "tile"): (256, 1), ("lion", "group8"): (256, 2)})
+    shapes = {**build._SHAPES, ("adam", "tile"): (256, 1), ("lion", "group8"): (256, 2)}
     flags = {name: defs for name, _, defs in build._units(shapes)}
     assert "-DFO_THREADS=256" in flags["fo_step_adam_quant_plain"] and "-DFO_THREADS=256" in flags["fo_step_lion_quant_group8"]
     assert flags["fo_step_sgd_quant_plain"] == {name: defs for name, _, defs in build._units()}["fo_step_sgd_quant_plain"]
