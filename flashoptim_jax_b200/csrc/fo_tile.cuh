@@ -61,6 +61,7 @@ template <int U>
 struct Units {
   static FO_DEVI uint32_t copy_to(uint32_t lane) { return (lane ^ ((lane >> 3) & (U - 1))) * 16u; }
   static FO_DEVI uint32_t read_at(uint32_t lane) { return (lane * U + (((lane * U) >> 3) & (U - 1))) * 16u; }  // unit j: ^ (j * 16)
+  static FO_DEVI uint32_t unit_at(uint32_t u) { return (u ^ ((u >> 3) & (U - 1))) * 16u; }
 };
 template <int U>
 FO_DEVI void copy_units(const uint32_t at, const char* src) {
@@ -109,38 +110,6 @@ FO_DEVI float2 table_pair(const char* table, const uint32_t w, const int b, cons
                      *reinterpret_cast<const float*>(table + __byte_perm(w, lane4, 0x5504u | (uint32_t)((b + 1) << 4))));
 }
 
-// A tile that holds a value outside the shortcuts' ranges: again from memory, in the two halves of 256 elements (sixteen lanes' worth) that
-// zero_chunk and warm_chunk take.  `rest`: bit k for a half k in which no new first moment differs from zero.  (Storing a half
-// that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28 elements.)
-template <int OPT, int PDT, int ECC_BITS, int MODE>
-__device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, uint32_t rest,
-                                       const uint32_t flags, const float wd, const float decay) {
-  if (rest != 0u && !rest_is_decay<OPT>(load_hyper<OPT>(dh))) rest = 0u;  // (asked here: in the loop it costs AdamW's kernels up to 5 %)
-#pragma unroll 1
-  for (uint32_t half = 0; half < 2u; ++half) {
-    const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
-    if constexpr ((MODE & ~(kClip | kGroup | kCoupled)) == 0) {
-      if ((rest >> half) & 1u) {
-        const Piece at = piece_at<PDT, ECC_BITS, FO_STATE_QUANT>(L, c.grad_dtype, (MODE & kGroup) != 0 ? c.group_shift : 5, i0);
-        if (zero_chunk<OPT, PDT, ECC_BITS>(flags, wd, decay, c.grad_dtype, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) continue;
-      }
-    }
-    warm_chunk<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE & ~kCoupled>(c, L, out, dh, i0, nullptr);
-  }
-}
-
-// 256 elements from i0 - 8 * lane on of a leaf's ragged end: the code of piece_kernel.
-template <int OPT, int PDT, int ECC_BITS, bool OUT>
-__device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t i0) {
-  const Hyp h = load_hyper<OPT>(dh);
-  if (OPT != FO_OPT_ADAM || (h.flags & kFlagTameAdam) != 0) {
-    const Clip clip = load_clip(c.sq_norm, c.max_norm, c.grad_dtype);
-    ragged_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT, OUT>(c, L, out, dh, h, clip, i0, (uint32_t)L.n);
-  } else {
-    cold_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT>(L, out, dh, c.grad_dtype, c.group_shift, i0, nullptr, c.sq_norm, c.max_norm);
-  }
-}
-
 // Where a lane's copies of a tile come from, and the copies.
 template <int OPT, int PDT, int ECC_BITS, int GDT>
 struct TileSource {
@@ -157,6 +126,9 @@ struct TileSource {
   // 750 us per 2^28 elements, as the compiler happened to assign it.)  Arrays that begin in the middle of a word still do that.
   const char* sc;
   bool sc_words, sc_mine;
+  static FO_DEVI bool in_words(const DevLeaf& L) {
+    return ((reinterpret_cast<uintptr_t>(L.mu_scales) | (kAdam ? reinterpret_cast<uintptr_t>(L.nu_scales) : 0)) & 3u) == 0;
+  }
   FO_DEVI TileSource(const DevLeaf& L, const uint32_t t, const int gsz, const int gshift, const uint32_t lane) {
     const size_t e0 = (size_t)t * kTileElems;
     grad = (const char*)L.grad + e0 * (size_t)gsz + lane * 16u;
@@ -165,7 +137,7 @@ struct TileSource {
     mu = (char*)L.mu + e0 + lane * 16u;
     nu = (char*)L.nu + e0 + lane * 16u;
     sc = (const char*)(kAdam && lane >= 16u ? L.nu_scales : L.mu_scales) + (e0 >> gshift) * 2u + (lane & 15u) * 4u;
-    sc_words = ((reinterpret_cast<uintptr_t>(L.mu_scales) | (kAdam ? reinterpret_cast<uintptr_t>(L.nu_scales) : 0)) & 3u) == 0;
+    sc_words = in_words(L);
     sc_mine = sc_words && (lane & 15u) < (256u >> gshift) && (kAdam || lane < 16u);
   }
   // the lane's units of the tile `ahead` steps on
@@ -180,6 +152,79 @@ struct TileSource {
     if (sc_mine) copy_async4(slot + S::kScales + lane * 4u, sc + ahead * ((kStep >> gshift) * 2));
   }
 };
+
+// What a lane owns of a tile's half in pieces of eight elements, from the warp's slot (the group scales of a leaf whose scales do not travel in words from
+// memory).
+template <int OPT, int PDT, int ECC_BITS, int GDT>
+FO_DEVI void slot_read(const DevLeaf& L, const uint32_t slot, const uint32_t half, const int gdt, const int gshift, const uint32_t i0, const bool sc_words,
+                       Raw<OPT, PDT, ECC_BITS, FO_STATE_QUANT>& r) {
+  using S = TileSlot<OPT, PDT, ECC_BITS, GDT>;
+  const uint32_t piece = half * 32u + (threadIdx.x & 31u);
+  if constexpr (PDT == FO_F32) {
+    r.p0 = lds128(slot + Units<4>::unit_at(2u * piece));
+    r.p1 = lds128(slot + Units<4>::unit_at(2u * piece + 1u));
+  } else {
+    r.p0 = lds128(slot + Units<2>::unit_at(piece));
+  }
+  if constexpr (ECC_BITS == 16) r.e = lds128(slot + S::kEcc + Units<2>::unit_at(piece));
+  if constexpr (ECC_BITS == 8) {
+    const uint2 e = lds64(slot + S::kEcc + piece * 8u);
+    r.e.x = e.x; r.e.y = e.y;
+  }
+  r.mq = lds64(slot + S::kMu + piece * 8u);
+  if constexpr (OPT == FO_OPT_ADAM) r.vq = lds64(slot + S::kNu + piece * 8u);
+  if (sc_words) {
+    const uint32_t at = slot + S::kScales + ((piece * 8u >> gshift) << 1);
+    r.msc = __float2half(lds_half(at));
+    if constexpr (OPT == FO_OPT_ADAM) r.vsc = __float2half(lds_half(at + 64u));
+  } else {
+    r.msc = ((const __half*)L.mu_scales)[i0 >> gshift];
+    if constexpr (OPT == FO_OPT_ADAM) r.vsc = ((const __half*)L.nu_scales)[i0 >> gshift];
+  }
+  if (gdt == FO_F32) {
+    r.g0 = lds128(slot + S::kGrad + Units<4>::unit_at(2u * piece));
+    r.g1 = lds128(slot + S::kGrad + Units<4>::unit_at(2u * piece + 1u));
+  } else {
+    r.g0 = lds128(slot + S::kGrad + Units<2>::unit_at(piece));
+  }
+}
+
+// A tile that holds a value outside the shortcuts' ranges, whose slot still holds what it was loaded from: once more, in the two halves of 256
+// elements (sixteen lanes' worth) that zero_chunk and the repairing pass take.  `rest`: bit k for a half k in which no new first moment differs from
+// zero.  (Storing a half that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28 elements;
+// under SGD and Lion it made such tiles themselves slower, 8192 x 8192 with 0.1 % zeros under SGD 233 -> 262.)
+template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE>
+__device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, const uint32_t slot, uint32_t rest,
+                                       const uint32_t flags, const float wd, const float decay) {
+  if (rest != 0u && !rest_is_decay<OPT>(load_hyper<OPT>(dh))) rest = 0u;  // (asked here: in the loop it costs AdamW's kernels up to 5 %)
+  const int gdt = GDT == kAnyGrad ? c.grad_dtype : GDT, gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;
+  const bool sc_words = TileSource<OPT, PDT, ECC_BITS, GDT>::in_words(L);
+#pragma unroll 1
+  for (uint32_t half = 0; half < 2u; ++half) {
+    const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
+    if constexpr ((MODE & ~(kClip | kGroup | kCoupled)) == 0) {
+      if ((rest >> half) & 1u) {
+        const Piece at = piece_at<PDT, ECC_BITS, FO_STATE_QUANT>(L, gdt, gshift, i0);
+        if (zero_chunk<OPT, PDT, ECC_BITS>(flags, wd, decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) continue;
+      }
+    }
+    Raw<OPT, PDT, ECC_BITS, FO_STATE_QUANT> raw;
+    slot_read<OPT, PDT, ECC_BITS, GDT>(L, slot, half, gdt, gshift, i0, sc_words, raw);
+    warm_finish<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE & ~kCoupled>(c, L, out, dh, i0, nullptr, raw);
+  }
+}
+
+// 256 elements from i0 - 8 * lane on of a leaf's ragged end: the code of piece_kernel.
+template <int OPT, int PDT, int ECC_BITS, bool OUT>
+__device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t i0) {
+  const Hyp h = load_hyper<OPT>(dh);
+  if (OPT != FO_OPT_ADAM || (h.flags & kFlagTameAdam) != 0) {
+    const Clip clip = load_clip(c.sq_norm, c.max_norm, c.grad_dtype);
+    ragged_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT, OUT>(c, L, out, dh, h, clip, i0, (uint32_t)L.n);
+  } else {
+    cold_piece<OPT, PDT, ECC_BITS, FO_STATE_QUANT>(L, out, dh, c.grad_dtype, c.group_shift, i0, nullptr, c.sq_norm, c.max_norm);
+  }
+}
 
 // One warp's tiles t, t + kWarps, ... below t1 of a leaf.  `primed`: the first one's copies are under way, in the first slot.
 template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE, typename OUT>
@@ -304,7 +349,7 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
         const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
         still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
       }
-      redo_tile<OPT, PDT, ECC_BITS, MODE>(c, L, out, dh, t * (uint32_t)kTileElems, still, h.flags, h.wd, h.decay);
+      redo_tile<OPT, PDT, ECC_BITS, GDT, MODE>(c, L, out, dh, t * (uint32_t)kTileElems, slot, still, h.flags, h.wd, h.decay);
     } else {
       // ---- stores: parameter and ECC, scales, codes -------------------------------------------------------------
       auto to = [&](char* base, long long DevOut::*d) {

@@ -206,3 +206,31 @@ def test_rows_at_rest_under_learning_rates_that_change_them(opt, lr, n):
     H.oracle_step(opt, g, ref, C.STATE_QUANT, 32, hp)
     _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, 32, hp, 0, 0, 0)
     H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, 32, np.empty(0, dtype=np.int64)), ref, f"n={n} lr={lr}")
+
+
+@pytest.mark.parametrize("n", [3000, MANY + 700])
+@pytest.mark.parametrize("opt,pdt,ecc_bits,group,conv", [
+    (C.ADAM, 1, 16, 32, O.FUSED), (C.ADAM, 1, 8, 128, O.FUSED), (C.ADAM, 2, 8, 32, O.UNFUSED), (C.ADAM, 0, 0, 16, O.FUSED), (C.LION, 1, 8, 32, O.FUSED),
+    (C.LION, 2, 16, 256, O.UNFUSED), (C.SGD, 1, 16, 32, O.FUSED), (C.SGD, 2, 8, 64, O.FUSED)])
+def test_scattered_odd_values(opt, pdt, ecc_bits, group, conv, n):
+    """Single elements outside the shortcuts' ranges among ordinary ones, which the repairs leave alone: parameters of zero, next to it and near
+    the largest, elements that never see a gradient, gradients whose square overflows."""
+    rng = np.random.default_rng(n + opt + group)
+    pick = lambda: rng.integers(0, n, 1 + n // 300)  # noqa: E731
+    p = rng.normal(0, 0.02, n).astype(np.float32)
+    for value in (0.0, -0.0, 1e-38, -3e-31, 6e4, -6e4):
+        p[pick()] = value
+    if pdt != 2:
+        p[pick()] = 2e38
+    never, huge = pick(), pick()
+    ref = H.fresh_leaf(p.astype(H.NP_OF_CODE[pdt]), opt, C.STATE_QUANT, ecc_bits, group)
+    dev = ref.copy().to_device()
+    for t in (1, 2):
+        g = H.make_grad(rng, n, 1e-2, np.float32)
+        if t == 2:  # (the fp16 scales of their groups are infinite then)
+            g[huge] = 1e20
+        g[never] = 0
+        hp = H.hyper_tuple(opt, conv, t, lr=1e-3, wd=1e-2)
+        H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+        _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 0, ecc_bits)
+        H.assert_leaf_equal(dev.to_host(), ref, f"step {t}")
