@@ -258,11 +258,13 @@ FO_DEVI Hyp load_hyper(const DevHyper& d) {
 }
 
 // Whether a step without gradients on moments of zero is the weight decay alone.  Its update term is the learning rate times +0 then: a NaN under
-// an infinite one, and -0, which turns a parameter of -0 into +0, under a learning rate or momentum with a sign.
+// an infinite one, and -0, which turns a parameter of -0 into +0, under a learning rate or momentum with a sign.  (Nor do factors of the
+// moments that are not finite leave them zero.)
 template <int OPT>
 FO_DEVI bool rest_is_decay(const Hyp& h) {
   const float lr = OPT == FO_OPT_ADAM ? h.lr_bc1 : h.lr;
-  return __float_as_int(lr) >= 0 && lr <= 1.0e30f && __float_as_int(h.b1) >= 0;
+  return __float_as_int(lr) >= 0 && lr <= 1.0e30f && __float_as_int(h.b1) >= 0 && h.b1 <= 1.0e30f && fabsf(h.b2) <= 1.0e30f && fabsf(h.omb1) <= 1.0e30f &&
+         fabsf(h.omb2) <= 1.0e30f;
 }
 
 FO_DEVI float sign_of(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : x); }
@@ -1442,10 +1444,6 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
   (void)rare;
   if constexpr (!REPAIR) {
     if (__any_sync(0xFFFFFFFFu, rare)) {
-      if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && (MODE & ~(kClip | kGroup)) == 0) {
-        // no new first moment of the warp differs from zero: look whether the whole piece is at rest
-        if (__all_sync(0xFFFFFFFFu, am_lane == 0.0f) && rest_is_decay<OPT>(h) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
-      }
       warm_chunk<OPT, PDT, ECC_BITS, STATE, MODE>(c, L, out, dh, i0, peers);
       return;
     }
@@ -1546,6 +1544,18 @@ FO_DEVI void hot_finish(const StepCommon& c, const DevLeaf& L, const DevOut* out
   }
 }
 
+// Takes a warp whose elements are at rest through zero_chunk; false where they are not (all lanes answer alike).
+template <int OPT, int PDT, int ECC_BITS>
+FO_DEVI bool step_at_rest(const Hyp& h, const int gdt, const Raw<OPT, PDT, ECC_BITS, FO_STATE_QUANT>& raw, const Unpacked& u, const Piece& at, const bool may) {
+  uint32_t codes = raw.mq.x | raw.mq.y;
+  if constexpr (OPT == FO_OPT_ADAM) codes |= raw.vq.x | raw.vq.y;
+  if (!__all_sync(0xFFFFFFFFu, may && codes == 0u)) return false;
+  bool rest = maxabs8(u.g) == 0.0f && maxabs8(u.m) == 0.0f;  // (no infinite scale, nothing that clipping made a NaN)
+  if constexpr (OPT == FO_OPT_ADAM) rest = rest && maxabs8(u.v) == 0.0f;
+  if (!__all_sync(0xFFFFFFFFu, rest) || !rest_is_decay<OPT>(h)) return false;
+  return zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc);
+}
+
 // Words of eight consecutive elements of which those behind number `last` (which may be negative) do not exist: their
 // places take the value of element `last`.
 template <int BYTES>
@@ -1625,12 +1635,8 @@ FO_DEVI void ragged_piece(const StepCommon& c, const DevLeaf& L, const DevOut* o
   hot_unpack<true, OPT, PDT, ECC_BITS, STATE>(raw, gdt, LutGlobal{}, u);
   if (clip.active) clip_grads<true>(u.g, gdt, clip);
   if constexpr (OPT == FO_OPT_ADAM && STATE == FO_STATE_QUANT && !OUT) {
-    // a whole warp at rest, as in step_kernel (one million elements at rest: 23.0 us with every element repaired, 5.8 so)
-    const bool codes_zero = n_valid == kPiece && (raw.mq.x | raw.mq.y | raw.vq.x | raw.vq.y) == 0u;
-    if (__all_sync(0xFFFFFFFFu, codes_zero && (h.flags & FO_FLAG_LP_DELTA) == 0) && rest_is_decay<OPT>(h)) {
-      const bool rest = maxabs8(u.g) == 0.0f && maxabs8(u.m) == 0.0f && maxabs8(u.v) == 0.0f;
-      if (__all_sync(0xFFFFFFFFu, rest) && zero_chunk<OPT, PDT, ECC_BITS>(h.flags, h.wd, h.decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) return;
-    }
+    // (one million elements at rest: 23.0 us with every element repaired, 5.8 so)
+    if (step_at_rest<OPT, PDT, ECC_BITS>(h, gdt, raw, u, at, n_valid == kPiece && (h.flags & FO_FLAG_LP_DELTA) == 0)) return;
   }
   constexpr int kMode = OUT ? kAll : kAll & ~kOut;
   hot_finish<true, OPT, PDT, ECC_BITS, STATE, kMode, true>(c, L, out, dh, h, gdt, i0, at, false, u, OutAt{out},
@@ -1666,6 +1672,9 @@ FO_DEVI void warm_finish(const StepCommon& c, const DevLeaf& L, const DevOut* ou
     if (clip.active) clip_grads<true>(u.g, gdt, clip);
   }
   const Piece at = piece_at<PDT, ECC_BITS, STATE>(L, gdt, gshift, i0);
+  if constexpr (STATE == FO_STATE_QUANT && (MODE & ~(kClip | kGroup)) == 0) {
+    if (step_at_rest<OPT, PDT, ECC_BITS>(h, gdt, raw, u, at, true)) return;
+  }
   hot_finish<true, OPT, PDT, ECC_BITS, STATE, MODE>(c, L, out, dh, h, gdt, i0, at, false, u, OutAt{out},
                                                     [&](uint4& w0, uint4& w1) { w0 = raw.p0; w1 = raw.p1; }, peers);
 }

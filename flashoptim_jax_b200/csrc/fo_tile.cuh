@@ -189,29 +189,17 @@ FO_DEVI void slot_read(const DevLeaf& L, const uint32_t slot, const uint32_t hal
   }
 }
 
-// A tile that holds a value outside the shortcuts' ranges, whose slot still holds what it was loaded from: once more, in the two halves of 256
-// elements (sixteen lanes' worth) that zero_chunk and the repairing pass take.  `rest`: bit k for a half k in which no new first moment differs from
-// zero.  (Storing a half that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28 elements;
-// under SGD and Lion it made such tiles themselves slower, 8192 x 8192 with 0.1 % zeros under SGD 233 -> 262.)
+// Half of a tile that holds a value outside the shortcuts' ranges, 256 elements (sixteen lanes' worth): once more, by the repairing pass, from the warp's slot,
+// which still holds it.  It works out for itself what only it needs, rows at rest among it: asked in the loop that cost ordinary tiles
+// up to 5 %.  (Storing a half that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28
+// elements; under SGD and Lion it made such tiles themselves slower, 8192 x 8192 with 0.1 % zeros under SGD 233 -> 262.)
 template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE>
-__device__ __noinline__ void redo_tile(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, const uint32_t slot, uint32_t rest,
-                                       const uint32_t flags, const float wd, const float decay) {
-  if (rest != 0u && !rest_is_decay<OPT>(load_hyper<OPT>(dh))) rest = 0u;  // (asked here: in the loop it costs AdamW's kernels up to 5 %)
+__device__ __noinline__ void redo_half(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t e0, const uint32_t slot, const uint32_t half) {
   const int gdt = GDT == kAnyGrad ? c.grad_dtype : GDT, gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;
-  const bool sc_words = TileSource<OPT, PDT, ECC_BITS, GDT>::in_words(L);
-#pragma unroll 1
-  for (uint32_t half = 0; half < 2u; ++half) {
-    const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
-    if constexpr ((MODE & ~(kClip | kGroup | kCoupled)) == 0) {
-      if ((rest >> half) & 1u) {
-        const Piece at = piece_at<PDT, ECC_BITS, FO_STATE_QUANT>(L, gdt, gshift, i0);
-        if (zero_chunk<OPT, PDT, ECC_BITS>(flags, wd, decay, gdt, at.grad, at.param, at.ecc, at.mu, at.nu, at.msc, at.vsc)) continue;
-      }
-    }
-    Raw<OPT, PDT, ECC_BITS, FO_STATE_QUANT> raw;
-    slot_read<OPT, PDT, ECC_BITS, GDT>(L, slot, half, gdt, gshift, i0, sc_words, raw);
-    warm_finish<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE & ~kCoupled>(c, L, out, dh, i0, nullptr, raw);
-  }
+  const uint32_t i0 = e0 + half * 256u + (threadIdx.x & 31u) * 8u;
+  Raw<OPT, PDT, ECC_BITS, FO_STATE_QUANT> raw;
+  slot_read<OPT, PDT, ECC_BITS, GDT>(L, slot, half, gdt, gshift, i0, TileSource<OPT, PDT, ECC_BITS, GDT>::in_words(L), raw);
+  warm_finish<OPT, PDT, ECC_BITS, FO_STATE_QUANT, MODE & ~kCoupled>(c, L, out, dh, i0, nullptr, raw);
 }
 
 // 256 elements from i0 - 8 * lane on of a leaf's ragged end: the code of piece_kernel.
@@ -331,7 +319,6 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
       for (int j = 0; j < 4; ++j) { m[k][j] = u.m[j]; theta[k][j] = u.theta[j]; }
     }
     // ---- group maxima, and one decision per warp ------------------------------------------------------------
-    const bool rest = am == 0.0f;
     if constexpr ((MODE & kGroup) != 0) {
       for (int o = 1; o < (1 << (gshift - 4)); o <<= 1) {
         am = max2<true>(am, __shfl_xor_sync(0xFFFFFFFFu, am, o));
@@ -344,12 +331,10 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
     rare = rare || !(am >= 1.0e-12f && am <= 1.0e30f);                           // an all-zero group, or beyond the reciprocal's range
     if constexpr (kAdam) rare = rare || !(av >= 1.0e-12f && av <= 1.0737418e9f);  // 2^30: also the limit of the packed division
     if (__any_sync(0xFFFFFFFFu, rare)) {
-      uint32_t still = 0u;
-      if constexpr ((MODE & ~(kClip | kGroup | kCoupled)) == 0) {
-        const uint32_t zero = __ballot_sync(0xFFFFFFFFu, rest);
-        still = ((zero & 0xFFFFu) == 0xFFFFu ? 1u : 0u) | (zero >> 16 == 0xFFFFu ? 2u : 0u);
-      }
-      redo_tile<OPT, PDT, ECC_BITS, GDT, MODE>(c, L, out, dh, t * (uint32_t)kTileElems, slot, still, h.flags, h.wd, h.decay);
+      // (A loop under Adam, two calls under Lion and SGD: which of them leaves the loop around it fewer instructions differs, AdamW 9 M elements in
+      // the L2 22.2 and 24.6 us, Lion 17.4 and 17.0, SGDW 15.1 and 14.9; through one call for both halves 24.1, 17.5 and 14.9.)
+#pragma unroll (kAdam ? 1 : 2)
+      for (uint32_t half = 0; half < 2u; ++half) redo_half<OPT, PDT, ECC_BITS, GDT, MODE>(c, L, out, dh, t * (uint32_t)kTileElems, slot, half);
     } else {
       // ---- stores: parameter and ECC, scales, codes -------------------------------------------------------------
       auto to = [&](char* base, long long DevOut::*d) {
