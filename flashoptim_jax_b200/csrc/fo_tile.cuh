@@ -528,6 +528,14 @@ cudaError_t launch_tiles(HostStep& hs, bool& chained, cudaStream_t s) {
   const unsigned int share = (total + grid - 1u) / grid;
   unsigned int run = share;
   if (share > 256u) run = (total + grid * 4u - 1u) / (grid * 4u);
+  else if (share <= 64u && ends <= 4u && total >= (unsigned int)kWarps) {
+    // A ragged end is cold code for one warp and lasts about as long as one and a half tiles of each warp.  A few ends get blocks with that much less to do:
+    // the others take a tile more where the last ones would be full.  (AdamW, 24-bit masters, 909412, 1137000, 1212000 elements 10.4, 9.4, 10.2 us
+    // with full last blocks, 7.2, 7.2, 7.7 so; Lion 1137000 5.8 and 5.3, SGDW 6.6 and 5.4.)
+    const unsigned int room = share > 5u * kWarps / 2u ? share - 3u * kWarps / 2u : (unsigned int)kWarps - 1u;
+    const unsigned int spare = (total - room + grid - ends - 1u) / (grid - ends);
+    if (spare > run) run = spare;
+  }
   p.run_chunks = run < 1u ? 1u : (run > 1536u ? 1536u : run);
   return launched(hs, launch_chained(kernel, grid, kThreads, smem, chained, s, p));
 }
