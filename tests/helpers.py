@@ -13,8 +13,8 @@ from oracle.driver import (BF16, NP_OF_CODE, LeafArrays, assert_leaf_equal, bits
 
 def abi_step(opt: int, grads: List, leaves: List[LeafArrays], state: int, group_size: int, hypers: List, hyper_of: List[int],
              param_dtype: int, grad_dtype: int, ecc_bits: int, stream: int = 0, expect_ok: bool = True,
-             peer_param_offsets=None, peer_grad_offsets=None, grad_sq_norm=None, max_grad_norm: float = 0.0) -> int:
-    """One fo_step call through the C ABI on torch device tensors (in place)."""
+             peer_param_offsets=None, peer_grad_offsets=None, grad_sq_norm=None, max_grad_norm: float = 0.0, outs=None) -> int:
+    """One fo_step call through the C ABI on torch device tensors (in place, or to the leaves `outs`)."""
     from flashoptim_jax_b200 import _lib
 
     L = (_lib.FoLeaf * len(leaves))()
@@ -44,7 +44,15 @@ def abi_step(opt: int, grads: List, leaves: List[LeafArrays], state: int, group_
             keep.append(arr)
             setattr(d, name, ctypes.cast(arr, ctypes.c_void_p))
             d.n_peers = len(offs)
-    rc = _lib.lib().fo_step(ctypes.byref(d), stream)
+    more = None
+    if outs is not None:
+        X = (_lib.FoLeafOut * len(outs))()
+        for i, lf in enumerate(outs):
+            for name in lf.fields():
+                t = getattr(lf, name)
+                setattr(X[i], name, None if t is None else t.data_ptr())
+        more = ctypes.byref(_lib.FoStepMore(struct_size=ctypes.sizeof(_lib.FoStepMore), outs=ctypes.cast(X, ctypes.c_void_p)))
+    rc = _lib.lib().fo_step_ex(ctypes.byref(d), more, stream)
     if expect_ok:
         _lib.check(rc)
     return rc

@@ -234,3 +234,36 @@ def test_scattered_odd_values(opt, pdt, ecc_bits, group, conv, n):
         H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
         _step(opt, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 0, ecc_bits)
         H.assert_leaf_equal(dev.to_host(), ref, f"step {t}")
+
+
+@pytest.mark.parametrize("first", ["outside", "inside"])
+@pytest.mark.parametrize("pdt,ecc_bits,group,max_norm,elsewhere", [(1, 16, 32, None, False), (2, 8, 32, 0.5, False), (0, 0, 128, None, False), (1, 8, 32, None, True)])
+def test_device_scalars_outside_the_proven_range_beside_ordinary_leaves(pdt, ecc_bits, group, max_norm, elsewhere, first):
+    """Leaves whose eps lies outside the range of the reciprocal shortcut, which tile_kernel learns while it runs (the scalars are the device's), in
+    turn with ordinary ones: first tiles that were asked for ahead and are dropped, later leaves in the same slots, ragged ends of both."""
+    import torch
+
+    from flashoptim_jax_b200 import _engine as eng
+
+    rng = np.random.default_rng(group + pdt)
+    sizes = (148 * 4096 + 700, 40 * 1024 + 9, 300 * 1024 + 513, 511, 64 * 1024, 700, 90 * 1024 + 255)
+    refs = [H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), C.ADAM, C.STATE_QUANT, ecc_bits, group) for n in sizes]
+    devs = [r.copy().to_device() for r in refs]
+    hyper_of = [(i + (first == "inside")) % 2 for i in range(len(sizes))]  # 0: outside
+    for t in (1, 2):
+        hps = [H.hyper_tuple(C.ADAM, O.FUSED, t, lr=1e-3, wd=1e-2, eps=eps) for eps in (1e-13, 1e-8)]
+        scalars = torch.tensor([hps[0][0], hps[0][7], hps[0][8]], device="cuda")
+        grads = [H.make_grad(rng, n, 1e-2, H.BF16) for n in sizes]
+        dev_g, sq = [H.to_torch(g) for g in grads], None
+        if max_norm is not None:
+            sq = eng.sq_norm_of(dev_g)
+            grads = O.clip_by_global_norm(grads, max_norm, sq_norm=float(sq.cpu()))
+        for g, r, h in zip(grads, refs, hyper_of):
+            H.oracle_step(C.ADAM, g, r, C.STATE_QUANT, group, hps[h])
+        outs = [H.LeafArrays(*[None if getattr(d, f) is None else torch.empty_like(getattr(d, f)) for f in d.fields()]) for d in devs] if elsewhere else None
+        H.abi_step(C.ADAM, dev_g, devs, C.STATE_QUANT, group, [hp + (scalars.data_ptr(),) for hp in hps], hyper_of, pdt, 1, ecc_bits,
+                   grad_sq_norm=sq, max_grad_norm=max_norm or 0.0, outs=outs)
+        torch.cuda.synchronize()
+        devs = outs if elsewhere else devs
+        for i, (d, r) in enumerate(zip(devs, refs)):
+            H.assert_leaf_equal(d.to_host(), r, f"step {t} leaf {i} n={sizes[i]}")
