@@ -39,8 +39,8 @@ UNIT = "params/s"
 
 # DRAM bytes per parameter (dram__bytes_read.sum + dram__bytes_write.sum) of one profiler capture of each
 # kernel on a 2^26-element bf16 leaf with bf16 gradients, keyed by (optimizer, ECC bits); traffic is
-# proportional to the parameter count.  AdamW / int16 ECC: 917.4 MB per 67,108,864 parameters.
-NCU_DRAM_BYTES_PER_PARAM = {("adamw", 16): 13.67, ("adamw", 8): 11.62, ("lion", 8): 9.56, ("sgdw", 8): 9.54}
+# proportional to the parameter count.  AdamW / int16 ECC: 899.7 MB per 67,108,864 parameters.
+NCU_DRAM_BYTES_PER_PARAM = {("adamw", 16): 13.41, ("adamw", 8): 11.40, ("lion", 8): 9.30, ("sgdw", 8): 9.31}
 
 
 def bytes_per_param(optimizer: str, param_bytes: int, ecc_bits: int, grad_bytes: int) -> float:

@@ -62,8 +62,10 @@ static PieceFn find_pieces(int opt, int pdt, int ecc_bits, int state) {
 #ifndef FO_SMALL_ELEMS
 #define FO_SMALL_ELEMS (148ull * 8192ull)
 #endif
-// The same where tile_kernel takes over, whose warps spread tiles of 512 elements (AdamW, 24-bit masters, in us with pieces and with tiles:
-// 2^19 elements 4.5 / 4.7, 2^20 6.8 / 5.5, 2^21 12.8 / 8.2).
+// The same where tile_kernel takes over, whose warps spread tiles of 512 elements.  In us with pieces and with tiles, whole steps in a graph, at 606720
+// elements: AdamW 24-bit masters 7.4 / 6.2, 32-bit 7.5 / 6.1, fp32 7.2 / 5.7, groups of 128 7.6 / 6.1, Lion 24-bit 5.1 / 4.8, fp32 5.1 / 4.5, SGDW 24-bit 5.1 / 4.7, fp32
+// 5.1 / 4.3, groups of 256 5.2 / 4.8; with a ragged end (620100) AdamW 8.0 / 7.0, Lion 5.4 / 5.5, SGDW 5.4 / 5.5.  At 2^19 pieces lead under AdamW (4.5 / 4.7,
+// the kernels alone).
 constexpr unsigned long long kSmallElemsTiles = 148ull * 4096ull;
 
 static DevHyper make_dev_hyper(const FoHyper& h, int opt) {

