@@ -431,7 +431,9 @@ FO_DEVI f2 reconstruct_ordinary2(f2 lpf, f2 ef) {
   // RN(e / MAX) for every integer e of the ECC type: e*hi + RN(e*lo) carries the quotient to
   // about 2^-48, which no e/MAX comes that close to a rounding boundary without being exact
   // (all 2^ECC_BITS values are compared with the IEEE division by the self-test)
-  f2 fr = fma2(ef, sp(K::rcp_hi()), mul2(ef, sp(K::rcp_lo())));
+  // (bf16 with 8-bit codes: lp has zeros where the products with RN(1 / 127) and the quotients differ, and the sums are the same for all values
+  // and codes.  With 16-bit codes the quotient's own rounding decides ties of the sum, and fp16 has values as small as the code's steps.)
+  f2 fr = PDT == FO_BF16 && ECC_BITS == 8 ? mul2(ef, sp(K::rcp_hi())) : fma2(ef, sp(K::rcp_hi()), mul2(ef, sp(K::rcp_lo())));
   f2 sc = mk(__uint_as_float(exp_field<PDT>(lpf.x)), __uint_as_float(exp_field<PDT>(lpf.y)));
   return fma2(fr, sc, lpf);
 }

@@ -104,6 +104,24 @@ __global__ void selftest_split(const float one, unsigned long long* out) {
   tally(bad, out);
 }
 
+// the parameter hand-back in 16-bit instructions, for every pair of an old and a new value (which NaN a NaN is stays open)
+template <int PDT>
+__global__ void selftest_hand_back(unsigned long long* out) {
+  unsigned long long bad = 0;
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 32); i += stride) {
+    const uint32_t old = (uint32_t)(i & 0xFFFFu), now = (uint32_t)(i >> 16);
+    const float o = Lp<PDT>::to_f32(old);
+    const uint32_t want = Lp<PDT>::from_f32(fadd(o, Lp<PDT>::to_f32(Lp<PDT>::from_f32(fsub(Lp<PDT>::to_f32(now), o)))));
+    const uint32_t got = hand_back2<PDT>(old | (now << 16), now | (old << 16));  // the same pair the other way round beside it
+    bad += !same_float(Lp<PDT>::to_f32(got & 0xFFFFu), Lp<PDT>::to_f32(want));
+    const float n = Lp<PDT>::to_f32(now);
+    const uint32_t back = Lp<PDT>::from_f32(fadd(n, Lp<PDT>::to_f32(Lp<PDT>::from_f32(fsub(o, n)))));
+    bad += !same_float(Lp<PDT>::to_f32(got >> 16), Lp<PDT>::to_f32(back));
+  }
+  tally(bad, out);
+}
+
 FO_DEVI uint32_t mix(uint64_t x) {
   x ^= x >> 33; x *= 0xff51afd7ed558ccdull; x ^= x >> 33; x *= 0xc4ceb9fe1a85ec53ull; x ^= x >> 33;
   return (uint32_t)x;
@@ -294,7 +312,10 @@ static void launch_sweep(int32_t which, int64_t arg, unsigned long long* d, cuda
 #define X(P, E)                                                                                  \
   if (pdt == P && eb == E) {                                                                     \
     if (which == FO_SELFTEST_RECONSTRUCT) selftest_reconstruct<P, E><<<grid, block, 0, s>>>(one, d); \
-    else selftest_split<P, E><<<grid, block, 0, s>>>(one, d);                                    \
+    else {                                                                                       \
+      selftest_split<P, E><<<grid, block, 0, s>>>(one, d);                                       \
+      if (E == 8) selftest_hand_back<P><<<grid, block, 0, s>>>(d);                               \
+    }                                                                                            \
     return;                                                                                      \
   }
       X(FO_BF16, 8) X(FO_BF16, 16) X(FO_F16, 8) X(FO_F16, 16)

@@ -226,6 +226,7 @@ struct Hyp {
   float lr, wd, b1, b2, omb1, omb2, eps;
   float decay, lr_bc1, sqrt_bc2, rcp_sqrt_bc2;
   float m_lo, m_hi;  // Adam: first moments between these keep the update's numerator lr/bc1 * m inside [2^-70, 2^60]
+  float least;       // smallest new parameter for which tile_kernel's first pass may leave out checks (tile_run); infinite: none
   uint32_t flags;
 };
 
@@ -253,7 +254,13 @@ FO_DEVI Hyp load_hyper(const DevHyper& d) {
     const float lrb = fabsf(h.lr_bc1);
     h.m_lo = fmul(fdiv(8.4703295e-22f, lrb), 1.0000005f);
     h.m_hi = fmul(fdiv(1.1529215e18f, lrb), 0.9999995f);
+    h.least = fmaxf(1.4551915e-11f, fmul(lrb, 2.3283064e-10f));  // 2^-36, lr/bc1 * 2^-32
+    const float b1 = fabsf(h.b1);
+    if (!((b1 >= 9.5367432e-7f || b1 == 0.0f) && fabsf(h.omb1) <= 2.0f)) h.least = __int_as_float(0x7F800000);
+  } else {
+    h.least = 1.4551915e-11f;
   }
+  if (!(fabsf(h.decay) <= 2.0f)) h.least = __int_as_float(0x7F800000);
   return h;
 }
 
@@ -268,6 +275,12 @@ FO_DEVI bool rest_is_decay(const Hyp& h) {
 }
 
 FO_DEVI float sign_of(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : x); }
+// the same in two instructions for x that is not NaN
+FO_DEVI float sign_or_zero(float x) {
+  float d;
+  asm("set.neu.f32.f32 %0, %1, 0f00000000;" : "=f"(d) : "f"(x));  // 1 or 0
+  return copysignf(d, x);
+}
 
 // ============================================================================================
 // cold path: one element at a time, IEEE arithmetic only
@@ -368,7 +381,8 @@ FO_DEVI Clip load_clip(const double* sq_norm, float max_norm, int gdt) {
   c.m_g = round_to_grad_dtype(max_norm, gdt);
   c.rcp_n = __frcp_rn(c.n_g);
   // Markstein's correction needs a correctly rounded reciprocal of a divisor whose mantissa is not all ones
-  c.div_ok = (__float_as_uint(c.n_g) & 0x7FFFFFu) != 0x7FFFFFu && c.n_g >= 9.5367432e-7f && c.n_g <= 1048576.0f;  // [2^-20, 2^20]
+  c.div_ok = (__float_as_uint(c.n_g) & 0x7FFFFFu) != 0x7FFFFFu && c.n_g >= 9.5367432e-7f && c.n_g <= 1048576.0f  // [2^-20, 2^20]
+             && fabsf(c.m_g) <= 2.0f * c.n_g;  // (a limit below zero: gradients do not grow)
   return c;
 }
 FO_DEVI float clip_ieee(float g, const Clip& c, int gdt) {
@@ -864,8 +878,8 @@ struct OutOf {
 };
 
 // master weights of a piece from the stored parameter words (p0, p1) and ECC words (e_in); same
-// contract for REPAIR as hot_unpack
-template <bool REPAIR, int PDT, int ECC_BITS>
+// contract for REPAIR as hot_unpack; CHECK = false: the caller answers for the values (tile_run)
+template <bool REPAIR, int PDT, int ECC_BITS, bool CHECK = true>
 FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, float2 (&theta)[4]) {
   using namespace fast2;
   bool rare = false;
@@ -911,7 +925,7 @@ FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, 
       // the first pass it leaves a theta that is not finite either, and stored_form sees that)
       [[maybe_unused]] constexpr float kLeast = PDT == FO_BF16 ? fast::Ordinary<FO_BF16>::kMin : 0.0f;
       bool odd = false;
-      if constexpr (PDT == FO_BF16) odd = !(minabs8(old_lp) >= kLeast);
+      if constexpr (PDT == FO_BF16 && CHECK) odd = !(minabs8(old_lp) >= kLeast);
       if constexpr (REPAIR) odd = odd || !(maxabs8(old_lp) <= 3.4e38f);
       if (odd) {
         rare = true;
@@ -930,8 +944,8 @@ FO_DEVI bool unpack_master(const uint4& p0, const uint4& p1, const uint4& e_in, 
   return rare;
 }
 
-// updated master weights -> parameter words and ECC words; same contract for REPAIR as hot_unpack
-template <bool REPAIR, int PDT, int ECC_BITS>
+// updated master weights -> parameter words and ECC words; same contract for REPAIR and CHECK as unpack_master
+template <bool REPAIR, int PDT, int ECC_BITS, bool CHECK = true>
 FO_DEVI bool stored_form(const float2 (&theta)[4], uint32_t (&nw)[4], uint4& ecc_out) {
   using namespace fast2;
   bool rare = false;
@@ -949,7 +963,7 @@ FO_DEVI bool stored_form(const float2 (&theta)[4], uint32_t (&nw)[4], uint4& ecc
       uint32_t ne[8];
 #pragma unroll
       for (int k = 0; k < 4; ++k) ecc_ordinary2<PDT, ECC_BITS>(theta[k], new_lp[k], ne[2 * k], ne[2 * k + 1]);
-      {
+      if constexpr (CHECK) {
         // outside these the exponent-field shortcut does not hold (tiny bf16 values), or the
         // update overflowed the 16-bit range and the reference clips the ECC
         [[maybe_unused]] constexpr float kLeast = PDT == FO_BF16 ? fast::Ordinary<FO_BF16>::kMin : 0.0f;
@@ -1140,8 +1154,8 @@ FO_DEVI bool mean_of_sum(float2 (&g)[4], const int gdt, const Peers& peers) {
 }
 
 // Global-norm clipping of a piece (see Clip), for gradients already known to be rescaled.
-// Same contract for REPAIR as hot_unpack.
-template <bool REPAIR, typename CLIP>
+// Same contract for REPAIR and CHECK as unpack_master.
+template <bool REPAIR, bool CHECK = true, typename CLIP>
 FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const CLIP& source) {
   using namespace fast2;
   const Clip c = source.get();
@@ -1155,11 +1169,13 @@ FO_DEVI bool clip_grads(float2 (&g)[4], const int gdt, const CLIP& source) {
     // normal: |g| >= 2^-100 (n_g <= 2^20), or zero.  Twice the magnitude bits minus one, as unsigned: zero wraps
     // to the top and passes.  (With the exact division and both conversions the same took 11 instructions per
     // element instead of 4.)
-    uint32_t lo = 0xFFFFFFFFu;
+    if constexpr (CHECK) {
+      uint32_t lo = 0xFFFFFFFFu;
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      lo = min(lo, min(2u * __float_as_uint(g[k].x) - 1u, 2u * __float_as_uint(g[k].y) - 1u));
-    rare = rare || lo < 2u * 0x0D800000u - 1u;
+      for (int k = 0; k < 4; ++k)
+        lo = min(lo, min(2u * __float_as_uint(g[k].x) - 1u, 2u * __float_as_uint(g[k].y) - 1u));
+      rare = rare || lo < 2u * 0x0D800000u - 1u;
+    }
     const __nv_bfloat162 mg = __float2bfloat162_rn(c.m_g);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -1213,6 +1229,15 @@ FO_DEVI float sign_of(float x);
 template <int OPT, int PDT, int ECC_BITS, int STATE, int MODE>
 __device__ __noinline__ void warm_chunk(const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const uint32_t i0, const Peers* peers);
 
+// old + (now - old) of two 16-bit values at a time, each operation rounded to their dtype
+template <int PDT>
+FO_DEVI uint32_t hand_back2(const uint32_t old, const uint32_t now) {
+  uint32_t r;
+  if constexpr (PDT == FO_BF16) asm("{.reg .b32 d; sub.rn.bf16x2 d, %2, %1; add.rn.bf16x2 %0, %1, d;}" : "=r"(r) : "r"(old), "r"(now));
+  else asm("{.reg .b32 d; sub.rn.f16x2 d, %2, %1; add.rn.f16x2 %0, %1, d;}" : "=r"(r) : "r"(old), "r"(now));
+  return r;
+}
+
 // FO_FLAG_LP_DELTA: the parameter handed back is old + lp(new - old), each operation rounded to the parameter's
 // dtype (flashoptim_jax/adamw.py:411,415,463); o0, o1 are the old parameter's words
 template <int PDT>
@@ -1224,25 +1249,18 @@ FO_DEVI void hand_back_delta(const uint4& o0, const uint4& o1, uint32_t (&nw)[4]
 #pragma unroll
     for (int k = 0; k < 4; ++k) theta[k] = add2(old[k], fma2(old[k], sp(-1.0f), theta[k]));
   } else {
-    float2 old[4];
-    pairs_of16<PDT>(o0, old);
+    // the 16-bit instructions round once, which is what fp32 operations rounded to 16 bits do (compared for all pairs of values by the self-test)
+    const uint32_t old[4] = {o0.x, o0.y, o0.z, o0.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float2 nv, d;
-      unpack2<PDT>(nw[k], nv.x, nv.y);
-      nv = fma2(old[k], sp(-1.0f), nv);
-      unpack2<PDT>(pack2<PDT>(nv.x, nv.y), d.x, d.y);
-      nv = add2(old[k], d);
-      nw[k] = pack2<PDT>(nv.x, nv.y);
-    }
+    for (int k = 0; k < 4; ++k) nw[k] = hand_back2<PDT>(old[k], nw[k]);
   }
 }
 
 // One step of eight elements: u.theta becomes the new master weight, u.m (and, kept in full, u.v) the new moments, nroot the negated
 // square root of the new second moment; am_lane and av_lane the largest magnitude of the first moment and of that root.
-// Same contract for REPAIR as hot_unpack.  COUPLED = false leaves out the weight decay that is added to the gradient: for calls in which
+// Same contract for REPAIR as hot_unpack; CHECK_M = false: the caller answers for the first moments.  COUPLED = false leaves out the weight decay that is added to the gradient: for calls in which
 // it is zero or decoupled.
-template <bool REPAIR, int OPT, int STATE, bool COUPLED>
+template <bool REPAIR, int OPT, int STATE, bool COUPLED, bool CHECK_M = true>
 FO_DEVI bool update_pairs(const Hyp& h, const float one, Unpacked& u, float2 (&nroot)[4], float& am_lane, float& av_lane) {
   using namespace fast2;
   const float2 one2 = sp(one);
@@ -1290,7 +1308,8 @@ FO_DEVI bool update_pairs(const Hyp& h, const float one, Unpacked& u, float2 (&n
     av_lane = -min8(nroot);
     // (with quantized moments the largest square root is checked once per group below, after the
     // shuffles; the repairing pass needs the answer per lane)
-    bool wild = !(max8(nv) <= -1.0e-30f) || !(minabs8(m) >= h.m_lo) || !(am_lane <= h.m_hi);
+    bool wild = !(max8(nv) <= -1.0e-30f);
+    if constexpr (CHECK_M) wild = wild || !(minabs8(m) >= h.m_lo) || !(am_lane <= h.m_hi);
     if constexpr (REPAIR || STATE != FO_STATE_QUANT) wild = wild || !(av_lane <= 1.0737418e9f);  // (an overflown second moment: NaN here)
     if (wild) {
       rare = true;
@@ -1309,25 +1328,27 @@ FO_DEVI bool update_pairs(const Hyp& h, const float one, Unpacked& u, float2 (&n
     for (int k = 0; k < 4; ++k) theta[k] = tn[k];
   } else if constexpr (OPT == FO_OPT_LION) {
     // flashoptim_jax/momentum_kernel.py:77-79 or flashoptim_jax/lion.py:50-52
+    // (With quantized moments a NaN fails the first pass by its group's maximum.)
+    auto direction = [](float x) { return !REPAIR && STATE == FO_STATE_QUANT ? sign_or_zero(x) : sign_of(x); };
     float2 upd[4];
     if (h.flags & FO_FLAG_LION_LERP) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float2 d = fma2(m[k], sp(-1.0f), g[k]);  // g - m
         const float2 c = sum2(mul2(sp(h.omb1), d), m[k], one2);
-        upd[k] = mk(sign_of(c.x), sign_of(c.y));
+        upd[k] = mk(direction(c.x), direction(c.y));
         m[k] = sum2(mul2(sp(h.omb2), d), m[k], one2);
       }
     } else {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float2 c = sum2(mul2(sp(h.b1), m[k]), mul2(sp(h.omb1), g[k]), one2);
-        upd[k] = mk(sign_of(c.x), sign_of(c.y));
+        upd[k] = mk(direction(c.x), direction(c.y));
         m[k] = sum2(mul2(sp(h.b2), m[k]), mul2(sp(h.omb2), g[k]), one2);
       }
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) theta[k] = sum2(mul2(theta[k], sp(h.decay)), mul2(sp(-h.lr), upd[k]), one2);  // theta*decay - lr*upd
+    for (int k = 0; k < 4; ++k) theta[k] = fma2(sp(-h.lr), upd[k], mul2(theta[k], sp(h.decay)));  // theta*decay - lr*upd; lr times +-1 or +-0 is exact
     am_lane = maxabs8(m);
   } else {
     // flashoptim_jax/momentum_kernel.py:74-75,80-86; flashoptim_jax/sgd.py:45-63

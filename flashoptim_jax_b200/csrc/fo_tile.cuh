@@ -189,6 +189,14 @@ FO_DEVI void slot_read(const DevLeaf& L, const uint32_t slot, const uint32_t hal
   }
 }
 
+// The magnitudes of new bf16 parameters that tile_run accepts, from `least` (rounded up) to 2^126: x = 2 w + range.x, in each half of a word of two parameters,
+// counts from twice the smallest and is below range.y for them only (a carry out of the lower half can make it one or two more).
+constexpr uint32_t kMostBits = 0x7E80u;  // 2^126
+FO_DEVI uint2 range_from(const float least) {
+  const uint32_t low = min((__float_as_uint(least) >> 16) + 2u, kMostBits);
+  return make_uint2((0x8000u - low) * 0x00020002u, 2u * (kMostBits - low));
+}
+
 // Half of a tile that holds a value outside the shortcuts' ranges, 256 elements (sixteen lanes' worth): once more, by the repairing pass, from the warp's slot,
 // which still holds it.  It works out for itself what only it needs, rows at rest among it: asked in the loop that cost ordinary tiles
 // up to 5 %.  (Storing a half that holds no such value from the first pass made the loop slower, AdamW with 8-bit codes 588 -> 623 us per 2^28
@@ -215,6 +223,20 @@ __device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, co
 }
 
 // One warp's tiles t, t + kWarps, ... below t1 of a leaf.  `primed`: the first one's copies are under way, in the first slot.
+//
+// bf16 parameters with codes (kLate; not under a decay added to the gradient): what the shortcuts ask of the old parameter and of the first moment follows
+// from the new parameter, so that one look at it takes the place of four range checks of every element.  Let it be |p| >= L, L = h.least >= 2^-36, and |decay| <= 2.
+//   * An old parameter below 2^-100, which the packed reconstruction may get wrong (it stays below 2^-99), has left nothing in p: the update it was
+//     decayed and added to is at least L / 2, 2^60 times as large.
+//   * A numerator below 2^-102, for which neg_div2 is not exact, makes an update below 2^-62 (eps >= 2^-40), exact or not, which is less than half a
+//     unit in the last place of anything that rounds to p: it adds nothing.  Above, up to 2^60 (am_most), neg_div2 is exact or its quotient as small.
+//   * Clipping a bf16 gradient below 2^-100, whose quotient may be off, makes a gradient below 2^-99.  The second moment is that of the element's past,
+//     or below the 1e-30 that is checked.  The first moment is that of the past too, or (|b1| >= 2^-20 or 0, |omb1| <= 2) below 2^-98: its code is 0 and its
+//     update, below 2^-58 lr / bc1, less than half a unit of p, which is why L is at least 2^-32 lr / bc1.
+// The look is taken at the packed words (range_from): an addition per word and a maximum per two.  (A test of single bits that passes 2^-31 to 2 with half
+// of that, and a comparison behind it for the rest, made leaves with larger parameters 5 % slower.)
+// AdamW with 8-bit codes, 2^28 elements 580 -> 560 us, with the power cap reached 662 -> 648, 4 M elements in the L2 12.3 -> 11.7; clipping 649 -> 597, 717 ->
+// 674, 14.4 -> 13.6; 16-bit codes 691 -> 682 at the cap; Lion 472 -> 441 and 9.1 -> 8.5, half of it by its sign in two instructions; SGDW 461 -> 454.
 template <int OPT, int PDT, int ECC_BITS, int GDT, int MODE, typename OUT>
 FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, const DevOut* out, const DevHyper& dh, const Hyp& h, const SharedClip& clip, uint32_t t,
                       const uint32_t t1, const uint32_t slots, const char* table, const OUT& distance) {
@@ -223,6 +245,7 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
   constexpr bool kAdam = OPT == FO_OPT_ADAM;
   constexpr int kStep = kWarps * kTileElems;  // elements from one of the warp's tiles to the next
   constexpr int kPsz = PDT == FO_F32 ? 4 : 2, kEsz = ECC_BITS / 8;
+  constexpr bool kLate = PDT == FO_BF16 && ECC_BITS != 0 && (MODE & kCoupled) == 0;
   const int gdt = GDT == kAnyGrad ? c.grad_dtype : GDT;
   const int gsz = gdt == FO_F32 ? 4 : 2;
   const int gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;  // 4 to 8 here
@@ -236,6 +259,14 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
   const int sc_step = (kStep >> gshift) * 2;
   bool wide = ((reinterpret_cast<uintptr_t>(L.param) | (ECC_BITS == 16 ? reinterpret_cast<uintptr_t>(L.ecc) : 0)) & 31u) == 0;
   if constexpr ((MODE & kOut) != 0) wide = wide && ((distance(&DevOut::param) | (ECC_BITS == 16 ? distance(&DevOut::ecc) : 0)) & 31) == 0;
+  // Where the range stands in the code it is 2^-28 and up, and a leaf that asks for more fails by its scales.  (That took AdamW with 8-bit codes, 4 M elements
+  // in the L2, 11.9 -> 11.7 us, clipping 13.8 -> 13.6, handing back 12.5 -> 12.1, Lion 8.55 -> 8.50, with 16-bit
+  // codes and fp32 gradients 10.8 -> 10.4, AdamW 4096 x 4096 in groups of 128 50.0 -> 49.3; but AdamW with 16-bit codes 12.4 -> 12.5, SGDW 8.5 -> 8.8.)
+  constexpr bool kFixed = OPT == FO_OPT_LION || (kAdam && (ECC_BITS == 8 || (MODE & kGroup) != 0));
+  constexpr float kFixedLeast = 3.7252903e-9f;
+  const uint2 range = kFixed ? range_from(kFixedLeast) : range_from(h.least);
+  float am_most = kAdam ? fminf(1.0e30f, h.m_hi) : 1.0e30f;  // of a group scale: the reciprocal's range, the update's numerator
+  if constexpr (kLate && kFixed) am_most = h.least <= kFixedLeast ? am_most : -1.0f;
   uint32_t slot = slots;
   if (!primed) {
     __syncwarp();
@@ -293,7 +324,7 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
       else p0 = lds128(p_at ^ (16u * k));
       if constexpr (ECC_BITS == 16) e = lds128((slot + S::kEcc + Units<2>::read_at(lane)) ^ (16u * k));
       if constexpr (ECC_BITS == 8) { e.x = k ? eq.z : eq.x; e.y = k ? eq.w : eq.y; }
-      bool odd = unpack_master<false, PDT, ECC_BITS>(p0, p1, e, u.theta);
+      bool odd = unpack_master<false, PDT, ECC_BITS, !kLate>(p0, p1, e, u.theta);
       const uint32_t mw[2] = {k ? mq.z : mq.x, k ? mq.w : mq.y}, vw[2] = {k ? vq.z : vq.x, k ? vq.w : vq.y};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -304,14 +335,14 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
         }
       }
       if constexpr ((MODE & kClip) != 0) {
-        if (clip.active) odd = clip_grads<false>(u.g, gdt, clip) || odd;
+        if (clip.active) odd = clip_grads<false, !(kLate && kAdam)>(u.g, gdt, clip) || odd;
       }
       float am_lane, av_lane;
-      odd = update_pairs<false, OPT, FO_STATE_QUANT, (MODE & kCoupled) != 0>(h, c.one, u, nroot[k], am_lane, av_lane) || odd;
+      odd = update_pairs<false, OPT, FO_STATE_QUANT, (MODE & kCoupled) != 0, !kLate>(h, c.one, u, nroot[k], am_lane, av_lane) || odd;
       // (Infinite parameters and NaNs take part in a weight decay of zero that is added to the gradient, which this pass leaves out.  Where there
       // is an error-correction code stored_form sees them.)
       if constexpr (ECC_BITS == 0 && OPT != FO_OPT_LION && (MODE & kCoupled) == 0) odd = odd || !(maxabs8(u.theta) <= 3.4e38f);
-      odd = stored_form<false, PDT, ECC_BITS>(u.theta, nw[k], ecc_out[k]) || odd;
+      odd = stored_form<false, PDT, ECC_BITS, !kLate>(u.theta, nw[k], ecc_out[k]) || odd;
       rare = rare || odd;
       am = k ? max2<true>(am, am_lane) : am_lane;
       av = k ? max2<true>(av, av_lane) : av_lane;
@@ -328,8 +359,16 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
       am = max2<true>(am, __shfl_xor_sync(0xFFFFFFFFu, am, 1));
       if constexpr (kAdam) av = max2<true>(av, __shfl_xor_sync(0xFFFFFFFFu, av, 1));
     }
-    rare = rare || !(am >= 1.0e-12f && am <= 1.0e30f);                           // an all-zero group, or beyond the reciprocal's range
+    rare = rare || !(am >= 1.0e-12f && am <= am_most);                           // an all-zero group, or beyond
     if constexpr (kAdam) rare = rare || !(av >= 1.0e-12f && av <= 1.0737418e9f);  // 2^30: also the limit of the packed division
+    if constexpr (kLate) {
+      uint32_t most = 0u;
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; j += 2) most = __vimax3_u16x2(most, 2u * nw[k][j] + range.x, 2u * nw[k][j + 1] + range.x);
+      rare = rare || (most & 0xFFFFu) >= range.y || (most >> 16) >= range.y;
+    }
     if (__any_sync(0xFFFFFFFFu, rare)) {
       // (A loop under Adam, two calls under Lion and SGD: which of them leaves the loop around it fewer instructions differs, AdamW 9 M elements in
       // the L2 22.2 and 24.6 us, Lion 17.4 and 17.0, SGDW 15.1 and 14.9; through one call for both halves 24.1, 17.5 and 14.9.)

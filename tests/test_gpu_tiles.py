@@ -267,3 +267,50 @@ def test_device_scalars_outside_the_proven_range_beside_ordinary_leaves(pdt, ecc
         devs = outs if elsewhere else devs
         for i, (d, r) in enumerate(zip(devs, refs)):
             H.assert_leaf_equal(d.to_host(), r, f"step {t} leaf {i} n={sizes[i]}")
+
+
+@pytest.mark.parametrize("opt,ecc_bits,group,gdt,more", [
+    (C.ADAM, 16, 32, 1, {}), (C.ADAM, 8, 32, 0, {}), (C.ADAM, 8, 128, 1, dict(conv=O.UNFUSED)), (C.ADAM, 16, 32, 1, dict(max_norm=0.5)),
+    (C.ADAM, 8, 32, 1, dict(max_norm=0.5, lr=20.0)), (C.ADAM, 8, 32, 1, dict(lr=0.0)), (C.ADAM, 16, 32, 1, dict(lr=1e-12, eps=1e-12)),
+    (C.ADAM, 8, 32, 1, dict(wd=4e3)), (C.ADAM, 8, 32, 1, dict(b1=1e-9, max_norm=0.5)), (C.ADAM, 16, 32, 1, dict(b1=0.0, max_norm=0.5)), (C.ADAM, 8, 32, 1, dict(decoupled=False)),
+    (C.ADAM, 8, 32, 0, dict(elsewhere=True)), (C.LION, 8, 32, 1, {}), (C.LION, 16, 64, 0, dict(conv=O.UNFUSED)), (C.LION, 8, 32, 1, dict(wd=4e3)),
+    (C.SGD, 8, 32, 1, {}), (C.SGD, 16, 32, 0, dict(nesterov=True)), (C.SGD, 8, 32, 1, dict(lr=1e-9))])
+def test_parameters_and_gradients_at_the_edges_of_the_first_pass(opt, ecc_bits, group, gdt, more):
+    """bf16 parameters of every power of two, and next to it, from the smallest to the largest, some of which the update crosses, beside tiny
+    gradients: alone in their tile and many in one."""
+    import torch
+
+    from flashoptim_jax_b200 import _engine as eng
+
+    kw = dict(dict(lr=1e-3, wd=1e-2), **more)
+    conv, max_norm, elsewhere = kw.pop("conv", O.FUSED), kw.pop("max_norm", None), kw.pop("elsewhere", False)
+    rng = np.random.default_rng(opt * 100 + ecc_bits + gdt + len(more))
+    n = 148 * 8192 + 700
+    p = rng.normal(0, 0.02, n).astype(np.float32)
+    edge = rng.random(n) < np.where(np.arange(n) < n // 2, 1 / 1000, 1 / 3)
+    exponent = rng.integers(-133, 120 if kw.get("decoupled", True) else 10, n)  # (a decay in the gradient: fp16 scales of the moments stay finite)
+    near = rng.random(n) < 0.5  # next to where the checks lie
+    exponent[near] = rng.choice([-126, -101, -100, -99, -64, -38, -37, -36, -35, -33, -32, -31, -30, 0, 1, 2], int(near.sum()))
+    edges = np.ldexp(rng.choice([1.0, 1.0 - 2.0**-8, 1.0 + 2.0**-7], n), exponent) * rng.choice([-1.0, 1.0], n)
+    p[edge] = edges[edge].astype(np.float32)
+    ref = H.fresh_leaf(p.astype(H.BF16), opt, C.STATE_QUANT, ecc_bits, group)
+    dev = ref.copy().to_device()
+    for t in (1, 2, 3):
+        g = H.make_grad(rng, n, 1e-2, np.float32)
+        tiny = rng.random(n) < 1 / 500
+        g[tiny] = np.ldexp(rng.choice([-1.0, 1.0], int(tiny.sum())), rng.integers(-140, -20, int(tiny.sum())))
+        g = g.astype(G_NP[gdt])
+        hp = H.hyper_tuple(opt, conv, t, **kw)
+        dev_g, sq = [H.to_torch(g)], None
+        if max_norm is not None:
+            sq = eng.sq_norm_of(dev_g)
+            g = O.clip_by_global_norm([g], max_norm, sq_norm=float(sq.cpu()))[0]
+        H.oracle_step(opt, g, ref, C.STATE_QUANT, group, hp)
+        outs = [H.LeafArrays(*[None if getattr(dev, f) is None else torch.empty_like(getattr(dev, f)) for f in dev.fields()])] if elsewhere else None
+        _step(opt, dev_g, [dev], outs, C.STATE_QUANT, group, hp, 1, gdt, ecc_bits, sq, max_norm or 0.0)
+        torch.cuda.synchronize()
+        dev = outs[0] if elsewhere else dev
+        got = dev.to_host()
+        both = np.isnan(got.param.astype(np.float32)) & np.isnan(ref.param.astype(np.float32))
+        got.param[both] = ref.param[both]  # (whichever NaN it is)
+        H.assert_leaf_equal(got, ref, f"step {t}")
