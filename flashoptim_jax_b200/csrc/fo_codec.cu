@@ -20,10 +20,21 @@ FO_DEVI void load8(const float* p, float (&v)[8]) {
   asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
 }
+// the same, giving way in the L2
+FO_DEVI void load8_once(const float* p, float (&v)[8]) {
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p));
+}
 FO_DEVI void store8(float* p, const float (&v)[8]) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
                "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
 }
+
+// Moments that are quantized are not read again, the codes are.  Up to about the size of the L2 the moments therefore give way in it, and what
+// dequantizes the codes, or the other moment, finds more of it there.  Both moments quantized and dequantized, 4.2 / 16.8 / 67 M elements: 20.5 / 62.8 / 222 us,
+// 19.8 / 59.6 / 223 with loads that give way; at 67 M a single quantization has 52.5 and 54.6.  (Blocks that stay and load a tile ahead 21.1 / 67.7 / 254, one
+// tile per block 20.4 / 64.8 / 227, blocks of 128 threads 22.0 / 73.3 / 275; the split of fp32 weights 306 and 318 with such loads.)
+constexpr unsigned long long kOnce = 1ull << 25;
 
 // Groups of 8 to 256 elements: 1 to 32 lanes.  (The maximum is taken over magnitude bits, so that a NaN survives.)
 template <bool VARIANCE>
@@ -39,7 +50,8 @@ __global__ void __launch_bounds__(kCodecThreads) quantize_kernel(const float* x,
     const bool whole = i0 + kPiece <= n;
     float v[8];
     if (whole && aligned) {
-      load8(x + i0, v);
+      if (n <= kOnce) load8_once(x + i0, v);
+      else load8(x + i0, v);
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = i0 + j < n ? x[i0 + j] : 0.0f;

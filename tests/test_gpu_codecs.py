@@ -171,3 +171,19 @@ def test_scales_of_another_group_size_are_refused():
         with pytest.raises(ValueError):
             fo.dequantize_momentum(bad, 32)
     assert torch.equal(fo.dequantize_momentum(q, 128), torch.ones(4096, device="cuda"))
+
+
+@pytest.mark.parametrize("group", [32, 256])
+@pytest.mark.parametrize("name", ["quantize_momentum", "quantize_variance"])
+def test_moments_on_either_side_of_the_size_from_which_loads_stay_in_the_l2(name, group):
+    """One call just above the size against two on its parts, which are below and at it."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    quantize, at = getattr(fo, name), 1 << 25
+    x = torch.randn(at + 256, device="cuda", generator=torch.Generator("cuda").manual_seed(group)).mul_(1e-3)
+    x = x.square_() if name == "quantize_variance" else x
+    whole, parts = quantize(x, group), (quantize(x[:at], group), quantize(x[at:], group))
+    for got, a, b in zip(whole, *parts):
+        assert torch.equal(got, torch.cat([a, b]))
