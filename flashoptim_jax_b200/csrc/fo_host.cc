@@ -318,6 +318,7 @@ struct Call {
   std::vector<FoHyper> hypers;
   std::vector<int> slots;  // group of each hyper set
   bool empty = true;       // no leaf has an element: nothing is launched
+  int64_t elems = 0;
 };
 struct Watched {  // a param-group dict as it was when the plan was made
   Ref dict;
@@ -333,6 +334,7 @@ struct Plan {
   std::vector<LeafSpec> leaves;
   std::vector<Group> groups;
   std::vector<Call> calls;
+  std::vector<int> order;          // in which they are issued
   Ref param_groups;
   std::vector<Watched> watched;
   bool dynamic = false;            // a selector that has to be asked at every step (a callable)
@@ -463,7 +465,13 @@ PyObject* make_plan(PyObject*, PyObject* args) {
     c.desc.n_hypers = (uint32_t)c.hypers.size();
     c.desc.leaves = c.leaves.data();
     c.desc.hypers = c.hypers.data();
+    plan->order.push_back((int)plan->order.size());
   }
+  // The largest first: the calls work on different leaves, and the launches of the small ones fill the SMs that are done with the large one.  In front
+  // of it they keep its blocks, which need an SM each, from beginning.  (ResNet-50, 25.5 M bf16 elements and 106 fp32 vectors, which the tree has first:
+  // SGDW 51.9 us a step in that order and 51.0 so, AdamW 71.2 and 66.6.)
+  for (const LeafSpec& l : plan->leaves) plan->calls[l.call].elems += l.n;
+  std::stable_sort(plan->order.begin(), plan->order.end(), [&](int a, int b) { return plan->calls[a].elems > plan->calls[b].elems; });
   return PyCapsule_New(plan.release(), kPlanName, [](PyObject* c) { delete (Plan*)PyCapsule_GetPointer(c, kPlanName); });
 }
 
@@ -748,7 +756,8 @@ PyObject* run(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const int status = on_device(plan->device, [&](cudaStream_t stream) {
     if (!plan->donate) allocate_results(*plan, made);
     uint32_t chain = 0u;
-    for (Call& c : plan->calls) {
+    for (const int at : plan->order) {
+      Call& c = plan->calls[at];
       for (size_t k = 0; k < c.slots.size(); ++k) c.hypers[k] = hyper[c.slots[k]];
       c.desc.grad_sq_norm = (const double*)sq;
       c.desc.max_grad_norm = f32(max_norm);

@@ -49,3 +49,47 @@ def test_dependent_calls_see_each_other(name, n):
     b = tree.tree_leaves(_chain(name, n, torch.cuda.synchronize))
     for x, y in zip(a, b):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("name", ["flash_adamw", "flash_lion", "flash_sgdw"])
+@pytest.mark.parametrize("n", [1000, 700_001, 2_000_003])
+def test_launches_of_one_step_in_a_graph(name, n):
+    """Leaves of three dtypes, the small ones first in the tree: their launches do not wait for that of the large one, the next gradients wait for all."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+    from flashoptim_jax_b200 import tree
+
+    def start():
+        g = torch.Generator(device="cuda").manual_seed(n)
+        p = {"a": torch.ones(4133, device="cuda"), "b": torch.ones(5, device="cuda", dtype=torch.float16),
+             "w": (torch.randn(n, device="cuda", generator=g) * 0.02).bfloat16()}
+        tx = getattr(fo, name)(learning_rate=1e-2, donate=True, capturable=True)
+        return tx, p, tx.init(p)
+
+    def steps(tx, p, s, pause):
+        for _ in range(3):
+            grads = {k: (v.float() * 0.1 + 1e-3).to(v.dtype) for k, v in p.items()}
+            pause()
+            p, s = tx.step(p, s, grads)
+            pause()
+        return p, s
+
+    side = torch.cuda.Stream()
+    tx, p, s = start()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        p, s = steps(tx, p, s, lambda: None)
+    torch.cuda.current_stream().wait_stream(side)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        p, s = steps(tx, p, s, lambda: None)
+    graph.replay()
+    graph.replay()
+    tx, q, t = start()
+    for _ in range(3):
+        q, t = steps(tx, q, t, torch.cuda.synchronize)
+    torch.cuda.synchronize()
+    for x, y in zip(tree.tree_leaves((p, s)), tree.tree_leaves((q, t))):
+        assert torch.equal(x, y)
