@@ -41,9 +41,9 @@ _KINDS = (("quant", 0), ("full", 1), ("generic", 3))
 # stream and one set of tables); the kernels that also read peers' gradients keep 256-thread blocks,
 # whose smaller stages leave room for a deeper copy pipeline.
 # "tile": the slices that run tile_kernel (quantized moments, one feature at most), one block per SM.  The 16 elements of a lane want 150 to
-# 168 registers under AdamW (2^28 elements, 24-bit masters: 588 us with 384 threads, 623 with 512; with the power cap reached
-# 672 and 704) and 138 under SGD (65 M elements, 32-bit masters, results elsewhere: 129 us with 384 threads, 143 with 512, 132 with 256);
-# Lion fits 512 (fp16, 2^28 elements: 435 us, 455 with 384).
+# 168 registers under AdamW (2^28 elements, 24-bit masters: 564 us with 384 threads, 585 with 512; with the power cap reached
+# 650 and 666; clipping 602 and 714) and 138 under SGD (65 M elements, 32-bit masters, results elsewhere: 129 us with 384 threads, 143 with 512, 132 with 256);
+# Lion fits 512 (2^28 elements at the cap, 24-bit masters: bf16 445 us, 462 with 384; fp16 479 and 493).
 _SHAPES = {("adam", "plain"): (512, 1), ("adam", "clip"): (512, 1), ("adam", "out"): (512, 1),
            ("adam", "delta"): (512, 1), ("adam", "all"): (384, 1), ("adam", "group8"): (512, 1), ("adam", "tile"): (384, 1),
            ("lion", "plain"): (768, 1), ("lion", "clip"): (512, 1), ("lion", "out"): (512, 1), ("lion", "all"): (512, 1), ("lion", "group8"): (512, 1),

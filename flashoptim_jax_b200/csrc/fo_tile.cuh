@@ -12,11 +12,15 @@
 //     look-up has a bank conflict.  64 KB of the SM's 227.
 //   * Slots: 16-byte units are stored at positions permuted inside 128 bytes (see Units), so that both the coalesced copies and
 //     the reads of a lane's 32 or 64 consecutive bytes fall on all banks.
-//   * All range checks are known once the group maxima are: one vote, then the stores of parameter and ECC, then the codes.
+//   * All range checks are known once the group maxima are: one vote, then the stores of parameter and ECC, then the codes.  For bf16 parameters
+//     with codes most of them are one look at the new parameters (tile_run).
 //   * Two slots per warp and a loop body that is not unrolled: three slots and an unrolled body measured the same.
 //
-// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 588 here; with the power cap reached
-// 798 and 675.  52 to 55 instructions per element instead of 63.
+// Measured (one bf16 leaf of 2^28 elements, AdamW, 32-bit master weights): 712 us with step_kernel, 588 here when it was written; with the power cap reached
+// 798 and 675 (691 -> 682 on another box when the checks moved).  51 instructions per element instead of 63; a packed one keeps the FMA pipe for two cycles (60 % busy, 64 % of
+// the issue slots).  Warps of a block, and blocks, end up to 10 % of a launch of 9 to 25 M elements apart.  Dealing the last tiles while the kernel runs
+// (clusterlaunchcontrol, a unit of one to four tiles for a warp that has nothing left) made 2^28 elements 3 to 8 % faster until the cap is reached, 1 to 2 %
+// slower then, and 9 M 24 -> 29 us: an answer takes a microsecond, and the device gives two per nanosecond.
 #pragma once
 
 namespace fo {
