@@ -187,3 +187,26 @@ def test_moments_on_either_side_of_the_size_from_which_loads_stay_in_the_l2(name
     whole, parts = quantize(x, group), (quantize(x[:at], group), quantize(x[at:], group))
     for got, a, b in zip(whole, *parts):
         assert torch.equal(got, torch.cat([a, b]))
+
+
+@pytest.mark.parametrize("n", [9472 * 2048, 9472 * 2048 + 1, 9473 * 2048 + 5, 9474 * 2048])
+def test_arrays_around_two_tiles_per_block(n):
+    """From 9472 tiles on the kernels that write more than they read have blocks of two tiles, the last of which may have one or part of one:
+    whole arrays against their halves."""
+    import torch
+
+    import flashoptim_jax_b200 as fo
+
+    x = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(n % 97)).mul_(0.02)
+    at = 4096 * 2048
+    for quantize, dequantize, y in ((fo.quantize_momentum, fo.dequantize_momentum, x), (fo.quantize_variance, fo.dequantize_variance, x * x)):
+        halves = [dequantize(quantize(y[:at], 32), 32), dequantize(quantize(y[at:], 32), 32)]
+        assert torch.equal(dequantize(quantize(y, 32), 32), torch.cat(halves))
+    for bits in (24, 32):
+        template = torch.empty(n, device="cuda", dtype=torch.bfloat16)
+        p, e = fo.set_fp32_params({"w": x}, {"w": template}, master_weight_bits=bits)
+        a, ea = fo.set_fp32_params({"w": x[:at]}, {"w": template[:at]}, master_weight_bits=bits)
+        b, eb = fo.set_fp32_params({"w": x[at:]}, {"w": template[at:]}, master_weight_bits=bits)
+        assert torch.equal(p["w"], torch.cat([a["w"], b["w"]])) and torch.equal(e["w"], torch.cat([ea["w"], eb["w"]]))
+        halves = [fo.reconstruct_weights(a, ea)["w"], fo.reconstruct_weights(b, eb)["w"]]
+        assert torch.equal(fo.reconstruct_weights(p, e)["w"], torch.cat(halves))
