@@ -290,6 +290,10 @@ extern "C" int fo_step_ex(const FoStepDesc* d, const FoStepMore* more, void* cud
       const DevHyper& dh = hyper[L.hyper];
       bool hot = aligned && !(mode == kPeer && (dh.flags & FO_FLAG_LP_DELTA) != 0);
       if (d->opt == FO_OPT_ADAM && dh.dyn == nullptr) hot = hot && (dh.flags & kFlagTameAdam) != 0;
+      // Lion's first pass on quantized moments takes the sign of a NaN for 1.  Moments and gradients that bring one show in the group's maximum; factors
+      // that do (finite ones only where both products overflow) are found here.  (Asked in the kernel, before the loop, that made Lion on fp16 parameters
+      // 2 to 5 % slower: 16.8 M elements 30.0 -> 30.6 us by a bound of the maxima, 31.6 by factors that make such moments NaN.)
+      if (d->opt == FO_OPT_LION && d->state == FO_STATE_QUANT) hot = hot && fabsf(dh.b1) <= 1.0e30f && fabsf(dh.omb1) <= 3.4e38f;
 #ifdef FO_NAIVE_MATH
       hot = false;
 #endif

@@ -1328,7 +1328,7 @@ FO_DEVI bool update_pairs(const Hyp& h, const float one, Unpacked& u, float2 (&n
     for (int k = 0; k < 4; ++k) theta[k] = tn[k];
   } else if constexpr (OPT == FO_OPT_LION) {
     // flashoptim_jax/momentum_kernel.py:77-79 or flashoptim_jax/lion.py:50-52
-    // (With quantized moments a NaN fails the first pass by its group's maximum.)
+    // (With quantized moments a NaN of the moment or the gradient fails the first pass by its group's maximum; factors that make one do not come here.)
     auto direction = [](float x) { return !REPAIR && STATE == FO_STATE_QUANT ? sign_or_zero(x) : sign_of(x); };
     float2 upd[4];
     if (h.flags & FO_FLAG_LION_LERP) {

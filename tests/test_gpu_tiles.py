@@ -314,3 +314,24 @@ def test_parameters_and_gradients_at_the_edges_of_the_first_pass(opt, ecc_bits, 
         both = np.isnan(got.param.astype(np.float32)) & np.isnan(ref.param.astype(np.float32))
         got.param[both] = ref.param[both]  # (whichever NaN it is)
         H.assert_leaf_equal(got, ref, f"step {t}")
+
+
+@pytest.mark.parametrize("n", [1000, MANY + 700])
+@pytest.mark.parametrize("conv", [O.FUSED, O.UNFUSED])
+@pytest.mark.parametrize("factors", [dict(b1=np.nan, omb1=np.nan), dict(b1=np.nan), dict(omb1=np.nan), dict(b1=np.inf), dict(omb1=-np.inf), dict(b1=3e38, omb1=-3e38)])
+@pytest.mark.parametrize("pdt,ecc_bits,group", [(1, 8, 32), (1, 16, 8), (2, 16, 64), (0, 0, 32)])
+def test_lion_under_factors_that_are_not_finite(pdt, ecc_bits, group, factors, conv, n):
+    """Factors that make the direction a NaN, and leave the moment what it is: so becomes the parameter, in pieces and in the first pass of tiles."""
+    rng = np.random.default_rng(n + group)
+    ref = H.fresh_leaf(rng.normal(0, 0.02, n).astype(np.float32).astype(H.NP_OF_CODE[pdt]), C.LION, C.STATE_QUANT, ecc_bits, group)
+    dev = ref.copy().to_device()
+    hp = list(H.hyper_tuple(C.LION, conv, 1, lr=1e-3, wd=1e-2))
+    for t in (1, 2):
+        g = H.make_grad(rng, n, 5e4, np.float32)
+        g[::50] = 0
+        if t == 2:  # (the first step gives moments)
+            hp[2], hp[4] = np.float32(factors.get("b1", hp[2])), np.float32(factors.get("omb1", hp[4]))
+        H.oracle_step(C.LION, g, ref, C.STATE_QUANT, group, hp)
+        _step(C.LION, [H.to_torch(g)], [dev], None, C.STATE_QUANT, group, hp, pdt, 0, ecc_bits)
+        H.assert_leaf_equal(_but_for_nans(dev.to_host(), ref, 32, np.empty(0, dtype=np.int64)), ref, f"step {t}")
+    assert conv is O.UNFUSED or np.isnan(ref.param.astype(np.float32)).any()
