@@ -83,6 +83,7 @@ static DevHyper make_dev_hyper(const FoHyper& h, int opt) {
     d.sqrt_bc2 = sqrtf(h.bc2);
     d.rcp_sqrt_bc2 = 1.0f / d.sqrt_bc2;
     if (adam_is_tame(h.eps, d.sqrt_bc2)) d.flags |= kFlagTameAdam;
+    d.least = adam_least_new(h.eps);
   }
   d.dyn = h.dev_scalars;
   return d;

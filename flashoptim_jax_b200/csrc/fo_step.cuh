@@ -97,6 +97,7 @@ struct DevHyper {
   // derived on the host with the same IEEE fp32 operations the kernel would use
   float decay, lr_bc1, sqrt_bc2, rcp_sqrt_bc2;
   uint32_t flags;
+  float least;       // Adam: see Hyp::least, for learning rates that do not count
   const float* dyn;  // optional device {lr, bc1, bc2}
 };
 
@@ -215,6 +216,10 @@ constexpr int kChunk = kThreads * kPiece;      // elements per chunk
 // would update the elements in between, in place and at the same time
 static_assert(kChunk % kPieceElems == 0, "a chunk is a whole number of pieces");
 
+// The smallest new parameter that tile_kernel may let answer for the values behind it (tile_run, where it is derived).
+constexpr float kLeastNew = 3.3881318e-21f;                                                      // 2^-68: Lion and SGD
+inline float adam_least_new(float eps) { return fmaxf(kLeastNew, 1.3234890e-23f / eps); }  // 2^-76 / eps
+
 // true when the quotient sqrt(nu)/sqrt(bc2) may be formed as div_by_rcp without changing
 // (quotient + eps): for sqrt(nu) >= 2^-100 the shortcut is exact, below it the quotient is
 // under half an ULP of eps either way.
@@ -226,7 +231,7 @@ struct Hyp {
   float lr, wd, b1, b2, omb1, omb2, eps;
   float decay, lr_bc1, sqrt_bc2, rcp_sqrt_bc2;
   float m_lo, m_hi;  // Adam: first moments between these keep the update's numerator lr/bc1 * m inside [2^-70, 2^60]
-  float least;       // smallest new parameter for which tile_kernel's first pass may leave out checks (tile_run); infinite: none
+  float least;       // Adam: smallest new parameter for which tile_kernel's first pass may leave out checks (tile_run); infinite: none
   uint32_t flags;
 };
 
@@ -250,17 +255,14 @@ FO_DEVI Hyp load_hyper(const DevHyper& d) {
   h.m_lo = 0.0f; h.m_hi = 0.0f;
   if constexpr (OPT == FO_OPT_ADAM) {
     // quotients nudged two places inwards, so that m >= m_lo implies RN(|lr_bc1| * m) >= 2^-70 and
-    // m <= m_hi implies RN(|lr_bc1| * m) <= 2^60; lr = 0 gives m_lo = inf (everything takes the IEEE repairs)
+    // m <= m_hi implies RN(|lr_bc1| * m) <= 2^60; lr = 0 gives m_lo = inf (all that ask for it take the IEEE repairs)
     const float lrb = fabsf(h.lr_bc1);
     h.m_lo = fmul(fdiv(8.4703295e-22f, lrb), 1.0000005f);
     h.m_hi = fmul(fdiv(1.1529215e18f, lrb), 0.9999995f);
-    h.least = fmaxf(1.4551915e-11f, fmul(lrb, 2.3283064e-10f));  // 2^-36, lr/bc1 * 2^-32
+    h.least = fmaxf(d.least, fmul(lrb, d.least * 16.0f));
     const float b1 = fabsf(h.b1);
-    if (!((b1 >= 9.5367432e-7f || b1 == 0.0f) && fabsf(h.omb1) <= 2.0f)) h.least = __int_as_float(0x7F800000);
-  } else {
-    h.least = 1.4551915e-11f;
+    if (!((b1 >= 9.5367432e-7f || b1 == 0.0f) && fabsf(h.omb1) <= 2.0f && fabsf(h.decay) <= 2.0f)) h.least = __int_as_float(0x7F800000);
   }
-  if (!(fabsf(h.decay) <= 2.0f)) h.least = __int_as_float(0x7F800000);
   return h;
 }
 

@@ -229,14 +229,16 @@ __device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, co
 // One warp's tiles t, t + kWarps, ... below t1 of a leaf.  `primed`: the first one's copies are under way, in the first slot.
 //
 // bf16 parameters with codes (kLate; not under a decay added to the gradient): what the shortcuts ask of the old parameter and of the first moment follows
-// from the new parameter, so that one look at it takes the place of four range checks of every element.  Let it be |p| >= L, L = h.least >= 2^-36, and |decay| <= 2.
-//   * An old parameter below 2^-100, which the packed reconstruction may get wrong (it stays below 2^-99), has left nothing in p: the update it was
-//     decayed and added to is at least L / 2, 2^60 times as large.
-//   * A numerator below 2^-102, for which neg_div2 is not exact, makes an update below 2^-62 (eps >= 2^-40), exact or not, which is less than half a
+// from the new parameter, so that one look at it takes the place of four range checks of every element.  Let it be |p| >= L, L >= 2^-68, and |decay| <= 2.
+//   * An old parameter below 2^-100, which the packed reconstruction may get wrong (it stays below 2^-99), has left nothing in p: decayed it is below 2^-98, and
+//     a quarter of a unit in the last place of the update that it was added to, which is above L / 2, is 2^-27 L at least.  (Lion and SGD ask for no more.)
+//   * A numerator below 2^-102, for which neg_div2 is not exact, makes an update below 2^-102 / eps, exact or not.  With L >= 2^-76 / eps that is less than half a
 //     unit in the last place of anything that rounds to p: it adds nothing.  Above, up to 2^60 (am_most), neg_div2 is exact or its quotient as small.
 //   * Clipping a bf16 gradient below 2^-100, whose quotient may be off, makes a gradient below 2^-99.  The second moment is that of the element's past,
 //     or below the 1e-30 that is checked.  The first moment is that of the past too, or (|b1| >= 2^-20 or 0, |omb1| <= 2) below 2^-98: its code is 0 and its
-//     update, below 2^-58 lr / bc1, less than half a unit of p, which is why L is at least 2^-32 lr / bc1.
+//     update, below 2^-98 lr / bc1 / eps, less than half a unit of p with L >= 2^-72 lr / bc1 / eps.
+// (Hyp::least.  With eps = 1e-8 and lr / bc1 up to 1/16 it is 2^-49.  A range that began at 2^-28 sent most tiles of a matrix that started at zero to the repairs:
+// AdamW with 8-bit codes, 4096 x 4096, the first 20 steps of a warm-up 954 -> 1572 us, Lion 698 -> 979.)
 // The look is taken at the packed words (range_from): an addition per word and a maximum per two.  (A test of single bits that passes 2^-31 to 2 with half
 // of that, and a comparison behind it for the rest, made leaves with larger parameters 5 % slower.)
 // AdamW with 8-bit codes, 2^28 elements 580 -> 560 us, with the power cap reached 662 -> 648, 4 M elements in the L2 12.3 -> 11.7; clipping 649 -> 597, 717 ->
@@ -263,14 +265,10 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
   const int sc_step = (kStep >> gshift) * 2;
   bool wide = ((reinterpret_cast<uintptr_t>(L.param) | (ECC_BITS == 16 ? reinterpret_cast<uintptr_t>(L.ecc) : 0)) & 31u) == 0;
   if constexpr ((MODE & kOut) != 0) wide = wide && ((distance(&DevOut::param) | (ECC_BITS == 16 ? distance(&DevOut::ecc) : 0)) & 31) == 0;
-  // Where the range stands in the code it is 2^-28 and up, and a leaf that asks for more fails by its scales.  (That took AdamW with 8-bit codes, 4 M elements
-  // in the L2, 11.9 -> 11.7 us, clipping 13.8 -> 13.6, handing back 12.5 -> 12.1, Lion 8.55 -> 8.50, with 16-bit
-  // codes and fp32 gradients 10.8 -> 10.4, AdamW 4096 x 4096 in groups of 128 50.0 -> 49.3; but AdamW with 16-bit codes 12.4 -> 12.5, SGDW 8.5 -> 8.8.)
-  constexpr bool kFixed = OPT == FO_OPT_LION || (kAdam && (ECC_BITS == 8 || (MODE & kGroup) != 0));
-  constexpr float kFixedLeast = 3.7252903e-9f;
-  const uint2 range = kFixed ? range_from(kFixedLeast) : range_from(h.least);
+  // Lion and SGD have the range in the code, and a leaf under another decay fails by its scales.
+  const uint2 range = range_from(kAdam ? h.least : kLeastNew);
   float am_most = kAdam ? fminf(1.0e30f, h.m_hi) : 1.0e30f;  // of a group scale: the reciprocal's range, the update's numerator
-  if constexpr (kLate && kFixed) am_most = h.least <= kFixedLeast ? am_most : -1.0f;
+  if constexpr (kLate && !kAdam) am_most = fabsf(h.decay) <= 2.0f ? am_most : -1.0f;
   uint32_t slot = slots;
   if (!primed) {
     __syncwarp();
