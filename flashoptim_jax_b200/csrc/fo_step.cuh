@@ -384,7 +384,7 @@ FO_DEVI Clip load_clip(const double* sq_norm, float max_norm, int gdt) {
   c.rcp_n = __frcp_rn(c.n_g);
   // Markstein's correction needs a correctly rounded reciprocal of a divisor whose mantissa is not all ones
   c.div_ok = (__float_as_uint(c.n_g) & 0x7FFFFFu) != 0x7FFFFFu && c.n_g >= 9.5367432e-7f && c.n_g <= 1048576.0f  // [2^-20, 2^20]
-             && fabsf(c.m_g) <= 2.0f * c.n_g;  // (a limit below zero: gradients do not grow)
+             && fabsf(c.m_g) <= 65536.0f * c.n_g;  // (a limit below zero can make gradients larger: tile_run counts with 2^16 times at most)
   return c;
 }
 FO_DEVI float clip_ieee(float g, const Clip& c, int gdt) {

@@ -234,9 +234,10 @@ __device__ __noinline__ void end_piece(const StepCommon& c, const DevLeaf& L, co
 //     a quarter of a unit in the last place of the update that it was added to, which is above L / 2, is 2^-27 L at least.  (Lion and SGD ask for no more.)
 //   * A numerator below 2^-102, for which neg_div2 is not exact, makes an update below 2^-102 / eps, exact or not.  With L >= 2^-76 / eps that is less than half a
 //     unit in the last place of anything that rounds to p: it adds nothing.  Above, up to 2^60 (am_most), neg_div2 is exact or its quotient as small.
-//   * Clipping a bf16 gradient below 2^-100, whose quotient may be off, makes a gradient below 2^-99.  The second moment is that of the element's past,
-//     or below the 1e-30 that is checked.  The first moment is that of the past too, or (|b1| >= 2^-20 or 0, |omb1| <= 2) below 2^-98: its code is 0 and its
-//     update, below 2^-98 lr / bc1 / eps, less than half a unit of p with L >= 2^-72 lr / bc1 / eps.
+//   * Clipping a bf16 gradient below 2^-100, whose quotient may be off, makes a gradient below 2^-100 G, where G is 2 or, under a limit below zero, up to 2^16
+//     (Clip::div_ok) times as large as the norm, |limit| / norm.  The second moment is that of the element's past, or below the 1e-30 that is checked.  The
+//     first moment is that of the past too, or (|b1| >= 2^-20 or 0, |omb1| <= 2) below 2^-99 G: its code is 0 and its update, below 2^-99 G lr / bc1 / eps, less
+//     than half a unit of p with L >= 2^-73 G lr / bc1 / eps.
 // (Hyp::least.  With eps = 1e-8 and lr / bc1 up to 1/16 it is 2^-49.  A range that began at 2^-28 sent most tiles of a matrix that started at zero to the repairs:
 // AdamW with 8-bit codes, 4096 x 4096, the first 20 steps of a warm-up 954 -> 1572 us, Lion 698 -> 979.)
 // The look is taken at the packed words (range_from): an addition per word and a maximum per two.  (A test of single bits that passes 2^-31 to 2 with half
@@ -266,7 +267,14 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
   bool wide = ((reinterpret_cast<uintptr_t>(L.param) | (ECC_BITS == 16 ? reinterpret_cast<uintptr_t>(L.ecc) : 0)) & 31u) == 0;
   if constexpr ((MODE & kOut) != 0) wide = wide && ((distance(&DevOut::param) | (ECC_BITS == 16 ? distance(&DevOut::ecc) : 0)) & 31) == 0;
   // Lion and SGD have the range in the code, and a leaf under another decay fails by its scales.
-  const uint2 range = range_from(kAdam ? h.least : kLeastNew);
+  float least = kAdam ? h.least : kLeastNew;
+  if constexpr (kLate && kAdam && (MODE & kClip) != 0) {
+    if (clip.active) {
+      const Clip k = clip.get();
+      least *= fmaxf(1.0f, 0.5f * fabsf(k.m_g) * k.rcp_n);
+    }
+  }
+  const uint2 range = range_from(least);
   float am_most = kAdam ? fminf(1.0e30f, h.m_hi) : 1.0e30f;  // of a group scale: the reciprocal's range, the update's numerator
   if constexpr (kLate && !kAdam) am_most = fabsf(h.decay) <= 2.0f ? am_most : -1.0f;
   uint32_t slot = slots;

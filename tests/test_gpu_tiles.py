@@ -274,6 +274,7 @@ def test_device_scalars_outside_the_proven_range_beside_ordinary_leaves(pdt, ecc
     (C.ADAM, 8, 32, 1, dict(max_norm=0.5, lr=20.0)), (C.ADAM, 8, 32, 1, dict(lr=0.0)), (C.ADAM, 16, 32, 1, dict(lr=1e-12, eps=1e-12)),
     (C.ADAM, 8, 32, 1, dict(wd=4e3)), (C.ADAM, 8, 32, 1, dict(b1=1e-9, max_norm=0.5)), (C.ADAM, 16, 32, 1, dict(b1=0.0, max_norm=0.5)), (C.ADAM, 8, 32, 1, dict(decoupled=False)),
     (C.ADAM, 8, 32, 0, dict(elsewhere=True)), (C.ADAM, 8, 32, 1, dict(lr=20.0, eps=1e-12)), (C.ADAM, 16, 32, 0, dict(lr=50.0, max_norm=0.5, eps=1e-12)),
+    (C.ADAM, 8, 32, 1, dict(max_norm=-300.0)), (C.ADAM, 16, 32, 1, dict(max_norm=-3e5, lr=1e-8)), (C.ADAM, 8, 32, 0, dict(max_norm=-300.0)), (C.SGD, 8, 32, 1, dict(max_norm=-300.0)),
     (C.ADAM, 8, 32, 1, dict(lr=1e-15, eps=1.0)), (C.ADAM, 16, 32, 1, dict(lr=1e-18, eps=1e-6, max_norm=0.5)), (C.LION, 16, 32, 1, dict(lr=1e-20)), (C.SGD, 16, 32, 1, dict(lr=1e-18)), (C.LION, 8, 32, 1, {}), (C.LION, 16, 64, 0, dict(conv=O.UNFUSED)), (C.LION, 8, 32, 1, dict(wd=4e3)),
     (C.SGD, 8, 32, 1, {}), (C.SGD, 16, 32, 0, dict(nesterov=True)), (C.SGD, 8, 32, 1, dict(lr=1e-9))])
 def test_parameters_and_gradients_at_the_edges_of_the_first_pass(opt, ecc_bits, group, gdt, more):
@@ -338,31 +339,53 @@ def test_lion_under_factors_that_are_not_finite(pdt, ecc_bits, group, factors, c
     assert conv is O.UNFUSED or np.isnan(ref.param.astype(np.float32)).any()
 
 
+def _in_turn(opt, ecc_bits, g, start, **runs):
+    """ms that 20 steps take from the parameters start[name] with (hyper-parameters, square of the norm, limit) of runs[name], the smallest of nine, in turn."""
+    import torch
+
+    n, best = g.numel(), {}
+    empty = H.fresh_leaf(np.zeros(0, H.BF16), opt, C.STATE_QUANT, ecc_bits)
+    state = lambda a: None if a is None else torch.zeros(n // 32 if a.dtype == np.float16 else n, device="cuda", dtype=H.to_torch(a).dtype)  # noqa: E731
+    leaves = {name: H.LeafArrays(start[name].clone(), *[state(getattr(empty, f)) for f in empty.fields()[1:]]) for name in runs}
+    for _ in range(9):
+        for name, (hp, sq, limit) in runs.items():
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            for _ in range(20):
+                _step(opt, [g], [leaves[name]], None, C.STATE_QUANT, 32, hp, 1, 1, ecc_bits, sq, limit)
+            end.record()
+            end.synchronize()
+            best[name] = min(best.get(name, 1e9), begin.elapsed_time(end))
+    return best
+
+
+def _normal(n, sigma, seed):
+    import torch
+
+    return (torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(seed)) * sigma).bfloat16()
+
+
 @pytest.mark.parametrize("opt,lr,eps", [(C.ADAM, 1e-14, 1e-8), (C.ADAM, 20.0, 1e-12), (C.LION, 1e-14, 0.0), (C.SGD, 1e-14, 0.0)])
 @pytest.mark.parametrize("ecc_bits", [8, 16])
 def test_small_parameters_and_large_rates_take_the_first_pass(opt, ecc_bits, lr, eps):
     """A leaf a tenth of which is 1e-10 (as a matrix that started at zero, or pruned weights), or whose learning rate is large, against the same leaf without:
-    not slower by more than half (repaired it takes twice as long and more).  Times of 20 steps, the smallest of nine, in turn."""
-    import torch
-
-    n, best = 1 << 24, {}
-    p = (torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(opt)) * 0.02).bfloat16()
-    g = (torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(9)) * 1e-3).bfloat16()
-    small = torch.where(torch.rand(n, device="cuda", generator=torch.Generator("cuda").manual_seed(5)) < 0.1, torch.full_like(p, 1e-10), p) if lr < 1 else p
-    kw = dict(eps=eps) if opt == C.ADAM else {}
-    leaves = {}
-    for name, start, rate in (("plain", p, 1e-14), ("odd", small, lr)):
-        host = H.fresh_leaf(np.zeros(0, H.BF16), opt, C.STATE_QUANT, ecc_bits)
-        leaf = H.LeafArrays(start.clone(), *[None if a is None else torch.zeros(n // 32 if a.dtype == np.float16 else n, device="cuda", dtype=H.to_torch(a).dtype)
-                                             for a in (host.ecc, host.mu, host.mu_scales, host.nu, host.nu_scales)])
-        leaves[name] = (leaf, H.hyper_tuple(opt, O.FUSED, 1, lr=rate, wd=1e-2 if rate < 1 else 0.0, **kw))
-    for _ in range(9):
-        for name, (leaf, hp) in leaves.items():
-            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            begin.record()
-            for _ in range(20):
-                _step(opt, [g], [leaf], None, C.STATE_QUANT, 32, hp, 1, 1, ecc_bits)
-            end.record()
-            end.synchronize()
-            best[name] = min(best.get(name, 1e9), begin.elapsed_time(end))
+    not slower by more than half (repaired it takes twice as long and more)."""
+    n = 1 << 24
+    p, kw = _normal(n, 0.02, opt), dict(eps=eps) if opt == C.ADAM else {}
+    odd = p.clone()
+    if lr < 1:
+        odd[::10] = 1e-10
+    best = _in_turn(opt, ecc_bits, _normal(n, 1e-3, 9), dict(plain=p, odd=odd), plain=(H.hyper_tuple(opt, O.FUSED, 1, lr=1e-14, wd=1e-2, **kw), None, 0.0),
+                    odd=(H.hyper_tuple(opt, O.FUSED, 1, lr=lr, wd=1e-2 if lr < 1 else 0.0, **kw), None, 0.0))
     assert best["odd"] <= 1.5 * best["plain"], best
+
+
+@pytest.mark.parametrize("opt", [C.ADAM, C.LION, C.SGD])
+def test_limits_below_zero_take_the_first_pass(opt):
+    """Clipping to a limit below zero (gradients are turned round), which is larger than the norm, against one above it."""
+    from flashoptim_jax_b200 import _engine as eng
+
+    p, g = _normal(1 << 24, 0.02, opt), _normal(1 << 24, 1e-3, 9)
+    hp, sq = H.hyper_tuple(opt, O.FUSED, 1, lr=1e-3), eng.sq_norm_of([g])
+    best = _in_turn(opt, 8, g, dict(above=p, below=p), above=(hp, sq, 1.0), below=(hp, sq, -100.0))
+    assert best["below"] <= 1.5 * best["above"], best
