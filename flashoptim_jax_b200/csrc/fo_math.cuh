@@ -383,7 +383,8 @@ FO_DEVI f2 neg_rcp2(f2 d) {
   return fma2(e, ny0, ny0);       // -(y0 + e*y0)
 }
 
-// RN(-a/d) per component.  Needs d in [1e-12, 2^47], |a| in [2^-70, 2^60] (so |a/d| stays a normal number).
+// RN(-a/d) per component.  Needs d in [1e-12, 2^47], |a| in [2^-102, 2^60] and |a/d| a normal number (which |a| >= 2^-70 makes it).  Below 2^-102 the
+// last place of the residual, at least 2^-47 |a|, can fall off; the result is then below 2^-102 (1 + 2^-20) / d, or 2^-125, in magnitude.
 // y = RN(1/d) (checked exhaustively), q = RN(a y) is off by 1.5 units in the last place at most.  What one correction leaves before its
 // rounding (mantissas scaled to [1, 2)): d y is 1 up to 2^-25 d and q is a/d up to a 2^-25 + 2^-24, whose product, less than 2^-47, the
 // correction misses; and where q is more than a unit off the residual can take 25 bits and is rounded itself, by 2^-47 / d at most.

@@ -167,6 +167,19 @@ __global__ void selftest_group_div(const float one, unsigned long long pairs, un
       const float2 q = fast2::neg_div2(make_float2(num, -num), make_float2(den, den2));
       bad += !same_float(q.x, fdiv(-num, den)) || !same_float(q.y, fdiv(num, den2));
     }
+    {
+      // smaller numerators, down to zero, which tile_run lets pass: the same from 2^-102 on where the quotient is a normal number, else next to nothing
+      const float num = __uint_as_float((r1 & 0x80000000u) | ((r2 % 58u) << 23) | (r0 & 0x7FFFFFu));
+      const float den = __uint_as_float(((87u + r3 % 87u) << 23) | (r1 & 0x7FFFFFu));  // [2^-40, 2^47)
+      const float den2 = __uint_as_float((87u << 23) | (r2 & 0x7FFFFFu));
+      const float2 q = fast2::neg_div2(make_float2(num, -num), make_float2(den, den2));
+      auto good = [](float got, float a, float d) {
+        const float want = fdiv(a, d);
+        if (fabsf(a) >= 1.9721523e-31f && fabsf(want) >= 1.1754944e-38f) return same_float(got, want);
+        return fabsf(got) <= fmaxf(fdiv(1.9721542e-31f, d), 2.3509887e-38f);  // 2^-102 (1 + 2^-20) / d, 2^-125
+      };
+      bad += !good(q.x, -num, den) || !good(q.y, num, den2);
+    }
     if (adam_is_tame(eps, sq)) {
       float a = fadd(fast::div_by_rcp(root, sq, __frcp_rn(sq)), eps);
       float b = fadd(fdiv(root, sq), eps);

@@ -57,7 +57,7 @@ def test_split_shortcut_exhaustive(pdt, ecc_bits):
 def test_group_scale_division_shortcut_on_random_pairs():
     from flashoptim_jax_b200 import _lib
 
-    # 4e9 random (value, scale) pairs: codes through the reciprocal shortcut vs IEEE divisions
+    # 4e9 random (value, scale) pairs: codes through the reciprocal shortcut vs IEEE divisions, the update division in and below its range
     assert _run(_lib.FO_SELFTEST_GROUP_DIV, 4000) == 0
 
 
