@@ -261,7 +261,8 @@ FO_DEVI Hyp load_hyper(const DevHyper& d) {
     h.m_hi = fmul(fdiv(1.1529215e18f, lrb), 0.9999995f);
     h.least = fmaxf(d.least, fmul(lrb, d.least * 16.0f));
     const float b1 = fabsf(h.b1);
-    if (!((b1 >= 9.5367432e-7f || b1 == 0.0f) && fabsf(h.omb1) <= 2.0f && fabsf(h.decay) <= 2.0f)) h.least = __int_as_float(0x7F800000);
+    if (!((b1 >= 9.5367432e-7f || b1 == 0.0f) && fabsf(h.omb1) <= 2.0f)) h.least = __int_as_float(0x7F800000);
+    if (!(fabsf(h.decay) <= 2.0f)) h.least = __int_as_float(0x7F800000);  // (in one condition the unfused text was 2 % slower: 16.8 M elements 41.2 -> 42.0 us)
   }
   return h;
 }
