@@ -32,7 +32,8 @@ FO_DEVI void store8(float* p, const float (&v)[8]) {
 
 // Moments that are quantized are not read again, the codes are.  Up to about the size of the L2 the moments therefore give way in it, and what
 // dequantizes the codes, or the other moment, finds more of it there.  Both moments quantized and dequantized, 4.2 / 16.8 / 67 M elements: 20.5 / 62.8 / 222 us,
-// 19.8 / 59.6 / 223 with loads that give way; at 67 M a single quantization has 52.5 and 54.6.  (Blocks that stay and load a tile ahead 21.1 / 67.7 / 254, one
+// 19.8 / 59.6 / 223 with loads that give way; 25 / 29 / 33.6 M 90.2 / 105.3 / 116.9 and 87.0 / 102.9 / 114.4.  A single quantization has 21.0 / 25.8 / 27.8 there and 20.0 /
+// 25.4 / 27.7, but at 42 / 50 / 67 M 34.0 / 40.1 / 52.5 and 35.0 / 41.6 / 54.6, where the four together still gain 1 % or nothing: the line lies between.  (Blocks that stay and load a tile ahead 21.1 / 67.7 / 254, one
 // tile per block 20.4 / 64.8 / 227, blocks of 128 threads 22.0 / 73.3 / 275; the split of fp32 weights 306 and 318 with such loads.)
 constexpr unsigned long long kOnce = 1ull << 25;
 
@@ -361,7 +362,8 @@ static unsigned int tile_grid(unsigned long long tiles) {
   const unsigned long long cap = 148ull * 8ull * 4ull;
   return (unsigned int)(tiles < cap ? (tiles ? tiles : 1) : cap);
 }
-// The same for the kernels that write as much as they read or more: above two tiles per block, blocks of two tiles.  In us, with the grid above and so:
+// The same for the kernels that write half of what they read or more (splitting, reconstructing, dequantizing): above two tiles per block, 9472 tiles, blocks of two.  In
+// us, with the grid above and so: split without codes 71 M elements 64.6 and 62.2, 160 M 144 and 138, back 67.5 and 64.9, 151 and 143;
 // split into 8- / 16-bit codes 71 M elements 77.0 / 88.2 and 75.7 / 84.2, 160 M 174 / 201 and 167 / 187; reconstructed from them 79.1 / 86.7 and 77.1 / 83.7, 177 / 195
 // and 171 / 187; moments dequantized 71 M 60.2 / 59.6 and 56.7 / 55.4.  25 M elements differ by 1 %, 16.8 M (1.7 tiles per block) have 18.6 / 20.3 and with blocks
 // of two 19.1 / 21.0.  Blocks of three and four tiles are no better.  Quantizing, which writes a quarter, is slower so: 71 M 55.9 / 59.8 and 56.9 / 61.1, 160 M 126 / 138 and 134 / 146.

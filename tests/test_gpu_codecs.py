@@ -191,8 +191,8 @@ def test_moments_on_either_side_of_the_size_from_which_loads_stay_in_the_l2(name
 
 @pytest.mark.parametrize("n", [9472 * 2048, 9472 * 2048 + 1, 9473 * 2048 + 5, 9474 * 2048])
 def test_arrays_around_two_tiles_per_block(n):
-    """From 9472 tiles on the kernels that write more than they read have blocks of two tiles, the last of which may have one or part of one:
-    whole arrays against their halves."""
+    """Above 9472 tiles splitting, reconstructing and dequantizing have blocks of two tiles, the last of which may have one or part of one: whole
+    arrays against their halves."""
     import torch
 
     import flashoptim_jax_b200 as fo
