@@ -253,14 +253,15 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
   constexpr int kStep = kWarps * kTileElems;  // elements from one of the warp's tiles to the next
   constexpr int kPsz = PDT == FO_F32 ? 4 : 2, kEsz = ECC_BITS / 8;
   constexpr bool kLate = PDT == FO_BF16 && ECC_BITS != 0 && (MODE & kCoupled) == 0;
-  // Where the look stands makes 2 to 5 % by what the compiler makes of the loop around it (repeats differ by 0.3 %).  8.4 M elements in the L2, us behind the
+  // Where the look stands makes 2 to 12 % by what the compiler makes of the loop around it (repeats differ by 0.3 %).  8.4 M elements in the L2, us behind the
   // maxima / in front of them / with each half: AdamW 8-bit codes 21.6 / 20.3 / 22.2, handing back 22.2 / 21.5 / 22.7, results elsewhere 21.8 / 23.2 / 21.7,
-  // clipping 23.1 / 23.4 / 23.6, groups of 128 22.3 / 22.9 / 22.2; 16-bit codes 21.7 / 21.9 / 22.8, handing back 22.1 / 22.3 / 22.5, clipping 24.0 / 24.1 / 23.9, groups
-  // 22.6 / 22.4 / 21.9; Lion 14.6 / 14.6 / 14.3, clipping 18.7 / 18.6 / 18.0, 16-bit codes 15.9 / 15.6 / 15.5; SGDW 14.8 / 15.0 / 14.9, 16-bit codes 14.6 / 15.0 / 14.9.
+  // clipping 23.1 / 23.4 / 23.6, under fp32 gradients 24.4 / 24.3 / 24.9, groups of 128 22.3 / 22.9 / 22.2; 16-bit codes 21.7 / 21.9 / 22.8, handing back 22.1 / 22.3 / 22.5,
+  // clipping 24.0 / 24.1 / 23.9, under gradients of any dtype 25.4 / 25.0 / 25.3, groups 22.6 / 22.4 / 21.9; Lion 14.6 / 14.6 / 14.3, clipping 18.7 / 18.6 / 18.0, 16-bit codes
+  // 15.9 / 15.6 / 15.5, results elsewhere 15.3 / - / 17.2; SGDW 14.8 / 15.0 / 14.9, 16-bit codes 14.6 / 15.0 / 14.9.
   enum { kNowhere, kBehind, kInFront, kWithEachHalf };
-  constexpr int kLook = !kLate ? kNowhere
-                        : OPT == FO_OPT_LION || (kAdam && (MODE & kGroup) != 0) ? kWithEachHalf
-                        : kAdam && ECC_BITS == 8 && (MODE & (kClip | kOut)) == 0 ? kInFront : kBehind;
+  constexpr bool kEachHalf = OPT == FO_OPT_LION ? (MODE & kOut) == 0 : kAdam && (MODE & kGroup) != 0;
+  constexpr bool kFront = kAdam && (MODE & kOut) == 0 && ((MODE & kClip) != 0 ? GDT != FO_BF16 : ECC_BITS == 8);
+  constexpr int kLook = !kLate ? kNowhere : kEachHalf ? kWithEachHalf : kFront ? kInFront : kBehind;
   const int gdt = GDT == kAnyGrad ? c.grad_dtype : GDT;
   const int gsz = gdt == FO_F32 ? 4 : 2;
   const int gshift = (MODE & kGroup) != 0 ? c.group_shift : 5;  // 4 to 8 here
