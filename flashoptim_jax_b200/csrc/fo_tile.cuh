@@ -257,9 +257,10 @@ FO_DEVI void tile_run(const bool primed, const StepCommon& c, const DevLeaf& L, 
   // maxima / in front of them / with each half: AdamW 8-bit codes 21.6 / 20.3 / 22.2, handing back 22.2 / 21.5 / 22.7, results elsewhere 21.8 / 23.2 / 21.7,
   // clipping 23.1 / 23.4 / 23.6, under fp32 gradients 24.4 / 24.3 / 24.9, groups of 128 22.3 / 22.9 / 22.2; 16-bit codes 21.7 / 21.9 / 22.8, handing back 22.1 / 22.3 / 22.5,
   // clipping 24.0 / 24.1 / 23.9, under gradients of any dtype 25.4 / 25.0 / 25.3, groups 22.6 / 22.4 / 21.9; Lion 14.6 / 14.6 / 14.3, clipping 18.7 / 18.6 / 18.0, 16-bit codes
-  // 15.9 / 15.6 / 15.5, results elsewhere 15.3 / - / 17.2; SGDW 14.8 / 15.0 / 14.9, 16-bit codes 14.6 / 15.0 / 14.9.
+  // 15.9 / 15.6 / 15.5, results elsewhere 15.3 / - / 17.2, groups 16.0 / 15.8 / 17.2; SGDW 14.8 / 15.0 / 14.9, 16-bit codes 14.6 / 15.0 / 14.9, groups of 256 15.4 / 16.3 / 15.9, under fp32 gradients
+  // 16.0 / 16.8 / 15.8.
   enum { kNowhere, kBehind, kInFront, kWithEachHalf };
-  constexpr bool kEachHalf = OPT == FO_OPT_LION ? (MODE & kOut) == 0 : kAdam && (MODE & kGroup) != 0;
+  constexpr bool kEachHalf = OPT == FO_OPT_LION ? (MODE & (kOut | kGroup)) == 0 : (MODE & kGroup) != 0 && (kAdam || (ECC_BITS == 8 && GDT == FO_F32));
   constexpr bool kFront = kAdam && (MODE & kOut) == 0 && ((MODE & kClip) != 0 ? GDT != FO_BF16 : ECC_BITS == 8);
   constexpr int kLook = !kLate ? kNowhere : kEachHalf ? kWithEachHalf : kFront ? kInFront : kBehind;
   const int gdt = GDT == kAnyGrad ? c.grad_dtype : GDT;
